@@ -40,11 +40,11 @@ extern "C" {
 #define NLFEM_ERR_TIMEOUT 6     /* a bounded device wait ran out */
 
 /* arithmetic of the quadrature */
-#define NLFEM_PREC_FP64 0       /* all FP64, the reference's arithmetic */
+#define NLFEM_PREC_FP64 0       /* all FP64 */
 #define NLFEM_PREC_MIXED 1      /* FP32 quadrature, FP64 cut geometry and accumulation */
-#define NLFEM_PREC_FP64_ONESIDED 2 /* FP64 arithmetic in the mixed path's algorithm (one-sided pass,
-                                      closed forms, fixed-point sums): 2D retriangulate only; it
-                                      measures what the precision alone costs */
+#define NLFEM_PREC_FP64_ONESIDED 2 /* the one-sided FP64 pass by name (2D retriangulate only), every
+                                      structural slot kept; NLFEM_PREC_FP64 takes the same pass where
+                                      it applies */
 
 /* One assembly problem. Arrays are borrowed host pointers, row-major. */
 typedef struct nlfem_problem {

@@ -20,6 +20,7 @@
 #include "quadrature.cuh"
 #include "passes.cuh"
 #include "passes_mix.cuh"
+#include "passes_f64.cuh"
 #include "passes_bary.cuh"
 #include "passes_vec.cuh"
 
@@ -994,6 +995,7 @@ struct FinishArgs {
     const unsigned char *touched;    // VAL_DF: slots that received a contribution
     const int *vprob;                // VAL_FX: problem of each row (fixed-point unit)
     const ProbParams *probs;
+    int keep_all;                    // VAL_F64: precision "fp64-onesided" keeps every structural slot
 };
 // Value of slot i of row u; keep says whether the slot survives (the reference drops exact
 // zeros; slots of the mixed passes are kept when they received any contribution).
@@ -1008,7 +1010,7 @@ __device__ __forceinline__ double slot_value(const FinishArgs &f, const double *
         keep = (v != 0.0) || f.touched[i];
     } else {
         v = vals[i];
-        keep = v != 0.0;
+        keep = v != 0.0 || f.keep_all;
     }
     return v;
 }

@@ -1,0 +1,628 @@
+// FP64 2D retriangulate pass: one-sided, work-compacted, deterministic integer sums.
+//
+// The same split as the mixed pass (passes_mix.cuh): one warp per outer element T taken from a
+// global counter, 32 pairs (T, b) per batch, each pair's geometry computed once from T, the
+// mirrored termNonloc from the symmetric completion, every diagonal entry from its row's sum
+// (kernels of |x - y| only; integrate_retriangulate, integration.cpp:345-540). All quadrature
+// arithmetic is FP64, and GB300 runs FP64 at 1/64 of its FP32 rate, so the FP64 pipe bounds the
+// kernel and everything that can leave it does:
+//   * The (pair, outer point) classes come from the certified FP32 test (certified.cuh): a ball
+//     holding the partner or missing it with a margin. All else is a cut item and takes the exact
+//     FP64 polygon.
+//   * Constant kernels: inside items need no quadrature loop. A pair's inside mask indexes a table
+//     (shared memory, one entry per mask byte) of the rule's outer sums over the mask; its blocks
+//     are those times kc |T| |b| and the rule's inner sums.
+//   * Cut items (and, for other kernels, inside items) are listed pair by pair, so a pair's items
+//     are neighbours: full warps integrate the items, then full warps fold them, one (pair, output)
+//     per lane, instead of every lane walking all outer points.
+// Measured (quadrature phase, against the two-sided colored pass that the path used before): constant
+// kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 51.6 ms against 1725 ms; 2 * 32^2
+// triangles: 1.1 against 66.6 ms; parabola, 2 * 57^2: 16.2 against 257 ms; fractional, 2 * 40^2:
+// 53 against 568 ms.
+//
+// Sums. Every contribution is rounded once to a 64-bit integer and added with an integer atomic,
+// so the result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
+// follows from a bound of that slot: the blocks' sum over the elements at t and at v is at most
+// 2^xN |patch t| |patch v|, with |patch| the elements' |det| sum at a vertex. Exponents are kept
+// in eighths of a bit (vexp = 8 log2 |patch|, rounded up), so that only their sum is rounded to a
+// whole power: the unit 2^((xN + vexp[t] + vexp[v]) / 8 - 62) is near 2^-55 of a pair that fills the
+// ball, whatever the mesh grading. The sums with many more terms keep a second integer 40 bits below
+// the first: termLocal in the diagonal-block slots (unit 2^(xD + vexp[t] - 62)), and per partner
+// element its termLocalPrime, of which a constant kernel's inside part is one number, the |T|
+// weighted sum of the outer rule over the inside masks. So do all sums of singular kernels, whose
+// bound is loose and whose near pairs are far above their far ones. A nonzero contribution that
+// rounds to zero counts one unit, so a slot is zero only when all its contributions are (the
+// reference drops exact zeros).
+#pragma once
+#include "passes_mix.cuh"
+
+namespace nlg {
+
+constexpr int F64_WARPS = 4;
+constexpr int F64_THREADS = 32 * F64_WARPS;
+constexpr int F64_CAP = 64;    // items integrated before their pairs are folded (>= MAXQ)
+constexpr int F64_RN = 7;      // per item: innerLocal, innerNonloc[3], off-diagonal termLocalPrime sums[3]
+constexpr int F64_OUT = 15;    // per pair: termNonloc[9], off-diagonal termLocal[3] and termLocalPrime[3]
+constexpr int F64_BITS = 62;   // a bound of 2^x has the unit 2^(x - 62)
+constexpr int F64_WIDE = 40;   // bits of a second integer
+constexpr int F64_ELP = 8;     // per element: inside sum (two integers), cut termLocalPrime[3], second integers[3]
+
+struct F64Args {
+    MixArgs m;                  // m.elp: F64_ELP integers per element
+    const int *vexp;            // per vertex, 8 log2 of its elements' |det| sum, rounded up
+    long long *valslo;          // second integers of vals
+    long long *valsNlo;         // second integers of valsN (singular kernels)
+};
+
+struct F64Warp {
+    long long rhb[3], rrb[3];   // T's rows (see MixWarp)
+    unsigned rmask[3];
+    int rlo[3], tvs[3];
+    int te[3];                  // vexp of T's vertices
+    int pid[32];                // partner element
+    int pe[32];                 // its eexp
+    int pve[32][3];             // vexp of its vertices
+    unsigned short list[F64_CAP];           // items: lane << 6 | inside << 5 | outer point
+    unsigned char pl[32], ps[32], pn[32];   // chunk's pairs: owner lane, first item, item count
+};
+template <int NW>
+struct F64Entry {   // one partner vertex of a batch and its integer sums over T's rows
+    int col, pad;
+    long long v[3 * NW];
+};
+__host__ __device__ constexpr int f64_words(int kind) { return kind == MIX_SINGULAR ? 2 : 1; }
+// per-pair sums of the folded items (15, and second integers: termLocalPrime[3], termNonloc[9]), then the item results; the scatter
+// list lies over both
+__host__ __device__ constexpr int f64_acc(int kind) { return F64_OUT + (kind == MIX_SINGULAR ? 12 : 3); }
+__host__ __device__ constexpr size_t f64_work_bytes(int kind) {
+    return (size_t)(32 * f64_acc(kind) + F64_CAP * F64_RN) * 8 > 96 * (8 + 24 * (size_t)f64_words(kind))
+               ? (size_t)(32 * f64_acc(kind) + F64_CAP * F64_RN) * 8
+               : 96 * (8 + 24 * (size_t)f64_words(kind));
+}
+__host__ __device__ constexpr size_t f64_warp_bytes(int kind, int nPx) {
+    return (sizeof(F64Warp) + 15) / 16 * 16 + (size_t)nPx * 24 + f64_work_bytes(kind) + 16;
+}
+// mask sums of the outer rule: one table of up to 256 entries per 8 outer points
+__host__ __device__ constexpr int f64_tab_entries(int nPx) { return nPx <= 8 ? 1 << nPx : 256 * ((nPx + 7) / 8); }
+__host__ __device__ constexpr size_t f64_smem_bytes(int kind, int nPx) {
+    return (size_t)nPx * 7 * 8 + (kind == MIX_CONST ? (size_t)f64_tab_entries(nPx) * 7 * 8 : 0) +
+           F64_WARPS * ((f64_warp_bytes(kind, nPx) + 15) / 16 * 16) + 16;
+}
+
+// 2^e, e in [-1022, 1023]
+__device__ __forceinline__ double pow2i(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// v 2^e by its exponent field, off the FP64 pipe (results below the normal range become 0, above it inf)
+__device__ __forceinline__ double scale2(double v, int e) {
+    const int hi = __double2hiint(v), x = (hi >> 20) & 0x7ff, y = x + e;
+    if (x == 0 || y <= 0) return 0.0;
+    return y >= 0x7ff ? __longlong_as_double(0x7ff0000000000000LL) : __hiloint2double(hi + (e << 20), __double2loint(v));
+}
+// e with |x| < 2^e (x normal; at least -900 for zeros and subnormals)
+__device__ __forceinline__ int exp_above(double x) {
+    const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1022;
+    return e < -900 ? -900 : e;
+}
+// q rounded to an integer (a nonzero one never to zero); |q| >= 2^62 or NaN sets bad
+__device__ __forceinline__ long long f64_fix(double q, bool &bad) {
+    const long long b = __double_as_longlong(q);
+    bad |= ((int)(b >> 52) & 0x7ff) >= 1023 + F64_BITS;
+    const long long i = __double2ll_rn(q);
+    return (i == 0 && (b << 1) != 0) ? (b < 0 ? -1LL : 1LL) : i;
+}
+// the second integer: what the first one's rounding left, 2^40 times finer
+__device__ __forceinline__ long long f64_fix_lo(double q, long long i) {
+    return __double2ll_rn((q - (double)i) * (double)(1LL << F64_WIDE));
+}
+__device__ __forceinline__ double f64_join(long long hi, long long lo) {
+    return (double)hi + (double)lo * (1.0 / (double)(1LL << F64_WIDE));
+}
+
+template <int KIND>
+__device__ __forceinline__ double f64_kernel(const ProbParams &P, double r2) {
+    if (KIND == MIX_CONST) return P.kc;
+    if (KIND == MIX_REGULAR && P.kernel == KER_PARABOLA) return P.kc * (P.sqdelta - r2);
+    return P.kc * exp2(-0.5 * P.expo * log2(r2));
+}
+
+// Inner sums of one item into res (see F64_RN), without the factor |T|: the quadrature over the
+// partner (inside) or over the fan of its polygon with the ball (cut).
+template <int KIND>
+__device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, const PassRuleT<double> &pr, bool inside,
+                                         const double *x, const double *Eb, double *res, unsigned &nsub) {
+    const double Q0x = Eb[0] - x[0], Q0y = Eb[1] - x[1];
+    const double e1x = Eb[2] - Eb[0], e1y = Eb[3] - Eb[1], e2x = Eb[4] - Eb[0], e2y = Eb[5] - Eb[1];
+    const double det = e1x * e2y - e1y * e2x;
+    double S0 = 0, S1[3] = {0, 0, 0}, S2[3] = {0, 0, 0};
+    if (KIND != MIX_CONST && inside) {
+        nsub++;
+        const double rT = fabs(det);
+        for (int i = 0; i < rule.nPy; i++) {
+            const double yx = Q0x + e1x * rule.Py[2 * i] + e2x * rule.Py[2 * i + 1];
+            const double yy = Q0y + e1y * rule.Py[2 * i] + e2y * rule.Py[2 * i + 1];
+            const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * rT;
+            S0 += kw * rule.dy[i];
+#pragma unroll
+            for (int c = 0; c < 3; c++) S1[c] += kw * pr.cy[3 * i + c];
+            S2[0] += kw * pr.cyy[6 * i + 1];
+            S2[1] += kw * pr.cyy[6 * i + 2];
+            S2[2] += kw * pr.cyy[6 * i + 4];
+        }
+    } else {
+        const double idet = 1.0 / det;
+        double R[18];
+        const int n = xretriangulate(x, Eb, P.sqdelta, P.caps, R);
+        for (int j = 0; j < n; j++) { R[2 * j] -= x[0]; R[2 * j + 1] -= x[1]; }
+        auto basis = [&](double yx, double yy, double *l) {   // psi_0..2 of b at y
+            const double dx = yx - Q0x, dy = yy - Q0y;
+            l[1] = (e2y * dx - e2x * dy) * idet;
+            l[2] = (e1x * dy - e1y * dx) * idet;
+            l[0] = 1.0 - l[1] - l[2];
+        };
+        if (KIND == MIX_CONST) {   // the rule's moments on each fan triangle (see item_cut_const)
+            const double m0 = pr.mom[0], mx = pr.mom[1], my = pr.mom[2], mxx = pr.mom[3], mxy = pr.mom[4], myy = pr.mom[5];
+            double la[3], lb[3], lc[3];
+            if (n >= 3) {
+                basis(R[0], R[1], la);
+                basis(R[2], R[3], lb);
+            }
+            for (int r = 0; r + 2 < n; r++) {
+                nsub++;
+                const double Bx = R[2 * r + 2] - R[0], By = R[2 * r + 3] - R[1], Cx = R[2 * r + 4] - R[0], Cy = R[2 * r + 5] - R[1];
+                const double rT = fabs(Bx * Cy - By * Cx);
+                basis(R[2 * r + 4], R[2 * r + 5], lc);
+                double t0[3], t1[3], t2[3], be[3], ga[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++) {
+                    be[q] = lb[q] - la[q];
+                    ga[q] = lc[q] - la[q];
+                    t0[q] = la[q] * m0 + (be[q] * mx + ga[q] * my);
+                    t1[q] = la[q] * mx + (be[q] * mxx + ga[q] * mxy);
+                    t2[q] = la[q] * my + (be[q] * mxy + ga[q] * myy);
+                    S1[q] += rT * t0[q];
+                    lb[q] = lc[q];
+                }
+                S0 += rT * m0;
+                S2[0] += rT * (la[0] * t0[1] + (be[0] * t1[1] + ga[0] * t2[1]));
+                S2[1] += rT * (la[0] * t0[2] + (be[0] * t1[2] + ga[0] * t2[2]));
+                S2[2] += rT * (la[1] * t0[2] + (be[1] * t1[2] + ga[1] * t2[2]));
+            }
+            S0 *= P.kc;
+#pragma unroll
+            for (int q = 0; q < 3; q++) { S1[q] *= P.kc; S2[q] *= P.kc; }
+        } else {
+            for (int r = 0; r + 2 < n; r++) {
+                nsub++;
+                const double Bx = R[2 * r + 2] - R[0], By = R[2 * r + 3] - R[1], Cx = R[2 * r + 4] - R[0], Cy = R[2 * r + 5] - R[1];
+                const double rT = fabs(Bx * Cy - By * Cx);
+                for (int i = 0; i < rule.nPy; i++) {
+                    const double yx = R[0] + Bx * rule.Py[2 * i] + Cx * rule.Py[2 * i + 1];
+                    const double yy = R[1] + By * rule.Py[2 * i] + Cy * rule.Py[2 * i + 1];
+                    const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * rT * rule.dy[i];
+                    double l[3];
+                    basis(yx, yy, l);
+                    S0 += kw;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) S1[c] += kw * l[c];
+                    S2[0] += kw * (l[0] * l[1]);
+                    S2[1] += kw * (l[0] * l[2]);
+                    S2[2] += kw * (l[1] * l[2]);
+                }
+            }
+        }
+    }
+    res[0] = S0;
+#pragma unroll
+    for (int q = 0; q < 3; q++) { res[1 + q] = S1[q]; res[4 + q] = S2[q]; }
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule rule, PassRuleT<double> pr) {
+    constexpr bool CK = KIND == MIX_CONST;
+    constexpr int NW = f64_words(KIND);
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const PassArgs &a = fa.m.p;
+    const SlotMap &sm = fa.m.m;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int nPx = rule.nPx;
+    // block: outer rule coefficients [nPx][7] (dx psi_r, off-diagonal dx psi_r psi_c, dx), mask sums
+    double *coef = reinterpret_cast<double *>(s_raw);
+    double *tab = coef + 7 * nPx;
+    unsigned char *wbase = reinterpret_cast<unsigned char *>(tab + (CK ? 7 * f64_tab_entries(nPx) : 0));
+    wbase = s_raw + ((wbase - s_raw) + 15) / 16 * 16 + (size_t)wib * ((f64_warp_bytes(KIND, nPx) + 15) / 16 * 16);
+    F64Warp &W = *reinterpret_cast<F64Warp *>(wbase);
+    double *x64 = reinterpret_cast<double *>(wbase + (sizeof(F64Warp) + 15) / 16 * 16);   // [nPx][2]
+    F2 *xf = reinterpret_cast<F2 *>(x64 + 2 * nPx);                                       // [nPx]
+    unsigned char *work = reinterpret_cast<unsigned char *>(xf + nPx);
+    long long *acc = reinterpret_cast<long long *>(work);                                 // [32][f64_acc]
+    double *res = reinterpret_cast<double *>(acc + 32 * f64_acc(KIND));                   // [F64_CAP][F64_RN]
+    F64Entry<NW> *slist = reinterpret_cast<F64Entry<NW> *>(work);
+    for (int i = threadIdx.x; i < 7 * nPx; i += F64_THREADS) {
+        const int k = i / 7, q = i - 7 * k;
+        coef[i] = q < 3 ? pr.cx[3 * k + q] : (q < 6 ? pr.cxx[6 * k + (q == 5 ? 4 : q - 2)] : pr.dxf[k]);
+    }
+    __syncthreads();
+    if (CK) {
+        for (int i = threadIdx.x; i < f64_tab_entries(nPx); i += F64_THREADS) {
+            double s[7] = {0, 0, 0, 0, 0, 0, 0};
+            for (int b = 0; b < 8; b++) {
+                const int k = 8 * (i >> 8) + b;
+                if (((i >> b) & 1) && k < nPx)
+#pragma unroll
+                    for (int q = 0; q < 7; q++) s[q] += coef[7 * k + q];
+            }
+#pragma unroll
+            for (int q = 0; q < 7; q++) tab[7 * i + q] = s[q];
+        }
+        __syncthreads();
+    }
+    long long *vals = reinterpret_cast<long long *>(a.vals);
+    bool bad = false;   // a contribution outside the fixed-point range (reported at the end)
+    bool miss = false;  // a matrix slot not found (reported at the end)
+    unsigned nsub = 0, nclose = 0, nitin = 0, nitcut = 0;
+    for (;;) {
+        int idx = 0;
+        if (lane == 0) idx = atomicAdd(fa.m.work, 1);
+        idx = __shfl_sync(FULL, idx, 0);
+        if (idx >= a.count) break;
+        const int T = a.list ? a.list[idx] : idx;
+        const long long lb = a.out_ptr[T], le = a.out_cnt ? lb + a.out_cnt[T] : a.out_ptr[T + 1];
+        if (lb == le || a.labT[T] == 0) continue;
+        int tv[3];
+        unsigned keepmask = 0;   // bit r: the row of T's vertex r exists
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            tv[r] = a.T32[(long long)T * 3 + r];
+            if (a.labV[tv[r]] > 0) keepmask |= 1u << r;
+        }
+        if (lane < 3) {   // T's rows, for the lookups of every batch
+            const int u = sel3(tv, lane);
+            RowHash h;
+            h.hb = h.rb = 0;
+            h.mask = 0xffffffffu;
+            h.lo = 0;
+            if (keepmask & (1u << lane)) h = row_hash(sm, u);
+            W.rhb[lane] = h.hb;
+            W.rrb[lane] = h.rb;
+            W.rmask[lane] = h.mask;
+            W.rlo[lane] = h.lo;
+            W.tvs[lane] = u;
+            W.te[lane] = fa.vexp[u];
+        }
+        const ProbParams P = a.probs[a.eprob[T]];
+        const double *ET64 = &a.EC[(long long)T * 6];
+        const float ohi0 = a.EChi[(long long)T * 6], ohi1 = a.EChi[(long long)T * 6 + 1];
+        const float olo0 = a.EClo[(long long)T * 6], olo1 = a.EClo[(long long)T * 6 + 1];
+        const double dT = a.adet[T];
+        for (int k = lane; k < nPx; k += 32) {
+            xtoPhys<2>(ET64, &rule.Px[2 * k], &x64[2 * k]);
+            xf[k] = f2((float)(x64[2 * k] - ET64[0]), (float)(x64[2 * k + 1] - ET64[1]));
+        }
+        __syncwarp();
+        int et[3];   // eighths of a bit: the unit exponent of T's rows
+#pragma unroll
+        for (int r = 0; r < 3; r++) et[r] = 8 * F64_BITS - P.xN - W.te[r];
+        const double dTs = scale2(dT, F64_BITS - P.xS);
+        double D[3] = {0, 0, 0};   // termLocal of T's pairs, off-diagonal
+        const bool frac_close = KIND == MIX_SINGULAR && duffy_close(P);
+        int part_next = lb + lane < le ? a.pB[lb + lane] : T;   // partners one batch ahead
+        for (long long p0 = lb; p0 < le; p0 += 32) {
+            const long long p = p0 + lane;
+            const bool act = p < le;
+            const int part = part_next;
+            part_next = p + 32 < le ? a.pB[p + 32] : T;
+            int pv[3];
+#pragma unroll
+            for (int r = 0; r < 3; r++) pv[r] = a.T32[(long long)part * 3 + r];
+            bool close = false;
+            if (frac_close && act) {
+                close = (part == T);
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) close |= (tv[i] == pv[j]);
+            }
+            const double rb = a.adet[part];
+            const int eb = exp_above(rb);
+            int ve[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) ve[c] = fa.vexp[pv[c]];
+            W.pid[lane] = part;
+            W.pe[lane] = eb;
+#pragma unroll
+            for (int c = 0; c < 3; c++) W.pve[lane][c] = ve[c];
+            unsigned inm = 0, cutm = 0;
+            if (act && !close) {
+                float pc[6];
+#pragma unroll
+                for (int j = 0; j < 6; j++)
+                    pc[j] = (a.EChi[(long long)part * 6 + j] - ((j & 1) ? ohi1 : ohi0)) + (a.EClo[(long long)part * 6 + j] - ((j & 1) ? olo1 : olo0));
+                for (int k = 0; k < nPx; k++) {
+                    const F2 x = xf[k];
+                    const F2 Q[3] = {f2(pc[0] - x.x, pc[1] - x.y), f2(pc[2] - x.x, pc[3] - x.y), f2(pc[4] - x.x, pc[5] - x.y)};
+                    const int c = fclassify(Q, P.sqdelta_f);
+                    inm |= (unsigned)(c == CLS_IN) << k;
+                    cutm |= (unsigned)(c == CLS_CUT) << k;
+                }
+            }
+            nitin += __popc(inm);
+            nitcut += __popc(cutm);
+            if (CK) nsub += __popc(inm);
+            // items, pair by pair, in chunks of whole pairs
+            const unsigned itm = CK ? cutm : inm | cutm;
+            const int cnt = __popc(itm);
+            const int incl = warp_incl_scan(cnt, lane), off = incl - cnt;
+            const int total = __shfl_sync(FULL, incl, 31);
+            for (int base = 0; base < total;) {
+                const bool mine = cnt > 0 && off >= base && off + cnt <= base + F64_CAP;
+                const unsigned who = __ballot_sync(FULL, mine);
+                const int end = __shfl_sync(FULL, incl, 31 - __clz(who));
+                if (mine) {
+                    int w = off - base;
+                    const int r = __popc(who & lanemask_lt());
+                    W.pl[r] = (unsigned char)lane;
+                    W.ps[r] = (unsigned char)w;
+                    W.pn[r] = (unsigned char)cnt;
+                    for (unsigned mm = itm; mm; mm &= mm - 1) {
+                        const int k = __ffs(mm) - 1;
+                        W.list[w++] = (unsigned short)(lane << 6 | ((inm >> k) & 1u) << 5 | k);
+                    }
+                }
+                __syncwarp();
+                for (int i = lane; i < end - base; i += 32) {
+                    const int it = W.list[i], k = it & 31;
+                    f64_item<KIND>(P, rule, pr, (it >> 5) & 1, &x64[2 * k], &a.EC[(long long)W.pid[it >> 6] * 6], &res[i * F64_RN], nsub);
+                }
+                __syncwarp();
+                const int nun = __popc(who) * F64_OUT;
+                for (int u = lane; u < nun; u += 32) {
+                    const int r = u / F64_OUT, o = u - r * F64_OUT, pl = W.pl[r];
+                    const int ci = o < 9 ? o / 3 : (o < 12 ? o - 6 : 6);
+                    const int ri = o < 9 ? 1 + o % 3 : (o < 12 ? 0 : o - 8);
+                    double v = 0;
+                    for (int i = W.ps[r], e = i + W.pn[r]; i < e; i++) v += coef[7 * (W.list[i] & 31) + ci] * res[i * F64_RN + ri];
+                    long long *A = &acc[pl * f64_acc(KIND)];
+                    if (o >= 9 && o < 12) {
+                        A[o] = __double_as_longlong(v * dT);
+                    } else {
+                        const int ex = o < 9 ? (8 * F64_BITS - P.xN - W.te[o / 3] - W.pve[pl][o % 3]) >> 3 : F64_BITS - P.xD - W.pe[pl];
+                        const double q = scale2(v * dT, ex);
+                        const long long iv = f64_fix(q, bad);
+                        A[o] = iv;
+                        if (o >= 12) A[o + 3] = f64_fix_lo(q, iv);
+                        else if (NW == 2) A[F64_OUT + 3 + o] = f64_fix_lo(q, iv);
+                    }
+                }
+                __syncwarp();
+                base = end;
+            }
+            // owner: the pair's blocks as integers (termLocal stays FP64, summed per lane)
+            long long nx[9 * NW];
+#pragma unroll
+            for (int i = 0; i < 9 * NW; i++) nx[i] = 0;
+            long long *ep = &fa.m.elp[(long long)part * F64_ELP];
+            if (CK && inm) {   // inside items: kc |T| |b| times the rule's sums
+                double m[7];
+#pragma unroll
+                for (int q = 0; q < 7; q++) m[q] = tab[7 * (inm & 255u) + q];
+                for (int b = 1; 8 * b < nPx; b++)
+#pragma unroll
+                    for (int q = 0; q < 7; q++) m[q] += tab[7 * (256 * b + ((inm >> (8 * b)) & 255u)) + q];
+                const double kr = P.kc * dT * rb;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const double iN = kr * pr.insum[1 + c];
+#pragma unroll
+                    for (int r = 0; r < 3; r++) nx[3 * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve[c]) >> 3), bad);
+                }
+                const double kl = kr * pr.insum[0];
+#pragma unroll
+                for (int q = 0; q < 3; q++) D[q] += m[3 + q] * kl;
+                const double q = m[6] * dTs;
+                const long long iv = f64_fix(q, bad);
+                red_add(ep, 0, iv);
+                red_add(ep, 1, f64_fix_lo(q, iv));
+            }
+            if (cnt) {
+                const long long *A = &acc[lane * f64_acc(KIND)];
+#pragma unroll
+                for (int i = 0; i < 9; i++) {
+                    nx[i] += A[i];
+                    if (NW == 2) nx[NW == 2 ? 9 + i : 0] += A[F64_OUT + 3 + i];
+                }
+#pragma unroll
+                for (int q = 0; q < 3; q++) D[q] += __longlong_as_double(A[9 + q]);
+#pragma unroll
+                for (int q = 0; q < 6; q++) red_add(ep, 2 + q, A[12 + q]);
+            }
+            if (KIND == MIX_SINGULAR && close) {   // Duffy blocks (their termNonlocPrime is termNonloc)
+                nclose++;
+                const long long cs = close_slot(a.xadj, a.adj, T, part);
+                if (cs < 0) {
+                    miss = true;
+                } else {
+                    const double *cb = &a.closebuf[cs * 36];
+                    D[0] += cb[1]; D[1] += cb[2]; D[2] += cb[5];
+#pragma unroll
+                    for (int q = 0; q < 3; q++) {
+                        const double v = scale2(cb[q == 2 ? 23 : 19 + q], F64_BITS - P.xD - eb);
+                        const long long iv = f64_fix(v, bad);
+                        red_add(ep, 2 + q, iv);
+                        red_add(ep, 5 + q, f64_fix_lo(v, iv));
+                    }
+#pragma unroll
+                    for (int i = 0; i < 9; i++) {
+                        const double q = scale2(cb[9 + i], (et[i / 3] - ve[i % 3]) >> 3);
+                        nx[i] = f64_fix(q, bad);
+                        if (NW == 2) nx[NW == 2 ? 9 + i : 0] = f64_fix_lo(q, nx[i]);
+                    }
+                }
+            }
+            // termNonloc into T's own rows: lanes sharing a partner vertex add their integers, all
+            // lanes share the (vertex, row) lookups; the mirrored entries come from k_sym_add_f64
+            __syncwarp();
+            int nent = 0;
+#pragma unroll 1
+            for (int c = 0; c < 3; c++) {
+                const int col = act ? sel3(pv, c) : -1;
+                const unsigned grp = __match_any_sync(FULL, col);
+                const bool leader = (__ffs(grp) - 1) == lane;
+                const int maxn = __reduce_max_sync(FULL, (unsigned)__popc(grp));
+                long long o[3 * NW], s[3 * NW];
+#pragma unroll
+                for (int r = 0; r < 3 * NW; r++) o[r] = s[r] = sel3(&nx[3 * r], c);
+                unsigned rest = grp & ~(1u << lane);
+                for (int it = 1; it < maxn; it++) {
+                    const int src = rest ? __ffs(rest) - 1 : lane;
+                    const bool use = rest != 0;
+                    if (rest) rest &= rest - 1;
+#pragma unroll
+                    for (int r = 0; r < 3 * NW; r++) {
+                        const long long t = shfl64(o[r], src);
+                        if (use) s[r] += t;
+                    }
+                }
+                const bool put = leader && col >= 0;
+                const unsigned m = __ballot_sync(FULL, put);
+                if (put) {
+                    F64Entry<NW> &e = slist[nent + __popc(m & lanemask_lt())];
+                    e.col = col;
+#pragma unroll
+                    for (int r = 0; r < 3 * NW; r++) e.v[r] = s[r];
+                }
+                nent += __popc(m);
+            }
+            __syncwarp();
+            for (int w = lane; w < 3 * nent; w += 32) {
+                const int e = w / 3, r = w - 3 * e;
+                const int col = slist[e].col;
+                if (col == W.tvs[r]) continue;   // the matrix diagonal: from the row sum
+                RowHash h;
+                h.hb = W.rhb[r]; h.rb = W.rrb[r]; h.mask = W.rmask[r]; h.lo = W.rlo[r];
+                long long s;
+                if (h.mask != 0xffffffffu) s = slot_find_row(sm, h, col);
+                else if (a.labV[col] > 0) s = slot_find(sm, col, W.tvs[r]);   // T's vertex has no row: the mirror
+                else continue;
+                if (s < 0) { miss = true; continue; }
+                red_add(fa.m.valsN, s, slist[e].v[r]);
+                if (NW == 2) red_add(fa.valsNlo, s, slist[e].v[3 + r]);
+            }
+            __syncwarp();
+        }
+        // termLocal of all of T's pairs into T's diagonal block
+#pragma unroll
+        for (int i = 0; i < 3; i++) D[i] = warp_sum(D[i]);
+        if (lane < 9 && lane / 3 != lane % 3) {   // off-diagonal entries (the diagonal: k_sym_add_f64)
+            const int r = lane / 3, c = lane % 3;
+            const int s = sm.dslot[(long long)T * 9 + lane];
+            const double d = r + c == 1 ? D[0] : (r + c == 2 ? D[1] : D[2]);
+            if (s >= 0) {
+                const double q = scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3));
+                const long long iv = f64_fix(q, bad);
+                red_add(vals, s, iv);
+                red_add(fa.valslo, s, f64_fix_lo(q, iv));
+            } else if (keepmask & (1u << r)) miss = true;
+        }
+        __syncwarp();
+    }
+    if (__any_sync(FULL, bad) && lane == 0) atomicOr(&a.err[5], 1);
+    if (__any_sync(FULL, miss) && lane == 0) atomicOr(&a.err[3], 1);
+    nsub = warp_sum(nsub);
+    nclose = warp_sum(nclose);
+    nitin = warp_sum(nitin);
+    nitcut = warp_sum(nitcut);
+    if (lane == 0) {
+        if (nsub && a.n_subtri) atomicAdd(a.n_subtri, (unsigned long long)nsub);
+        if (nclose && a.n_close) atomicAdd(a.n_close, (unsigned long long)nclose);
+        if (nitin && a.n_in) atomicAdd(a.n_in, (unsigned long long)nitin);
+        if (nitcut && a.n_cut) atomicAdd(a.n_cut, (unsigned long long)nitcut);
+    }
+}
+
+// vexp of every vertex: 8 log2 of its elements' |det| sum, rounded up (with a margin far above the
+// logarithm's rounding).
+__global__ void k_vexp(const long long *__restrict__ vptr, const int *__restrict__ vel, const double *__restrict__ adet,
+                       long long nV, int *__restrict__ vexp) {
+    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nV) return;
+    double s = 0;
+    for (long long i = vptr[v]; i < vptr[v + 1]; i++) s += adet[vel[i]];
+    vexp[v] = s > 1e-270 ? (int)ceil(8.0 * log2(s) + 1e-3) : -7200;
+}
+
+// termLocalPrime sums of each element into its diagonal-block slots, in their rows' units. The
+// inside part of a constant kernel is kc |b| times its summed outer weights times the inner rule's
+// sums in01, in02, in12 of psi_r psi_c.
+__global__ void k_elem_blocks_f64(const long long *__restrict__ elp, const double *__restrict__ adet,
+                                  const int *__restrict__ vexp, const int *__restrict__ dslot,
+                                  const int *__restrict__ T32, const int *__restrict__ labV,
+                                  const int *__restrict__ eprob, const ProbParams *__restrict__ probs, double in01,
+                                  double in02, double in12, long long nE, long long *__restrict__ vals,
+                                  long long *__restrict__ valslo, int *__restrict__ err) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nE) return;
+    const long long *p = &elp[e * F64_ELP];
+    if ((p[0] | p[1] | p[2] | p[3] | p[4] | p[5] | p[6] | p[7]) == 0) return;
+    const ProbParams &P = probs[eprob[e]];
+    const double in[3] = {in01, in02, in12};
+    const double kin = scale2(f64_join(p[0], p[1]), P.xS - F64_BITS) * (P.kc * adet[e]);
+    const int eb = exp_above(adet[e]);
+    double b[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) b[q] = kin * in[q] + scale2(f64_join(p[2 + q], p[5 + q]), P.xD + eb - F64_BITS);
+    bool bad = false;
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            if (r == c) continue;   // the diagonal comes from the row sum (k_sym_add_f64)
+            const int v = T32[e * 3 + r], s = dslot[e * 9 + 3 * r + c];
+            if (s >= 0) {
+                const double q = scale2(b[r + c - 1], F64_BITS - P.xD - ((vexp[v] + 7) >> 3));
+                const long long iv = f64_fix(q, bad);
+                red_add(vals, s, iv);
+                red_add(valslo, s, f64_fix_lo(q, iv));
+            } else if (labV[v] > 0) {
+                atomicOr(&err[3], 1);
+            }
+        }
+    if (bad) atomicOr(&err[5], 1);
+}
+
+// The FP64 matrix from the sums: entry (t, v) is the diagonal blocks' part minus the termNonloc sums
+// of the slot and of its transposed slot; each diagonal entry is minus its row's other entries. vals
+// is replaced in place by FP64 values. One warp per row; HBM-bound (each slot's sums are read
+// twice).
+__global__ void k_sym_add_f64(const long long *__restrict__ rowptr, const int *__restrict__ cols,
+                              const int *__restrict__ tpos, const long long *__restrict__ valsN,
+                              const long long *__restrict__ valsNlo, const long long *__restrict__ valslo,
+                              const int *__restrict__ vexp, const int *__restrict__ vprob,
+                              const ProbParams *__restrict__ probs, long long nrows, double *__restrict__ vals) {
+    const int lane = threadIdx.x & 31;
+    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long t = gw; t < nrows; t += nw) {
+        const long long b = rowptr[t], e = rowptr[t + 1];
+        if (b == e) continue;
+        const ProbParams &P = probs[vprob[t]];
+        const int et = vexp[t], eN = 8 * F64_BITS - P.xN - et, eD = P.xD + ((et + 7) >> 3) - F64_BITS;
+        double off = 0;
+        long long dslot = -1;
+        for (long long s = b + lane; s < e; s += 32) {
+            const int v = cols[s];
+            if (v == (int)t) { dslot = s; continue; }
+            const int tp = tpos[s];
+            const long long ts = tp >= 0 ? rowptr[v] + tp : -1;
+            double q = valsNlo ? f64_join(valsN[s], valsNlo[s]) : (double)valsN[s];
+            if (ts >= 0) q += valsNlo ? f64_join(valsN[ts], valsNlo[ts]) : (double)valsN[ts];
+            const long long dh = reinterpret_cast<const long long *>(vals)[s];
+            double x = -scale2(q, -((eN - vexp[v]) >> 3));
+            if (dh) x += scale2(f64_join(dh, valslo[s]), eD);   // a slot of a diagonal block
+            vals[s] = x;
+            off += x;
+        }
+        off = warp_sum(off);
+        if (dslot >= 0) vals[dslot] = -off;   // the row sums to zero
+    }
+}
+
+}  // namespace nlg

@@ -186,6 +186,56 @@ static long zeta_common(const long *idx, const long *ptr, long a, long b) {
     return n;
 }
 
+// Whether the one-sided FP64 pass (passes_f64.cuh) takes the problem, and the bounds its units
+// follow from. A pair's blocks are at most kbound |T| |b| times the rules' absolute sums (CN, CD:
+// basis functions at inner points of polygons inside the element are at most the largest absolute
+// row sum of the rule's own); for singular kernels kbound is the value at the mean element size
+// times 2^20, and contributions beyond it are detected. Elements near degenerate (where the
+// reference's solve2x2 may abort), bounds far outside the exponent range and options that
+// need the general pass go there. fp64-onesided, which has no such pass to match, is bound only by
+// the range.
+static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, double kbound) {
+    P.f64ok = 0;
+    if (!P.cert || p.dim != 2 || p.outdim != 1 || p.is_dg) return;
+    double atot = 0, amin = 1e300, amax = 0;
+    bool sound = true;
+    for (long e = 0; e < p.nE; e++) {
+        const long *t = &p.elements[3 * e];
+        for (int a = 0; a < 3; a++)
+            if (t[a] < 0 || t[a] >= p.nV) return;
+        const double *x = &p.vertices[2 * t[0]], *y = &p.vertices[2 * t[1]], *z = &p.vertices[2 * t[2]];
+        const double a = y[0] - x[0], b = z[0] - x[0], c = y[1] - x[1], d = z[1] - x[1];
+        const double det = fabs(a * d - b * c), scale = (fabs(a) + fabs(c)) * (fabs(b) + fabs(d));
+        sound = sound && det > 1e-10 * scale && std::max(fabs(a), fabs(c)) > 1e-14;
+        atot += det;
+        amin = std::min(amin, det);
+        amax = std::max(amax, det);
+    }
+    double cx = 1, cy = 1, sx = 0, sy = 0, px[3] = {0, 0, 0};
+    for (int k = 0; k < p.nPx; k++) {
+        const double ps[3] = {1.0 - p.Px[2 * k] - p.Px[2 * k + 1], p.Px[2 * k], p.Px[2 * k + 1]};
+        cx = std::max(cx, fabs(ps[0]) + fabs(ps[1]) + fabs(ps[2]));
+        sx += fabs(p.dx[k]);
+        for (int r = 0; r < 3; r++) px[r] += fabs(p.dx[k] * ps[r]);
+    }
+    for (int k = 0; k < p.nPy; k++) {
+        cy = std::max(cy, fabs(1.0 - p.Py[2 * k] - p.Py[2 * k + 1]) + fabs(p.Py[2 * k]) + fabs(p.Py[2 * k + 1]));
+        sy += fabs(p.dy[k]);
+    }
+    if (P.kernel == KER_PARABOLA) kbound *= cy * cy;   // inner points outside the polygon
+    if (P.singular) kbound *= 1048576.0;
+    const double CN = kbound * std::max(px[0], std::max(px[1], px[2])) * sy * cy, CD = 2 * kbound * sx * cx * cx * sy * cy * cy * atot;
+    if (!(CN > 1e-120 && CN < 1e120 && CD > 1e-120 && CD < 1e120 && sx > 1e-30 && atot > 1e-60 && atot < 1e60 && amax < 1e60)) return;
+    if (P.kernel != KER_CONSTANT && P.kernel != KER_PARABOLA && P.kernel != KER_FRACTIONAL) return;
+    P.xN = (int)ceil(8.0 * log2(CN) + 1e-3);
+    P.xD = exact_ceil_log2(CD);
+    P.xS = exact_ceil_log2(sx * atot);
+    if (p.precision == NLFEM_PREC_FP64)
+        P.f64ok = sound && amin > 1e-60 && !P.full_search && !P.zeta && (!P.singular || duffy_close(P));
+    else
+        P.f64ok = 1;
+}
+
 static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     memset(&P, 0, sizeof(P));
     if (p.dim != 2 && p.dim != 3) return fail(NLFEM_ERR_INVALID, "Dimension is not equal to 2 or 3.");
@@ -324,13 +374,14 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     for (int j = 0; j < p.dim; j++) vol *= std::max(hi[j] - lo[j], 1e-300);
     const double el = vol / (double)p.nE;
     P.el = el;
-    // The one-sided passes decide their geometry with margins (certified.cuh; 2^-40 for the FP64
-    // instance). The rounding of coordinates local to an outer element grows with the element
-    // size relative to the ball: the FP32 vertex tests stay inside their margin while every element
-    // diameter is at most MIX_MAX_H_OVER_DELTA times delta (the FP64 ones up to 512 delta).
-    if (system && (p.precision == NLFEM_PREC_MIXED || p.precision == NLFEM_PREC_FP64_ONESIDED)) {
+    // The one-sided passes and the filtered search decide their geometry with FP32 margins
+    // (certified.cuh). The rounding of coordinates local to an outer element grows with the element
+    // size relative to the ball: the vertex tests stay inside their margin while every element
+    // diameter is at most MIX_MAX_H_OVER_DELTA times delta. The mixed path refuses larger elements,
+    // the FP64 paths take their FP64 routines for them.
+    double hmax2 = 0;
+    if (system) {
         const int dV = p.dim + 1;
-        double hmax2 = 0;
         for (long e = 0; e < p.nE; e++)
             for (int a = 0; a < dV; a++)
                 for (int b = a + 1; b < dV; b++) {
@@ -344,12 +395,17 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
                     hmax2 = std::max(hmax2, d2);
                 }
         const double lim = p.precision == NLFEM_PREC_MIXED ? MIX_MAX_H_OVER_DELTA : 512.0;
-        if (hmax2 > lim * lim * p.sqdelta)
+        if (p.precision != NLFEM_PREC_FP64 && hmax2 > lim * lim * p.sqdelta)
             return fail(NLFEM_ERR_UNSUPPORTED, std::string("precision \"") + (p.precision == NLFEM_PREC_MIXED ? "mixed" : "fp64-onesided") +
                         "\" needs elements no larger than " + std::to_string((int)lim) +
                         " times the horizon (the margins of its geometry tests); precision \"fp64\" has no such bound");
     }
-    double mag;
+    if (system) {
+        bool finite = std::isfinite(p.sqdelta);
+        for (long v = 0; v < p.nV * p.dim; v++) finite = finite && std::isfinite(p.vertices[v]);
+        P.cert = finite && hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta;
+    }
+    double mag, kbound = 0;   // kbound: bound of |kernel| inside the ball (estimate for singular kernels)
     if (system) {
         const double h = pow(el, 1.0 / p.dim);
         const double ball = p.dim == 2 ? M_PI * p.sqdelta : 4.0 / 3.0 * M_PI * p.sqdelta * P.delta;
@@ -359,6 +415,7 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
         if (P.kernel == KER_FRACTIONAL || P.kernel == KER_MICROFIELD || P.kernel == KER_MICROFIELD3D)
             kmax = P.kc / pow(std::min(h, P.delta), P.expo);
         mag = fabs(kmax) * el * std::max(ball, el);
+        kbound = fabs(kmax);
     } else {
         double fm = 1.0;
         for (int j = 0; j < p.dim; j++) fm = std::max(fm, std::max(fabs(lo[j]), fabs(hi[j])));
@@ -366,6 +423,7 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     }
     if (!(mag > 0) || !std::isfinite(mag)) mag = 1.0;
     P.scale_exp = exact_ceil_log2(mag);
+    if (system && p.precision != NLFEM_PREC_MIXED) set_f64_bounds(p, P, kbound);
     return set_fx_unit(P, 0);
 }
 
@@ -426,7 +484,10 @@ struct Session {
     DevBuf color, color2, colorlist, closeA, closeB, closebuf, touched;
     std::vector<int> color_off;
     int prec = 0;
-    bool onesided64 = false;   // PM_RETRI pass in FP64 (the mixed path's algorithm, FP64 arithmetic)
+    bool onesided64 = false;   // precision "fp64-onesided": every structural slot is kept
+    bool f64 = false;          // PM_RETRI in FP64 (passes_f64.cuh)
+    bool cert = false;         // the pair search takes the certified FP32 geometry
+    DevBuf vexp, valsNlo, valslo;   // FP64 one-sided pass: vertex exponents, second integers (singular kernels)
     DevBuf vcnt, vptr, vel, adjcnt, xadj, adj;
     DevBuf stamp_epoch;   // per-warp stamp epochs of the search
     long long stamp_layout[3] = {0, 0, 0};   // warps, element and vertex stride the stamps were laid out for
@@ -487,7 +548,7 @@ struct Session {
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
                 &hcap, &hptr, &htab, &tpos, &dslot, &rwords, &rbase, &rlo, &rankmap, &eid_ptr, &eid, &vp_cnt, &vp_off, &vp_ptr, &vp_scratch, &pscratch, &rowoff, &kclist, &valsN, &elp,
                 &po_cnt, &po_off, &po_ptr, &po_scratch, &tcnt, &tptr, &tcols, &sv_vec, &sv_part, &zptr, &zidx, &vacc, &vtiny,
-                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel};
+                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo};
     }
     ~Session() {
         for (DevBuf *b : buffers()) b->release();
@@ -551,6 +612,15 @@ static int d2h(Session &S, T *host, const T *dev, size_t n) {
 }
 
 static int device_ok();
+constexpr size_t F64_MAX_SMEM = 227 * 1024;
+constexpr int F64_REFUSED = -100;   // internal: the call goes to the colored passes
+
+// Kernel class of a problem for the one-sided passes: 0 constant kernel (closed forms), 1 other
+// regular kernel, 2 singular kernel with Duffy close pairs.
+static int kernel_class(const ProbParams &q) {
+    if (q.kernel == KER_CONSTANT || q.kernel == KER_CONSTANT3D) return 0;
+    return duffy_close(q) ? 2 : 1;
+}
 
 // Host checks of the problems first (they need no device, so a configuration error is reported as
 // such on any machine), then the device: stream, events, uploads.
@@ -616,12 +686,22 @@ static int session_init(Session &S, const nlfem_problem *probs, int n, bool syst
         if (S.prec == PREC_MIX && S.dim == 2 && all_retri && !any_zeta) S.pmode = PM_RETRI;
         if (S.prec == PREC_MIX && all_bary && !any_singular && !any_zeta) S.pmode = PM_BARY;
         if (S.od > 1) S.pmode = PM_VEC;
-        if (S.onesided64) {
-            if (!(S.dim == 2 && all_retri && !any_zeta))
-                return fail(NLFEM_ERR_UNSUPPORTED, "precision \"fp64-onesided\" covers the 2D retriangulate rule "
-                                                   "without domain-decomposition weights");
-            S.pmode = PM_RETRI;
+        if (S.onesided64 && !(S.dim == 2 && all_retri && !any_zeta))
+            return fail(NLFEM_ERR_UNSUPPORTED, "precision \"fp64-onesided\" covers the 2D retriangulate rule "
+                                               "without domain-decomposition weights");
+        // FP64: the one-sided pass where it covers every problem of the call and its rule's tables
+        // fit an SM's shared memory (16 to 41 times the colored passes' speed on 2 * 32^2 to 2 * 128^2
+        // triangles, see passes_f64.cuh), the colored passes for everything else
+        bool all_f64 = system && S.prec == PREC_F64 && all_retri;
+        S.cert = system;
+        for (const ProbParams &q : S.hprm) {
+            all_f64 = all_f64 && q.f64ok && f64_smem_bytes(kernel_class(q), S.rule.nPx) <= F64_MAX_SMEM;
+            const bool known = (q.remote == MTH_RETRIANGULATE || q.remote == MTH_BARYCENTER) &&
+                               (q.close == MTH_RETRIANGULATE || q.close == MTH_BARYCENTER || duffy_close(q));
+            S.cert = S.cert && q.cert && known;   // the filtered search knows these rules' tests
         }
+        S.f64 = all_f64;
+        if (all_f64) S.pmode = PM_RETRI;
     }
     r = device_ok();
     if (r) return r;
@@ -866,7 +946,8 @@ static int run_bfs(Session &S) {
     // visited set: per-warp stamp arrays in global memory. (A shared-memory bitmap over the
     // problem's elements was measured slower: neighbouring candidates share a word, so the
     // shared-memory atomics serialise, and the bitmaps cap the occupancy.)
-    auto kfn = S.prec == PREC_MIX ? k_bfs<DIM, PREC_MIX> : k_bfs<DIM, PREC_F64>;
+    // the certified FP32 tests give the FP64 predicate's pairs (exact routine inside the margins)
+    auto kfn = S.prec == PREC_MIX || S.cert ? k_bfs<DIM, PREC_MIX> : k_bfs<DIM, PREC_F64>;
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, BFS_THREADS, 0));
     per_sm = std::max(per_sm, 1);
@@ -1114,6 +1195,7 @@ static int run_slot_maps(Session &S) {
         return NLFEM_OK;
     }
     ENS(S.tpos, sizeof(int) * (nnz + 1));
+    if (nnz >= 0x7fffffffLL && S.f64 && !S.onesided64) return F64_REFUSED;
     if (nnz >= 0x7fffffffLL)
         return fail(NLFEM_ERR_UNSUPPORTED, "the one-sided pass indexes matrix slots with 32-bit integers (2^31 - 1 slots at most)");
     ENS(S.dslot, sizeof(int) * (nE * dV * dV + 1));
@@ -1507,54 +1589,51 @@ static int run_close(Session &S) {
 // first), so every problem goes through the same code as its single assembly and the batch matrices
 // equal the single ones bit for bit. A contribution outside the fixed-point range sets err[5]; the
 // pass is then redone with a unit 2^16 times coarser.
-template <typename PR>
-using OneSidedKernelT = void (*)(MixArgs, Rule, PR);
-typedef OneSidedKernelT<PassRule> OneSidedKernel;
-// Kernel class of a problem for the one-sided passes: 0 constant kernel (closed forms), 1 other
-// regular kernel, 2 singular kernel with Duffy close pairs.
-static int kernel_class(const ProbParams &q) {
-    if (q.kernel == KER_CONSTANT || q.kernel == KER_CONSTANT3D) return 0;
-    return duffy_close(q) ? 2 : 1;
-}
-
-template <typename PR>
-static int run_pass_one_sided(Session &S, const PassArgs &pa, const PR &pr, const OneSidedKernelT<PR> *kfn,
-                              int threads, size_t smem) {
-    const long long nnz = S.nnz_struct;
+typedef void (*OneSidedKernel)(MixArgs, Rule, PassRule);
+// One launch per kernel class of the call's problems: the class and its element list (null: every
+// element).
+struct ClassLaunch { int cls; const int *list; int count; };
+static int class_launches(Session &S, ClassLaunch *L, int *nl) {
     int ncls[3] = {0, 0, 0};
     for (const ProbParams &q : S.hprm) ncls[kernel_class(q)]++;
-    struct Launch { OneSidedKernelT<PR> k; const int *list; int count; int per_sm; };
-    Launch L[3];
-    int nl = 0;
+    *nl = 0;
     for (int c = 0; c < 3; c++)
-        if (ncls[c] == (int)S.hprm.size()) L[nl++] = Launch{kfn[c], nullptr, (int)S.nE, 0};
-    if (nl == 0) {   // several classes: one launch per class over its problems' elements
-        if (S.kc_off[0] < 0) {
-            if (S.replay) return fail(NLFEM_ERR_UNSUPPORTED, "element list by kernel class missing in graph capture");
-            std::vector<int> h;
-            h.reserve((size_t)S.nE);
-            for (int c = 0; c < 3; c++) {
-                S.kc_off[c] = (long long)h.size();
-                for (const ProbParams &q : S.hprm)
-                    if (kernel_class(q) == c)
-                        for (int e = 0; e < q.nE; e++) h.push_back(q.elem_off + e);
-            }
-            S.kc_off[3] = (long long)h.size();
-            ENS(S.kclist, sizeof(int) * (h.size() + 1));
-            CK(cudaMemcpyAsync(S.kclist.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, S.st));
-            CK(cudaStreamSynchronize(S.st));
+        if (ncls[c] == (int)S.hprm.size()) L[(*nl)++] = ClassLaunch{c, nullptr, (int)S.nE};
+    if (*nl) return NLFEM_OK;
+    if (S.kc_off[0] < 0) {
+        if (S.replay) return fail(NLFEM_ERR_UNSUPPORTED, "element list by kernel class missing in graph capture");
+        std::vector<int> h;
+        h.reserve((size_t)S.nE);
+        for (int c = 0; c < 3; c++) {
+            S.kc_off[c] = (long long)h.size();
+            for (const ProbParams &q : S.hprm)
+                if (kernel_class(q) == c)
+                    for (int e = 0; e < q.nE; e++) h.push_back(q.elem_off + e);
         }
-        const int *lst = S.kclist.get<int>();
-        for (int c = 0; c < 3; c++)
-            if (S.kc_off[c + 1] > S.kc_off[c])
-                L[nl++] = Launch{kfn[c], lst + S.kc_off[c], (int)(S.kc_off[c + 1] - S.kc_off[c]), 0};
+        S.kc_off[3] = (long long)h.size();
+        ENS(S.kclist, sizeof(int) * (h.size() + 1));
+        CK(cudaMemcpyAsync(S.kclist.p, h.data(), sizeof(int) * h.size(), cudaMemcpyHostToDevice, S.st));
+        CK(cudaStreamSynchronize(S.st));
     }
+    for (int c = 0; c < 3; c++)
+        if (S.kc_off[c + 1] > S.kc_off[c])
+            L[(*nl)++] = ClassLaunch{c, S.kclist.get<int>() + S.kc_off[c], (int)(S.kc_off[c + 1] - S.kc_off[c])};
+    return NLFEM_OK;
+}
+
+static int run_pass_one_sided(Session &S, const PassArgs &pa, const PassRule &pr, const OneSidedKernel *kfn,
+                              int threads, size_t smem) {
+    const long long nnz = S.nnz_struct;
+    ClassLaunch L[3];
+    int nl = 0, per_sm[3] = {0, 0, 0};
+    int rc = class_launches(S, L, &nl);
+    if (rc) return rc;
     for (int i = 0; i < nl; i++) {
-        CK(cudaFuncSetAttribute(L[i].k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&L[i].per_sm, L[i].k, threads, smem));
-        if (L[i].per_sm < 1) return fail(NLFEM_ERR_UNSUPPORTED, "quadrature rule too large for the pass's shared memory");
-        if (S.tune_pass > 0) L[i].per_sm = std::min(L[i].per_sm, S.tune_pass);   // autotuned
-        S.used_pass = std::max(i ? S.used_pass : 0, L[i].per_sm);
+        CK(cudaFuncSetAttribute(kfn[L[i].cls], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[i], kfn[L[i].cls], threads, smem));
+        if (per_sm[i] < 1) return fail(NLFEM_ERR_UNSUPPORTED, "quadrature rule too large for the pass's shared memory");
+        if (S.tune_pass > 0) per_sm[i] = std::min(per_sm[i], S.tune_pass);   // autotuned
+        S.used_pass = std::max(i ? S.used_pass : 0, per_sm[i]);
     }
     MixArgs ma;
     ma.p = pa;
@@ -1583,7 +1662,7 @@ static int run_pass_one_sided(Session &S, const PassArgs &pa, const PR &pr, cons
             ma.p.list = L[i].list;
             ma.p.count = L[i].count;
             CK(cudaMemsetAsync(ma.work, 0, sizeof(int), S.st));
-            L[i].k<<<(unsigned)(S.nSM * L[i].per_sm), threads, smem, S.st>>>(ma, S.rule, pr); ++S.nlaunch;
+            kfn[L[i].cls]<<<(unsigned)(S.nSM * per_sm[i]), threads, smem, S.st>>>(ma, S.rule, pr); ++S.nlaunch;
             CK(cudaGetLastError());
         }
         if (retri) {   // termLocalPrime blocks, then the transposed termNonloc sums
@@ -1608,6 +1687,69 @@ static int run_pass_one_sided(Session &S, const PassArgs &pa, const PR &pr, cons
         }
         CK(cudaMemcpyAsync(S.prm.p, S.hprm.data(), sizeof(ProbParams) * S.hprm.size(), cudaMemcpyHostToDevice, S.st));
     }
+    return fail(NLFEM_ERR_NUMERIC, "contribution outside the fixed-point range (non-finite value?)");
+}
+
+// One-sided FP64 pass (passes_f64.cuh): vertex exponents, one persistent launch per kernel class,
+// then the partner blocks and the symmetric completion. A value outside the fixed-point range
+// (a singular kernel on a mesh with extreme grading, non-finite values) hands the call to the
+// colored passes (precision "fp64"; "fp64-onesided" reports it).
+static int run_pass_f64(Session &S, const PassArgs &pa) {
+    const long long nnz = S.nnz_struct;
+    const PassRuleT<double> pr = make_pass_rule<double>(S.rule, 2);
+    typedef void (*Kernel)(F64Args, Rule, PassRuleT<double>);
+    const Kernel kfn[3] = {k_pass_f64<MIX_CONST>, k_pass_f64<MIX_REGULAR>, k_pass_f64<MIX_SINGULAR>};
+    ClassLaunch L[3];
+    int nl = 0;
+    int r = class_launches(S, L, &nl);
+    if (r) return r;
+    bool wide = false;
+    for (int i = 0; i < nl; i++) wide = wide || L[i].cls == MIX_SINGULAR;
+    ENS(S.vexp, sizeof(int) * (S.nV + 1));
+    ENS(S.valsN, sizeof(long long) * (nnz + 1));
+    const size_t elp_bytes = sizeof(long long) * F64_ELP * (S.nE + 1);
+    ENS(S.elp, elp_bytes);
+    ENS(S.valslo, sizeof(long long) * (nnz + 1));
+    if (wide) ENS(S.valsNlo, sizeof(long long) * (nnz + 1));
+    k_vexp<<<grid_for(S.nV, 256), 256, 0, S.st>>>(S.vptr.get<long long>(), S.vel.get<int>(), S.adet.get<double>(), S.nV, S.vexp.get<int>()); ++S.nlaunch;
+    CK(cudaMemsetAsync(S.valsN.p, 0, sizeof(long long) * (nnz + 1), S.st));
+    CK(cudaMemsetAsync(S.elp.p, 0, elp_bytes, S.st));
+    CK(cudaMemsetAsync(S.valslo.p, 0, sizeof(long long) * (nnz + 1), S.st));
+    if (wide) CK(cudaMemsetAsync(S.valsNlo.p, 0, sizeof(long long) * (nnz + 1), S.st));
+    CK(cudaMemsetAsync(S.err.get<int>() + 5, 0, sizeof(int), S.st));
+    F64Args fa;
+    fa.m.p = pa;
+    fa.m.m = slot_map(S);
+    fa.m.work = reinterpret_cast<int *>(S.counters.get<unsigned long long>() + 10);
+    fa.m.valsN = S.valsN.get<long long>();
+    fa.m.elp = S.elp.get<long long>();
+    fa.vexp = S.vexp.get<int>();
+    fa.valsNlo = wide ? S.valsNlo.get<long long>() : nullptr;
+    fa.valslo = S.valslo.get<long long>();
+    for (int i = 0; i < nl; i++) {
+        if (L[i].count == 0) continue;
+        const size_t smem = f64_smem_bytes(L[i].cls, S.rule.nPx);
+        int per_sm = 0;
+        CK(cudaFuncSetAttribute(kfn[L[i].cls], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn[L[i].cls], F64_THREADS, smem));
+        per_sm = std::max(per_sm, 1);
+        if (S.tune_pass > 0) per_sm = std::min(per_sm, S.tune_pass);   // autotuned
+        S.used_pass = std::max(i ? S.used_pass : 0, per_sm);
+        fa.m.p.list = L[i].list;
+        fa.m.p.count = L[i].count;
+        CK(cudaMemsetAsync(fa.m.work, 0, sizeof(int), S.st));
+        kfn[L[i].cls]<<<(unsigned)(S.nSM * per_sm), F64_THREADS, smem, S.st>>>(fa, S.rule, pr); ++S.nlaunch;
+        CK(cudaGetLastError());
+    }
+    k_elem_blocks_f64<<<grid_for(S.nE, 256), 256, 0, S.st>>>(fa.m.elp, S.adet.get<double>(), fa.vexp, S.dslot.get<int>(), S.T32.get<int>(), S.labV.get<int>(), S.eprob.get<int>(), S.prm.get<ProbParams>(), pr.insum[5], pr.insum[6], pr.insum[8], S.nE, S.vals.get<long long>(), fa.valslo, S.err.get<int>()); ++S.nlaunch;
+    k_sym_add_f64<<<S.nSM * 16, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.cols.get<int>(), S.tpos.get<int>(), fa.m.valsN, fa.valsNlo, fa.valslo, fa.vexp, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.nV, S.vals.get<double>()); ++S.nlaunch;
+    CK(cudaGetLastError());
+    if (S.replay) return NLFEM_OK;   // the flag is checked after the replay
+    int ovf = 0;
+    r = d2h(S, &ovf, S.err.get<int>() + 5, 1);
+    if (r) return r;
+    if (!ovf) return NLFEM_OK;
+    if (!S.onesided64) return F64_REFUSED;
     return fail(NLFEM_ERR_NUMERIC, "contribution outside the fixed-point range (non-finite value?)");
 }
 
@@ -1698,16 +1840,10 @@ static int run_passes(Session &S) {
     a.touched = S.prec == PREC_MIX && S.pmode == PM_COLORED ? S.touched.get<unsigned char>() : nullptr;
     if (S.pmode == PM_VEC) return run_pass_vec<DIM>(S);
     const PassRule pr = make_pass_rule<float>(S.rule, DIM);
-    if (S.pmode == PM_RETRI && S.onesided64) {
-        const PassRuleT<double> pr64 = make_pass_rule<double>(S.rule, DIM);
-        const OneSidedKernelT<PassRuleT<double>> k[3] = {k_pass_mix2d<MIX_CONST, double>, k_pass_mix2d<MIX_REGULAR, double>,
-                                                        k_pass_mix2d<MIX_SINGULAR, double>};
-        return run_pass_one_sided(S, a, pr64, k, MIX_THREADS, mix_warp_bytes<double>(S.rule.nPx) * MIX_WARPS);
-    }
+    if (S.pmode == PM_RETRI && S.f64) return run_pass_f64(S, a);
     if (S.pmode == PM_RETRI) {
-        const OneSidedKernel k[3] = {k_pass_mix2d<MIX_CONST, float>, k_pass_mix2d<MIX_REGULAR, float>,
-                                     k_pass_mix2d<MIX_SINGULAR, float>};
-        return run_pass_one_sided(S, a, pr, k, MIX_THREADS, mix_warp_bytes<float>(S.rule.nPx) * MIX_WARPS);
+        const OneSidedKernel k[3] = {k_pass_mix2d<MIX_CONST>, k_pass_mix2d<MIX_REGULAR>, k_pass_mix2d<MIX_SINGULAR>};
+        return run_pass_one_sided(S, a, pr, k, MIX_THREADS, mix_warp_bytes(S.rule.nPx) * MIX_WARPS);
     }
     if (S.pmode == PM_BARY) {   // no singular kernels here
         const OneSidedKernel k[3] = {k_pass_bary<DIM, true>, k_pass_bary<DIM, false>, k_pass_bary<DIM, false>};
@@ -1737,9 +1873,9 @@ static int run_finish(Session &S) {
     ENS(S.fptr, sizeof(long long) * (nV + 1));
     // values: FP64 sums, double-float sums with touched flags (two-sided mixed passes), or
     // fixed-point sums of the one-sided pass (every structural slot received a contribution)
-    const int vmode = S.pmode != PM_COLORED ? VAL_FX : (S.prec == PREC_MIX ? VAL_DF : VAL_F64);
+    const int vmode = S.prec == PREC_F64 ? VAL_F64 : (S.pmode != PM_COLORED ? VAL_FX : VAL_DF);
     const unsigned char *tch = vmode == VAL_DF ? S.touched.get<unsigned char>() : nullptr;
-    const FinishArgs fa{vmode, tch, S.vprob.get<int>(), S.prm.get<ProbParams>()};
+    const FinishArgs fa{vmode, tch, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.onesided64};
     k_finish_count<<<grid_for(nV * 32, 256), 256, 0, S.st>>>(S.rowptr.get<long long>(), nV, S.vals.get<double>(), fa, S.keepcnt.get<int>()); ++S.nlaunch;
     int r = scan_excl<int>(S, S.keepcnt.get<int>(), nV, S.fptr.get<long long>());
     if (r) return r;
@@ -1825,6 +1961,11 @@ static int run_system_post(Session &S) {
 template <int DIM>
 static int run_system_t(Session &S) {
     int r = run_system_body<DIM>(S);
+    if (r == F64_REFUSED) {   // the colored passes hold what the one-sided FP64 pass cannot
+        S.f64 = false;
+        S.pmode = PM_COLORED;
+        r = run_system_body<DIM>(S);
+    }
     return r ? r : run_system_post(S);
 }
 
@@ -2264,7 +2405,7 @@ static std::string tune_key(const Session &S, const char *stage) {
     for (const ProbParams &q : S.hprm) kc |= 1 << kernel_class(q);
     for (char &c : name) if (c == ' ') c = '_';
     return name + "|" + stage + "|d" + std::to_string(S.dim) + "|m" + std::to_string(S.pmode) + "|p" +
-           std::to_string(S.prec) + (S.onesided64 ? "o" : "") + "|k" + std::to_string(kc);
+           std::to_string(S.prec) + "|k" + std::to_string(kc);
 }
 
 static void tune_load_locked() {

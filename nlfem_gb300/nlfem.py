@@ -16,9 +16,9 @@ reference raises it (output dimension mismatch, bad arma header) and ``NlfemErro
 reference would abort the process.
 
 Extra configuration keys (absent from the reference): ``"precision"``: ``"fp64"`` (default,
-the reference's arithmetic), ``"mixed"`` (FP32 quadrature with FP64 cut geometry and FP64
-accumulation), or ``"fp64-onesided"`` (the mixed path's algorithm in FP64 arithmetic, 2D
-retriangulate only: it separates what the precision costs from what the algorithm saves).
+FP64 arithmetic throughout), ``"mixed"`` (FP32 quadrature with FP64 cut geometry and exact integer
+accumulation), or ``"fp64-onesided"`` (the one-sided FP64 pass by name, 2D retriangulate only, with
+every structural matrix slot kept; ``"fp64"`` takes the same pass where it applies).
 """
 import ctypes
 import os

@@ -1130,3 +1130,68 @@ def test_mixed_refuses_elements_far_larger_than_the_horizon(nl, orc):
     if B.nnz:
         fro, mx = rel_errors(A, B)
         assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+
+
+def _split_rule(n):
+    """n-point rules of the reference triangle for the FP64 pass's mask tables: the centroid, the 7- and
+    16-point rules, and the 7-point rule on each of the four midpoint triangles (28 points)."""
+    from nlfem_gb300 import quadrules
+    if n == 1:
+        return quadrules.centroid1()
+    if n in (7, 16):
+        return quadrules.dunavant7() if n == 7 else quadrules.dunavant16()
+    P, w = quadrules.dunavant7()
+    corners = [((0, 0), (.5, 0), (0, .5)), ((.5, 0), (1, 0), (.5, .5)), ((0, .5), (.5, .5), (0, 1)), ((.5, .5), (0, .5), (.5, 0))]
+    pts = [np.array(a) + P[:, :1] * (np.array(b) - np.array(a)) + P[:, 1:] * (np.array(c) - np.array(a)) for a, b, c in corners]
+    return np.concatenate(pts), np.tile(w / 4, 4)
+
+
+@pytest.mark.parametrize("nq,kern", [(1, "constant"), (16, "constant"), (28, "constant"), (1, "parabola"), (28, "parabola"), (7, "constant")])
+def test_fp64_pass_rules_numberings_and_graph(nl, orc, nq, kern):
+    """The one-sided FP64 pass at outer rules of one to four mask bytes, on a graded mesh (element
+    measures over two decades) with a random vertex numbering (hash slot maps), against the oracle;
+    normal runs, graph replays and a batch give the same bits."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(14, 0.1, jitter=0.15, seed=71)
+    v = np.sign(v) * np.abs(v) ** 1.7
+    perm = np.random.default_rng(5).permutation(len(v))
+    v2 = np.empty_like(v)
+    v2[perm] = v
+    m = meshes.mesh_dict(v2, perm[e], l)
+    P, w = _split_rule(nq)
+    c = conf2d()
+    c["quadrature"] = {"outer": {"points": P, "weights": w}, "inner": {"points": P, "weights": w}}
+    k = {"function": kern, "horizon": 0.11, "outputdim": 1}
+    A = nl.stiffnessMatrix(dict(m), k, c)
+    B = orc.assemble(m, k, c)["A"]
+    assert same_pattern(A, B)
+    fro, mx = rel_errors(A, B)
+    assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+    s = nl.Session([(dict(m), k, c), (square_mesh(9, 0.1, jitter=0.2, seed=72), KC, c)])
+    try:
+        for graph in (False, True, True):
+            s.assemble(graph=graph)
+            C = s.download(0)
+            assert same_pattern(A, C) and np.array_equal(A.tocsr().data, C.data)
+    finally:
+        s.close()
+
+
+def test_fp64_general_pass_still_taken(nl, orc):
+    """Calls outside the one-sided FP64 pass (a sliver element, an element far above the horizon beside
+    ordinary ones) take the general FP64 passes, alone and in a batch with an ordinary problem."""
+    m = square_mesh(10, 0.1, jitter=0.1, seed=73)
+    v = m["vertices"].copy()
+    v[0] = 0.5 * (v[1] + v[11]) + 1e-13   # a corner moved onto the diagonal of its cell: slivers
+    from nlfem_gb300 import meshes
+    sliver = meshes.mesh_dict(v, m["elements"], m["elementLabels"])
+    A = nl.stiffnessMatrix(dict(sliver), KC, conf2d())
+    B = orc.assemble(sliver, KC, conf2d())["A"]
+    assert same_pattern(A, B)
+    fro, mx = rel_errors(A, B)
+    assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+    As = nl.stiffnessMatrix_batch([(dict(sliver), KC, conf2d()), (dict(m), KC, conf2d())])
+    assert same_pattern(As[0], A) and abs(As[0] - A).max() == 0
+    R = orc.assemble(m, KC, conf2d())["A"]
+    fro, mx = rel_errors(As[1], R)
+    assert same_pattern(As[1], R) and fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
