@@ -22,6 +22,7 @@
 #include "passes_mix.cuh"
 #include "passes_f64.cuh"
 #include "passes_bary.cuh"
+#include "passes_f64_bary.cuh"
 #include "passes_vec.cuh"
 
 #include <algorithm>

@@ -52,6 +52,7 @@ struct F64Args {
     const int *vexp;            // per vertex, 8 log2 of its elements' |det| sum, rounded up
     long long *valslo;          // second integers of vals
     long long *valsNlo;         // second integers of valsN (singular kernels)
+    const double *mtab;         // constant kernels: the mask table (k_mask_table)
 };
 
 struct F64Warp {
@@ -115,6 +116,45 @@ __device__ __forceinline__ long long f64_fix_lo(double q, long long i) {
 }
 __device__ __forceinline__ double f64_join(long long hi, long long lo) {
     return (double)hi + (double)lo * (1.0 / (double)(1LL << F64_WIDE));
+}
+
+// s + c += x y, c the low part of the sum (product and sum without loss to second order)
+__device__ __forceinline__ void f64_acc2(double &s, double &c, double x, double y) {
+    const double p = x * y, t = s + p, z = t - s;
+    c += ((s - (t - z)) + (p - z)) + fma(x, y, -p);
+    s = t;
+}
+// Outer sum over the mask byte of table entry i (8 outer points from 8 (i >> 8) on) of dx_k f_k, f a
+// product of up to two basis functions: r < 0 leaves out the first, c < 0 the second. Every entry of
+// the matrix takes these sums, so they are summed with compensation.
+__device__ __forceinline__ double f64_mask_sum(const Rule &rule, int dV, int i, int r, int c) {
+    double s = 0, e = 0;
+    for (int b = 0; b < 8; b++) {
+        const int k = 8 * (i >> 8) + b;
+        if (!((i >> b) & 1) || k >= rule.nPx) continue;
+        const double pr = r < 0 ? 1.0 : rule.psix[dV * k + r], pc = c < 0 ? 1.0 : rule.psix[dV * k + c];
+        const double w = rule.dx[k] * pr;
+        f64_acc2(s, e, w, pc);
+        e += fma(rule.dx[k], pr, -w) * pc;
+    }
+    return s + e;
+}
+
+// Mask table of the rule, TS numbers per entry: the sums over dx psi_r, then over dx psi_r psi_c (r < c),
+// and in 2D over dx. Built once per assembly: the compensated sums on the FP64 pipe would cost each
+// block of the pass 0.2 ms with 11 points, copying them costs it a few microseconds.
+__global__ void k_mask_table(Rule rule, int dV, int TS, int n, double *__restrict__ tab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n * TS) return;
+    const int m = i / TS;
+    int q = i - TS * m, r = q, c = -1;
+    if (q >= dV) {   // (r, c) of the q-th product, or past them
+        r = 0;
+        for (q -= dV; r < dV - 1 && q >= dV - 1 - r; r++) q -= dV - 1 - r;
+        c = r + 1 + q;
+        if (r == dV - 1) r = c = -1;
+    }
+    tab[i] = f64_mask_sum(rule, dV, m, r, c);
 }
 
 template <int KIND>
@@ -242,17 +282,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
     }
     __syncthreads();
     if (CK) {
-        for (int i = threadIdx.x; i < f64_tab_entries(nPx); i += F64_THREADS) {
-            double s[7] = {0, 0, 0, 0, 0, 0, 0};
-            for (int b = 0; b < 8; b++) {
-                const int k = 8 * (i >> 8) + b;
-                if (((i >> b) & 1) && k < nPx)
-#pragma unroll
-                    for (int q = 0; q < 7; q++) s[q] += coef[7 * k + q];
-            }
-#pragma unroll
-            for (int q = 0; q < 7; q++) tab[7 * i + q] = s[q];
-        }
+        for (int i = threadIdx.x; i < 7 * f64_tab_entries(nPx); i += F64_THREADS) tab[i] = fa.mtab[i];
         __syncthreads();
     }
     long long *vals = reinterpret_cast<long long *>(a.vals);
@@ -589,7 +619,7 @@ __global__ void k_elem_blocks_f64(const long long *__restrict__ elp, const doubl
 }
 
 // The FP64 matrix from the sums: entry (t, v) is the diagonal blocks' part minus the termNonloc sums
-// of the slot and of its transposed slot; each diagonal entry is minus its row's other entries. vals
+// of the slot and of its transposed slot (tpos null: rules without Prime blocks have none); each diagonal entry is minus its row's other entries. vals
 // is replaced in place by FP64 values. One warp per row; HBM-bound (each slot's sums are read
 // twice).
 __global__ void k_sym_add_f64(const long long *__restrict__ rowptr, const int *__restrict__ cols,
@@ -610,7 +640,7 @@ __global__ void k_sym_add_f64(const long long *__restrict__ rowptr, const int *_
         for (long long s = b + lane; s < e; s += 32) {
             const int v = cols[s];
             if (v == (int)t) { dslot = s; continue; }
-            const int tp = tpos[s];
+            const int tp = tpos ? tpos[s] : -1;
             const long long ts = tp >= 0 ? rowptr[v] + tp : -1;
             double q = valsNlo ? f64_join(valsN[s], valsNlo[s]) : (double)valsN[s];
             if (ts >= 0) q += valsNlo ? f64_join(valsN[ts], valsNlo[ts]) : (double)valsN[ts];

@@ -1,6 +1,7 @@
 // Host orchestration of the assembly pipeline and the C ABI (included by assemble.cu).
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace nlg {
 
@@ -186,52 +187,70 @@ static long zeta_common(const long *idx, const long *ptr, long a, long b) {
     return n;
 }
 
-// Whether the one-sided FP64 pass (passes_f64.cuh) takes the problem, and the bounds its units
-// follow from. A pair's blocks are at most kbound |T| |b| times the rules' absolute sums (CN, CD:
-// basis functions at inner points of polygons inside the element are at most the largest absolute
-// row sum of the rule's own); for singular kernels kbound is the value at the mean element size
-// times 2^20, and contributions beyond it are detected. Elements near degenerate (where the
-// reference's solve2x2 may abort), bounds far outside the exponent range and options that
-// need the general pass go there. fp64-onesided, which has no such pass to match, is bound only by
-// the range.
+// Whether a one-sided FP64 pass takes the problem (passes_f64.cuh, the 2D retriangulate rule;
+// passes_f64_bary.cuh, the barycenter rule with a constant kernel), and the bounds its units follow
+// from. A pair's blocks are at most kbound |T| |b| times the rules' absolute sums (CN, CD: basis
+// functions at inner points of polygons inside the element are at most the largest absolute row
+// sum of the rule's own); for singular kernels kbound is the value at the mean element size times
+// 2^20, and contributions beyond it are detected. Elements near degenerate (where the reference's
+// solve2x2 may abort; the barycenter rule never calls it), bounds far outside the exponent range
+// and options that need the general pass go there. fp64-onesided, which has no such pass to match,
+// is bound only by the range.
 static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, double kbound) {
     P.f64ok = 0;
-    if (!P.cert || p.dim != 2 || p.outdim != 1 || p.is_dg) return;
+    if (!P.cert || p.outdim != 1 || p.is_dg) return;
+    const bool bary = P.remote == MTH_BARYCENTER;
+    if (bary ? P.kernel != KER_CONSTANT && P.kernel != KER_CONSTANT3D
+             : p.dim != 2 || (P.kernel != KER_CONSTANT && P.kernel != KER_PARABOLA && P.kernel != KER_FRACTIONAL)) return;
+    const int dim = p.dim, dV = dim + 1;
     double atot = 0, amin = 1e300, amax = 0;
     bool sound = true;
     for (long e = 0; e < p.nE; e++) {
-        const long *t = &p.elements[3 * e];
-        for (int a = 0; a < 3; a++)
+        const long *t = &p.elements[dV * e];
+        for (int a = 0; a < dV; a++)
             if (t[a] < 0 || t[a] >= p.nV) return;
-        const double *x = &p.vertices[2 * t[0]], *y = &p.vertices[2 * t[1]], *z = &p.vertices[2 * t[2]];
-        const double a = y[0] - x[0], b = z[0] - x[0], c = y[1] - x[1], d = z[1] - x[1];
-        const double det = fabs(a * d - b * c), scale = (fabs(a) + fabs(c)) * (fabs(b) + fabs(d));
-        sound = sound && det > 1e-10 * scale && std::max(fabs(a), fabs(c)) > 1e-14;
+        double m[3][3];
+        for (int c = 1; c < dV; c++)
+            for (int j = 0; j < dim; j++) m[c - 1][j] = p.vertices[dim * t[c] + j] - p.vertices[dim * t[0] + j];
+        double det;
+        if (dim == 2) {
+            det = fabs(m[0][0] * m[1][1] - m[1][0] * m[0][1]);
+            const double l0 = fabs(m[0][0]) + fabs(m[0][1]), l1 = fabs(m[1][0]) + fabs(m[1][1]);
+            sound = sound && det > 1e-10 * l0 * l1 && std::max(fabs(m[0][0]), fabs(m[0][1])) > 1e-14;
+        } else {
+            det = fabs(m[0][0] * (m[1][1] * m[2][2] - m[1][2] * m[2][1]) - m[0][1] * (m[1][0] * m[2][2] - m[1][2] * m[2][0]) +
+                       m[0][2] * (m[1][0] * m[2][1] - m[1][1] * m[2][0]));
+        }
         atot += det;
         amin = std::min(amin, det);
         amax = std::max(amax, det);
     }
-    double cx = 1, cy = 1, sx = 0, sy = 0, px[3] = {0, 0, 0};
-    for (int k = 0; k < p.nPx; k++) {
-        const double ps[3] = {1.0 - p.Px[2 * k] - p.Px[2 * k + 1], p.Px[2 * k], p.Px[2 * k + 1]};
-        cx = std::max(cx, fabs(ps[0]) + fabs(ps[1]) + fabs(ps[2]));
-        sx += fabs(p.dx[k]);
-        for (int r = 0; r < 3; r++) px[r] += fabs(p.dx[k] * ps[r]);
+    double cx = 1, cy = 1, sx = 0, sy = 0, px[4] = {0, 0, 0, 0};
+    for (int q = 0; q < 2; q++) {   // the outer rule, then the inner rule
+        const int n = q ? p.nPy : p.nPx;
+        const double *X = q ? p.Py : p.Px, *w = q ? p.dy : p.dx;
+        for (int k = 0; k < n; k++) {
+            double ps[4] = {1.0, 0, 0, 0}, sum = 0;
+            for (int j = 0; j < dim; j++) {
+                ps[j + 1] = X[dim * k + j];
+                ps[0] -= X[dim * k + j];
+            }
+            for (int r = 0; r < dV; r++) sum += fabs(ps[r]);
+            (q ? cy : cx) = std::max(q ? cy : cx, sum);
+            (q ? sy : sx) += fabs(w[k]);
+            for (int r = 0; r < dV && !q; r++) px[r] += fabs(w[k] * ps[r]);
+        }
     }
-    for (int k = 0; k < p.nPy; k++) {
-        cy = std::max(cy, fabs(1.0 - p.Py[2 * k] - p.Py[2 * k + 1]) + fabs(p.Py[2 * k]) + fabs(p.Py[2 * k + 1]));
-        sy += fabs(p.dy[k]);
-    }
+    if (bary) kbound *= 2.0;   // the rule's weight 2
     if (P.kernel == KER_PARABOLA) kbound *= cy * cy;   // inner points outside the polygon
     if (P.singular) kbound *= 1048576.0;
-    const double CN = kbound * std::max(px[0], std::max(px[1], px[2])) * sy * cy, CD = 2 * kbound * sx * cx * cx * sy * cy * cy * atot;
+    const double CN = kbound * *std::max_element(px, px + 4) * sy * cy, CD = 2 * kbound * sx * cx * cx * sy * cy * cy * atot;
     if (!(CN > 1e-120 && CN < 1e120 && CD > 1e-120 && CD < 1e120 && sx > 1e-30 && atot > 1e-60 && atot < 1e60 && amax < 1e60)) return;
-    if (P.kernel != KER_CONSTANT && P.kernel != KER_PARABOLA && P.kernel != KER_FRACTIONAL) return;
     P.xN = (int)ceil(8.0 * log2(CN) + 1e-3);
     P.xD = exact_ceil_log2(CD);
     P.xS = exact_ceil_log2(sx * atot);
     if (p.precision == NLFEM_PREC_FP64)
-        P.f64ok = sound && amin > 1e-60 && !P.full_search && !P.zeta && (!P.singular || duffy_close(P));
+        P.f64ok = sound && amin > (bary ? -1.0 : 1e-60) && !P.full_search && !P.zeta && (!P.singular || duffy_close(P));
     else
         P.f64ok = 1;
 }
@@ -485,9 +504,9 @@ struct Session {
     std::vector<int> color_off;
     int prec = 0;
     bool onesided64 = false;   // precision "fp64-onesided": every structural slot is kept
-    bool f64 = false;          // PM_RETRI in FP64 (passes_f64.cuh)
+    bool f64 = false;          // PM_RETRI or PM_BARY in FP64 (passes_f64.cuh, passes_f64_bary.cuh)
     bool cert = false;         // the pair search takes the certified FP32 geometry
-    DevBuf vexp, valsNlo, valslo;   // FP64 one-sided pass: vertex exponents, second integers (singular kernels)
+    DevBuf vexp, valsNlo, valslo, mtab;   // FP64 one-sided passes: vertex exponents, second integers, mask table
     DevBuf vcnt, vptr, vel, adjcnt, xadj, adj;
     DevBuf stamp_epoch;   // per-warp stamp epochs of the search
     long long stamp_layout[3] = {0, 0, 0};   // warps, element and vertex stride the stamps were laid out for
@@ -548,7 +567,7 @@ struct Session {
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
                 &hcap, &hptr, &htab, &tpos, &dslot, &rwords, &rbase, &rlo, &rankmap, &eid_ptr, &eid, &vp_cnt, &vp_off, &vp_ptr, &vp_scratch, &pscratch, &rowoff, &kclist, &valsN, &elp,
                 &po_cnt, &po_off, &po_ptr, &po_scratch, &tcnt, &tptr, &tcols, &sv_vec, &sv_part, &zptr, &zidx, &vacc, &vtiny,
-                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo};
+                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo, &mtab};
     }
     ~Session() {
         for (DevBuf *b : buffers()) b->release();
@@ -692,16 +711,18 @@ static int session_init(Session &S, const nlfem_problem *probs, int n, bool syst
         // FP64: the one-sided pass where it covers every problem of the call and its rule's tables
         // fit an SM's shared memory (16 to 41 times the colored passes' speed on 2 * 32^2 to 2 * 128^2
         // triangles, see passes_f64.cuh), the colored passes for everything else
-        bool all_f64 = system && S.prec == PREC_F64 && all_retri;
+        bool all_f64 = system && S.prec == PREC_F64 && (all_retri || all_bary);
         S.cert = system;
         for (const ProbParams &q : S.hprm) {
-            all_f64 = all_f64 && q.f64ok && f64_smem_bytes(kernel_class(q), S.rule.nPx) <= F64_MAX_SMEM;
+            const size_t smem = all_retri ? f64_smem_bytes(kernel_class(q), S.rule.nPx)
+                                          : (S.dim == 2 ? f64_bary_smem<2>(S.rule.nPx) : f64_bary_smem<3>(S.rule.nPx));
+            all_f64 = all_f64 && q.f64ok && smem <= F64_MAX_SMEM;
             const bool known = (q.remote == MTH_RETRIANGULATE || q.remote == MTH_BARYCENTER) &&
                                (q.close == MTH_RETRIANGULATE || q.close == MTH_BARYCENTER || duffy_close(q));
             S.cert = S.cert && q.cert && known;   // the filtered search knows these rules' tests
         }
         S.f64 = all_f64;
-        if (all_f64) S.pmode = PM_RETRI;
+        if (all_f64) S.pmode = all_retri ? PM_RETRI : PM_BARY;
     }
     r = device_ok();
     if (r) return r;
@@ -1505,8 +1526,10 @@ static int run_pair_blocks(Session &S, long long n, const long *pairs, int close
     return d2h(S, ret, S.keepcnt.get<int>(), (size_t)n);
 }
 
+// Rule constants in type R. The sums enter every entry alike, so FP64 takes them in long double.
 template <typename R>
 static PassRuleT<R> make_pass_rule(const Rule &r, int dim) {
+    typedef typename std::conditional<sizeof(R) == 8, long double, double>::type A;
     PassRuleT<R> pr;
     memset(&pr, 0, sizeof(pr));
     const int dV = dim + 1, NS = dV * (dV + 1) / 2;
@@ -1518,21 +1541,21 @@ static PassRuleT<R> make_pass_rule(const Rule &r, int dim) {
             for (int b = a; b < dV; b++) pr.cxx[NS * k + t++] = (R)(r.dx[k] * r.psix[dV * k + a] * r.psix[dV * k + b]);
         }
     }
-    double insum[1 + 4 + 10] = {0}, mom[6] = {0};
+    A insum[1 + 4 + 10] = {0}, mom[6] = {0};
     for (int i = 0; i < r.nPy; i++) {
         for (int c = 0; c < dim; c++) pr.pyf[dim * i + c] = (R)r.Py[dim * i + c];
         int t = 0;
         insum[0] += r.dy[i];
         for (int a = 0; a < dV; a++) {
             pr.cy[dV * i + a] = (R)(r.dy[i] * r.psiy[dV * i + a]);
-            insum[1 + a] += r.dy[i] * r.psiy[dV * i + a];
+            insum[1 + a] += (A)r.dy[i] * r.psiy[dV * i + a];
             for (int b = a; b < dV; b++) {
-                insum[1 + dV + t] += r.dy[i] * r.psiy[dV * i + a] * r.psiy[dV * i + b];
+                insum[1 + dV + t] += (A)r.dy[i] * r.psiy[dV * i + a] * r.psiy[dV * i + b];
                 pr.cyy[NS * i + t++] = (R)(r.dy[i] * r.psiy[dV * i + a] * r.psiy[dV * i + b]);
             }
         }
         if (dim == 2) {
-            const double px = r.Py[2 * i], py = r.Py[2 * i + 1], w = r.dy[i];
+            const A px = r.Py[2 * i], py = r.Py[2 * i + 1], w = r.dy[i];
             mom[0] += w; mom[1] += w * px; mom[2] += w * py;
             mom[3] += w * px * px; mom[4] += w * px * py; mom[5] += w * py * py;
         }
@@ -1694,11 +1717,13 @@ static int run_pass_one_sided(Session &S, const PassArgs &pa, const PassRule &pr
 // then the partner blocks and the symmetric completion. A value outside the fixed-point range
 // (a singular kernel on a mesh with extreme grading, non-finite values) hands the call to the
 // colored passes (precision "fp64"; "fp64-onesided" reports it).
+template <int DIM>
 static int run_pass_f64(Session &S, const PassArgs &pa) {
     const long long nnz = S.nnz_struct;
-    const PassRuleT<double> pr = make_pass_rule<double>(S.rule, 2);
+    const PassRuleT<double> pr = make_pass_rule<double>(S.rule, DIM);
+    const bool retri = S.pmode == PM_RETRI;
     typedef void (*Kernel)(F64Args, Rule, PassRuleT<double>);
-    const Kernel kfn[3] = {k_pass_f64<MIX_CONST>, k_pass_f64<MIX_REGULAR>, k_pass_f64<MIX_SINGULAR>};
+    const Kernel kfn[3] = {retri ? k_pass_f64<MIX_CONST> : k_pass_bary_f64<DIM>, k_pass_f64<MIX_REGULAR>, k_pass_f64<MIX_SINGULAR>};
     ClassLaunch L[3];
     int nl = 0;
     int r = class_launches(S, L, &nl);
@@ -1708,17 +1733,25 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     ENS(S.vexp, sizeof(int) * (S.nV + 1));
     ENS(S.valsN, sizeof(long long) * (nnz + 1));
     const size_t elp_bytes = sizeof(long long) * F64_ELP * (S.nE + 1);
-    ENS(S.elp, elp_bytes);
+    if (retri) ENS(S.elp, elp_bytes);
     ENS(S.valslo, sizeof(long long) * (nnz + 1));
     if (wide) ENS(S.valsNlo, sizeof(long long) * (nnz + 1));
     k_vexp<<<grid_for(S.nV, 256), 256, 0, S.st>>>(S.vptr.get<long long>(), S.vel.get<int>(), S.adet.get<double>(), S.nV, S.vexp.get<int>()); ++S.nlaunch;
     CK(cudaMemsetAsync(S.valsN.p, 0, sizeof(long long) * (nnz + 1), S.st));
-    CK(cudaMemsetAsync(S.elp.p, 0, elp_bytes, S.st));
+    if (retri) CK(cudaMemsetAsync(S.elp.p, 0, elp_bytes, S.st));
     CK(cudaMemsetAsync(S.valslo.p, 0, sizeof(long long) * (nnz + 1), S.st));
     if (wide) CK(cudaMemsetAsync(S.valsNlo.p, 0, sizeof(long long) * (nnz + 1), S.st));
     CK(cudaMemsetAsync(S.err.get<int>() + 5, 0, sizeof(int), S.st));
+    const int tab_n = f64_tab_entries(S.rule.nPx), tab_ts = retri ? 7 : f64_bary_tab<DIM>();
+    ENS(S.mtab, sizeof(double) * tab_n * tab_ts);
+    for (int i = 0; i < nl; i++)
+        if (L[i].cls == MIX_CONST) {
+            k_mask_table<<<grid_for((long long)tab_n * tab_ts, 64), 64, 0, S.st>>>(S.rule, DIM + 1, tab_ts, tab_n, S.mtab.get<double>());
+            ++S.nlaunch;
+        }
     F64Args fa;
     fa.m.p = pa;
+    fa.mtab = S.mtab.get<double>();
     fa.m.m = slot_map(S);
     fa.m.work = reinterpret_cast<int *>(S.counters.get<unsigned long long>() + 10);
     fa.m.valsN = S.valsN.get<long long>();
@@ -1728,7 +1761,7 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     fa.valslo = S.valslo.get<long long>();
     for (int i = 0; i < nl; i++) {
         if (L[i].count == 0) continue;
-        const size_t smem = f64_smem_bytes(L[i].cls, S.rule.nPx);
+        const size_t smem = retri ? f64_smem_bytes(L[i].cls, S.rule.nPx) : f64_bary_smem<DIM>(S.rule.nPx);
         int per_sm = 0;
         CK(cudaFuncSetAttribute(kfn[L[i].cls], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn[L[i].cls], F64_THREADS, smem));
@@ -1741,8 +1774,9 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
         kfn[L[i].cls]<<<(unsigned)(S.nSM * per_sm), F64_THREADS, smem, S.st>>>(fa, S.rule, pr); ++S.nlaunch;
         CK(cudaGetLastError());
     }
-    k_elem_blocks_f64<<<grid_for(S.nE, 256), 256, 0, S.st>>>(fa.m.elp, S.adet.get<double>(), fa.vexp, S.dslot.get<int>(), S.T32.get<int>(), S.labV.get<int>(), S.eprob.get<int>(), S.prm.get<ProbParams>(), pr.insum[5], pr.insum[6], pr.insum[8], S.nE, S.vals.get<long long>(), fa.valslo, S.err.get<int>()); ++S.nlaunch;
-    k_sym_add_f64<<<S.nSM * 16, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.cols.get<int>(), S.tpos.get<int>(), fa.m.valsN, fa.valsNlo, fa.valslo, fa.vexp, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.nV, S.vals.get<double>()); ++S.nlaunch;
+    if (retri) k_elem_blocks_f64<<<grid_for(S.nE, 256), 256, 0, S.st>>>(fa.m.elp, S.adet.get<double>(), fa.vexp, S.dslot.get<int>(), S.T32.get<int>(), S.labV.get<int>(), S.eprob.get<int>(), S.prm.get<ProbParams>(), pr.insum[5], pr.insum[6], pr.insum[8], S.nE, S.vals.get<long long>(), fa.valslo, S.err.get<int>());
+    S.nlaunch += retri;
+    k_sym_add_f64<<<S.nSM * 16, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.cols.get<int>(), retri ? S.tpos.get<int>() : nullptr, fa.m.valsN, fa.valsNlo, fa.valslo, fa.vexp, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.nV, S.vals.get<double>()); ++S.nlaunch;
     CK(cudaGetLastError());
     if (S.replay) return NLFEM_OK;   // the flag is checked after the replay
     int ovf = 0;
@@ -1840,7 +1874,7 @@ static int run_passes(Session &S) {
     a.touched = S.prec == PREC_MIX && S.pmode == PM_COLORED ? S.touched.get<unsigned char>() : nullptr;
     if (S.pmode == PM_VEC) return run_pass_vec<DIM>(S);
     const PassRule pr = make_pass_rule<float>(S.rule, DIM);
-    if (S.pmode == PM_RETRI && S.f64) return run_pass_f64(S, a);
+    if (S.f64) return run_pass_f64<DIM>(S, a);
     if (S.pmode == PM_RETRI) {
         const OneSidedKernel k[3] = {k_pass_mix2d<MIX_CONST>, k_pass_mix2d<MIX_REGULAR>, k_pass_mix2d<MIX_SINGULAR>};
         return run_pass_one_sided(S, a, pr, k, MIX_THREADS, mix_warp_bytes(S.rule.nPx) * MIX_WARPS);

@@ -1195,3 +1195,29 @@ def test_fp64_general_pass_still_taken(nl, orc):
     R = orc.assemble(m, KC, conf2d())["A"]
     fro, mx = rel_errors(As[1], R)
     assert same_pattern(As[1], R) and fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+
+
+@pytest.mark.parametrize("dim,n,delta,nq", [(3, 3, 0.5, 11), (3, 7, 0.2, 11), (2, 13, 0.15, 1), (2, 12, 0.2, 28)])
+def test_fp64_barycenter_pass(nl, orc, dim, n, delta, nq):
+    """The one-sided FP64 barycenter pass (constant kernels; one to four mask bytes, a partly filled
+    batch on the smallest mesh) against the oracle; graph replays give the same bits."""
+    if dim == 3:
+        m, c, kern = cube_mesh(n, 0.1, jitter=0.15, seed=n), conf3d(), "constant3D"
+    else:
+        m, c, kern = square_mesh(n, 0.1, jitter=0.15, seed=n), conf2d(method="baryCenter"), "constant"
+        P, w = _split_rule(nq)
+        c["quadrature"] = {"outer": {"points": P, "weights": w}, "inner": {"points": P, "weights": w}}
+    k = {"function": kern, "horizon": delta, "outputdim": 1}
+    A = nl.stiffnessMatrix(dict(m), k, c)
+    B = orc.assemble(m, k, c)["A"]
+    assert same_pattern(A, B)
+    fro, mx = rel_errors(A, B)
+    assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+    s = nl.Session([(dict(m), k, c)])
+    try:
+        for graph in (False, True, True):
+            s.assemble(graph=graph)
+            C = s.download(0)
+            assert same_pattern(A, C) and np.array_equal(A.tocsr().data, C.data)
+    finally:
+        s.close()
