@@ -81,8 +81,14 @@ struct FPoly {
     FPt first, last;
 };
 
-__device__ __forceinline__ void fpush(FPoly &Y, const FPt &p, bool &amb) {
+// What the polygon's points are, in order, four bits each (FP64 pass): vertex k (k), the root r of
+// edge k (3 + 2 k + r), a cap point (9).
+enum { FCODE_X = 3, FCODE_CAP = 9 };
+
+template <bool CODES>
+__device__ __forceinline__ void fpush(FPoly &Y, const FPt &p, bool &amb, int code, unsigned long long *codes) {
     if (Y.n >= 9) { amb = true; return; }
+    if (CODES) *codes |= (unsigned long long)code << (4 * Y.n);
     if (Y.R) Y.R[Y.n] = p.y;   // null R: the count only
     if (Y.n == 0) Y.first = p;
     Y.last = p;
@@ -96,8 +102,10 @@ __device__ __forceinline__ void fpush(FPoly &Y, const FPt &p, bool &amb) {
 // bisector of a chord passes through the center), on the side sign(n . m). This form turns the
 // chord ends' position errors into a cap error of the same size instead of amplifying them by
 // delta / |chord|.
+template <bool CODES>
 __device__ __forceinline__ void fplace_cap(FPoly &Y, const FPt &a, const FPt &b, float sq, const F2 *P,
-                                           const F2 *nu, float orientation, bool &amb, unsigned *why = nullptr) {
+                                           const F2 *nu, float orientation, bool &amb, unsigned *why,
+                                           unsigned long long *codes) {
     const F2 n = f2((a.y.y - b.y.y) * orientation, (b.y.x - a.y.x) * orientation);
     const F2 m = f2(0.5f * (a.y.x + b.y.x), 0.5f * (a.y.y + b.y.y));
     const float mm = dot(m, m), nn = dot(n, n);
@@ -109,15 +117,16 @@ __device__ __forceinline__ void fplace_cap(FPoly &Y, const FPt &a, const FPt &b,
     const F2 y = f2(m.x * s, m.y * s);
     const float em = 0.5f * (a.eperp + a.ealong + b.eperp + b.ealong);
     const float ey = delta * em * rsqrtf(mm) + em + 8.f * U32 * delta;
-    if (fin_triangle(y, ey, P, nu, amb, why)) fpush(Y, FPt{y, ey, 0.f}, amb);
+    if (fin_triangle(y, ey, P, nu, amb, why)) fpush<CODES>(Y, FPt{y, ey, 0.f}, amb, FCODE_CAP, codes);
 }
 
 // FP32 method_retriangulate with the triangle P given relative to the ball center. Returns the
 // polygon point count (sub-triangles: fan (R0, R[j+1], R[j+2])); amb = true when a decision was
 // within its margin (the result must then be recomputed in FP64). With R null only the count is
-// kept (the interaction test of the pair search).
+// kept (the interaction test of the pair search); with CODES also what each point is.
+template <bool CODES = false>
 __device__ __forceinline__ int fretriangulate(const F2 *P, float sq, int caps, F2 *R, bool &amb,
-                                              unsigned *why = nullptr) {
+                                              unsigned *why = nullptr, unsigned long long *codes = nullptr) {
     FPoly Y;
     Y.R = R;
     Y.n = 0;
@@ -140,7 +149,7 @@ __device__ __forceinline__ int fretriangulate(const F2 *P, float sq, int caps, F
         const float dp = dot(p, p);
         if (dp > sqlo && dp < sqhi) { amb = true; if (why) *why |= 2u; }
         if (dp <= sq) {
-            fpush(Y, FPt{p, 4.f * U32 * (fabsf(p.x) + fabsf(p.y)), 0.f}, amb);
+            fpush<CODES>(Y, FPt{p, 4.f * U32 * (fabsf(p.x) + fabsf(p.y)), 0.f}, amb, k, codes);
             is_onEdge = false;
         }
         const float ab = dot(q, b), aa = dot(q, q), bb = dot(b, b);
@@ -180,15 +189,15 @@ __device__ __forceinline__ int fretriangulate(const F2 *P, float sq, int caps, F
                 if (!(lam >= 0.f && lam <= 1.f && (qi == 0 || v > 0.f))) continue;
                 is_firstPointLiesOnVertex = is_firstPointLiesOnVertex && (Y.n != 0);
                 const FPt y{f2(fmaf(lam, b.x, q.x), fmaf(lam, b.y, q.y)), eperp, ealong};
-                if (is_onEdge && caps) fplace_cap(Y, Y.last, y, sq, P, nu, orientation, amb, why);
-                fpush(Y, y, amb);
+                if (is_onEdge && caps) fplace_cap<CODES>(Y, Y.last, y, sq, P, nu, orientation, amb, why, codes);
+                fpush<CODES>(Y, y, amb, FCODE_X + 2 * k + qi, codes);
                 is_onEdge = true;
             }
         }
     }
     if (is_onEdge && (!is_firstPointLiesOnVertex && Y.n > 1) && caps) {
         const FPt last = Y.last, first = Y.first;
-        fplace_cap(Y, last, first, sq, P, nu, orientation, amb, why);
+        fplace_cap<CODES>(Y, last, first, sq, P, nu, orientation, amb, why, codes);
     }
     return Y.n;
 }

@@ -333,8 +333,8 @@ struct ProbParams {
     float fx_mul;     // 2^-fx_ue
     int fx_ue;        // scale_exp + guard bits - 62
     double el;        // mean element measure (bounding box / nE), for capacity estimates
-    int cert;         // finite coordinates, elements at most MIX_MAX_H_OVER_DELTA delta: the certified
-                      // FP32 geometry decides the search and the classes (certified.cuh)
+    int cert;         // the certified FP32 geometry may decide the search and the classes (certified.cuh):
+                      // element sizes, horizon and coordinates in its range
     int f64ok;        // the one-sided FP64 pass takes this problem (passes_f64.cuh)
     int xN, xD, xS;   // its fixed-point bounds: 2^(xN / 8) above a pair's termNonloc per |T| |b|, 2^xD above
                       // its diagonal blocks times the mesh's |det| sum, 2^xS above the outer weights' sum times that

@@ -7,8 +7,8 @@
 // arithmetic is FP64, and GB300 runs FP64 at 1/64 of its FP32 rate, so the FP64 pipe bounds the
 // kernel and everything that can leave it does:
 //   * The (pair, outer point) classes come from the certified FP32 test (certified.cuh): a ball
-//     holding the partner or missing it with a margin. All else is a cut item and takes the exact
-//     FP64 polygon.
+//     holding the partner or missing it with a margin. All else is a cut item. Its polygon's structure
+//     comes from the certified FP32 run too, only its points are FP64 (f64_polygon).
 //   * Constant kernels: inside items need no quadrature loop. A pair's inside mask indexes a table
 //     (shared memory, one entry per mask byte) of the rule's outer sums over the mask; its blocks
 //     are those times kc |T| |b| and the rule's inner sums.
@@ -16,9 +16,9 @@
 //     are neighbours: full warps integrate the items, then full warps fold them, one (pair, output)
 //     per lane, instead of every lane walking all outer points.
 // Measured (quadrature phase, against the two-sided colored pass that the path used before): constant
-// kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 51.6 ms against 1725 ms; 2 * 32^2
-// triangles: 1.1 against 66.6 ms; parabola, 2 * 57^2: 16.2 against 257 ms; fractional, 2 * 40^2:
-// 53 against 568 ms.
+// kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 24.5 ms against 1725 ms; 2 * 32^2
+// triangles: 0.54 against 66.6 ms; parabola, 2 * 57^2: 12.2 against 257 ms; fractional, 2 * 40^2:
+// 49.5 against 568 ms.
 //
 // Sums. Every contribution is rounded once to a 64-bit integer and added with an integer atomic,
 // so the result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
@@ -53,6 +53,7 @@ struct F64Args {
     long long *valslo;          // second integers of vals
     long long *valsNlo;         // second integers of valsN (singular kernels)
     const double *mtab;         // constant kernels: the mask table (k_mask_table)
+    int exact2;                 // the inner rule integrates degree two exactly (see f64_item)
 };
 
 struct F64Warp {
@@ -164,21 +165,132 @@ __device__ __forceinline__ double f64_kernel(const ProbParams &P, double r2) {
     return P.kc * exp2(-0.5 * P.expo * log2(r2));
 }
 
+// Square root, reciprocal and reciprocal square root by Newton's iteration from an FP32 seed (24 bits,
+// so two steps reach FP64; the last step of the square root and of the quotient is the residual
+// correction). A CUDA division or square root keeps the FP64 pipe busy about twice as long: they
+// serve arguments whose FP32 seed would leave the FP32 range.
+__device__ __forceinline__ bool f64_seedable(float v) { return v > 1e-30f && v < 1e30f; }
+__device__ __forceinline__ double f64_rsqrt(double v) {
+    const float s = (float)v;
+    if (!f64_seedable(s)) return 1.0 / sqrt(v);
+    double y = (double)rsqrtf(s);
+    y = fma(0.5 * y, fma(-(v * y), y, 1.0), y);
+    return fma(0.5 * y, fma(-(v * y), y, 1.0), y);
+}
+__device__ __forceinline__ double f64_sqrt(double v) {
+    const float s = (float)v;
+    if (!f64_seedable(s)) return sqrt(v);
+    double y = (double)rsqrtf(s);
+    y = fma(0.5 * y, fma(-(v * y), y, 1.0), y);
+    const double g = v * y;
+    return fma(0.5 * y, fma(-g, g, v), g);
+}
+__device__ __forceinline__ double f64_div(double a, double b) {
+    const float s = (float)b;
+    if (!f64_seedable(fabsf(s))) return a / b;
+    double y = (double)(1.f / s);
+    y = fma(y, fma(-b, y, 1.0), y);
+    const double q = a * y;
+    return fma(y, fma(-b, q, a), q);
+}
+
+// Polygon of a cut item: points relative to the ball's center in R, and in the partner's reference
+// coordinates in L (n of each, at most 9).
+struct F64Poly {
+    double R[18], L[18];
+    int n;
+};
+
+// The polygon of B(x) and the triangle Q (relative to x), e1, e2 its edges from Q0. The certified FP32
+// run fixes what the points are (which vertices, which roots of which edges, which caps: the
+// reference's branches); only the points themselves are FP64: per crossing a square root and a
+// quotient, per cap a reciprocal square root. In reference coordinates vertices are constants and
+// a crossing is its root. Against the exact routine, which takes both roots of all three edges with
+// their divisions for every item, that is about a third of the FP64 instructions: with the boundary
+// moments of f64_item 51.5 -> 24.5 ms on 2 * 128^2 triangles (constant kernel). Near-tangent cases
+// go to the exact routine (its points are the reference's bit for bit).
+template <bool PHYS>
+__device__ __forceinline__ void f64_polygon(const ProbParams &P, const double *x, const double *Eb, const double *Q,
+                                            const double *e, double idet, F64Poly &Y) {
+    const F2 Qf[3] = {f2((float)Q[0], (float)Q[1]), f2((float)Q[2], (float)Q[3]), f2((float)Q[4], (float)Q[5])};
+    bool amb = false;
+    unsigned long long codes = 0;
+    Y.n = fretriangulate<true>(Qf, P.sqdelta_f, P.caps, nullptr, amb, nullptr, &codes);
+    auto to_ref = [&](double yx, double yy, double *l) {
+        const double dx = yx - Q[0], dy = yy - Q[1];
+        l[0] = (e[3] * dx - e[2] * dy) * idet;
+        l[1] = (e[0] * dy - e[1] * dx) * idet;
+    };
+    if (amb) {
+        Y.n = xretriangulate(x, Eb, P.sqdelta, P.caps, Y.R);
+        for (int j = 0; j < Y.n; j++) {
+            Y.R[2 * j] -= x[0];
+            Y.R[2 * j + 1] -= x[1];
+            to_ref(Y.R[2 * j], Y.R[2 * j + 1], &Y.L[2 * j]);
+        }
+        return;
+    }
+    unsigned xm = 0, cm = 0;
+    for (int j = 0; j < Y.n; j++) {
+        const int c = (int)(codes >> (4 * j)) & 15;
+        xm |= (unsigned)(c >= FCODE_X && c < FCODE_CAP) << j;
+        cm |= (unsigned)(c == FCODE_CAP) << j;
+        if (c < 3) {
+            Y.L[2 * j] = c == 1 ? 1.0 : 0.0;
+            Y.L[2 * j + 1] = c == 2 ? 1.0 : 0.0;
+            if (PHYS) {
+                Y.R[2 * j] = c == 0 ? Q[0] : (c == 1 ? Q[2] : Q[4]);
+                Y.R[2 * j + 1] = c == 0 ? Q[1] : (c == 1 ? Q[3] : Q[5]);
+            }
+        }
+    }
+#pragma unroll 1
+    for (; xm; xm &= xm - 1) {
+        const int j = __ffs(xm) - 1, c = ((int)(codes >> (4 * j)) & 15) - FCODE_X, k = c >> 1, r = c & 1;
+        const double px = k == 0 ? Q[0] : (k == 1 ? Q[2] : Q[4]), py = k == 0 ? Q[1] : (k == 1 ? Q[3] : Q[5]);
+        const double qx = k == 0 ? Q[2] : (k == 1 ? Q[4] : Q[0]), qy = k == 0 ? Q[3] : (k == 1 ? Q[5] : Q[1]);
+        const double bx = px - qx, by = py - qy;
+        const double ab = qx * bx + qy * by, aad = (qx * qx + qy * qy) - P.sqdelta, bb = bx * bx + by * by;
+        const double sv = f64_sqrt(fmax(ab * ab - aad * bb, 0.0));
+        // the root of larger size has no cancellation, the other is aad / bb over it (as the reference)
+        const bool pos = ab < 0.0;
+        const double big = pos ? sv - ab : -(ab + sv);
+        const bool direct = pos == (r == 0);
+        const double lam = f64_div(direct ? big : aad, direct ? bb : big);
+        Y.R[2 * j] = fma(lam, bx, qx);
+        Y.R[2 * j + 1] = fma(lam, by, qy);
+        Y.L[2 * j] = k == 0 ? 1.0 - lam : (k == 1 ? lam : 0.0);
+        Y.L[2 * j + 1] = k == 0 ? 0.0 : (k == 1 ? 1.0 - lam : lam);
+    }
+#pragma unroll 1
+    for (; cm; cm &= cm - 1) {   // between two crossings (placePointOnCap, integration.cpp:1353-1377)
+        const int j = __ffs(cm) - 1, i = j ? j - 1 : 0, h = j + 1 < Y.n ? j + 1 : 0;
+        const double o = idet > 0 ? -1.0 : 1.0;
+        const double nx = (Y.R[2 * i + 1] - Y.R[2 * h + 1]) * o, ny = (Y.R[2 * h] - Y.R[2 * i]) * o;
+        const double s = P.delta * f64_rsqrt(nx * nx + ny * ny);
+        Y.R[2 * j] = nx * s;
+        Y.R[2 * j + 1] = ny * s;
+        to_ref(Y.R[2 * j], Y.R[2 * j + 1], &Y.L[2 * j]);
+    }
+}
+
 // Inner sums of one item into res (see F64_RN), without the factor |T|: the quadrature over the
-// partner (inside) or over the fan of its polygon with the ball (cut).
+// partner (inside) or over the fan of its polygon with the ball (cut). exact2: the inner rule integrates
+// polynomials of degree two exactly, so a constant kernel's sums over the fan are the polygon's
+// moments, taken from its boundary in reference coordinates (Green's theorem, one term per edge).
 template <int KIND>
 __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, const PassRuleT<double> &pr, bool inside,
-                                         const double *x, const double *Eb, double *res, unsigned &nsub) {
-    const double Q0x = Eb[0] - x[0], Q0y = Eb[1] - x[1];
-    const double e1x = Eb[2] - Eb[0], e1y = Eb[3] - Eb[1], e2x = Eb[4] - Eb[0], e2y = Eb[5] - Eb[1];
-    const double det = e1x * e2y - e1y * e2x;
+                                         bool exact2, const double *x, const double *Eb, double *res, unsigned &nsub) {
+    const double Q[6] = {Eb[0] - x[0], Eb[1] - x[1], Eb[2] - x[0], Eb[3] - x[1], Eb[4] - x[0], Eb[5] - x[1]};
+    const double e[4] = {Eb[2] - Eb[0], Eb[3] - Eb[1], Eb[4] - Eb[0], Eb[5] - Eb[1]};
+    const double det = e[0] * e[3] - e[1] * e[2];
     double S0 = 0, S1[3] = {0, 0, 0}, S2[3] = {0, 0, 0};
     if (KIND != MIX_CONST && inside) {
         nsub++;
         const double rT = fabs(det);
         for (int i = 0; i < rule.nPy; i++) {
-            const double yx = Q0x + e1x * rule.Py[2 * i] + e2x * rule.Py[2 * i + 1];
-            const double yy = Q0y + e1y * rule.Py[2 * i] + e2y * rule.Py[2 * i + 1];
+            const double yx = Q[0] + e[0] * rule.Py[2 * i] + e[2] * rule.Py[2 * i + 1];
+            const double yy = Q[1] + e[1] * rule.Py[2 * i] + e[3] * rule.Py[2 * i + 1];
             const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * rT;
             S0 += kw * rule.dy[i];
 #pragma unroll
@@ -188,64 +300,80 @@ __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, 
             S2[2] += kw * pr.cyy[6 * i + 4];
         }
     } else {
-        const double idet = 1.0 / det;
-        double R[18];
-        const int n = xretriangulate(x, Eb, P.sqdelta, P.caps, R);
-        for (int j = 0; j < n; j++) { R[2 * j] -= x[0]; R[2 * j + 1] -= x[1]; }
-        auto basis = [&](double yx, double yy, double *l) {   // psi_0..2 of b at y
-            const double dx = yx - Q0x, dy = yy - Q0y;
-            l[1] = (e2y * dx - e2x * dy) * idet;
-            l[2] = (e1x * dy - e1y * dx) * idet;
-            l[0] = 1.0 - l[1] - l[2];
-        };
-        if (KIND == MIX_CONST) {   // the rule's moments on each fan triangle (see item_cut_const)
-            const double m0 = pr.mom[0], mx = pr.mom[1], my = pr.mom[2], mxx = pr.mom[3], mxy = pr.mom[4], myy = pr.mom[5];
-            double la[3], lb[3], lc[3];
-            if (n >= 3) {
-                basis(R[0], R[1], la);
-                basis(R[2], R[3], lb);
+        F64Poly Y;
+        f64_polygon<KIND != MIX_CONST>(P, x, Eb, Q, e, f64_div(1.0, det), Y);
+        const double adet = fabs(det);
+        if (Y.n >= 3) nsub += Y.n - 2;
+        if (KIND == MIX_CONST && exact2) {
+            if (Y.n >= 3) {
+                double A = 0, Mx = 0, My = 0, Mxx = 0, Mxy = 0, Myy = 0;
+                double x0 = Y.L[2 * Y.n - 2], y0 = Y.L[2 * Y.n - 1];
+#pragma unroll 1
+                for (int j = 0; j < Y.n; j++) {
+                    const double x1 = Y.L[2 * j], y1 = Y.L[2 * j + 1];
+                    const double c = x0 * y1 - x1 * y0, sx = x0 + x1, sy = y0 + y1;
+                    A += c;
+                    Mx = fma(c, sx, Mx);
+                    My = fma(c, sy, My);
+                    Mxx = fma(c, fma(sx, sx, -(x0 * x1)), Mxx);
+                    Myy = fma(c, fma(sy, sy, -(y0 * y1)), Myy);
+                    Mxy = fma(c, fma(sx, sy, fma(x0, y0, x1 * y1)), Mxy);
+                    x0 = x1;
+                    y0 = y1;
+                }
+                const double f = P.kc * adet;
+                A *= 0.5 * f;
+                Mx *= (1.0 / 6.0) * f;
+                My *= (1.0 / 6.0) * f;
+                Mxx *= (1.0 / 12.0) * f;
+                Myy *= (1.0 / 12.0) * f;
+                Mxy *= (1.0 / 24.0) * f;
+                S0 = A;
+                S1[0] = A - Mx - My; S1[1] = Mx; S1[2] = My;
+                S2[0] = Mx - Mxx - Mxy; S2[1] = My - Mxy - Myy; S2[2] = Mxy;
             }
-            for (int r = 0; r + 2 < n; r++) {
-                nsub++;
-                const double Bx = R[2 * r + 2] - R[0], By = R[2 * r + 3] - R[1], Cx = R[2 * r + 4] - R[0], Cy = R[2 * r + 5] - R[1];
-                const double rT = fabs(Bx * Cy - By * Cx);
-                basis(R[2 * r + 4], R[2 * r + 5], lc);
-                double t0[3], t1[3], t2[3], be[3], ga[3];
+        } else if (KIND == MIX_CONST) {   // the rule's moments on each fan triangle (see item_cut_const)
+            const double m0 = pr.mom[0], mx = pr.mom[1], my = pr.mom[2], mxx = pr.mom[3], mxy = pr.mom[4], myy = pr.mom[5];
+            const double la[3] = {1.0 - Y.L[0] - Y.L[1], Y.L[0], Y.L[1]};
+            for (int r = 0; r + 2 < Y.n; r++) {
+                const double *b = &Y.L[2 * r + 2], *c = &Y.L[2 * r + 4];
+                double be[3], ga[3];
+                be[1] = b[0] - la[1]; be[2] = b[1] - la[2]; be[0] = -be[1] - be[2];
+                ga[1] = c[0] - la[1]; ga[2] = c[1] - la[2]; ga[0] = -ga[1] - ga[2];
+                const double rT = adet * P.kc * fabs(be[1] * ga[2] - be[2] * ga[1]);
+                double t0[3], t1[3], t2[3];
 #pragma unroll
                 for (int q = 0; q < 3; q++) {
-                    be[q] = lb[q] - la[q];
-                    ga[q] = lc[q] - la[q];
                     t0[q] = la[q] * m0 + (be[q] * mx + ga[q] * my);
                     t1[q] = la[q] * mx + (be[q] * mxx + ga[q] * mxy);
                     t2[q] = la[q] * my + (be[q] * mxy + ga[q] * myy);
                     S1[q] += rT * t0[q];
-                    lb[q] = lc[q];
                 }
                 S0 += rT * m0;
                 S2[0] += rT * (la[0] * t0[1] + (be[0] * t1[1] + ga[0] * t2[1]));
                 S2[1] += rT * (la[0] * t0[2] + (be[0] * t1[2] + ga[0] * t2[2]));
                 S2[2] += rT * (la[1] * t0[2] + (be[1] * t1[2] + ga[1] * t2[2]));
             }
-            S0 *= P.kc;
-#pragma unroll
-            for (int q = 0; q < 3; q++) { S1[q] *= P.kc; S2[q] *= P.kc; }
         } else {
-            for (int r = 0; r + 2 < n; r++) {
-                nsub++;
-                const double Bx = R[2 * r + 2] - R[0], By = R[2 * r + 3] - R[1], Cx = R[2 * r + 4] - R[0], Cy = R[2 * r + 5] - R[1];
+            for (int r = 0; r + 2 < Y.n; r++) {
+                const double Bx = Y.R[2 * r + 2] - Y.R[0], By = Y.R[2 * r + 3] - Y.R[1];
+                const double Cx = Y.R[2 * r + 4] - Y.R[0], Cy = Y.R[2 * r + 5] - Y.R[1];
+                const double b1 = Y.L[2 * r + 2] - Y.L[0], b2 = Y.L[2 * r + 3] - Y.L[1];
+                const double c1 = Y.L[2 * r + 4] - Y.L[0], c2 = Y.L[2 * r + 5] - Y.L[1];
                 const double rT = fabs(Bx * Cy - By * Cx);
                 for (int i = 0; i < rule.nPy; i++) {
-                    const double yx = R[0] + Bx * rule.Py[2 * i] + Cx * rule.Py[2 * i + 1];
-                    const double yy = R[1] + By * rule.Py[2 * i] + Cy * rule.Py[2 * i + 1];
-                    const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * rT * rule.dy[i];
-                    double l[3];
-                    basis(yx, yy, l);
+                    const double px = rule.Py[2 * i], py = rule.Py[2 * i + 1];
+                    const double yx = Y.R[0] + Bx * px + Cx * py, yy = Y.R[1] + By * px + Cy * py;
+                    const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * (rT * rule.dy[i]);
+                    const double l1 = Y.L[0] + b1 * px + c1 * py, l2 = Y.L[1] + b2 * px + c2 * py, l0 = 1.0 - l1 - l2;
+                    const double k1 = kw * l1, k2 = kw * l2;
                     S0 += kw;
-#pragma unroll
-                    for (int c = 0; c < 3; c++) S1[c] += kw * l[c];
-                    S2[0] += kw * (l[0] * l[1]);
-                    S2[1] += kw * (l[0] * l[2]);
-                    S2[2] += kw * (l[1] * l[2]);
+                    S1[0] += kw * l0;
+                    S1[1] += k1;
+                    S1[2] += k2;
+                    S2[0] += k1 * l0;
+                    S2[1] += k2 * l0;
+                    S2[2] += k1 * l2;
                 }
             }
         }
@@ -400,7 +528,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                 __syncwarp();
                 for (int i = lane; i < end - base; i += 32) {
                     const int it = W.list[i], k = it & 31;
-                    f64_item<KIND>(P, rule, pr, (it >> 5) & 1, &x64[2 * k], &a.EC[(long long)W.pid[it >> 6] * 6], &res[i * F64_RN], nsub);
+                    f64_item<KIND>(P, rule, pr, (it >> 5) & 1, fa.exact2, &x64[2 * k], &a.EC[(long long)W.pid[it >> 6] * 6], &res[i * F64_RN], nsub);
                 }
                 __syncwarp();
                 const int nun = __popc(who) * F64_OUT;

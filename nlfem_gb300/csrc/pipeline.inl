@@ -398,7 +398,7 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     // size relative to the ball: the vertex tests stay inside their margin while every element
     // diameter is at most MIX_MAX_H_OVER_DELTA times delta. The mixed path refuses larger elements,
     // the FP64 paths take their FP64 routines for them.
-    double hmax2 = 0;
+    double hmax2 = 0, hmin2 = 1e300;
     if (system) {
         const int dV = p.dim + 1;
         for (long e = 0; e < p.nE; e++)
@@ -412,6 +412,7 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
                         d2 += d * d;
                     }
                     hmax2 = std::max(hmax2, d2);
+                    hmin2 = std::min(hmin2, d2);
                 }
         const double lim = p.precision == NLFEM_PREC_MIXED ? MIX_MAX_H_OVER_DELTA : 512.0;
         if (p.precision != NLFEM_PREC_FP64 && hmax2 > lim * lim * p.sqdelta)
@@ -420,9 +421,13 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
                         " times the horizon (the margins of its geometry tests); precision \"fp64\" has no such bound");
     }
     if (system) {
-        bool finite = std::isfinite(p.sqdelta);
-        for (long v = 0; v < p.nV * p.dim; v++) finite = finite && std::isfinite(p.vertices[v]);
-        P.cert = finite && hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta;
+        // The margins also assume that the squares and products of the tests stay normal FP32
+        // numbers, and that a double-float pair holds a coordinate to far below 2^-24 delta (its own
+        // rounding is 2^-48 of the coordinate). The FP64 paths check both.
+        double cmax = 0;
+        for (long v = 0; v < p.nV * p.dim; v++) cmax = fabs(p.vertices[v]) <= cmax ? cmax : fabs(p.vertices[v]);   // a NaN stays
+        P.cert = hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
+                 p.sqdelta < 1e14 && std::min(hmin2, p.sqdelta) > 1e-24 && hmin2 * p.sqdelta > 1e-28;
     }
     double mag, kbound = 0;   // kbound: bound of |kernel| inside the ball (estimate for singular kernels)
     if (system) {
@@ -1752,6 +1757,11 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     F64Args fa;
     fa.m.p = pa;
     fa.mtab = S.mtab.get<double>();
+    fa.exact2 = 1;   // the rule's moments are the triangle's to rounding (2^-53; the 7-point rule's are)
+    {
+        const double m[6] = {1.0 / 2, 1.0 / 6, 1.0 / 6, 1.0 / 12, 1.0 / 24, 1.0 / 12};
+        for (int q = 0; q < 6; q++) fa.exact2 = fa.exact2 && fabs(pr.mom[q] - m[q]) <= 1.2e-16 * m[q];
+    }
     fa.m.m = slot_map(S);
     fa.m.work = reinterpret_cast<int *>(S.counters.get<unsigned long long>() + 10);
     fa.m.valsN = S.valsN.get<long long>();

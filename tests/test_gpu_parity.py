@@ -1221,3 +1221,21 @@ def test_fp64_barycenter_pass(nl, orc, dim, n, delta, nq):
             assert same_pattern(A, C) and np.array_equal(A.tocsr().data, C.data)
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("scale,shift", [(1e-5, 0.0), (1e5, 5.0), (1e-11, 0.0), (1.0, 1e5)])
+def test_fp64_pass_scales(nl, orc, scale, shift):
+    """The FP64 path on meshes of other units and far from the origin: inside the range of the FP32
+    class tests and of the Newton seeds (1e-5, 1e5), and outside of it (horizons of 1e-12, coordinates
+    of 1e6 horizons), where the FP64 predicates run. The reference takes its polygon points in absolute
+    coordinates, so the bar grows with the coordinates' rounding over the element size (h = 0.1)."""
+    m = square_mesh(12, 0.1, jitter=0.2, seed=81)
+    from nlfem_gb300 import meshes
+    m = meshes.mesh_dict((m["vertices"] + shift) * scale, m["elements"], m["elementLabels"])
+    k = {"function": "constant", "horizon": 0.1 * scale, "outputdim": 1}
+    A = nl.stiffnessMatrix(dict(m), k, conf2d())
+    B = orc.assemble(m, k, conf2d())["A"]
+    assert same_pattern(A, B)
+    fro, mx = rel_errors(A, B)
+    tol = FP64_TOL + 64 * 1.1e-16 * shift / 0.1
+    assert fro < tol and mx < tol, (fro, mx)
