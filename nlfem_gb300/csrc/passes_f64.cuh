@@ -18,7 +18,7 @@
 // Measured (quadrature phase, against the two-sided colored pass that the path used before): constant
 // kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 24.5 ms against 1725 ms; 2 * 32^2
 // triangles: 0.54 against 66.6 ms; parabola, 2 * 57^2: 12.2 against 257 ms; fractional, 2 * 40^2:
-// 49.5 against 568 ms.
+// 15.4 against about 540 ms.
 //
 // Sums. Every contribution is rounded once to a 64-bit integer and added with an integer atomic,
 // so the result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
@@ -53,6 +53,7 @@ struct F64Args {
     long long *valslo;          // second integers of vals
     long long *valsNlo;         // second integers of valsN (singular kernels)
     const double *mtab;         // constant kernels: the mask table (k_mask_table)
+    const double *pw;           // singular kernels: power tables (primitives.cuh)
     int exact2;                 // the inner rule integrates degree two exactly (see f64_item)
 };
 
@@ -158,13 +159,6 @@ __global__ void k_mask_table(Rule rule, int dV, int TS, int n, double *__restric
     tab[i] = f64_mask_sum(rule, dV, m, r, c);
 }
 
-template <int KIND>
-__device__ __forceinline__ double f64_kernel(const ProbParams &P, double r2) {
-    if (KIND == MIX_CONST) return P.kc;
-    if (KIND == MIX_REGULAR && P.kernel == KER_PARABOLA) return P.kc * (P.sqdelta - r2);
-    return P.kc * exp2(-0.5 * P.expo * log2(r2));
-}
-
 // Square root, reciprocal and reciprocal square root by Newton's iteration from an FP32 seed (24 bits,
 // so two steps reach FP64; the last step of the square root and of the quotient is the residual
 // correction). A CUDA division or square root keeps the FP64 pipe busy about twice as long: they
@@ -192,6 +186,15 @@ __device__ __forceinline__ double f64_div(double a, double b) {
     y = fma(y, fma(-b, y, 1.0), y);
     const double q = a * y;
     return fma(y, fma(-b, q, a), q);
+}
+
+// Kernel value from r2 = |x - y|^2; pw the problem's power table (singular kernels).
+template <int KIND>
+__device__ __forceinline__ double f64_kernel(const ProbParams &P, const double *pw, double r2) {
+    if (KIND == MIX_CONST) return P.kc;
+    if (KIND == MIX_SINGULAR) return pw_eval(pw, r2);
+    if (P.kernel == KER_PARABOLA) return P.kc * (P.sqdelta - r2);
+    return P.kc * exp2(-0.5 * P.expo * log2(r2));
 }
 
 // Polygon of a cut item: points relative to the ball's center in R, and in the partner's reference
@@ -280,7 +283,7 @@ __device__ __forceinline__ void f64_polygon(const ProbParams &P, const double *x
 // moments, taken from its boundary in reference coordinates (Green's theorem, one term per edge).
 template <int KIND>
 __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, const PassRuleT<double> &pr, bool inside,
-                                         bool exact2, const double *x, const double *Eb, double *res, unsigned &nsub) {
+                                         bool exact2, const double *pw, const double *x, const double *Eb, double *res, unsigned &nsub) {
     const double Q[6] = {Eb[0] - x[0], Eb[1] - x[1], Eb[2] - x[0], Eb[3] - x[1], Eb[4] - x[0], Eb[5] - x[1]};
     const double e[4] = {Eb[2] - Eb[0], Eb[3] - Eb[1], Eb[4] - Eb[0], Eb[5] - Eb[1]};
     const double det = e[0] * e[3] - e[1] * e[2];
@@ -291,7 +294,7 @@ __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, 
         for (int i = 0; i < rule.nPy; i++) {
             const double yx = Q[0] + e[0] * rule.Py[2 * i] + e[2] * rule.Py[2 * i + 1];
             const double yy = Q[1] + e[1] * rule.Py[2 * i] + e[3] * rule.Py[2 * i + 1];
-            const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * rT;
+            const double kw = f64_kernel<KIND>(P, pw, yx * yx + yy * yy) * rT;
             S0 += kw * rule.dy[i];
 #pragma unroll
             for (int c = 0; c < 3; c++) S1[c] += kw * pr.cy[3 * i + c];
@@ -364,7 +367,7 @@ __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, 
                 for (int i = 0; i < rule.nPy; i++) {
                     const double px = rule.Py[2 * i], py = rule.Py[2 * i + 1];
                     const double yx = Y.R[0] + Bx * px + Cx * py, yy = Y.R[1] + By * px + Cy * py;
-                    const double kw = f64_kernel<KIND>(P, yx * yx + yy * yy) * (rT * rule.dy[i]);
+                    const double kw = f64_kernel<KIND>(P, pw, yx * yx + yy * yy) * (rT * rule.dy[i]);
                     const double l1 = Y.L[0] + b1 * px + c1 * py, l2 = Y.L[1] + b2 * px + c2 * py, l0 = 1.0 - l1 - l2;
                     const double k1 = kw * l1, k2 = kw * l2;
                     S0 += kw;
@@ -447,6 +450,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
             W.te[lane] = fa.vexp[u];
         }
         const ProbParams P = a.probs[a.eprob[T]];
+        const double *pw = KIND == MIX_SINGULAR ? fa.pw + (long long)a.eprob[T] * PW_N : nullptr;
         const double *ET64 = &a.EC[(long long)T * 6];
         const float ohi0 = a.EChi[(long long)T * 6], ohi1 = a.EChi[(long long)T * 6 + 1];
         const float olo0 = a.EClo[(long long)T * 6], olo1 = a.EClo[(long long)T * 6 + 1];
@@ -528,7 +532,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                 __syncwarp();
                 for (int i = lane; i < end - base; i += 32) {
                     const int it = W.list[i], k = it & 31;
-                    f64_item<KIND>(P, rule, pr, (it >> 5) & 1, fa.exact2, &x64[2 * k], &a.EC[(long long)W.pid[it >> 6] * 6], &res[i * F64_RN], nsub);
+                    f64_item<KIND>(P, rule, pr, (it >> 5) & 1, fa.exact2, pw, &x64[2 * k], &a.EC[(long long)W.pid[it >> 6] * 6], &res[i * F64_RN], nsub);
                 }
                 __syncwarp();
                 const int nun = __popc(who) * F64_OUT;

@@ -511,6 +511,7 @@ struct Session {
     bool onesided64 = false;   // precision "fp64-onesided": every structural slot is kept
     bool f64 = false;          // PM_RETRI or PM_BARY in FP64 (passes_f64.cuh, passes_f64_bary.cuh)
     bool cert = false;         // the pair search takes the certified FP32 geometry
+    DevBuf pw;                 // power tables of the singular kernels (FP64), PW_N numbers per problem
     DevBuf vexp, valsNlo, valslo, mtab;   // FP64 one-sided passes: vertex exponents, second integers, mask table
     DevBuf vcnt, vptr, vel, adjcnt, xadj, adj;
     DevBuf stamp_epoch;   // per-warp stamp epochs of the search
@@ -572,7 +573,7 @@ struct Session {
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
                 &hcap, &hptr, &htab, &tpos, &dslot, &rwords, &rbase, &rlo, &rankmap, &eid_ptr, &eid, &vp_cnt, &vp_off, &vp_ptr, &vp_scratch, &pscratch, &rowoff, &kclist, &valsN, &elp,
                 &po_cnt, &po_off, &po_ptr, &po_scratch, &tcnt, &tptr, &tcols, &sv_vec, &sv_part, &zptr, &zidx, &vacc, &vtiny,
-                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo, &mtab};
+                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo, &mtab, &pw};
     }
     ~Session() {
         for (DevBuf *b : buffers()) b->release();
@@ -1477,6 +1478,36 @@ static Duffy duffy_view(const Session &S) {
     return d;
 }
 
+// Power tables (pw_eval): table p for problem p's kernel kc |z|^-expo.
+__global__ void k_pw_table(const ProbParams *__restrict__ probs, int nProb, double *__restrict__ tab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, p = i / PW_N, q = i - p * PW_N;
+    if (p >= nProb || !probs[p].singular) return;
+    const double h = -0.5 * probs[p].expo;
+    double v = 0;
+    if (q < 6) {   // binomial coefficients of (1 + t)^h
+        v = 1.0;
+        for (int n = 0; n <= q; n++) v *= (h - n) / (n + 1.0);
+    } else if (q >= PW_E && q < PW_M) {   // kc 2^(E h); zero and subnormal arguments give infinity
+        const int e = q - PW_E;
+        const double E = e - 1023.0, hi = E * h, lo = fma(E, h, -hi), I = rint(hi);
+        v = e == 0 ? __longlong_as_double(0x7ff0000000000000LL)
+                   : (e == 2047 ? __longlong_as_double(0x7ff8000000000000LL)
+                                : probs[p].kc * ldexp(exp2(hi - I) * fma(lo, 0.6931471805599453, 1.0), (int)I));
+    } else if (q >= PW_M) {
+        const int j = (q - PW_M) >> 1;
+        const double inv = rint(4096.0 / (1.0 + (j + 0.5) / 256.0)) / 4096.0;
+        v = (q & 1) ? pow(inv, -h) : inv;
+    }
+    tab[i] = v;
+}
+static int run_pw_tables(Session &S) {
+    const long long n = (long long)S.nProb * PW_N;
+    ENS(S.pw, sizeof(double) * n);
+    k_pw_table<<<grid_for(n, 64), 64, 0, S.st>>>(S.prm.get<ProbParams>(), S.nProb, S.pw.get<double>()); ++S.nlaunch;
+    CK(cudaGetLastError());
+    return NLFEM_OK;
+}
+
 __global__ void k_iota(int *l, long long n) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) l[i] = (int)i;
@@ -1518,6 +1549,8 @@ static int run_pair_blocks(Session &S, long long n, const long *pairs, int close
         k_iota<<<grid_for(n, 256), 256, 0, S.st>>>(S.closelist.get<int>(), n); ++S.nlaunch;
         a.list = S.closelist.get<int>();
         a.nlist = n;
+        if ((r = run_pw_tables(S))) return r;
+        a.pw = S.pw.get<double>();
         k_quad_close<false><<<grid_for(n * 32, 128), 128, 0, S.st>>>(a, duffy_view(S)); ++S.nlaunch;
     } else {
         k_quad_fp64<DIM><<<grid_for(n, 128), 128, 0, S.st>>>(a, S.rule); ++S.nlaunch;
@@ -1603,7 +1636,11 @@ static int run_close(Session &S) {
     k_iota<<<grid_for(nslot, 256), 256, 0, S.st>>>(S.closelist.get<int>(), nslot); ++S.nlaunch;
     a.list = S.closelist.get<int>();
     a.nlist = nslot;
-    // the mixed path takes the kernel power in FP32 after an exact binary range reduction
+    if (S.prec != PREC_MIX) {
+        const int r = run_pw_tables(S);
+        if (r) return r;
+        a.pw = S.pw.get<double>();
+    }
     if (S.prec == PREC_MIX) k_quad_close<true><<<grid_for(nslot * 32, 128), 128, 0, S.st>>>(a, duffy_view(S));
     else k_quad_close<false><<<grid_for(nslot * 32, 128), 128, 0, S.st>>>(a, duffy_view(S));
     ++S.nlaunch;
@@ -1757,6 +1794,7 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     F64Args fa;
     fa.m.p = pa;
     fa.mtab = S.mtab.get<double>();
+    fa.pw = S.pw.get<double>();   // singular kernels: made with the close pairs (run_close)
     fa.exact2 = 1;   // the rule's moments are the triangle's to rounding (2^-53; the 7-point rule's are)
     {
         const double m[6] = {1.0 / 2, 1.0 / 6, 1.0 / 6, 1.0 / 12, 1.0 / 24, 1.0 / 12};

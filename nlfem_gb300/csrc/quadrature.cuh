@@ -54,6 +54,7 @@ struct QuadArgs {
     int *ret_out;             // explicit-pair mode: doesInteract
     int force_close;          // explicit-pair mode: use the close-pair rule
     unsigned long long *n_subtri;
+    const double *pw;         // power tables of the singular kernels, PW_N numbers per problem
 };
 
 __device__ __forceinline__ long long find_slot(const long long *__restrict__ rowptr,
@@ -500,27 +501,12 @@ __global__ void k_close_list(QuadArgs a, int *list, unsigned long long *count) {
 
 // One warp per close pair: integrate_fractional (integration.cpp:187-288) with join()
 // (:1913-1958), FP64 throughout; lanes stride over the Duffy points, warp-reduce the blocks.
-// r2^h (h < 0) for the mixed path: r2 = m 2^E exactly (frexp, m in [1/2, 1)), and h E = I + f
-// with I = floor(h E) an integer, so r2^h = 2^I 2^(f + h log2 m) where only the last power, of an
-// argument in [0, 1 - h), is evaluated in FP32 (exp2f, log2f). Its relative error is a few units
-// of 2^-24 times (1 + |h|), about 3e-7, far inside the mixed path's 1e-6; the binary exponent
-// is exact. Range reduction by the exact power of two, as in any pow implementation.
-__device__ __forceinline__ double pow_split(double r2, double h) {
-    int E;
-    const double m = frexp(r2, &E);
-    const double t = h * (double)E;
-    const double I = floor(t);
-    const float g = fmaf((float)h, log2f((float)m), (float)(t - I));
-    return ldexp((double)exp2f(g), (int)I);
-}
-
 // Sum over the Duffy points of one close pair (integration.cpp:187-288) of w pxy pxy^T, upper
 // triangle of the nL x nL matrix, nL = 6 - NEQ: the lanes take the (map, Gauss point) items in
-// turn. The kernel value |x - y|^-(d+2s) is taken as exp2(-(d+2s)/2 log2 |x - y|^2), the same
-// function as the reference's 1/pow(sqrt(r), d+2s) without the power's extra work; FAST (mixed
-// path) evaluates it with pow_split and sums in compensated FP32.
-template <int NEQ, bool FAST>
-__device__ __forceinline__ void close_accumulate(const ProbParams &P, const Duffy &d, int c, int nT,
+// turn. The kernel value c |x - y|^-(d+2s) comes from the power table (pw_eval). FP64-bound: with exp2
+// and log2 the power was more than half of the instructions.
+template <int NEQ>
+__device__ __forceinline__ void close_accumulate(const Duffy &d, const double *pw, int c, int nT,
                                                  const double *EA, const double *EB, double dAB, double *M) {
     constexpr int NL = 6 - NEQ, SH = 3 - NEQ;
     const int lane = threadIdx.x & 31;
@@ -529,10 +515,6 @@ __device__ __forceinline__ void close_accumulate(const ProbParams &P, const Duff
     const double *td_base = d.tdet[c];
     const double a0 = EA[2] - EA[0], a1 = EA[4] - EA[0], a2 = EA[3] - EA[1], a3 = EA[5] - EA[1];
     const double b0 = EB[2] - EB[0], b1 = EB[4] - EB[0], b2 = EB[3] - EB[1], b3 = EB[5] - EB[1];
-    const double hexp = -0.5 * P.expo;
-    float Mf[FAST ? 21 : 1], Mc[FAST ? 21 : 1];   // FAST: FP32 sums and their compensation
-#pragma unroll
-    for (int q = 0; q < (FAST ? 21 : 1); q++) Mf[q] = Mc[q] = 0.f;
     for (int idx = lane; idx < total; idx += 32) {
         const int k = idx % d.nPg;
         const double *al = &al_base[(long long)idx * 4];
@@ -541,7 +523,7 @@ __device__ __forceinline__ void close_accumulate(const ProbParams &P, const Duff
         const double y0 = al[2] * b0 + al[3] * b1 + EB[0], y1 = al[2] * b2 + al[3] * b3 + EB[1];
         const double z0 = x0 - y0, z1 = x1 - y1;
         const double r2 = z0 * z0 + z1 * z1;
-        const double ker = P.kc * (FAST ? pow_split(r2, hexp) : exp2(hexp * log2(r2)));
+        const double ker = pw_eval(pw, r2);
         const double px[3] = {1.0 - al[0] - al[1], al[0], al[1]};
         const double py[3] = {1.0 - al[2] - al[3], al[2], al[3]};
         double v[NL];
@@ -555,38 +537,12 @@ __device__ __forceinline__ void close_accumulate(const ProbParams &P, const Duff
             }
         }
         const double base = ker * tf * d.dg[k] * dAB;
-        if (FAST) {
-            // mixed path: the summands, each a product of FP64 values rounded once to FP32, are
-            // added with Kahan compensation (error about 2^-23 of the sum, independent of the
-            // point count); the lanes' sums are combined in FP64 by the caller
-            float vf[NL];
 #pragma unroll
-            for (int aa = 0; aa < NL; aa++) vf[aa] = (float)v[aa];
-            const float bf = (float)base;
+        for (int aa = 0; aa < NL; aa++) {
+            const double fa = base * v[aa];
 #pragma unroll
-            for (int aa = 0; aa < NL; aa++) {
-                const float fa = bf * vf[aa];
-#pragma unroll
-                for (int b = aa; b < NL; b++) {
-                    const int q = sym_idx<6>(aa, b);
-                    const float y = fmaf(fa, vf[b], -Mc[q]);
-                    const float t = Mf[q] + y;
-                    Mc[q] = (t - Mf[q]) - y;
-                    Mf[q] = t;
-                }
-            }
-        } else {
-#pragma unroll
-            for (int aa = 0; aa < NL; aa++) {
-                const double fa = base * v[aa];
-#pragma unroll
-                for (int b = aa; b < NL; b++) M[sym_idx<6>(aa, b)] += fa * v[b];
-            }
+            for (int b = aa; b < NL; b++) M[sym_idx<6>(aa, b)] += fa * v[b];
         }
-    }
-    if (FAST) {
-#pragma unroll
-        for (int q = 0; q < 21; q++) M[q] = (double)Mf[q] - (double)Mc[q];
     }
 }
 
@@ -672,13 +628,12 @@ __device__ __forceinline__ void close_accumulate_f32(const ProbParams &P, const 
 // in turn: the kernel at the canceled points (as in the fractional rule), the basis functions at
 // the points with xi kept, the weight xi^(1 - 2s). W holds termLocal and termLocalPrime (upper
 // triangles) and termNonloc (3 x 3), all in the order of the join's sorted vertices.
-__device__ __forceinline__ void weak_accumulate(const ProbParams &P, const Duffy &d, int c, int nT,
+__device__ __forceinline__ void weak_accumulate(const Duffy &d, const double *pw, int c, int nT,
                                                 const double *EA, const double *EB, double dAB, double *W) {
     const int lane = threadIdx.x & 31;
     const int total = nT * d.nPg;
     const double a0 = EA[2] - EA[0], a1 = EA[4] - EA[0], a2 = EA[3] - EA[1], a3 = EA[5] - EA[1];
     const double b0 = EB[2] - EB[0], b1 = EB[4] - EB[0], b2 = EB[3] - EB[1], b3 = EB[5] - EB[1];
-    const double hexp = -0.5 * P.expo;
     for (int idx = lane; idx < total; idx += 32) {
         const int k = idx % d.nPg;
         const double *ac = &d.alpha[c][(long long)idx * 4];
@@ -686,7 +641,7 @@ __device__ __forceinline__ void weak_accumulate(const ProbParams &P, const Duffy
         const double x0 = ac[0] * a0 + ac[1] * a1 + EA[0], x1 = ac[0] * a2 + ac[1] * a3 + EA[1];
         const double y0 = ac[2] * b0 + ac[3] * b1 + EB[0], y1 = ac[2] * b2 + ac[3] * b3 + EB[1];
         const double z0 = x0 - y0, z1 = x1 - y1;
-        const double ker = P.kc * exp2(hexp * log2(z0 * z0 + z1 * z1));
+        const double ker = pw_eval(pw, z0 * z0 + z1 * z1);
         const double f = ker * d.tdetW[c][idx] * d.dg[k] * dAB;
         const double px[3] = {1.0 - au[0] - au[1], au[0], au[1]};
         const double py[3] = {1.0 - au[2] - au[3], au[2], au[3]};
@@ -772,7 +727,9 @@ __global__ void __launch_bounds__(128) k_quad_close(QuadArgs a, Duffy d) {
     if (w >= a.nlist) return;
     const long long p = a.list[w];
     const int aT = a.pA[p], bT = a.pB[p];
-    const ProbParams P = a.probs[a.eprob[aT]];
+    const int prob = a.eprob[aT];
+    const ProbParams P = a.probs[prob];
+    const double *pw = FAST ? nullptr : a.pw + (long long)prob * PW_N;
     const int *aV = &a.T32[(long long)aT * 3];
     const int *bV = &a.T32[(long long)bT * 3];
     // join
@@ -809,7 +766,7 @@ __global__ void __launch_bounds__(128) k_quad_close(QuadArgs a, Duffy d) {
 #pragma unroll
         for (int i = 0; i < 21; i++) W[i] = 0.0;
         if (FAST) weak_accumulate_f32(P, d, c, nT, EA, EB, dA * dB, W);
-        else weak_accumulate(P, d, c, nT, EA, EB, dA * dB, W);
+        else weak_accumulate(d, pw, c, nT, EA, EB, dA * dB, W);
 #pragma unroll
         for (int i = 0; i < 21; i++) W[i] = warp_sum(W[i]);
         // termLocal[argA a][argA b], termLocalPrime[argB a][argB b], termNonloc and
@@ -850,9 +807,9 @@ __global__ void __launch_bounds__(128) k_quad_close(QuadArgs a, Duffy d) {
         else if (nEqual == 2) close_accumulate_f32<2>(P, d, c, nT, EA, EB, dA * dB, M);
         else close_accumulate_f32<3>(P, d, c, nT, EA, EB, dA * dB, M);
     } else {
-        if (nEqual == 1) close_accumulate<1, false>(P, d, c, nT, EA, EB, dA * dB, M);
-        else if (nEqual == 2) close_accumulate<2, false>(P, d, c, nT, EA, EB, dA * dB, M);
-        else close_accumulate<3, false>(P, d, c, nT, EA, EB, dA * dB, M);
+        if (nEqual == 1) close_accumulate<1>(d, pw, c, nT, EA, EB, dA * dB, M);
+        else if (nEqual == 2) close_accumulate<2>(d, pw, c, nT, EA, EB, dA * dB, M);
+        else close_accumulate<3>(d, pw, c, nT, EA, EB, dA * dB, M);
     }
 #pragma unroll
     for (int i = 0; i < 21; i++) M[i] = warp_sum(M[i]);
