@@ -52,7 +52,7 @@ __global__ void k_prep_elements(const long long *__restrict__ T64, const long lo
                                 int *__restrict__ T32, int *__restrict__ labT, int *__restrict__ eprob,
                                 double *__restrict__ EC, double *__restrict__ adet,
                                 float *__restrict__ EChi, float *__restrict__ EClo,
-                                float *__restrict__ adetf, float *__restrict__ BCf) {
+                                float *__restrict__ adetf, float *__restrict__ BCf, double *__restrict__ idet) {
     constexpr int dV = DIM + 1;
     long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nE) return;
@@ -104,6 +104,7 @@ __global__ void k_prep_elements(const long long *__restrict__ T64, const long lo
     }
     adet[e] = fabs(det);
     adetf[e] = (float)fabs(det);
+    if (idet) idet[e] = 1.0 / det;
 }
 
 __global__ void k_prep_vertices(const long long *__restrict__ lab64, const int *__restrict__ voff,

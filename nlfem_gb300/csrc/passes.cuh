@@ -266,6 +266,7 @@ struct PassRuleT {
     // py^2) over the reference triangle.
     R insum[1 + 4 + 10];
     R mom[6];
+    R mom4[9];   // the moments of degree three and four: px^3, px^2 py, px py^2, py^3, px^4, ..., py^4
     // sums over the outer points of cxx (upper triangle), cx and dxf, in that order: an outer
     // element's folds when every outer point's ball contains the partner (constant kernels)
     R xsum[10 + 4 + 1];

@@ -16,9 +16,9 @@
 //     are neighbours: full warps integrate the items, then full warps fold them, one (pair, output)
 //     per lane, instead of every lane walking all outer points.
 // Measured (quadrature phase, against the two-sided colored pass that the path used before): constant
-// kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 24.5 ms against 1725 ms; 2 * 32^2
-// triangles: 0.54 against 66.6 ms; parabola, 2 * 57^2: 12.2 against 257 ms; fractional, 2 * 40^2:
-// 15.4 against about 540 ms.
+// kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 21.4 ms against 1725 ms; 2 * 32^2
+// triangles: 0.52 against 66.6 ms; parabola, 2 * 57^2: 5.4 against 257 ms; fractional, 2 * 40^2:
+// 9.6 against about 540 ms. The FP64 pipe is 70 to 89% busy in these.
 //
 // Sums. Every contribution is rounded once to a 64-bit integer and added with an integer atomic,
 // so the result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
@@ -40,7 +40,7 @@ namespace nlg {
 
 constexpr int F64_WARPS = 4;
 constexpr int F64_THREADS = 32 * F64_WARPS;
-constexpr int F64_CAP = 64;    // items integrated before their pairs are folded (>= MAXQ)
+constexpr int F64_CAP = 128;   // items integrated before their pairs are folded (>= MAXQ)
 constexpr int F64_RN = 7;      // per item: innerLocal, innerNonloc[3], off-diagonal termLocalPrime sums[3]
 constexpr int F64_OUT = 15;    // per pair: termNonloc[9], off-diagonal termLocal[3] and termLocalPrime[3]
 constexpr int F64_BITS = 62;   // a bound of 2^x has the unit 2^(x - 62)
@@ -52,9 +52,10 @@ struct F64Args {
     const int *vexp;            // per vertex, 8 log2 of its elements' |det| sum, rounded up
     long long *valslo;          // second integers of vals
     long long *valsNlo;         // second integers of valsN (singular kernels)
+    const double *idet;         // per element, 1 / det (signed)
     const double *mtab;         // constant kernels: the mask table (k_mask_table)
     const double *pw;           // singular kernels: power tables (primitives.cuh)
-    int exact2;                 // the inner rule integrates degree two exactly (see f64_item)
+    int exact;                  // the inner rule integrates degree two (bit 0), four (bit 1) exactly (see f64_item)
 };
 
 struct F64Warp {
@@ -65,7 +66,9 @@ struct F64Warp {
     int pid[32];                // partner element
     int pe[32];                 // its eexp
     int pve[32][3];             // vexp of its vertices
-    unsigned short list[F64_CAP];           // items: lane << 6 | inside << 5 | outer point
+    F2 pc[32][3];               // its vertices relative to T's vertex 0, FP32
+    unsigned short list[F64_CAP];           // items, pair by pair: lane << 6 | inside << 5 | outer point
+    unsigned char order[F64_CAP];           // the inside items, then the cut items (kernels that list both)
     unsigned char pl[32], ps[32], pn[32];   // chunk's pairs: owner lane, first item, item count
 };
 template <int NW>
@@ -83,12 +86,12 @@ __host__ __device__ constexpr size_t f64_work_bytes(int kind) {
                : 96 * (8 + 24 * (size_t)f64_words(kind));
 }
 __host__ __device__ constexpr size_t f64_warp_bytes(int kind, int nPx) {
-    return (sizeof(F64Warp) + 15) / 16 * 16 + (size_t)nPx * 24 + f64_work_bytes(kind) + 16;
+    return (sizeof(F64Warp) + 15) / 16 * 16 + (size_t)nPx * (24 + 56) + f64_work_bytes(kind) + 16;
 }
 // mask sums of the outer rule: one table of up to 256 entries per 8 outer points
 __host__ __device__ constexpr int f64_tab_entries(int nPx) { return nPx <= 8 ? 1 << nPx : 256 * ((nPx + 7) / 8); }
 __host__ __device__ constexpr size_t f64_smem_bytes(int kind, int nPx) {
-    return (size_t)nPx * 7 * 8 + (kind == MIX_CONST ? (size_t)f64_tab_entries(nPx) * 7 * 8 : 0) +
+    return (kind == MIX_CONST ? (size_t)f64_tab_entries(nPx) * 7 * 8 : 0) +
            F64_WARPS * ((f64_warp_bytes(kind, nPx) + 15) / 16 * 16) + 16;
 }
 
@@ -159,30 +162,37 @@ __global__ void k_mask_table(Rule rule, int dV, int TS, int n, double *__restric
     tab[i] = f64_mask_sum(rule, dV, m, r, c);
 }
 
-// Square root, reciprocal and reciprocal square root by Newton's iteration from an FP32 seed (24 bits,
-// so two steps reach FP64; the last step of the square root and of the quotient is the residual
-// correction). A CUDA division or square root keeps the FP64 pipe busy about twice as long: they
-// serve arguments whose FP32 seed would leave the FP32 range.
-__device__ __forceinline__ bool f64_seedable(float v) { return v > 1e-30f && v < 1e30f; }
+// Square root, quotient and reciprocal square root by Newton's iteration from an FP32 seed (22 bits or
+// more, so two steps reach FP64; the last step of the square root and of the quotient is the residual
+// correction). The seed's conversions go through the integer pipe (conversions from and to FP64 run
+// at its rate). CUDA's division and square root, which keep the FP64 pipe busy about twice as long,
+// serve arguments outside [2^-98, 2^98], where the seed would leave the FP32 range.
+__device__ __forceinline__ bool f64_seedable(double v) {   // v > 0
+    return (unsigned)((__double2hiint(v) >> 20) - (1023 - 98)) < 196u;
+}
+__device__ __forceinline__ float f64_to_seed(double v) {
+    const int hi = __double2hiint(v);
+    return __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)__double2loint(v) >> 29));
+}
+__device__ __forceinline__ double f64_from_seed(float s) {
+    const int b = __float_as_int(s);
+    return __hiloint2double((b >> 3) + (896 << 20), b << 29);
+}
+__device__ __forceinline__ double f64_rsqrt_step(double v, double y) { return fma(0.5 * y, fma(-(v * y), y, 1.0), y); }
 __device__ __forceinline__ double f64_rsqrt(double v) {
-    const float s = (float)v;
-    if (!f64_seedable(s)) return 1.0 / sqrt(v);
-    double y = (double)rsqrtf(s);
-    y = fma(0.5 * y, fma(-(v * y), y, 1.0), y);
-    return fma(0.5 * y, fma(-(v * y), y, 1.0), y);
+    if (!f64_seedable(v)) return 1.0 / sqrt(v);
+    return f64_rsqrt_step(v, f64_rsqrt_step(v, f64_from_seed(rsqrtf(f64_to_seed(v)))));
 }
 __device__ __forceinline__ double f64_sqrt(double v) {
-    const float s = (float)v;
-    if (!f64_seedable(s)) return sqrt(v);
-    double y = (double)rsqrtf(s);
-    y = fma(0.5 * y, fma(-(v * y), y, 1.0), y);
-    const double g = v * y;
+    if (!f64_seedable(v)) return sqrt(v);
+    const double y = f64_rsqrt_step(v, f64_from_seed(rsqrtf(f64_to_seed(v)))), g = v * y;
     return fma(0.5 * y, fma(-g, g, v), g);
 }
 __device__ __forceinline__ double f64_div(double a, double b) {
-    const float s = (float)b;
-    if (!f64_seedable(fabsf(s))) return a / b;
-    double y = (double)(1.f / s);
+    const double m = fabs(b);
+    if (!f64_seedable(m)) return a / b;
+    double y = f64_from_seed(__fdividef(1.f, f64_to_seed(m)));
+    y = __hiloint2double(__double2hiint(y) | (__double2hiint(b) & 0x80000000), __double2loint(y));
     y = fma(y, fma(-b, y, 1.0), y);
     const double q = a * y;
     return fma(y, fma(-b, q, a), q);
@@ -197,11 +207,47 @@ __device__ __forceinline__ double f64_kernel(const ProbParams &P, const double *
     return P.kc * exp2(-0.5 * P.expo * log2(r2));
 }
 
+// A cut item in the general pass's arithmetic (out_retri_f64, in_retri_f64), step by step in absolute
+// coordinates: the rare items whose polygon the certified run leaves open and which is tiny (a sphere
+// through a vertex, a near-tangent edge). Such a polygon may lie below the rounding of the partner's
+// reference coordinates, and which of its sums vanish decides which matrix entries exist.
+template <int KIND>
+__device__ __forceinline__ void f64_item_exact(const ProbParams &P, const Rule &rule, const double *pw, const double *x,
+                                            const double *Eb, double *res, unsigned &nsub) {
+    double R[18], S0 = 0, S1[3] = {0, 0, 0}, S2[3] = {0, 0, 0};
+    const int n = xretriangulate(x, Eb, P.sqdelta, P.caps, R);
+    for (int r = 0; r + 2 < n; r++) {
+        nsub++;
+        const double tri[6] = {R[0], R[1], R[2 * r + 2], R[2 * r + 3], R[2 * r + 4], R[2 * r + 5]};
+        const double rTdet = xabsDet2(tri);
+        for (int i = 0; i < rule.nPy; i++) {
+            double y[2], ref[2] = {0, 0};
+            y[0] = (tri[2] - tri[0]) * rule.Py[2 * i] + (tri[4] - tri[0]) * rule.Py[2 * i + 1] + tri[0];
+            y[1] = (tri[3] - tri[1]) * rule.Py[2 * i] + (tri[5] - tri[1]) * rule.Py[2 * i + 1] + tri[1];
+            const double z0 = x[0] - y[0], z1 = x[1] - y[1];
+            const double w = f64_kernel<KIND>(P, pw, z0 * z0 + z1 * z1) * rule.dy[i] * rTdet;
+            xtoRef(Eb, y, ref);
+            const double l0 = 1.0 - ref[0] - ref[1];
+            S0 += w;
+            S1[0] += l0 * w;
+            S1[1] += ref[0] * w;
+            S1[2] += ref[1] * w;
+            S2[0] += l0 * ref[0] * w;
+            S2[1] += l0 * ref[1] * w;
+            S2[2] += ref[0] * ref[1] * w;
+        }
+    }
+    res[0] = S0;
+#pragma unroll
+    for (int q = 0; q < 3; q++) { res[1 + q] = S1[q]; res[4 + q] = S2[q]; }
+}
+
 // Polygon of a cut item: points relative to the ball's center in R, and in the partner's reference
 // coordinates in L (n of each, at most 9).
 struct F64Poly {
     double R[18], L[18];
     int n;
+    unsigned seg;   // bit j: the side from point j - 1 (cyclic) to j may lie off the two edges through vertex 0
 };
 
 // The polygon of B(x) and the triangle Q (relative to x), e1, e2 its edges from Q0. The certified FP32
@@ -210,32 +256,45 @@ struct F64Poly {
 // quotient, per cap a reciprocal square root. In reference coordinates vertices are constants and
 // a crossing is its root. Against the exact routine, which takes both roots of all three edges with
 // their divisions for every item, that is about a third of the FP64 instructions: with the boundary
-// moments of f64_item 51.5 -> 24.5 ms on 2 * 128^2 triangles (constant kernel). Near-tangent cases
-// go to the exact routine (its points are the reference's bit for bit).
-template <bool PHYS>
-__device__ __forceinline__ void f64_polygon(const ProbParams &P, const double *x, const double *Eb, const double *Q,
-                                            const double *e, double idet, F64Poly &Y) {
-    const F2 Qf[3] = {f2((float)Q[0], (float)Q[1]), f2((float)Q[2], (float)Q[3]), f2((float)Q[4], (float)Q[5])};
-    bool amb = false;
-    unsigned long long codes = 0;
-    Y.n = fretriangulate<true>(Qf, P.sqdelta_f, P.caps, nullptr, amb, nullptr, &codes);
+// moments of f64_item 51.5 -> 20.5 ms on 2 * 128^2 triangles (constant kernel). False where a decision
+// is within its margin. LATE takes such an item's polygon from the exact routine instead, and is false
+// where that holds less than 1e-5 of the partner (f64_item_exact then; above, every sum of the item is
+// far above its rounding).
+template <bool PHYS, bool LATE>
+__device__ __forceinline__ bool f64_polygon(const ProbParams &P, const double *x, const double *Eb, const F2 *Qf, const double *Q,
+                                            const double *e, double adet, double idet, F64Poly &Y) {
     auto to_ref = [&](double yx, double yy, double *l) {
         const double dx = yx - Q[0], dy = yy - Q[1];
         l[0] = (e[3] * dx - e[2] * dy) * idet;
         l[1] = (e[0] * dy - e[1] * dx) * idet;
     };
-    if (amb) {
+    if (LATE) {
         Y.n = xretriangulate(x, Eb, P.sqdelta, P.caps, Y.R);
+        double area = 0;
         for (int j = 0; j < Y.n; j++) {
             Y.R[2 * j] -= x[0];
             Y.R[2 * j + 1] -= x[1];
             to_ref(Y.R[2 * j], Y.R[2 * j + 1], &Y.L[2 * j]);
+            if (j >= 2)
+                area += fabs((Y.R[2 * j - 2] - Y.R[0]) * (Y.R[2 * j + 1] - Y.R[1]) - (Y.R[2 * j - 1] - Y.R[1]) * (Y.R[2 * j] - Y.R[0]));
         }
-        return;
+        Y.seg = (1u << Y.n) - 1u;
+        return Y.n < 3 || area >= 1e-5 * adet;
     }
+    bool amb = false;
+    unsigned long long codes = 0;
+    Y.n = fretriangulate<true>(Qf, P.sqdelta_f, P.caps, nullptr, amb, nullptr, &codes);
+    if (amb) return false;
     unsigned xm = 0, cm = 0;
+    // by code, whether the point lies on edge 0 (bit c) and edge 2 (bit c + 16): vertices 0, 1 and the
+    // roots 3, 4 of edge 0; vertices 0, 2 and the roots 7, 8 of edge 2
+    constexpr unsigned ON = 0x0000001bu | 0x01850000u;
+    Y.seg = 0;
+    int cp = Y.n ? (int)(codes >> (4 * Y.n - 4)) & 15 : 0;
     for (int j = 0; j < Y.n; j++) {
         const int c = (int)(codes >> (4 * j)) & 15;
+        Y.seg |= (unsigned)(((ON >> c) & (ON >> cp) & 0x10001u) == 0) << j;
+        cp = c;
         xm |= (unsigned)(c >= FCODE_X && c < FCODE_CAP) << j;
         cm |= (unsigned)(c == FCODE_CAP) << j;
         if (c < 3) {
@@ -254,7 +313,7 @@ __device__ __forceinline__ void f64_polygon(const ProbParams &P, const double *x
         const double qx = k == 0 ? Q[2] : (k == 1 ? Q[4] : Q[0]), qy = k == 0 ? Q[3] : (k == 1 ? Q[5] : Q[1]);
         const double bx = px - qx, by = py - qy;
         const double ab = qx * bx + qy * by, aad = (qx * qx + qy * qy) - P.sqdelta, bb = bx * bx + by * by;
-        const double sv = f64_sqrt(fmax(ab * ab - aad * bb, 0.0));
+        const double v = ab * ab - aad * bb, sv = __double2hiint(v) > 0 ? f64_sqrt(v) : 0.0;
         // the root of larger size has no cancellation, the other is aad / bb over it (as the reference)
         const bool pos = ab < 0.0;
         const double big = pos ? sv - ab : -(ab + sv);
@@ -275,45 +334,83 @@ __device__ __forceinline__ void f64_polygon(const ProbParams &P, const double *x
         Y.R[2 * j + 1] = ny * s;
         to_ref(Y.R[2 * j], Y.R[2 * j + 1], &Y.L[2 * j]);
     }
+    return true;
 }
 
 // Inner sums of one item into res (see F64_RN), without the factor |T|: the quadrature over the
-// partner (inside) or over the fan of its polygon with the ball (cut). exact2: the inner rule integrates
-// polynomials of degree two exactly, so a constant kernel's sums over the fan are the polygon's
-// moments, taken from its boundary in reference coordinates (Green's theorem, one term per edge).
-template <int KIND>
-__device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, const PassRuleT<double> &pr, bool inside,
-                                         bool exact2, const double *pw, const double *x, const double *Eb, double *res, unsigned &nsub) {
+// partner (inside) or over the fan of its polygon with the ball (cut).
+// Polynomial kernels need no inner points. An inside item of the parabola kernel is a combination of
+// the rule's moments to degree four. Where the inner rule integrates the polynomials exactly (degree two
+// for constant kernels, four for the parabola), the sums over the fan are the polygon's integrals,
+// taken from its boundary in reference coordinates (Green's theorem with the origin in vertex 0, so that
+// sides on the two edges through it add nothing): closed forms per side for constant kernels; for
+// the parabola the integral over the triangle (0, P0, P1) of a monomial of degree d is
+// (P0 x P1) / (d + 2) times its mean over the side, by the 3-point Gauss rule (exact to degree five).
+// Returns false for a cut item whose polygon the certified run leaves open, which takes LATE.
+template <int KIND, bool LATE>
+__device__ __forceinline__ bool f64_item(const ProbParams &P, const Rule &rule, const PassRuleT<double> &pr, bool inside,
+                                         int exact, const double *pw, const double *x, const F2 *Qf, const double *Eb, double adet, double idet,
+                                         double *res, unsigned &nsub) {
     const double Q[6] = {Eb[0] - x[0], Eb[1] - x[1], Eb[2] - x[0], Eb[3] - x[1], Eb[4] - x[0], Eb[5] - x[1]};
     const double e[4] = {Eb[2] - Eb[0], Eb[3] - Eb[1], Eb[4] - Eb[0], Eb[5] - Eb[1]};
-    const double det = e[0] * e[3] - e[1] * e[2];
     double S0 = 0, S1[3] = {0, 0, 0}, S2[3] = {0, 0, 0};
-    if (KIND != MIX_CONST && inside) {
+    const bool parab = KIND == MIX_REGULAR && P.kernel == KER_PARABOLA;
+    // parabola: kernel kc (k0 - k1 . r - (ka r1^2 + 2 kb r1 r2 + kd r2^2)) in reference coordinates r
+    double k0 = 0, k1x = 0, k1y = 0, ka = 0, kb2 = 0, kd = 0;
+    if (parab) {
+        k0 = P.sqdelta - (Q[0] * Q[0] + Q[1] * Q[1]);
+        k1x = 2.0 * (Q[0] * e[0] + Q[1] * e[1]);
+        k1y = 2.0 * (Q[0] * e[2] + Q[1] * e[3]);
+        ka = e[0] * e[0] + e[1] * e[1];
+        kb2 = 2.0 * (e[0] * e[2] + e[1] * e[3]);
+        kd = e[2] * e[2] + e[3] * e[3];
+    }
+    auto from_moments = [&](double f, const double *I) {   // I: integrals of the kernel times 1, r1, r2, r1^2, r1 r2, r2^2
+        S0 = f * I[0];
+        S1[0] = f * (I[0] - I[1] - I[2]); S1[1] = f * I[1]; S1[2] = f * I[2];
+        S2[0] = f * (I[1] - I[3] - I[4]); S2[1] = f * (I[2] - I[4] - I[5]); S2[2] = f * I[4];
+    };
+    auto sum_point = [&](double k, int i, double *I) {   // inner point i with kernel value k
+        I[0] += k * rule.dy[i];
+        I[1] += k * pr.cy[3 * i + 1];
+        I[2] += k * pr.cy[3 * i + 2];
+        I[3] += k * pr.cyy[6 * i + 3];
+        I[4] += k * pr.cyy[6 * i + 4];
+        I[5] += k * pr.cyy[6 * i + 5];
+    };
+    if (KIND == MIX_REGULAR && parab && inside) {
         nsub++;
-        const double rT = fabs(det);
+        const double *m = pr.mom, *h = pr.mom4;
+        auto sum = [&](double c, double cx, double cy, double cxx, double cxy, double cyy) {
+            return k0 * c - (k1x * cx + k1y * cy) - (ka * cxx + kb2 * cxy + kd * cyy);
+        };
+        const double I[6] = {sum(m[0], m[1], m[2], m[3], m[4], m[5]), sum(m[1], m[3], m[4], h[0], h[1], h[2]),
+                             sum(m[2], m[4], m[5], h[1], h[2], h[3]), sum(m[3], h[0], h[1], h[4], h[5], h[6]),
+                             sum(m[4], h[1], h[2], h[5], h[6], h[7]), sum(m[5], h[2], h[3], h[6], h[7], h[8])};
+        from_moments(P.kc * adet, I);
+    } else if (KIND != MIX_CONST && inside) {
+        nsub++;
+        double I[6] = {0, 0, 0, 0, 0, 0};
         for (int i = 0; i < rule.nPy; i++) {
             const double yx = Q[0] + e[0] * rule.Py[2 * i] + e[2] * rule.Py[2 * i + 1];
             const double yy = Q[1] + e[1] * rule.Py[2 * i] + e[3] * rule.Py[2 * i + 1];
-            const double kw = f64_kernel<KIND>(P, pw, yx * yx + yy * yy) * rT;
-            S0 += kw * rule.dy[i];
-#pragma unroll
-            for (int c = 0; c < 3; c++) S1[c] += kw * pr.cy[3 * i + c];
-            S2[0] += kw * pr.cyy[6 * i + 1];
-            S2[1] += kw * pr.cyy[6 * i + 2];
-            S2[2] += kw * pr.cyy[6 * i + 4];
+            sum_point(f64_kernel<KIND>(P, pw, yx * yx + yy * yy), i, I);
         }
+        from_moments(adet, I);
     } else {
         F64Poly Y;
-        f64_polygon<KIND != MIX_CONST>(P, x, Eb, Q, e, f64_div(1.0, det), Y);
-        const double adet = fabs(det);
+        if (!f64_polygon<KIND != MIX_CONST, LATE>(P, x, Eb, Qf, Q, e, adet, idet, Y)) {
+            if (LATE) f64_item_exact<KIND>(P, rule, pw, x, Eb, res, nsub);
+            return LATE;
+        }
         if (Y.n >= 3) nsub += Y.n - 2;
-        if (KIND == MIX_CONST && exact2) {
+        if (KIND == MIX_CONST && (exact & 1)) {
             if (Y.n >= 3) {
                 double A = 0, Mx = 0, My = 0, Mxx = 0, Mxy = 0, Myy = 0;
-                double x0 = Y.L[2 * Y.n - 2], y0 = Y.L[2 * Y.n - 1];
 #pragma unroll 1
-                for (int j = 0; j < Y.n; j++) {
-                    const double x1 = Y.L[2 * j], y1 = Y.L[2 * j + 1];
+                for (unsigned sg = Y.seg; sg; sg &= sg - 1) {   // sides through the origin's edges add nothing
+                    const int j = __ffs(sg) - 1, i = j ? j - 1 : Y.n - 1;
+                    const double x0 = Y.L[2 * i], y0 = Y.L[2 * i + 1], x1 = Y.L[2 * j], y1 = Y.L[2 * j + 1];
                     const double c = x0 * y1 - x1 * y0, sx = x0 + x1, sy = y0 + y1;
                     A += c;
                     Mx = fma(c, sx, Mx);
@@ -321,8 +418,6 @@ __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, 
                     Mxx = fma(c, fma(sx, sx, -(x0 * x1)), Mxx);
                     Myy = fma(c, fma(sy, sy, -(y0 * y1)), Myy);
                     Mxy = fma(c, fma(sx, sy, fma(x0, y0, x1 * y1)), Mxy);
-                    x0 = x1;
-                    y0 = y1;
                 }
                 const double f = P.kc * adet;
                 A *= 0.5 * f;
@@ -335,6 +430,31 @@ __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, 
                 S1[0] = A - Mx - My; S1[1] = Mx; S1[2] = My;
                 S2[0] = Mx - Mxx - Mxy; S2[1] = My - Mxy - Myy; S2[2] = Mxy;
             }
+        } else if (KIND == MIX_REGULAR && parab && (exact & 2)) {
+            double I[6] = {0, 0, 0, 0, 0, 0};
+            const double k02 = 0.5 * k0, k03 = (1.0 / 3.0) * k0, k04 = 0.25 * k0;
+            if (Y.n < 3) Y.seg = 0;
+#pragma unroll 1
+            for (unsigned sg = Y.seg; sg; sg &= sg - 1) {
+                const int j = __ffs(sg) - 1, i = j ? j - 1 : Y.n - 1;
+                const double x0 = Y.L[2 * i], y0 = Y.L[2 * i + 1], dx = Y.L[2 * j] - x0, dy = Y.L[2 * j + 1] - y0;
+                const double c = x0 * dy - dx * y0;
+#pragma unroll
+                for (int g = 0; g < 3; g++) {
+                    const double t = g == 1 ? 0.5 : (g == 0 ? 0.11270166537925831 : 0.8872983346207417);
+                    const double zx = fma(t, dx, x0), zy = fma(t, dy, y0), cg = c * (g == 1 ? 4.0 / 9.0 : 5.0 / 18.0);
+                    const double k1 = k1x * zx + k1y * zy, k2 = zx * (ka * zx) + zy * (kb2 * zx + kd * zy);
+                    const double w0 = cg * (k02 - (1.0 / 3.0) * k1 - 0.25 * k2), w1 = cg * (k03 - 0.25 * k1 - 0.2 * k2);
+                    const double w2 = cg * (k04 - 0.2 * k1 - (1.0 / 6.0) * k2), tx = w2 * zx;
+                    I[0] += w0;
+                    I[1] += w1 * zx;
+                    I[2] += w1 * zy;
+                    I[3] += tx * zx;
+                    I[4] += tx * zy;
+                    I[5] += (w2 * zy) * zy;
+                }
+            }
+            from_moments(P.kc * adet, I);
         } else if (KIND == MIX_CONST) {   // the rule's moments on each fan triangle (see item_cut_const)
             const double m0 = pr.mom[0], mx = pr.mom[1], my = pr.mom[2], mxx = pr.mom[3], mxy = pr.mom[4], myy = pr.mom[5];
             const double la[3] = {1.0 - Y.L[0] - Y.L[1], Y.L[0], Y.L[1]};
@@ -358,32 +478,47 @@ __device__ __forceinline__ void f64_item(const ProbParams &P, const Rule &rule, 
                 S2[2] += rT * (la[1] * t0[2] + (be[1] * t1[2] + ga[1] * t2[2]));
             }
         } else {
+            double M[6] = {0, 0, 0, 0, 0, 0};
             for (int r = 0; r + 2 < Y.n; r++) {
                 const double Bx = Y.R[2 * r + 2] - Y.R[0], By = Y.R[2 * r + 3] - Y.R[1];
                 const double Cx = Y.R[2 * r + 4] - Y.R[0], Cy = Y.R[2 * r + 5] - Y.R[1];
-                const double b1 = Y.L[2 * r + 2] - Y.L[0], b2 = Y.L[2 * r + 3] - Y.L[1];
-                const double c1 = Y.L[2 * r + 4] - Y.L[0], c2 = Y.L[2 * r + 5] - Y.L[1];
                 const double rT = fabs(Bx * Cy - By * Cx);
+                double I[6] = {0, 0, 0, 0, 0, 0};   // in the fan triangle's own reference coordinates
                 for (int i = 0; i < rule.nPy; i++) {
                     const double px = rule.Py[2 * i], py = rule.Py[2 * i + 1];
                     const double yx = Y.R[0] + Bx * px + Cx * py, yy = Y.R[1] + By * px + Cy * py;
-                    const double kw = f64_kernel<KIND>(P, pw, yx * yx + yy * yy) * (rT * rule.dy[i]);
-                    const double l1 = Y.L[0] + b1 * px + c1 * py, l2 = Y.L[1] + b2 * px + c2 * py, l0 = 1.0 - l1 - l2;
-                    const double k1 = kw * l1, k2 = kw * l2;
-                    S0 += kw;
-                    S1[0] += kw * l0;
-                    S1[1] += k1;
-                    S1[2] += k2;
-                    S2[0] += k1 * l0;
-                    S2[1] += k2 * l0;
-                    S2[2] += k1 * l2;
+                    sum_point(f64_kernel<KIND>(P, pw, yx * yx + yy * yy), i, I);
                 }
+                // r1, r2 of the partner are affine in them
+                const double a1 = Y.L[0], a2 = Y.L[1], b1 = Y.L[2 * r + 2] - a1, b2 = Y.L[2 * r + 3] - a2;
+                const double c1 = Y.L[2 * r + 4] - a1, c2 = Y.L[2 * r + 5] - a2;
+                const double u0 = a1 * I[0] + b1 * I[1] + c1 * I[2], v0 = a2 * I[0] + b2 * I[1] + c2 * I[2];
+                const double ux = a1 * I[1] + b1 * I[3] + c1 * I[4], vx = a2 * I[1] + b2 * I[3] + c2 * I[4];
+                const double uy = a1 * I[2] + b1 * I[4] + c1 * I[5], vy = a2 * I[2] + b2 * I[4] + c2 * I[5];
+                M[0] += rT * I[0];
+                M[1] += rT * u0;
+                M[2] += rT * v0;
+                M[3] += rT * (a1 * u0 + b1 * ux + c1 * uy);
+                M[4] += rT * (a1 * v0 + b1 * vx + c1 * vy);
+                M[5] += rT * (a2 * v0 + b2 * vx + c2 * vy);
             }
+            from_moments(1.0, M);
         }
     }
     res[0] = S0;
 #pragma unroll
     for (int q = 0; q < 3; q++) { res[1 + q] = S1[q]; res[4 + q] = S2[q]; }
+    return true;
+}
+// About one cut item in 400 on the mesh above. Out of line, after the others of its chunk: inlined, the
+// exact routines' registers and code cost the ordinary items 5 to 10%.
+template <int KIND>
+__device__ __noinline__ unsigned f64_item_late(const ProbParams *P, const Rule &rule, const PassRuleT<double> &pr, int exact,
+                                               const double *pw, const double *x, const double *Eb, double adet, double idet,
+                                               double *res) {
+    unsigned nsub = 0;
+    f64_item<KIND, true>(*P, rule, pr, false, exact, pw, x, nullptr, Eb, adet, idet, res, nsub);
+    return nsub;
 }
 
 template <int KIND>
@@ -395,23 +530,17 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
     const SlotMap &sm = fa.m.m;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int nPx = rule.nPx;
-    // block: outer rule coefficients [nPx][7] (dx psi_r, off-diagonal dx psi_r psi_c, dx), mask sums
-    double *coef = reinterpret_cast<double *>(s_raw);
-    double *tab = coef + 7 * nPx;
+    double *tab = reinterpret_cast<double *>(s_raw);   // mask sums (constant kernels)
     unsigned char *wbase = reinterpret_cast<unsigned char *>(tab + (CK ? 7 * f64_tab_entries(nPx) : 0));
     wbase = s_raw + ((wbase - s_raw) + 15) / 16 * 16 + (size_t)wib * ((f64_warp_bytes(KIND, nPx) + 15) / 16 * 16);
     F64Warp &W = *reinterpret_cast<F64Warp *>(wbase);
     double *x64 = reinterpret_cast<double *>(wbase + (sizeof(F64Warp) + 15) / 16 * 16);   // [nPx][2]
     F2 *xf = reinterpret_cast<F2 *>(x64 + 2 * nPx);                                       // [nPx]
-    unsigned char *work = reinterpret_cast<unsigned char *>(xf + nPx);
+    double *coef = reinterpret_cast<double *>(xf + nPx);   // [nPx][7]: |T| dx times psi_r, psi_r psi_c (r < c), 1
+    unsigned char *work = reinterpret_cast<unsigned char *>(coef + 7 * nPx);
     long long *acc = reinterpret_cast<long long *>(work);                                 // [32][f64_acc]
     double *res = reinterpret_cast<double *>(acc + 32 * f64_acc(KIND));                   // [F64_CAP][F64_RN]
     F64Entry<NW> *slist = reinterpret_cast<F64Entry<NW> *>(work);
-    for (int i = threadIdx.x; i < 7 * nPx; i += F64_THREADS) {
-        const int k = i / 7, q = i - 7 * k;
-        coef[i] = q < 3 ? pr.cx[3 * k + q] : (q < 6 ? pr.cxx[6 * k + (q == 5 ? 4 : q - 2)] : pr.dxf[k]);
-    }
-    __syncthreads();
     if (CK) {
         for (int i = threadIdx.x; i < 7 * f64_tab_entries(nPx); i += F64_THREADS) tab[i] = fa.mtab[i];
         __syncthreads();
@@ -459,6 +588,10 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
             xtoPhys<2>(ET64, &rule.Px[2 * k], &x64[2 * k]);
             xf[k] = f2((float)(x64[2 * k] - ET64[0]), (float)(x64[2 * k + 1] - ET64[1]));
         }
+        for (int i = lane; i < 7 * nPx; i += 32) {
+            const int k = i / 7, q = i - 7 * k;
+            coef[i] = dT * (q < 3 ? pr.cx[3 * k + q] : (q < 6 ? pr.cxx[6 * k + (q == 5 ? 4 : q - 2)] : pr.dxf[k]));
+        }
         __syncwarp();
         int et[3];   // eighths of a bit: the unit exponent of T's rows
 #pragma unroll
@@ -498,6 +631,8 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
 #pragma unroll
                 for (int j = 0; j < 6; j++)
                     pc[j] = (a.EChi[(long long)part * 6 + j] - ((j & 1) ? ohi1 : ohi0)) + (a.EClo[(long long)part * 6 + j] - ((j & 1) ? olo1 : olo0));
+#pragma unroll
+                for (int j = 0; j < 3; j++) W.pc[lane][j] = f2(pc[2 * j], pc[2 * j + 1]);
                 for (int k = 0; k < nPx; k++) {
                     const F2 x = xf[k];
                     const F2 Q[3] = {f2(pc[0] - x.x, pc[1] - x.y), f2(pc[2] - x.x, pc[3] - x.y), f2(pc[4] - x.x, pc[5] - x.y)};
@@ -509,30 +644,49 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
             nitin += __popc(inm);
             nitcut += __popc(cutm);
             if (CK) nsub += __popc(inm);
-            // items, pair by pair, in chunks of whole pairs
+            // items, pair by pair, in chunks of whole pairs; inside and cut items are integrated apart,
+            // so that a warp does not run both paths
             const unsigned itm = CK ? cutm : inm | cutm;
-            const int cnt = __popc(itm);
-            const int incl = warp_incl_scan(cnt, lane), off = incl - cnt;
+            const int cnt = __popc(itm), cin = CK ? 0 : __popc(inm);
+            const int sc = warp_incl_scan(cnt | cin << 16, lane);
+            const int incl = sc & 0xffff, off = incl - cnt, offin = (sc >> 16) - cin;
             const int total = __shfl_sync(FULL, incl, 31);
-            for (int base = 0; base < total;) {
+            for (int base = 0, basein = 0; base < total;) {
                 const bool mine = cnt > 0 && off >= base && off + cnt <= base + F64_CAP;
                 const unsigned who = __ballot_sync(FULL, mine);
-                const int end = __shfl_sync(FULL, incl, 31 - __clz(who));
+                const int last = 31 - __clz(who);
+                const int end = __shfl_sync(FULL, incl, last), endin = __shfl_sync(FULL, sc >> 16, last);
+                const int n = end - base, nin = endin - basein;
                 if (mine) {
-                    int w = off - base;
+                    int w = off - base, wi = offin - basein, wc = nin + w - wi;
                     const int r = __popc(who & lanemask_lt());
                     W.pl[r] = (unsigned char)lane;
                     W.ps[r] = (unsigned char)w;
                     W.pn[r] = (unsigned char)cnt;
                     for (unsigned mm = itm; mm; mm &= mm - 1) {
                         const int k = __ffs(mm) - 1;
-                        W.list[w++] = (unsigned short)(lane << 6 | ((inm >> k) & 1u) << 5 | k);
+                        const unsigned in = (inm >> k) & 1u;
+                        if (!CK) W.order[in ? wi++ : wc++] = (unsigned char)w;
+                        W.list[w++] = (unsigned short)(lane << 6 | in << 5 | k);
                     }
                 }
                 __syncwarp();
-                for (int i = lane; i < end - base; i += 32) {
-                    const int it = W.list[i], k = it & 31;
-                    f64_item<KIND>(P, rule, pr, (it >> 5) & 1, fa.exact2, pw, &x64[2 * k], &a.EC[(long long)W.pid[it >> 6] * 6], &res[i * F64_RN], nsub);
+                unsigned late = 0;   // bit r: this lane's r-th item of the chunk needs the exact routine
+                for (int part0 = 0; part0 < (CK ? 1 : 2); part0++) {   // inside items, then cut items
+                    const int first = CK || part0 == 0 ? 0 : nin, past = CK || part0 ? n : nin;
+                    for (int i0 = first + lane, r = 0; i0 < past; i0 += 32, r++) {
+                        const int i = CK ? i0 : W.order[i0], it = W.list[i], k = it & 31, j = it >> 6, b = W.pid[j];
+                        const F2 xk = xf[k], Qf[3] = {W.pc[j][0] - xk, W.pc[j][1] - xk, W.pc[j][2] - xk};
+                        if (!f64_item<KIND, false>(P, rule, pr, !CK && part0 == 0, fa.exact, pw, &x64[2 * k], Qf, &a.EC[(long long)b * 6],
+                                                   a.adet[b], fa.idet[b], &res[i * F64_RN], nsub))
+                            late |= 1u << r;
+                    }
+                }
+                for (; late; late &= late - 1) {
+                    const int i0 = (CK ? 0 : nin) + lane + 32 * (__ffs(late) - 1);
+                    const int i = CK ? i0 : W.order[i0], it = W.list[i], b = W.pid[it >> 6];
+                    nsub += f64_item_late<KIND>(&a.probs[a.eprob[T]], rule, pr, fa.exact, pw, &x64[2 * (it & 31)],
+                                                &a.EC[(long long)b * 6], a.adet[b], fa.idet[b], &res[i * F64_RN]);
                 }
                 __syncwarp();
                 const int nun = __popc(who) * F64_OUT;
@@ -544,10 +698,10 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                     for (int i = W.ps[r], e = i + W.pn[r]; i < e; i++) v += coef[7 * (W.list[i] & 31) + ci] * res[i * F64_RN + ri];
                     long long *A = &acc[pl * f64_acc(KIND)];
                     if (o >= 9 && o < 12) {
-                        A[o] = __double_as_longlong(v * dT);
+                        A[o] = __double_as_longlong(v);
                     } else {
                         const int ex = o < 9 ? (8 * F64_BITS - P.xN - W.te[o / 3] - W.pve[pl][o % 3]) >> 3 : F64_BITS - P.xD - W.pe[pl];
-                        const double q = scale2(v * dT, ex);
+                        const double q = scale2(v, ex);
                         const long long iv = f64_fix(q, bad);
                         A[o] = iv;
                         if (o >= 12) A[o + 3] = f64_fix_lo(q, iv);
@@ -556,6 +710,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                 }
                 __syncwarp();
                 base = end;
+                basein = endin;
             }
             // owner: the pair's blocks as integers (termLocal stays FP64, summed per lane)
             long long nx[9 * NW];

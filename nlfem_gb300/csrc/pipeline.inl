@@ -383,9 +383,11 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     }
     // fixed-point scale: typical magnitude of an entry
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    double finite = 0;   // stays 0 unless a coordinate is not finite
     for (long v = 0; v < p.nV; v++)
         for (int j = 0; j < p.dim; j++) {
             double x = p.vertices[v * p.dim + j];
+            finite += x - x;
             lo[j] = std::min(lo[j], x);
             hi[j] = std::max(hi[j], x);
         }
@@ -425,8 +427,8 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
         // numbers, and that a double-float pair holds a coordinate to far below 2^-24 delta (its own
         // rounding is 2^-48 of the coordinate). The FP64 paths check both.
         double cmax = 0;
-        for (long v = 0; v < p.nV * p.dim; v++) cmax = fabs(p.vertices[v]) <= cmax ? cmax : fabs(p.vertices[v]);   // a NaN stays
-        P.cert = hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
+        for (int j = 0; j < p.dim; j++) cmax = std::max(cmax, std::max(fabs(lo[j]), fabs(hi[j])));
+        P.cert = finite == 0 && hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
                  p.sqdelta < 1e14 && std::min(hmin2, p.sqdelta) > 1e-24 && hmin2 * p.sqdelta > 1e-28;
     }
     double mag, kbound = 0;   // kbound: bound of |kernel| inside the ball (estimate for singular kernels)
@@ -512,6 +514,7 @@ struct Session {
     bool f64 = false;          // PM_RETRI or PM_BARY in FP64 (passes_f64.cuh, passes_f64_bary.cuh)
     bool cert = false;         // the pair search takes the certified FP32 geometry
     DevBuf pw;                 // power tables of the singular kernels (FP64), PW_N numbers per problem
+    DevBuf idet;               // 1 / det per element (FP64 retriangulate pass)
     DevBuf vexp, valsNlo, valslo, mtab;   // FP64 one-sided passes: vertex exponents, second integers, mask table
     DevBuf vcnt, vptr, vel, adjcnt, xadj, adj;
     DevBuf stamp_epoch;   // per-warp stamp epochs of the search
@@ -573,7 +576,7 @@ struct Session {
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
                 &hcap, &hptr, &htab, &tpos, &dslot, &rwords, &rbase, &rlo, &rankmap, &eid_ptr, &eid, &vp_cnt, &vp_off, &vp_ptr, &vp_scratch, &pscratch, &rowoff, &kclist, &valsN, &elp,
                 &po_cnt, &po_off, &po_ptr, &po_scratch, &tcnt, &tptr, &tcols, &sv_vec, &sv_part, &zptr, &zidx, &vacc, &vtiny,
-                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo, &mtab, &pw};
+                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo, &mtab, &pw, &idet};
     }
     ~Session() {
         for (DevBuf *b : buffers()) b->release();
@@ -910,6 +913,8 @@ static int run_prep(Session &S) {
     ENS(S.adetf, sizeof(float) * nE);
     ENS(S.EClo, sizeof(float) * nE * DIM * dV);
     ENS(S.BCf, sizeof(float) * nE * BC_STRIDE<DIM>);
+    const bool want_idet = S.f64 && S.pmode == PM_RETRI;
+    if (want_idet) ENS(S.idet, sizeof(double) * nE);
     ENS(S.labV, sizeof(int) * nV);
     ENS(S.vprob, sizeof(int) * nV);
     ENS(S.counters, sizeof(unsigned long long) * 16);
@@ -919,7 +924,8 @@ static int run_prep(Session &S) {
     k_prep_elements<DIM><<<grid_for(nE, 256), 256, 0, S.st>>>(
         S.T64.get<long long>(), S.labT64.get<long long>(), S.V.get<double>(), S.eoffd.get<int>(),
         S.voffd.get<int>(), S.nProb, nE, S.T32.get<int>(), S.labT.get<int>(), S.eprob.get<int>(),
-        S.EC.get<double>(), S.adet.get<double>(), S.EChi.get<float>(), S.EClo.get<float>(), S.adetf.get<float>(), S.BCf.get<float>()); ++S.nlaunch;
+        S.EC.get<double>(), S.adet.get<double>(), S.EChi.get<float>(), S.EClo.get<float>(), S.adetf.get<float>(), S.BCf.get<float>(),
+        want_idet ? S.idet.get<double>() : nullptr); ++S.nlaunch;
     k_prep_vertices<<<grid_for(nV, 256), 256, 0, S.st>>>(S.labV64.get<long long>(), S.voffd.get<int>(),
         S.nProb, nV, S.labV.get<int>(), S.vprob.get<int>()); ++S.nlaunch;
     CK(cudaGetLastError());
@@ -1484,7 +1490,7 @@ __global__ void k_pw_table(const ProbParams *__restrict__ probs, int nProb, doub
     if (p >= nProb || !probs[p].singular) return;
     const double h = -0.5 * probs[p].expo;
     double v = 0;
-    if (q < 6) {   // binomial coefficients of (1 + t)^h
+    if (q < 5) {   // binomial coefficients of (1 + t)^h
         v = 1.0;
         for (int n = 0; n <= q; n++) v *= (h - n) / (n + 1.0);
     } else if (q >= PW_E && q < PW_M) {   // kc 2^(E h); zero and subnormal arguments give infinity
@@ -1495,7 +1501,7 @@ __global__ void k_pw_table(const ProbParams *__restrict__ probs, int nProb, doub
                                 : probs[p].kc * ldexp(exp2(hi - I) * fma(lo, 0.6931471805599453, 1.0), (int)I));
     } else if (q >= PW_M) {
         const int j = (q - PW_M) >> 1;
-        const double inv = rint(4096.0 / (1.0 + (j + 0.5) / 256.0)) / 4096.0;
+        const double inv = rint(8192.0 / (1.0 + (j + 0.5) / PW_J)) / 8192.0;
         v = (q & 1) ? pow(inv, -h) : inv;
     }
     tab[i] = v;
@@ -1579,7 +1585,7 @@ static PassRuleT<R> make_pass_rule(const Rule &r, int dim) {
             for (int b = a; b < dV; b++) pr.cxx[NS * k + t++] = (R)(r.dx[k] * r.psix[dV * k + a] * r.psix[dV * k + b]);
         }
     }
-    A insum[1 + 4 + 10] = {0}, mom[6] = {0};
+    A insum[1 + 4 + 10] = {0}, mom[6] = {0}, mom4[9] = {0};
     for (int i = 0; i < r.nPy; i++) {
         for (int c = 0; c < dim; c++) pr.pyf[dim * i + c] = (R)r.Py[dim * i + c];
         int t = 0;
@@ -1596,10 +1602,14 @@ static PassRuleT<R> make_pass_rule(const Rule &r, int dim) {
             const A px = r.Py[2 * i], py = r.Py[2 * i + 1], w = r.dy[i];
             mom[0] += w; mom[1] += w * px; mom[2] += w * py;
             mom[3] += w * px * px; mom[4] += w * px * py; mom[5] += w * py * py;
+            mom4[0] += w * px * px * px; mom4[1] += w * px * px * py; mom4[2] += w * px * py * py; mom4[3] += w * py * py * py;
+            mom4[4] += w * px * px * px * px; mom4[5] += w * px * px * px * py; mom4[6] += w * px * px * py * py;
+            mom4[7] += w * px * py * py * py; mom4[8] += w * py * py * py * py;
         }
     }
     for (int q = 0; q < 1 + 4 + 10; q++) pr.insum[q] = (R)insum[q];
     for (int q = 0; q < 6; q++) pr.mom[q] = (R)mom[q];
+    for (int q = 0; q < 9; q++) pr.mom4[q] = (R)mom4[q];
     double xsum[10 + 4 + 1] = {0};
     for (int k = 0; k < r.nPx; k++) {
         int t = 0;
@@ -1795,16 +1805,23 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     fa.m.p = pa;
     fa.mtab = S.mtab.get<double>();
     fa.pw = S.pw.get<double>();   // singular kernels: made with the close pairs (run_close)
-    fa.exact2 = 1;   // the rule's moments are the triangle's to rounding (2^-53; the 7-point rule's are)
-    {
-        const double m[6] = {1.0 / 2, 1.0 / 6, 1.0 / 6, 1.0 / 12, 1.0 / 24, 1.0 / 12};
-        for (int q = 0; q < 6; q++) fa.exact2 = fa.exact2 && fabs(pr.mom[q] - m[q]) <= 1.2e-16 * m[q];
-    }
+    // whether the inner rule's moments are the triangle's to rounding (the 7-point rule's are): degree two
+    // for constant kernels, four for the parabola
+    bool ex2 = true, ex4 = true;
+    for (int d = 0, q2 = 0, q4 = 0; d <= 4; d++)
+        for (int b = 0; b <= d; b++) {   // integral of px^(d-b) py^b: (d-b)! b! / (d+2)!
+            static const double f[7] = {1, 1, 2, 6, 24, 120, 720};
+            const double m = f[d - b] * f[b] / f[d + 2], got = d <= 2 ? pr.mom[q2++] : pr.mom4[q4++];
+            if (d <= 2) ex2 = ex2 && fabs(got - m) <= 1.2e-16 * m;
+            ex4 = ex4 && fabs(got - m) <= 4e-16 * m;
+        }
+    fa.exact = (ex2 ? 1 : 0) | (ex4 ? 2 : 0);
     fa.m.m = slot_map(S);
     fa.m.work = reinterpret_cast<int *>(S.counters.get<unsigned long long>() + 10);
     fa.m.valsN = S.valsN.get<long long>();
     fa.m.elp = S.elp.get<long long>();
     fa.vexp = S.vexp.get<int>();
+    fa.idet = S.idet.get<double>();
     fa.valsNlo = wide ? S.valsNlo.get<long long>() : nullptr;
     fa.valslo = S.valslo.get<long long>();
     for (int i = 0; i < nl; i++) {

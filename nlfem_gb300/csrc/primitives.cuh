@@ -190,19 +190,18 @@ __device__ __forceinline__ double fx_to_double(unsigned long long lo, unsigned l
 }
 
 // ---------------------------------------------------------------- c r2^h by table
-// The singular kernels' c |z|^(2h) in FP64, r2 = |z|^2 = 2^E m: the top eight bits j of the mantissa
-// pick inv_j near 1 / m (twelve fraction bits, so t = m inv_j - 1 takes one rounding and |t| < 0.0023),
-// and c r2^h = (c 2^(E h)) inv_j^(-h) (1 + t)^h, the last factor by its binomial series to t^6 (the
-// next term is below 2^-60). Table-driven range reduction after Tang (1990). About 10 FP64
-// instructions where exp2(h log2 r2) takes about 75; the largest error over r2 in [1e-13, 1] and s in
-// [0.1, 0.9] is 4.6e-16 (1 / pow(sqrt(r2), 2 + 2s): 5.7e-16). One table per problem.
-constexpr int PW_E = 8, PW_M = PW_E + 2048, PW_N = PW_M + 512;   // b_1..b_6; c 2^(E h); pairs inv_j, inv_j^(-h)
+// The singular kernels' c |z|^(2h) in FP64, r2 = |z|^2 = 2^E m: the top nine bits j of the mantissa
+// pick inv_j near 1 / m (thirteen fraction bits, so t = m inv_j - 1 takes one rounding and |t| < 0.0012),
+// and c r2^h = (c 2^(E h)) inv_j^(-h) (1 + t)^h, the last factor by its binomial series to t^5 (the
+// next term is below 2^-55). Table-driven range reduction after Tang (1990). 8 FP64 instructions
+// where exp2(h log2 r2) takes about 75; the largest error over r2 in [1e-13, 1] and s in [0.1, 0.9] is
+// 4.6e-16 (1 / pow(sqrt(r2), 2 + 2s): 5.7e-16). One table per problem.
+constexpr int PW_E = 8, PW_M = PW_E + 2048, PW_J = 512, PW_N = PW_M + 2 * PW_J;   // b_1..b_5; c 2^(E h); pairs inv_j, inv_j^(-h)
 __device__ __forceinline__ double pw_eval(const double *__restrict__ tab, double r2) {
-    const int hi = __double2hiint(r2), j = (hi >> 12) & 255;
+    const int hi = __double2hiint(r2), j = (hi >> 11) & (PW_J - 1);
     const double2 q = reinterpret_cast<const double2 *>(tab + PW_M)[j];
     const double t = fma(__hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(r2)), q.x, -1.0);
-    double p = fma(tab[5], t, tab[4]);
-    p = fma(p, t, tab[3]);
+    double p = fma(tab[4], t, tab[3]);
     p = fma(p, t, tab[2]);
     p = fma(p, t, tab[1]);
     p = fma(p, t, tab[0]);

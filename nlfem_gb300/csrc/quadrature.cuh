@@ -502,48 +502,52 @@ __global__ void k_close_list(QuadArgs a, int *list, unsigned long long *count) {
 // One warp per close pair: integrate_fractional (integration.cpp:187-288) with join()
 // (:1913-1958), FP64 throughout; lanes stride over the Duffy points, warp-reduce the blocks.
 // Sum over the Duffy points of one close pair (integration.cpp:187-288) of w pxy pxy^T, upper
-// triangle of the nL x nL matrix, nL = 6 - NEQ: the lanes take the (map, Gauss point) items in
-// turn. The kernel value c |x - y|^-(d+2s) comes from the power table (pw_eval). FP64-bound: with exp2
-// and log2 the power was more than half of the instructions.
+// triangle of the nL x nL matrix, nL = 6 - NEQ, without the factor |A| |B|: the lanes take the (map,
+// Gauss point) items in turn. FP64-bound, so the loop keeps to what each point needs: x - y from the
+// elements' edge vectors at the shared first vertex (the join puts the common vertices first), the
+// kernel from the power table (pw_eval), and only rows and columns 1.. of the sums. The entries of pxy
+// add up to zero (both elements' basis functions sum to one), so close_row0 completes row 0. That
+// is 27 to 34 FP64 instructions per point; with exp2, log2 and the whole matrix it was 120.
 template <int NEQ>
 __device__ __forceinline__ void close_accumulate(const Duffy &d, const double *pw, int c, int nT,
-                                                 const double *EA, const double *EB, double dAB, double *M) {
-    constexpr int NL = 6 - NEQ, SH = 3 - NEQ;
+                                                 const double *EA, const double *EB, double *M) {
     const int lane = threadIdx.x & 31;
     const int total = nT * d.nPg;
-    const double *al_base = d.alpha[c];
+    const double2 *al_base = reinterpret_cast<const double2 *>(d.alpha[c]);
     const double *td_base = d.tdet[c];
     const double a0 = EA[2] - EA[0], a1 = EA[4] - EA[0], a2 = EA[3] - EA[1], a3 = EA[5] - EA[1];
     const double b0 = EB[2] - EB[0], b1 = EB[4] - EB[0], b2 = EB[3] - EB[1], b3 = EB[5] - EB[1];
     for (int idx = lane; idx < total; idx += 32) {
-        const int k = idx % d.nPg;
-        const double *al = &al_base[(long long)idx * 4];
-        const double tf = td_base[idx];
-        const double x0 = al[0] * a0 + al[1] * a1 + EA[0], x1 = al[0] * a2 + al[1] * a3 + EA[1];
-        const double y0 = al[2] * b0 + al[3] * b1 + EB[0], y1 = al[2] * b2 + al[3] * b3 + EB[1];
-        const double z0 = x0 - y0, z1 = x1 - y1;
-        const double r2 = z0 * z0 + z1 * z1;
-        const double ker = pw_eval(pw, r2);
-        const double px[3] = {1.0 - al[0] - al[1], al[0], al[1]};
-        const double py[3] = {1.0 - al[2] - al[3], al[2], al[3]};
-        double v[NL];
+        const double2 x = al_base[2 * idx], y = al_base[2 * idx + 1];
+        const double z0 = (x.x * a0 + x.y * a1) - (y.x * b0 + y.y * b1);
+        const double z1 = (x.x * a2 + x.y * a3) - (y.x * b2 + y.y * b3);
+        const double base = pw_eval(pw, z0 * z0 + z1 * z1) * (td_base[idx] * d.dg[idx % d.nPg]);
+        double v[6] = {0, 0, 0, 0, 0, 0};
+        if (NEQ == 1) { v[1] = x.x; v[2] = x.y; v[3] = -y.x; v[4] = -y.y; }
+        if (NEQ == 2) { v[1] = x.x - y.x; v[2] = x.y; v[3] = -y.y; }
+        if (NEQ == 3) { v[1] = x.x - y.x; v[2] = x.y - y.y; }
 #pragma unroll
-        for (int i = 0; i < 3; i++) {
-            if (i < NEQ) {
-                v[i] = px[i] - py[i];
-            } else {
-                v[i] = px[i];
-                v[i + SH] = -py[i];
-            }
-        }
-        const double base = ker * tf * d.dg[k] * dAB;
+        for (int i = 1; i < 6 - NEQ; i++) {
+            const double f = base * v[i];
 #pragma unroll
-        for (int aa = 0; aa < NL; aa++) {
-            const double fa = base * v[aa];
-#pragma unroll
-            for (int b = aa; b < NL; b++) M[sym_idx<6>(aa, b)] += fa * v[b];
+            for (int j = i; j < 6 - NEQ; j++) M[sym_idx<6>(i, j)] += f * v[j];
         }
     }
+}
+// Row 0 of the sums from the others (every row of w pxy pxy^T sums to zero).
+__device__ __forceinline__ void close_row0(int nL, double *M) {
+    double r0[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int j = 1; j < 6; j++)
+#pragma unroll
+        for (int i = 1; i < 6; i++)
+            if (j < nL && i < nL) r0[j] -= M[i <= j ? sym_idx<6>(i, j) : sym_idx<6>(j, i)];
+#pragma unroll
+    for (int j = 1; j < 6; j++) {
+        if (j < nL) M[j] = r0[j];
+        r0[0] -= r0[j];
+    }
+    M[0] = r0[0];
 }
 
 // The same sum on the mixed path with FP32 arithmetic throughout the point loop (FP64 runs at
@@ -807,12 +811,17 @@ __global__ void __launch_bounds__(128) k_quad_close(QuadArgs a, Duffy d) {
         else if (nEqual == 2) close_accumulate_f32<2>(P, d, c, nT, EA, EB, dA * dB, M);
         else close_accumulate_f32<3>(P, d, c, nT, EA, EB, dA * dB, M);
     } else {
-        if (nEqual == 1) close_accumulate<1>(d, pw, c, nT, EA, EB, dA * dB, M);
-        else if (nEqual == 2) close_accumulate<2>(d, pw, c, nT, EA, EB, dA * dB, M);
-        else close_accumulate<3>(d, pw, c, nT, EA, EB, dA * dB, M);
+        if (nEqual == 1) close_accumulate<1>(d, pw, c, nT, EA, EB, M);
+        else if (nEqual == 2) close_accumulate<2>(d, pw, c, nT, EA, EB, M);
+        else close_accumulate<3>(d, pw, c, nT, EA, EB, M);
     }
 #pragma unroll
     for (int i = 0; i < 21; i++) M[i] = warp_sum(M[i]);
+    if (!FAST) {
+#pragma unroll
+        for (int i = 0; i < 21; i++) M[i] *= dA * dB;
+        close_row0(nLocal, M);
+    }
     for (int aa = 0; aa < nLocal; aa++)
         for (int b = 0; b < nLocal; b++) acc[tgt[aa * 6 + b]] += sgn[aa * 6 + b] * M[aa <= b ? sym_idx<6>(aa, b) : sym_idx<6>(b, aa)];
     }

@@ -1239,3 +1239,21 @@ def test_fp64_pass_scales(nl, orc, scale, shift):
     fro, mx = rel_errors(A, B)
     tol = FP64_TOL + 64 * 1.1e-16 * shift / 0.1
     assert fro < tol and mx < tol, (fro, mx)
+
+
+def test_fp64_pass_keeps_vanishing_entries(nl, orc):
+    """A sphere within rounding of a vertex: the pair's polygon is far below the elements' own rounding
+    and one matrix entry is 1e-24 of the largest. The reference keeps it (only exact zeros are dropped)."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(26, 0.1099, jitter=0.2, seed=26)
+    rng = np.random.Generator(np.random.PCG64(475299725))
+    s, t = int(rng.integers(1, len(v))), int(rng.integers(1, len(e)))
+    v = v + rng.uniform(-0.5, 0.5, 2)
+    m = meshes.mesh_dict(np.roll(v, s, axis=0), np.roll((e + s) % len(v), t, axis=0), np.roll(l, t))
+    k = {"function": "parabola", "horizon": 0.1099, "outputdim": 1}
+    A = nl.stiffnessMatrix(m, k, conf2d())
+    B = orc.assemble(m, k, conf2d())["A"]
+    assert abs(B.tocsr().data).min() < 1e-20 * abs(B).max()   # the entry is there
+    assert same_pattern(A, B)
+    fro, mx = rel_errors(A, B)
+    assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
