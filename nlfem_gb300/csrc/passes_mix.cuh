@@ -22,7 +22,10 @@ namespace nlg {
 
 constexpr int MIX_WARPS = 4;
 constexpr int MIX_THREADS = 32 * MIX_WARPS;
-constexpr int RES_N = 10;   // per item: innerLocal, innerNonloc[3], inner termLocalPrime sums[6]
+constexpr int RES_N = 7;    // per item: innerLocal, innerNonloc[3], off-diagonal termLocalPrime sums[3] (the matrix
+                            // diagonal comes from the row sums); the odd stride keeps the banks apart
+// upper-triangle positions of the off-diagonal entries (0, 1), (0, 2), (1, 2)
+__host__ __device__ __forceinline__ constexpr int off3(int q) { return q == 2 ? 4 : q + 1; }
 constexpr int SCAT_U = 1;   // slot lookups per lane whose first accesses are issued together (more
                             // unrolling overflows the instruction cache of this kernel)
 
@@ -74,7 +77,7 @@ __device__ __forceinline__ void item_in(const ProbParams &P, const Rule &rule, c
     const F2 p0 = f2(pc[0] - x.x, pc[1] - x.y);
     const F2 e1 = f2(pc[2] - pc[0], pc[3] - pc[1]), e2 = f2(pc[4] - pc[0], pc[5] - pc[1]);
     float iL = 0, i0 = 0, i1 = 0, i2 = 0;
-    float lp[6] = {0, 0, 0, 0, 0, 0};
+    float lp[3] = {0, 0, 0};
     for (int i = 0; i < rule.nPy; i++) {
         const float px = Py[2 * i], py = Py[2 * i + 1];
         const float yx = p0.x + e1.x * px + e2.x * py;
@@ -85,11 +88,11 @@ __device__ __forceinline__ void item_in(const ProbParams &P, const Rule &rule, c
         i1 = fmaf(kw, pr.cy[3 * i + 1], i1);
         i2 = fmaf(kw, pr.cy[3 * i + 2], i2);
 #pragma unroll
-        for (int ab = 0; ab < 6; ab++) lp[ab] = fmaf(kw, pr.cyy[6 * i + ab], lp[ab]);
+        for (int q = 0; q < 3; q++) lp[q] = fmaf(kw, pr.cyy[6 * i + off3(q)], lp[q]);
     }
     res[0] = iL; res[1] = i0; res[2] = i1; res[3] = i2;
 #pragma unroll
-    for (int ab = 0; ab < 6; ab++) res[4 + ab] = lp[ab];
+    for (int q = 0; q < 3; q++) res[4 + q] = lp[q];
 }
 
 // Inner sums of one "cut" item: polygon of B(x) and b (certified FP32 with the exact FP64
@@ -104,7 +107,7 @@ __device__ __forceinline__ void item_cut(const ProbParams &P, const Rule &rule, 
     F2 Rp[9];
     const int n = cut_polygon(Q, P.sqdelta_f, P, x64, Eb64, Rp, namb);
     float iL = 0, i0 = 0, i1 = 0, i2 = 0;
-    float lp[6] = {0, 0, 0, 0, 0, 0};
+    float lp[3] = {0, 0, 0};
     for (int r = 0; r + 2 < n; r++) {
         nsub++;
         const F2 Av = Rp[0], B = Rp[r + 1] - Rp[0], C = Rp[r + 2] - Rp[0];
@@ -122,14 +125,14 @@ __device__ __forceinline__ void item_cut(const ProbParams &P, const Rule &rule, 
             i0 = fmaf(kw, s0, i0);
             i1 = fmaf(kw, r0, i1);
             i2 = fmaf(kw, r1, i2);
-            lp[0] = fmaf(kw, s0 * s0, lp[0]); lp[1] = fmaf(kw, s0 * r0, lp[1]);
-            lp[2] = fmaf(kw, s0 * r1, lp[2]); lp[3] = fmaf(kw, r0 * r0, lp[3]);
-            lp[4] = fmaf(kw, r0 * r1, lp[4]); lp[5] = fmaf(kw, r1 * r1, lp[5]);
+            lp[0] = fmaf(kw, s0 * r0, lp[0]);
+            lp[1] = fmaf(kw, s0 * r1, lp[1]);
+            lp[2] = fmaf(kw, r0 * r1, lp[2]);
         }
     }
     res[0] = iL; res[1] = i0; res[2] = i1; res[3] = i2;
 #pragma unroll
-    for (int ab = 0; ab < 6; ab++) res[4 + ab] = lp[ab];
+    for (int q = 0; q < 3; q++) res[4 + q] = lp[q];
 }
 
 // Inner sums of one "cut" item for a constant kernel. The kernel weight of every inner point is
@@ -157,7 +160,7 @@ __device__ __forceinline__ void item_cut_const(const ProbParams &P, const PassRu
         l[2] = (e1.x * dyr - e1.y * dxr) * idet;
         l[0] = 1.f - l[1] - l[2];
     };
-    float S0 = 0, S1[3] = {0, 0, 0}, S2[6] = {0, 0, 0, 0, 0, 0};
+    float S0 = 0, S1[3] = {0, 0, 0}, S2[3] = {0, 0, 0};
     float la[3], lb[3], lc[3];
     if (n >= 3) {
         basis(Rp[0], la);
@@ -177,13 +180,13 @@ __device__ __forceinline__ void item_cut_const(const ProbParams &P, const PassRu
             t2[q] = fmaf(al, my, fmaf(be, mxy, ga * myy));
         }
         S0 = fmaf(rT, m0, S0);
-        int t = 0;
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             S1[q] = fmaf(rT, t0[q], S1[q]);
             const float al = la[q], be = lb[q] - la[q], ga = lc[q] - la[q];
 #pragma unroll
-            for (int q2 = q; q2 < 3; q2++, t++) S2[t] = fmaf(rT, fmaf(al, t0[q2], fmaf(be, t1[q2], ga * t2[q2])), S2[t]);
+            for (int q2 = q + 1; q2 < 3; q2++)
+                S2[q + q2 - 1] = fmaf(rT, fmaf(al, t0[q2], fmaf(be, t1[q2], ga * t2[q2])), S2[q + q2 - 1]);
         }
 #pragma unroll
         for (int q = 0; q < 3; q++) lb[q] = lc[q];
@@ -193,7 +196,7 @@ __device__ __forceinline__ void item_cut_const(const ProbParams &P, const PassRu
 #pragma unroll
     for (int q = 0; q < 3; q++) res[1 + q] = kc * S1[q];
 #pragma unroll
-    for (int q = 0; q < 6; q++) res[4 + q] = kc * S2[q];
+    for (int q = 0; q < 3; q++) res[4 + q] = kc * S2[q];
 }
 
 // Appends this lane's items of class cls (one per outer point k with that class) to list, in
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 4) k_pass_mix2d(MixArgs ma, Rule 
                     }
                 } else {
                     float L[6] = {0, 0, 0, 0, 0, 0}, N[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-                    float LP[6] = {0, 0, 0, 0, 0, 0};
+                    float LP[3] = {0, 0, 0};
                     // the outer-point loop is warp-uniform (the rule's constants are read at one
                     // address per warp); each lane adds the items its classes select
                     float Axx[6] = {0, 0, 0, 0, 0, 0}, Ax[3] = {0, 0, 0}, Ad = 0;   // inside items (constant kernel)
@@ -445,14 +448,14 @@ __global__ void __launch_bounds__(MIX_THREADS, 4) k_pass_mix2d(MixArgs ma, Rule 
                                 N[3 * r + 2] = fmaf(c, rr[3], N[3 * r + 2]);
                             }
 #pragma unroll
-                            for (int ab = 0; ab < 6; ab++) LP[ab] = fmaf(dk, rr[4 + ab], LP[ab]);
+                            for (int q = 0; q < 3; q++) LP[q] = fmaf(dk, rr[4 + q], LP[q]);
                         }
                     }
                     if (CK) {   // an inside item's sums are kc |b| times the rule's element sums
-                        float inv[RES_N];
+                        float inv[RES_N];   // innerLocal, innerNonloc[3], off-diagonal termLocalPrime[3]
                         const float kr = P.kc_f * W.prt[lane];
 #pragma unroll
-                        for (int q = 0; q < RES_N; q++) inv[q] = kr * pr.insum[q];
+                        for (int q = 0; q < RES_N; q++) inv[q] = kr * pr.insum[q < 4 ? q : 4 + off3(q - 4)];
 #pragma unroll
                         for (int ab = 0; ab < 6; ab++) L[ab] = fmaf(Axx[ab], inv[0], L[ab]);
 #pragma unroll
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 4) k_pass_mix2d(MixArgs ma, Rule 
                             N[3 * r + 2] = fmaf(Ax[r], inv[3], N[3 * r + 2]);
                         }
 #pragma unroll
-                        for (int ab = 0; ab < 6; ab++) LP[ab] = fmaf(Ad, inv[4 + ab], LP[ab]);
+                        for (int q = 0; q < 3; q++) LP[q] = fmaf(Ad, inv[4 + q], LP[q]);
                     }
 #pragma unroll
                     for (int i = 0; i < 6; i++)   // the diagonal entries come from the row sums (k_sym_add)
@@ -470,8 +473,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 4) k_pass_mix2d(MixArgs ma, Rule 
 #pragma unroll
                     for (int i = 0; i < 9; i++) mx[i] = nx[i] = fx64(N[i] * rTT, P.fx_mul, bad);
 #pragma unroll
-                    for (int i = 0; i < 6; i++)
-                        if (i != 0 && i != 3 && i != 5) lpx[i] = fx64(LP[i] * rTT, P.fx_mul, bad);
+                    for (int q = 0; q < 3; q++) lpx[off3(q)] = fx64(LP[q] * rTT, P.fx_mul, bad);
                 }
                 // Only off-diagonal entries of the matrix are accumulated: every kept row of the
                 // assembled operator sums to zero (for kernels of |x - y| each pair's blocks do, the
