@@ -537,7 +537,7 @@ struct Session {
     DevBuf valsN, elp;                      // one-sided retriangulate pass: own-row termNonloc, LP blocks
     DevBuf po_cnt, po_off, po_ptr, po_scratch, tcnt, tptr, tcols;   // transposed pattern construction
     long long po_cap = 0, t_nnz = 0;
-    DevBuf sv_vec, sv_part;                 // CG solve: f, g, b, x, r, p, Ap; dot partials
+    DevBuf sv_vec, sv_part;                 // CG solve: f, g, x, r, p, Ap, u; scalars and dot partials
     DevBuf zptr, zidx;                      // domain-decomposition indicator (element -> subdomains)
     DevBuf vacc, vtiny;                     // vector path: 128-bit sums per expanded slot
     DevBuf kclist;                          // elements grouped by kernel class (pass launches)
@@ -2351,132 +2351,228 @@ static void cache_give(Session &S) {
 // A_Omega u = f_Omega - A_Gamma g for problem i of a session (computeRates2D.py:47-70): rows and
 // unknowns are the vertices with label > 0, g holds the Dirichlet values of the vertices with
 // label < 0 (label-0 columns are left out, as the reference's masks do). Conjugate gradients in
-// FP64 on the session's CSR: one warp per row for the products, dot products as fixed-grid block
-// partials summed on the host in a fixed order, so the iterates are deterministic.
-constexpr int SOLVE_DOT_BLOCKS = 256;
+// FP64 on the session's CSR, three launches per iteration and no host read inside a batch of them: the
+// dot products stay on the device as one partial per block, which every block of a later launch sums
+// in the same order (so all of them, and every run, get the same scalars).
+//   k_solve_a  stops when r.r has fallen below the bound; else Ap and p.Ap
+//   k_solve_b  x += alpha p, r -= alpha Ap, r.r
+//   k_solve_p  p = r + beta p
+// Launches past the stop return at once. The product is bound by the FP64 pipe where the matrix sits in
+// L2 and by HBM beyond (at 1/64 rate one FMA per entry takes about the time of its 12 bytes), so eight
+// lanes share a row (a 32-lane tree per row would add half as many FP64 instructions again), only one
+// warp per block sums the partials, and p is formed once rather than at every gather (forming it there
+// saved a launch but made the product 2.2 times slower). Per-iteration host reads of the two dot
+// products left the GPU idle most of the time (figures at session_solve).
+constexpr int SOLVE_THREADS = 256;
+constexpr int SOLVE_LANES = 8;    // lanes per matrix row
+constexpr int SOLVE_BATCH = 16;   // iterations queued between two looks at the state
 
-__global__ void k_solve_rhs(const long long *__restrict__ fptr, const int *__restrict__ fcols,
-                            const double *__restrict__ fvals, const int *__restrict__ labV, long long r0,
-                            long long n, const double *__restrict__ f, const double *__restrict__ g,
-                            double *__restrict__ b) {
-    const int lane = threadIdx.x & 31;
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w >= n) return;
-    const long long row = r0 + w;
-    double s = 0.0;
-    if (labV[row] > 0)
-        for (long long k = fptr[row] + lane; k < fptr[row + 1]; k += 32) {
-            const int c = fcols[k];
-            if (labV[c] < 0) s += fvals[k] * g[c - r0];
-        }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-    if (lane == 0) b[w] = labV[row] > 0 ? f[w] - s : 0.0;
-}
+struct SolveArgs {
+    const long long *fptr;
+    const int *fcols, *labV;
+    const double *fvals, *f, *g;
+    double *x, *r, *p, *Ap, *pa, *pb, *rs;   // pa: partials of p.Ap; pb: of r.r; rs[2]: r.r of even / odd iterations
+    int *state;                              // [0] iterations + 1 when stopped, [1] breakdown
+    double *stop;                            // the bound on r.r
+    long long r0, n;
+    int nba, nbb;                            // partials in pa, pb
+    double rtol2;
+    double *u;
+};
 
-__global__ void k_solve_spmv(const long long *__restrict__ fptr, const int *__restrict__ fcols,
-                             const double *__restrict__ fvals, const int *__restrict__ labV, long long r0,
-                             long long n, const double *__restrict__ x, double *__restrict__ y) {
-    const int lane = threadIdx.x & 31;
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w >= n) return;
-    const long long row = r0 + w;
-    double s = 0.0;
-    if (labV[row] > 0)
-        for (long long k = fptr[row] + lane; k < fptr[row + 1]; k += 32) {
-            const int c = fcols[k];
-            if (labV[c] > 0) s += fvals[k] * x[c - r0];
-        }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-    if (lane == 0) y[w] = s;
-}
-
-__global__ void k_solve_dot(const double *__restrict__ a, const double *__restrict__ b, long long n,
-                            double *__restrict__ part) {
-    __shared__ double sh[256];
-    double s = 0.0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        s += a[i] * b[i];
-    sh[threadIdx.x] = s;
+// Sum of n partials, the same in every block (fixed strides, fixed tree); sh: one double.
+__device__ __forceinline__ double solve_sum(const double *part, int n, double *sh) {
+    if (threadIdx.x < 32) {
+        double s = 0.0;
+        for (int i = threadIdx.x; i < n; i += 32) s += part[i];
+        s = warp_sum(s);
+        if (threadIdx.x == 0) *sh = s;
+    }
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+    return *sh;
 }
-
-// x += alpha p, r -= alpha Ap
-__global__ void k_solve_update(double alpha, const double *__restrict__ p, const double *__restrict__ Ap,
-                               double *__restrict__ x, double *__restrict__ r, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        x[i] += alpha * p[i];
-        r[i] -= alpha * Ap[i];
+// This block's partial: the threads' values by a fixed tree; sh: one double per warp.
+__device__ __forceinline__ void solve_partial(double v, double *sh, double *out) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < SOLVE_THREADS / 32; w++) s += sh[w];
+        *out = s;
     }
 }
-// p = r + beta p
-__global__ void k_solve_dir(double beta, const double *__restrict__ r, double *__restrict__ p, long long n) {
+__device__ __forceinline__ double solve_row_sum(double s) {
+#pragma unroll
+    for (int o = SOLVE_LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+    return s;
+}
+
+// b = f - A_Gamma g (0 where the vertex has no unknown), r = p = b, x = 0, partials of b.b.
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_rhs(SolveArgs a) {
+    __shared__ double sh[SOLVE_THREADS / 32];
+    const int sub = threadIdx.x & (SOLVE_LANES - 1);
+    double dot = 0.0;
+    const long long step = (long long)gridDim.x * (SOLVE_THREADS / SOLVE_LANES);
+    for (long long w = ((long long)blockIdx.x * SOLVE_THREADS + threadIdx.x) / SOLVE_LANES, e = (a.n + step - 1) / step * step; w < e;
+         w += step) {   // every lane takes the same number of turns
+        const long long row = a.r0 + w;
+        const bool un = w < a.n && a.labV[row] > 0;
+        double s = 0.0;
+        if (un)
+            for (long long k = a.fptr[row] + sub; k < a.fptr[row + 1]; k += SOLVE_LANES) {
+                const int c = a.fcols[k];
+                if (a.labV[c] < 0) s += a.fvals[k] * a.g[c - a.r0];
+            }
+        s = solve_row_sum(s);
+        if (w < a.n && sub == 0) {
+            const double b = un ? a.f[w] - s : 0.0;
+            a.r[w] = b;
+            a.p[w] = b;
+            a.x[w] = 0.0;
+            dot += b * b;
+        }
+    }
+    solve_partial(dot, sh, &a.pb[blockIdx.x]);
+}
+
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_a(SolveArgs a, int it) {
+    __shared__ double sh[SOLVE_THREADS / 32], sh1;
+    if (a.state[0]) return;   // stopped in an earlier launch
+    const double rs = solve_sum(a.pb, a.nbb, &sh1);
+    const double stop = it ? *a.stop : a.rtol2 * rs;
+    if (!(rs > stop && rs > 0.0)) {   // every block decides alike
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.state[0] = it + 1;
+        return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.rs[it & 1] = rs;
+        if (it == 0) *a.stop = stop;
+    }
+    const int sub = threadIdx.x & (SOLVE_LANES - 1);
+    const long long step = (long long)gridDim.x * (SOLVE_THREADS / SOLVE_LANES);
+    double dot = 0.0;
+    for (long long w = ((long long)blockIdx.x * SOLVE_THREADS + threadIdx.x) / SOLVE_LANES, e = (a.n + step - 1) / step * step; w < e;
+         w += step) {
+        const long long row = a.r0 + w;
+        double s = 0.0, s2 = 0.0;
+        if (w < a.n && a.labV[row] > 0) {   // p is zero where the column's vertex has no unknown
+            const long long b = a.fptr[row], end = a.fptr[row + 1];
+            long long k = b + sub;
+            for (; k + 3 * SOLVE_LANES < end; k += 4 * SOLVE_LANES) {   // four gathers in flight
+                int c[4];
+                double v[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    c[q] = a.fcols[k + q * SOLVE_LANES];
+                    v[q] = a.fvals[k + q * SOLVE_LANES];
+                }
+                s = fma(v[0], a.p[c[0] - a.r0], s);
+                s2 = fma(v[1], a.p[c[1] - a.r0], s2);
+                s = fma(v[2], a.p[c[2] - a.r0], s);
+                s2 = fma(v[3], a.p[c[3] - a.r0], s2);
+            }
+            for (; k < end; k += SOLVE_LANES) s = fma(a.fvals[k], a.p[a.fcols[k] - a.r0], s);
+        }
+        s = solve_row_sum(s + s2);
+        if (w < a.n && sub == 0) {
+            a.Ap[w] = s;
+            dot = fma(a.p[w], s, dot);
+        }
+    }
+    solve_partial(dot, sh, &a.pa[blockIdx.x]);
+}
+
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_b(SolveArgs a, int it) {
+    __shared__ double sh[SOLVE_THREADS / 32], sh1;
+    if (a.state[0]) return;
+    const double pAp = solve_sum(a.pa, a.nba, &sh1);
+    if (!(pAp > 0.0)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            a.state[1] = 1;
+            a.state[0] = it + 1;
+        }
+        return;
+    }
+    const double alpha = a.rs[it & 1] / pAp;
+    double dot = 0.0;
+    for (long long i = (long long)blockIdx.x * SOLVE_THREADS + threadIdx.x; i < a.n; i += (long long)gridDim.x * SOLVE_THREADS) {
+        a.x[i] += alpha * a.p[i];
+        const double r = a.r[i] - alpha * a.Ap[i];
+        a.r[i] = r;
+        dot += r * r;
+    }
+    solve_partial(dot, sh, &a.pb[blockIdx.x]);
+}
+
+__global__ void __launch_bounds__(SOLVE_THREADS) k_solve_p(SolveArgs a, int it) {
+    __shared__ double sh1;
+    if (a.state[0]) return;
+    const double beta = solve_sum(a.pb, a.nbb, &sh1) / a.rs[it & 1];
+    for (long long i = (long long)blockIdx.x * SOLVE_THREADS + threadIdx.x; i < a.n; i += (long long)gridDim.x * SOLVE_THREADS)
+        a.p[i] = a.r[i] + beta * a.p[i];
+}
+
+// u: the solution, g where the label is negative
+__global__ void k_solve_out(SolveArgs a) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = r[i] + beta * p[i];
+    if (i < a.n) a.u[i] = a.labV[a.r0 + i] < 0 ? a.g[i] : a.x[i];
 }
 
-static int solve_dot(Session &S, const double *a, const double *b, long long n, double *out) {
-    k_solve_dot<<<SOLVE_DOT_BLOCKS, 256, 0, S.st>>>(a, b, n, S.sv_part.get<double>());
-    CK(cudaGetLastError());
-    double part[SOLVE_DOT_BLOCKS];
-    int r = d2h(S, part, S.sv_part.get<double>(), SOLVE_DOT_BLOCKS);
-    if (r) return r;
-    double s = 0.0;
-    for (int k = 0; k < SOLVE_DOT_BLOCKS; k++) s += part[k];
-    *out = s;
-    return NLFEM_OK;
-}
-
+// 2 * 96^2 triangles, 2.0e6 entries, 45 iterations: 1.37 ms a solve (2.87 ms with host reads of the dot
+// products); per iteration 12 us for the product (half of it FP64 pipe time), 5.6 and 4.2 us for the
+// vector updates, which are launch and latency chains. 4, 16 or 32 lanes a row: 1.56, 1.49, 1.55 ms.
 static int session_solve(Session &S, int i, const double *f, const double *g, double rtol, int maxit,
                          double *u, int *iters) {
     if (S.nnz <= 0) return fail(NLFEM_ERR_INVALID, "solve needs an assembled session");
     const long long r0 = S.voff[i], n = S.voff[i + 1] - S.voff[i];
+    SolveArgs a;
+    memset(&a, 0, sizeof(a));
+    a.r0 = r0;
+    a.n = n;
+    const long long rows = SOLVE_THREADS / SOLVE_LANES;
+    a.nba = (int)std::min<long long>((n + rows - 1) / rows, (long long)S.nSM * 4);
+    a.nbb = (int)std::min<long long>((n + SOLVE_THREADS - 1) / SOLVE_THREADS, (long long)S.nSM * 2);
+    a.rtol2 = rtol * rtol;
     ENS(S.sv_vec, sizeof(double) * 7 * (n + 1));
-    ENS(S.sv_part, sizeof(double) * SOLVE_DOT_BLOCKS);
-    double *vf = S.sv_vec.get<double>(), *vg = vf + (n + 1), *b = vg + (n + 1), *x = b + (n + 1);
-    double *rr = x + (n + 1), *p = rr + (n + 1), *Ap = p + (n + 1);
+    ENS(S.sv_part, sizeof(double) * (2 * (size_t)a.nba + a.nbb + 8));
+    double *v = S.sv_vec.get<double>();
+    double *vf = v, *vg = v + (n + 1);
+    a.f = vf; a.g = vg;
+    a.x = v + 2 * (n + 1); a.r = v + 3 * (n + 1); a.p = v + 4 * (n + 1);
+    a.Ap = v + 5 * (n + 1); a.u = v + 6 * (n + 1);
+    a.rs = S.sv_part.get<double>();
+    a.stop = a.rs + 2;
+    a.state = reinterpret_cast<int *>(a.rs + 4);
+    a.pa = a.rs + 8;
+    a.pb = a.pa + a.nba;   // the first r.r has nba partials, later ones nbb
+    a.fptr = S.fptr.get<long long>(); a.fcols = S.fcols.get<int>(); a.fvals = S.fvals.get<double>();
+    a.labV = S.labV.get<int>();
     CK(cudaMemcpyAsync(vf, f, sizeof(double) * n, cudaMemcpyHostToDevice, S.st));
     CK(cudaMemcpyAsync(vg, g, sizeof(double) * n, cudaMemcpyHostToDevice, S.st));
-    CK(cudaMemsetAsync(x, 0, sizeof(double) * n, S.st));
-    const long long *fp = S.fptr.get<long long>();
-    const int *fc = S.fcols.get<int>(), *lab = S.labV.get<int>();
-    const double *fv = S.fvals.get<double>();
-    const unsigned gw = grid_for(n * 32, 256), ge = grid_for(n, 256);
-    k_solve_rhs<<<gw, 256, 0, S.st>>>(fp, fc, fv, lab, r0, n, vf, vg, b);
-    CK(cudaMemcpyAsync(rr, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, S.st));
-    CK(cudaMemcpyAsync(p, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, S.st));
-    double bb = 0.0, rs = 0.0;
-    int r = solve_dot(S, b, b, n, &bb);
-    if (r) return r;
-    rs = bb;
-    const double stop = rtol * rtol * bb;
-    int it = 0;
-    while (it < maxit && rs > stop && rs > 0.0) {
-        k_solve_spmv<<<gw, 256, 0, S.st>>>(fp, fc, fv, lab, r0, n, p, Ap);
-        double pAp = 0.0;
-        if ((r = solve_dot(S, p, Ap, n, &pAp))) return r;
-        if (!(pAp > 0.0)) return fail(NLFEM_ERR_NUMERIC, "CG breakdown: the operator is not positive definite on the search direction");
-        const double alpha = rs / pAp;
-        k_solve_update<<<ge, 256, 0, S.st>>>(alpha, p, Ap, x, rr, n);
-        double rs2 = 0.0;
-        if ((r = solve_dot(S, rr, rr, n, &rs2))) return r;
-        k_solve_dir<<<ge, 256, 0, S.st>>>(rs2 / rs, rr, p, n);
-        rs = rs2;
-        it++;
+    CK(cudaMemsetAsync(a.state, 0, 2 * sizeof(int), S.st));
+    const int nbb = a.nbb;
+    k_solve_rhs<<<a.nba, SOLVE_THREADS, 0, S.st>>>(a);
+    int r, state[2] = {0, 0}, it = 0;
+    while (!state[0] && it <= maxit) {   // the launch of iteration maxit only sees whether it has stopped
+        for (int k = 0; k < SOLVE_BATCH && it <= maxit; k++, it++) {
+            a.nbb = it ? nbb : a.nba;   // partials of r.r that this iteration sums
+            k_solve_a<<<a.nba, SOLVE_THREADS, 0, S.st>>>(a, it);
+            if (it == maxit) continue;
+            k_solve_b<<<nbb, SOLVE_THREADS, 0, S.st>>>(a, it);
+            a.nbb = nbb;
+            k_solve_p<<<nbb, SOLVE_THREADS, 0, S.st>>>(a, it);
+        }
+        CK(cudaGetLastError());
+        if ((r = d2h(S, state, a.state, 2))) return r;
     }
+    if (state[1]) return fail(NLFEM_ERR_NUMERIC, "CG breakdown: the operator is not positive definite on the search direction");
+    k_solve_out<<<grid_for(n, 256), 256, 0, S.st>>>(a);
     CK(cudaGetLastError());
-    std::vector<int> hl(n);
-    if ((r = d2h(S, u, x, n))) return r;
-    if ((r = d2h(S, hl.data(), lab + r0, n))) return r;
-    for (long long k = 0; k < n; k++)
-        if (hl[k] < 0) u[k] = g[k];
-    if (iters) *iters = it;
-    if (it >= maxit && rs > stop) return fail(NLFEM_ERR_NUMERIC, "CG did not reach the tolerance within maxit iterations");
+    if ((r = d2h(S, u, a.u, n))) return r;
+    const int its = state[0] ? state[0] - 1 : maxit;
+    if (iters) *iters = its;
+    if (!state[0]) return fail(NLFEM_ERR_NUMERIC, "CG did not reach the tolerance within maxit iterations");
     return NLFEM_OK;
 }
 }  // namespace nlg
