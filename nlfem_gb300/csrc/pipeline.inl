@@ -500,7 +500,7 @@ struct Session {
     Rule rule;
     int duffy_nPg = 0;
     cudaStream_t st = nullptr;
-    cudaEvent_t ev[8];
+    cudaEvent_t ev[8] = {};
     // inputs
     DevBuf T64, labT64, V, labV64, eoffd, voffd, prm, duffy;
     DevBuf duffyf;   // FP32 Duffy tables of the mixed close-pair rule: points (float4), weights
@@ -582,7 +582,8 @@ struct Session {
         for (DevBuf *b : buffers()) b->release();
         if (gexec) cudaGraphExecDestroy(gexec);
         if (st) {
-            for (int i = 0; i < 8; i++) cudaEventDestroy(ev[i]);
+            for (int i = 0; i < 8; i++)
+                if (ev[i]) cudaEventDestroy(ev[i]);
             cudaStreamDestroy(st);
         }
     }
@@ -635,6 +636,16 @@ template <typename T>
 static int d2h(Session &S, T *host, const T *dev, size_t n) {
     if (S.replay) return NLFEM_OK;   // captured sequence: the host values are those of the last run
     CK(cudaMemcpyAsync(host, dev, n * sizeof(T), cudaMemcpyDeviceToHost, S.st));
+    CK(cudaStreamSynchronize(S.st));
+    return NLFEM_OK;
+}
+
+// Two reads with one wait.
+template <typename T, typename U>
+static int d2h2(Session &S, T *h1, const T *d1, size_t n1, U *h2, const U *d2, size_t n2) {
+    if (S.replay) return NLFEM_OK;
+    CK(cudaMemcpyAsync(h1, d1, n1 * sizeof(T), cudaMemcpyDeviceToHost, S.st));
+    CK(cudaMemcpyAsync(h2, d2, n2 * sizeof(U), cudaMemcpyDeviceToHost, S.st));
     CK(cudaStreamSynchronize(S.st));
     return NLFEM_OK;
 }
@@ -739,8 +750,10 @@ static int session_init(Session &S, const nlfem_problem *probs, int n, bool syst
         int dev = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&S.nSM, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaStreamCreateWithFlags(&S.st, cudaStreamNonBlocking));
-        for (int i = 0; i < 8; i++) CK(cudaEventCreate(&S.ev[i]));
+        if (!S.st) {   // one-shot calls bring the last one's (cache_take)
+            CK(cudaStreamCreateWithFlags(&S.st, cudaStreamNonBlocking));
+            for (int i = 0; i < 8; i++) CK(cudaEventCreate(&S.ev[i]));
+        }
     }
     const int dV = S.dV, dim = S.dim;
     ENS(S.T64, sizeof(long long) * S.nE * dV);
@@ -1001,13 +1014,15 @@ static int run_bfs(Session &S) {
         }
         S.pool_cap = std::max<long long>((long long)(1.1 * est), 1 << 20);
     }
-    {   // stamps: zeroed only when first laid out (a new layout or a larger buffer)
+    {   // stamps: zeroed only when first laid out (a new layout or a larger buffer). With the layout
+        // unchanged, what an earlier search (of any mesh) left lies below the warps' epochs.
         const size_t be = sizeof(unsigned short) * (size_t)nwarps * S.maxNE;
         const size_t bv = sizeof(unsigned short) * (size_t)nwarps * S.maxNV;
         const size_t bw = sizeof(unsigned) * (size_t)nwarps;
         const bool relayout = be > S.visited.cap || bv > S.vvisited.cap || bw > S.stamp_epoch.cap ||
                               S.stamp_layout[0] != nwarps || S.stamp_layout[1] != S.maxNE ||
                               S.stamp_layout[2] != S.maxNV;
+        if (relayout) S.stamp_layout[0] = 0;   // until the stamps are cleared below
         ENS(S.visited, be);
         ENS(S.vvisited, bv);
         ENS(S.stamp_epoch, bw);
@@ -1051,10 +1066,9 @@ static int run_bfs(Session &S) {
         if (S.replay) return NLFEM_OK;   // overflow flags are checked after the replay
         unsigned long long hc[3];
         int he[2];
-        int r = d2h(S, hc, cnt, 3);
+        int r = d2h2(S, hc, cnt, 3, he, S.err.get<int>(), 2);
         if (r) return r;
-        r = d2h(S, he, S.err.get<int>(), 2);
-        if (r) return r;
+        S.P = (long long)hc[0];   // pool cursor: the pairs found
         if (he[0]) { S.qcap = std::max<long long>((long long)hc[2] * 3 / 2, S.qcap * 2); continue; }
         if (he[1]) { S.pool_cap = (long long)hc[0] + (long long)hc[0] / 8 + 1024; continue; }
         S.stats.n_candidates = (long)hc[1];
@@ -1090,9 +1104,7 @@ static int run_pairs(Session &S) {
     S.pairs_pool = !S.want_pair_arrays &&
                    (S.pmode == PM_BARY || S.pmode == PM_RETRI) && pattern_bitmap_threads(S);
     if (S.pairs_pool) {
-        int r = d2h(S, &S.P, reinterpret_cast<long long *>(S.counters.get<unsigned long long>()), 1);   // pool cursor
-        if (r) return r;
-        S.stats.n_pairs = (long)S.P;
+        S.stats.n_pairs = (long)S.P;   // read with the search's flags
         CK(cudaGetLastError());
         return NLFEM_OK;
     }
@@ -1389,9 +1401,8 @@ static int run_pattern_bm(Session &S, int words, int threads) {
         int r = scan_excl<int>(S, S.rowcnt.get<int>(), nV, S.rowptr.get<long long>());
         if (r) return r;
         int ovf = 0;
-        if ((r = d2h(S, &ovf, S.err.get<int>() + 6, 1))) return r;
+        if ((r = d2h2(S, &ovf, S.err.get<int>() + 6, 1, &S.nnz_struct, S.rowptr.get<long long>() + nV, 1))) return r;
         if (!ovf) {
-            if ((r = d2h(S, &S.nnz_struct, S.rowptr.get<long long>() + nV, 1))) return r;
             ENS(S.cols, sizeof(int) * (S.nnz_struct + 1));
             k_row_copy<<<S.nSM * 8, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.rowoff.get<long long>(), nV,
                                                     S.pscratch.get<int>(), S.cols.get<int>()); ++S.nlaunch;
@@ -1843,13 +1854,7 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     S.nlaunch += retri;
     k_sym_add_f64<<<S.nSM * 16, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.cols.get<int>(), retri ? S.tpos.get<int>() : nullptr, fa.m.valsN, fa.valsNlo, fa.valslo, fa.vexp, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.nV, S.vals.get<double>()); ++S.nlaunch;
     CK(cudaGetLastError());
-    if (S.replay) return NLFEM_OK;   // the flag is checked after the replay
-    int ovf = 0;
-    r = d2h(S, &ovf, S.err.get<int>() + 5, 1);
-    if (r) return r;
-    if (!ovf) return NLFEM_OK;
-    if (!S.onesided64) return F64_REFUSED;
-    return fail(NLFEM_ERR_NUMERIC, "contribution outside the fixed-point range (non-finite value?)");
+    return NLFEM_OK;   // the range flag (err[5]) is read with the number of entries (run_finish)
 }
 
 // Vector-valued kernels: one thread per ordered pair, FP64 blocks, 128-bit fixed-point sums in the
@@ -1978,8 +1983,13 @@ static int run_finish(Session &S) {
     k_finish_count<<<grid_for(nV * 32, 256), 256, 0, S.st>>>(S.rowptr.get<long long>(), nV, S.vals.get<double>(), fa, S.keepcnt.get<int>()); ++S.nlaunch;
     int r = scan_excl<int>(S, S.keepcnt.get<int>(), nV, S.fptr.get<long long>());
     if (r) return r;
-    r = d2h(S, &S.nnz, S.fptr.get<long long>() + nV, 1);
+    int ovf = 0;   // a contribution outside the fixed-point range (the mixed passes have read theirs)
+    r = d2h2(S, &S.nnz, S.fptr.get<long long>() + nV, 1, &ovf, S.err.get<int>() + 5, 1);
     if (r) return r;
+    if (S.f64 && ovf) {
+        if (!S.onesided64) return F64_REFUSED;
+        return fail(NLFEM_ERR_NUMERIC, "contribution outside the fixed-point range (non-finite value?)");
+    }
     ENS(S.fcols, sizeof(int) * (S.nnz + 1));
     ENS(S.fvals, sizeof(double) * (S.nnz + 1));
     k_finish_compact<<<grid_for(nV * 32, 256), 256, 0, S.st>>>(S.rowptr.get<long long>(), nV, S.cols.get<int>(), S.vals.get<double>(), fa, S.fptr.get<long long>(), S.fcols.get<int>(), S.fvals.get<double>()); ++S.nlaunch;
@@ -1987,10 +1997,13 @@ static int run_finish(Session &S) {
     return NLFEM_OK;
 }
 
+static int flag_errors(const int *he);
 static int check_errors(Session &S) {
     int he[8];
     int r = d2h(S, he, S.err.get<int>(), 8);
-    if (r) return r;
+    return r ? r : flag_errors(he);
+}
+static int flag_errors(const int *he) {
     if (he[3]) return fail(NLFEM_ERR_CUDA, "internal: CSR slot not found during scatter");
     if (he[4]) return fail(NLFEM_ERR_NUMERIC, "in solve2x2. Matrix not invertible.");
     if (he[7]) return fail(NLFEM_ERR_NUMERIC, "kernel evaluated outside its domain (labeled: |x - y| >= delta, or 10 labelx + labely in 14..20)");
@@ -2027,18 +2040,17 @@ static int run_system_body(Session &S) {
 // After the sequence: errors, timings (CUDA events on the assembly stream) and counters.
 static int run_system_post(Session &S) {
     int r;
-    CK(cudaStreamSynchronize(S.st));
-    if ((r = check_errors(S))) return r;
+    int he[8];
+    unsigned long long cnt[16];
+    if ((r = d2h2(S, he, S.err.get<int>(), 8, cnt, S.counters.get<unsigned long long>(), 16))) return r;
+    if ((r = flag_errors(he))) return r;
     float t[4];
     for (int i = 0; i < 4; i++) CK(cudaEventElapsedTime(&t[i], S.ev[i], S.ev[i + 1]));
-    unsigned long long ncl[7] = {0, 0, 0, 0, 0, 0, 0};
-    if ((r = d2h(S, ncl, S.counters.get<unsigned long long>() + 4, 4))) return r;
-    if ((r = d2h(S, &ncl[4], S.counters.get<unsigned long long>() + 1, 1))) return r;
-    if ((r = d2h(S, &ncl[5], S.counters.get<unsigned long long>() + 12, 2))) return r;
-    S.stats.n_items_in = (long)ncl[5];
-    S.stats.n_items_cut = (long)ncl[6];
+    const unsigned long long *ncl = cnt + 4;
+    S.stats.n_items_in = (long)cnt[12];
+    S.stats.n_items_cut = (long)cnt[13];
     S.stats.slot_map = (S.pmode == PM_RETRI || S.pmode == PM_BARY) ? (S.use_rank ? 1 : 2) : 0;
-    S.stats.n_candidates = (long)ncl[4];
+    S.stats.n_candidates = (long)cnt[1];
     S.stats.n_close = (long)ncl[0];
     S.stats.n_subtri = (long)ncl[1];
     S.stats.n_ambiguous = (long)(ncl[2] + ncl[3]);
@@ -2137,7 +2149,6 @@ static int run_forcing_t(Session &S) {
     ++S.nlaunch;
     k_forcing_finish<<<grid_for(K, 256), 256, 0, S.st>>>(S.facc.get<unsigned long long>(), K, S.od, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.fd.get<double>()); ++S.nlaunch;
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(S.st));
     return NLFEM_OK;
 }
 
@@ -2220,10 +2231,9 @@ static void host_release_free() {
 
 static int download32(Session &S, int i, nlfem_csr32 *out) {
     const long long r0 = (long long)S.od * S.voff[i], nrows = (long long)S.od * (S.voff[i + 1] - S.voff[i]);
-    long long b[2];
-    int r = d2h(S, &b[0], S.fptr.get<long long>() + r0, 1);
-    if (r) return r;
-    r = d2h(S, &b[1], S.fptr.get<long long>() + r0 + nrows, 1);
+    long long b[2] = {0, S.nnz};
+    int r = NLFEM_OK;
+    if (S.nProb > 1) r = d2h2(S, &b[0], S.fptr.get<long long>() + r0, 1, &b[1], S.fptr.get<long long>() + r0 + nrows, 1);
     if (r) return r;
     const long long nnz = b[1] - b[0];
     if (nnz > 0x7fffffffLL || nrows > 0x7fffffffLL)
@@ -2254,10 +2264,9 @@ static int download32(Session &S, int i, nlfem_csr32 *out) {
 
 static int download(Session &S, int i, nlfem_csr *out) {
     const long long r0 = (long long)S.od * S.voff[i], nrows = (long long)S.od * (S.voff[i + 1] - S.voff[i]);
-    long long b[2];
-    int r = d2h(S, &b[0], S.fptr.get<long long>() + r0, 1);
-    if (r) return r;
-    r = d2h(S, &b[1], S.fptr.get<long long>() + r0 + nrows, 1);
+    long long b[2] = {0, S.nnz};
+    int r = NLFEM_OK;
+    if (S.nProb > 1) r = d2h2(S, &b[0], S.fptr.get<long long>() + r0, 1, &b[1], S.fptr.get<long long>() + r0 + nrows, 1);
     if (r) return r;
     const long long nnz = b[1] - b[0];
     ENS(S.out64a, sizeof(long long) * (nrows + 1));
@@ -2307,9 +2316,10 @@ struct nlfem_session {
     std::vector<nlfem_problem> probs;
 };
 
-// Device buffers of the last one-shot assembly (nlfem_stiffness_matrix / _batch), kept for the
-// next one on the same device so repeated calls do not allocate: buffers only grow, and every
-// stage initialises what it reads. nlfem_cache_release frees them.
+// Device buffers, stream and events of the last one-shot call (nlfem_stiffness_matrix / _batch,
+// nlfem_load_vector), kept for the next one on the same device so repeated calls neither allocate nor
+// create: buffers only grow, and every stage initialises what it reads. One set is kept; a call that
+// overlaps another makes its own and frees it. nlfem_cache_release frees the kept one.
 namespace nlg {
 static std::mutex g_cache_mu;
 static Session *g_cache = nullptr;
@@ -2322,6 +2332,9 @@ static void cache_take(Session &S) {
     if (!g_cache || g_cache_dev != dev) return;
     std::vector<DevBuf *> from = g_cache->buffers(), to = S.buffers();
     for (size_t i = 0; i < to.size(); i++) std::swap(*to[i], *from[i]);
+    std::swap(S.st, g_cache->st);
+    std::swap(S.ev, g_cache->ev);
+    std::swap(S.stamp_layout, g_cache->stamp_layout);   // the search's stamps stay valid (see run_bfs)
     S.hint_pat_cap = g_cache->hint_pat_cap;
     S.hint_po_cap = g_cache->hint_po_cap;
     S.hint_vp_cap = g_cache->hint_vp_cap;
@@ -2340,11 +2353,15 @@ static void cache_give(Session &S) {
     g_cache_dev = dev;
     std::vector<DevBuf *> from = S.buffers(), to = g_cache->buffers();
     for (size_t i = 0; i < to.size(); i++) std::swap(*to[i], *from[i]);
-    g_cache->hint_pat_cap = S.pat_cap;
-    g_cache->hint_po_cap = S.po_cap;
-    g_cache->hint_vp_cap = S.vp_cap;
-    g_cache->hint_nE = S.nE;
-    g_cache->hint_nV = S.nV;
+    std::swap(S.st, g_cache->st);
+    std::swap(S.ev, g_cache->ev);
+    std::swap(S.stamp_layout, g_cache->stamp_layout);
+    // a load vector has no pattern: the last matrix's sizes stay
+    g_cache->hint_pat_cap = S.system ? S.pat_cap : S.hint_pat_cap;
+    g_cache->hint_po_cap = S.system ? S.po_cap : S.hint_po_cap;
+    g_cache->hint_vp_cap = S.system ? S.vp_cap : S.hint_vp_cap;
+    g_cache->hint_nE = S.system ? S.nE : S.hint_nE;
+    g_cache->hint_nV = S.system ? S.nV : S.hint_nV;
 }
 
 // ---------------------------------------------------------------- CG solve on the assembled matrix
@@ -2774,30 +2791,31 @@ int nlfem_session_set_search_epoch(nlfem_session *s, unsigned epoch) {
 }
 
 // One-shot session on the cached buffers of the previous one-shot call.
-static int session_create_cached(const nlfem_problem *probs, int n, nlfem_session **out) {
-    if (!probs || n <= 0 || !out) return fail(NLFEM_ERR_INVALID, "no problems");
-    nlfem_session *s = new nlfem_session();
-    cache_take(s->S);
-    s->probs.assign(probs, probs + n);
-    int r = session_init(s->S, probs, n, true);
-    if (!r) r = session_upload(s->S, probs);
-    if (r) { cache_give(s->S); delete s; return r; }
-    *out = s;
-    return NLFEM_OK;
-}
-
 static void session_destroy_cached(nlfem_session *s) {
     if (!s) return;
-    cudaStreamSynchronize(s->S.st);
+    if (s->S.st) cudaStreamSynchronize(s->S.st);
     cudaGetLastError();
     cache_give(s->S);
     delete s;
 }
 
+static int session_create_cached(const nlfem_problem *probs, int n, bool system, nlfem_session **out) {
+    if (!probs || n <= 0 || !out) return fail(NLFEM_ERR_INVALID, "no problems");
+    nlfem_session *s = new nlfem_session();
+    s->S.system = system;
+    cache_take(s->S);
+    s->probs.assign(probs, probs + n);
+    int r = session_init(s->S, probs, n, system);
+    if (!r) r = session_upload(s->S, probs);
+    if (r) { session_destroy_cached(s); return r; }
+    *out = s;
+    return NLFEM_OK;
+}
+
 int nlfem_stiffness_batch(const nlfem_problem *probs, int n, nlfem_csr *outs) {
     if (!outs) return fail(NLFEM_ERR_INVALID, "null output");
     nlfem_session *s = nullptr;
-    int r = session_create_cached(probs, n, &s);
+    int r = session_create_cached(probs, n, true, &s);
     if (r) return r;
     r = run_system(s->S);
     for (int i = 0; !r && i < n; i++) r = download(s->S, i, &outs[i]);
@@ -2808,7 +2826,7 @@ int nlfem_stiffness_batch(const nlfem_problem *probs, int n, nlfem_csr *outs) {
 int nlfem_stiffness_batch32(const nlfem_problem *probs, int n, nlfem_csr32 *outs) {
     if (!outs) return fail(NLFEM_ERR_INVALID, "null output");
     nlfem_session *s = nullptr;
-    int r = session_create_cached(probs, n, &s);
+    int r = session_create_cached(probs, n, true, &s);
     if (r) return r;
     r = run_system(s->S);
     for (int i = 0; !r && i < n; i++) r = download32(s->S, i, &outs[i]);
@@ -2837,11 +2855,13 @@ int nlfem_stiffness_matrix(const nlfem_problem *prob, nlfem_csr *out) {
 
 int nlfem_load_vector(const nlfem_problem *prob, double *fd) {
     if (!prob || !fd) return fail(NLFEM_ERR_INVALID, "null argument");
-    Session S;
-    int r = session_init(S, prob, 1, false);
-    if (!r) r = session_upload(S, prob);
-    if (!r) r = (S.dim == 2) ? run_forcing_t<2>(S) : run_forcing_t<3>(S);
+    nlfem_session *s = nullptr;
+    int r = session_create_cached(prob, 1, false, &s);
+    if (r) return r;
+    Session &S = s->S;
+    r = (S.dim == 2) ? run_forcing_t<2>(S) : run_forcing_t<3>(S);
     if (!r) r = d2h(S, fd, S.fd.get<double>(), (size_t)S.od * S.nV);
+    session_destroy_cached(s);
     return r;
 }
 
