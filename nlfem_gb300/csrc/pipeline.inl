@@ -187,6 +187,56 @@ static long zeta_common(const long *idx, const long *ptr, long a, long b) {
     return n;
 }
 
+// One walk over a problem's elements: squared edge lengths, |det| (sum, least, largest), and whether
+// every element is clear of degenerate (where the reference's solve2x2 may abort, 2D). known: every
+// vertex index is in range.
+struct MeshScan {
+    double hmin2 = 1e300, hmax2 = 0, atot = 0, amin = 1e300, amax = 0;
+    bool sound = true, known = true;
+};
+template <int DIM>
+static MeshScan scan_mesh(const nlfem_problem &p) {
+    MeshScan m;
+    constexpr int dV = DIM + 1;
+    for (long e = 0; e < p.nE; e++) {
+        const long *t = &p.elements[dV * e];
+        double X[dV][DIM];
+        bool ok = true;
+        for (int a = 0; a < dV; a++) ok = ok && t[a] >= 0 && t[a] < p.nV;
+        if (!ok) {   // rejected by the mesh checks
+            m.known = false;
+            continue;
+        }
+        for (int a = 0; a < dV; a++)
+            for (int j = 0; j < DIM; j++) X[a][j] = p.vertices[DIM * t[a] + j];
+        double lo = 1e300, hi = 0;
+        for (int a = 0; a < dV; a++)
+            for (int b = a + 1; b < dV; b++) {
+                double d2 = 0;
+                for (int j = 0; j < DIM; j++) d2 += (X[a][j] - X[b][j]) * (X[a][j] - X[b][j]);
+                lo = d2 < lo ? d2 : lo;
+                hi = d2 > hi ? d2 : hi;
+            }
+        m.hmin2 = lo < m.hmin2 ? lo : m.hmin2;
+        m.hmax2 = hi > m.hmax2 ? hi : m.hmax2;
+        double E[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, det;
+        for (int c = 0; c < DIM; c++)
+            for (int j = 0; j < DIM; j++) E[c][j] = X[c + 1][j] - X[0][j];
+        if (DIM == 2) {
+            det = fabs(E[0][0] * E[1][1] - E[1][0] * E[0][1]);
+            const double l0 = fabs(E[0][0]) + fabs(E[0][1]), l1 = fabs(E[1][0]) + fabs(E[1][1]);
+            m.sound = m.sound && det > 1e-10 * l0 * l1 && (fabs(E[0][0]) > 1e-14 || fabs(E[0][1]) > 1e-14);
+        } else {
+            det = fabs(E[0][0] * (E[1][1] * E[2][2] - E[1][2] * E[2][1]) - E[0][1] * (E[1][0] * E[2][2] - E[1][2] * E[2][0]) +
+                       E[0][2] * (E[1][0] * E[2][1] - E[1][1] * E[2][0]));
+        }
+        m.atot += det;
+        m.amin = det < m.amin ? det : m.amin;
+        m.amax = det > m.amax ? det : m.amax;
+    }
+    return m;
+}
+
 // Whether a one-sided FP64 pass takes the problem (passes_f64.cuh, the 2D retriangulate rule;
 // passes_f64_bary.cuh, the barycenter rule with a constant kernel), and the bounds its units follow
 // from. A pair's blocks are at most kbound |T| |b| times the rules' absolute sums (CN, CD: basis
@@ -196,35 +246,15 @@ static long zeta_common(const long *idx, const long *ptr, long a, long b) {
 // solve2x2 may abort; the barycenter rule never calls it), bounds far outside the exponent range
 // and options that need the general pass go there. fp64-onesided, which has no such pass to match,
 // is bound only by the range.
-static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, double kbound) {
+static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, const MeshScan &m, double kbound) {
     P.f64ok = 0;
-    if (!P.cert || p.outdim != 1 || p.is_dg) return;
+    if (!P.cert || !m.known || p.outdim != 1 || p.is_dg) return;
+    if (p.nPx <= 0 || p.nPx > MAXQ || p.nPy <= 0 || p.nPy > MAXQ || !p.Px || !p.dx || !p.Py || !p.dy) return;   // make_rule reports it
     const bool bary = P.remote == MTH_BARYCENTER;
     if (bary ? P.kernel != KER_CONSTANT && P.kernel != KER_CONSTANT3D
              : p.dim != 2 || (P.kernel != KER_CONSTANT && P.kernel != KER_PARABOLA && P.kernel != KER_FRACTIONAL)) return;
     const int dim = p.dim, dV = dim + 1;
-    double atot = 0, amin = 1e300, amax = 0;
-    bool sound = true;
-    for (long e = 0; e < p.nE; e++) {
-        const long *t = &p.elements[dV * e];
-        for (int a = 0; a < dV; a++)
-            if (t[a] < 0 || t[a] >= p.nV) return;
-        double m[3][3];
-        for (int c = 1; c < dV; c++)
-            for (int j = 0; j < dim; j++) m[c - 1][j] = p.vertices[dim * t[c] + j] - p.vertices[dim * t[0] + j];
-        double det;
-        if (dim == 2) {
-            det = fabs(m[0][0] * m[1][1] - m[1][0] * m[0][1]);
-            const double l0 = fabs(m[0][0]) + fabs(m[0][1]), l1 = fabs(m[1][0]) + fabs(m[1][1]);
-            sound = sound && det > 1e-10 * l0 * l1 && std::max(fabs(m[0][0]), fabs(m[0][1])) > 1e-14;
-        } else {
-            det = fabs(m[0][0] * (m[1][1] * m[2][2] - m[1][2] * m[2][1]) - m[0][1] * (m[1][0] * m[2][2] - m[1][2] * m[2][0]) +
-                       m[0][2] * (m[1][0] * m[2][1] - m[1][1] * m[2][0]));
-        }
-        atot += det;
-        amin = std::min(amin, det);
-        amax = std::max(amax, det);
-    }
+    const double atot = m.atot;
     double cx = 1, cy = 1, sx = 0, sy = 0, px[4] = {0, 0, 0, 0};
     for (int q = 0; q < 2; q++) {   // the outer rule, then the inner rule
         const int n = q ? p.nPy : p.nPx;
@@ -245,12 +275,12 @@ static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, double kbound)
     if (P.kernel == KER_PARABOLA) kbound *= cy * cy;   // inner points outside the polygon
     if (P.singular) kbound *= 1048576.0;
     const double CN = kbound * *std::max_element(px, px + 4) * sy * cy, CD = 2 * kbound * sx * cx * cx * sy * cy * cy * atot;
-    if (!(CN > 1e-120 && CN < 1e120 && CD > 1e-120 && CD < 1e120 && sx > 1e-30 && atot > 1e-60 && atot < 1e60 && amax < 1e60)) return;
+    if (!(CN > 1e-120 && CN < 1e120 && CD > 1e-120 && CD < 1e120 && sx > 1e-30 && atot > 1e-60 && atot < 1e60 && m.amax < 1e60)) return;
     P.xN = (int)ceil(8.0 * log2(CN) + 1e-3);
     P.xD = exact_ceil_log2(CD);
     P.xS = exact_ceil_log2(sx * atot);
     if (p.precision == NLFEM_PREC_FP64)
-        P.f64ok = sound && amin > (bary ? -1.0 : 1e-60) && !P.full_search && !P.zeta && (!P.singular || duffy_close(P));
+        P.f64ok = m.sound && m.amin > (bary ? -1.0 : 1e-60) && !P.full_search && !P.zeta && (!P.singular || duffy_close(P));
     else
         P.f64ok = 1;
 }
@@ -400,24 +430,11 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     // size relative to the ball: the vertex tests stay inside their margin while every element
     // diameter is at most MIX_MAX_H_OVER_DELTA times delta. The mixed path refuses larger elements,
     // the FP64 paths take their FP64 routines for them.
-    double hmax2 = 0, hmin2 = 1e300;
+    MeshScan scan;
     if (system) {
-        const int dV = p.dim + 1;
-        for (long e = 0; e < p.nE; e++)
-            for (int a = 0; a < dV; a++)
-                for (int b = a + 1; b < dV; b++) {
-                    const long va = p.elements[e * dV + a], vb = p.elements[e * dV + b];
-                    if (va < 0 || vb < 0 || va >= p.nV || vb >= p.nV) continue;   // rejected by the mesh checks
-                    double d2 = 0;
-                    for (int j = 0; j < p.dim; j++) {
-                        const double d = p.vertices[va * p.dim + j] - p.vertices[vb * p.dim + j];
-                        d2 += d * d;
-                    }
-                    hmax2 = std::max(hmax2, d2);
-                    hmin2 = std::min(hmin2, d2);
-                }
+        scan = p.dim == 2 ? scan_mesh<2>(p) : scan_mesh<3>(p);
         const double lim = p.precision == NLFEM_PREC_MIXED ? MIX_MAX_H_OVER_DELTA : 512.0;
-        if (p.precision != NLFEM_PREC_FP64 && hmax2 > lim * lim * p.sqdelta)
+        if (p.precision != NLFEM_PREC_FP64 && scan.hmax2 > lim * lim * p.sqdelta)
             return fail(NLFEM_ERR_UNSUPPORTED, std::string("precision \"") + (p.precision == NLFEM_PREC_MIXED ? "mixed" : "fp64-onesided") +
                         "\" needs elements no larger than " + std::to_string((int)lim) +
                         " times the horizon (the margins of its geometry tests); precision \"fp64\" has no such bound");
@@ -428,8 +445,8 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
         // rounding is 2^-48 of the coordinate). The FP64 paths check both.
         double cmax = 0;
         for (int j = 0; j < p.dim; j++) cmax = std::max(cmax, std::max(fabs(lo[j]), fabs(hi[j])));
-        P.cert = finite == 0 && hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
-                 p.sqdelta < 1e14 && std::min(hmin2, p.sqdelta) > 1e-24 && hmin2 * p.sqdelta > 1e-28;
+        P.cert = finite == 0 && scan.hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
+                 p.sqdelta < 1e14 && std::min(scan.hmin2, p.sqdelta) > 1e-24 && scan.hmin2 * p.sqdelta > 1e-28;
     }
     double mag, kbound = 0;   // kbound: bound of |kernel| inside the ball (estimate for singular kernels)
     if (system) {
@@ -449,7 +466,7 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     }
     if (!(mag > 0) || !std::isfinite(mag)) mag = 1.0;
     P.scale_exp = exact_ceil_log2(mag);
-    if (system && p.precision != NLFEM_PREC_MIXED) set_f64_bounds(p, P, kbound);
+    if (system && p.precision != NLFEM_PREC_MIXED) set_f64_bounds(p, P, scan, kbound);
     return set_fx_unit(P, 0);
 }
 
