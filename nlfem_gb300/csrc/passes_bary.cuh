@@ -32,20 +32,24 @@ struct BaryWarp {
     int rlo[DIM + 1];                   // T's rows: first window word (window-rank map)
     int tvs[DIM + 1];                   // T's vertices
 };
-template <int DIM>
-struct BaryEntry {   // one partner vertex of a batch and its integer sums over T's rows
-    int col, pad;
-    long long v[DIM + 1];
+struct BaryGroup {   // lanes of a batch whose partners share a vertex (as local vertex c)
+    int col, c;
+    unsigned lanes;
 };
+// integers of a lane's pair, padded to an odd count so that the lanes' words fall in different banks
+__host__ __device__ constexpr int bary_vals(int dim) { return (dim + 1) * (dim + 1) + (dim == 3); }
 template <int DIM>
 __host__ __device__ constexpr size_t bary_res_bytes(int nPx) {
-    return (size_t)32 * nPx * (DIM + 2) * 4 > (size_t)32 * (DIM + 1) * sizeof(BaryEntry<DIM>)
+    return (size_t)32 * nPx * (DIM + 2) * 4 > 32 * (bary_vals(DIM) * 8 + (DIM + 1) * sizeof(BaryGroup))
                ? (size_t)32 * nPx * (DIM + 2) * 4
-               : (size_t)32 * (DIM + 1) * sizeof(BaryEntry<DIM>);
+               : 32 * (bary_vals(DIM) * 8 + (DIM + 1) * sizeof(BaryGroup));
 }
+// outer rule coefficients per point, read at lane-dependent points: dx psi_r, then dx psi_r psi_c (r < c)
+template <int DIM>
+__host__ __device__ constexpr int bary_coef() { return DIM == 2 ? 8 : 12; }
 template <int DIM>
 __host__ __device__ constexpr size_t bary_warp_bytes(int nPx) {
-    // BaryWarp + item results [32][nPx][DIM+2] (or the scatter list) + inside list [32*nPx] shorts
+    // BaryWarp + item results [32][nPx][DIM+2] (or the scatter values and groups) + inside list [32*nPx] shorts
     return ((sizeof(BaryWarp<DIM>) + 15) / 16) * 16 + bary_res_bytes<DIM>(nPx) + (size_t)32 * nPx * 2 + 16;
 }
 
@@ -59,9 +63,13 @@ __device__ __forceinline__ float kernel_f32_r2(const ProbParams &P, float r2) {
 }
 
 // CK: the launch covers constant-kernel problems only; an item's sums over the full inner element
-// are then kc |b| times the rule's precomputed element sums.
+// are then kc |b| times the rule's precomputed element sums. The sums over a pair's inside points read
+// the outer rule at points that differ from lane to lane: from shared memory (the constant cache
+// serves one address at a time). Five blocks
+// per SM at 96 registers: 4 and 6 were 1.1 and 0.4 ms slower at 6 * 32^3 tetrahedra, 1.26e8 pairs, where
+// the pass takes 10.2 ms (15.7 with the constant cache and group sums by shuffles).
 template <int DIM, bool CK>
-__global__ void __launch_bounds__(BARY_THREADS) k_pass_bary(MixArgs ma, Rule rule, PassRule pr) {
+__global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs ma, Rule rule, PassRule pr) {
     constexpr int dV = DIM + 1, NS = dV * (dV + 1) / 2, RN = DIM + 2;
     extern __shared__ __align__(16) unsigned char s_raw[];
     const PassArgs &a = ma.p;
@@ -72,7 +80,22 @@ __global__ void __launch_bounds__(BARY_THREADS) k_pass_bary(MixArgs ma, Rule rul
     BaryWarp<DIM> &W = *reinterpret_cast<BaryWarp<DIM> *>(wbase);
     float *res = reinterpret_cast<float *>(wbase + ((sizeof(BaryWarp<DIM>) + 15) / 16) * 16);   // [32][nPx][RN]
     unsigned short *lst = reinterpret_cast<unsigned short *>(reinterpret_cast<unsigned char *>(res) + bary_res_bytes<DIM>(nPx));
-    BaryEntry<DIM> *slist = reinterpret_cast<BaryEntry<DIM> *>(res);
+    constexpr int VS = bary_vals(DIM);
+    long long *sval = reinterpret_cast<long long *>(res);                  // [32][VS], after the fold
+    BaryGroup *slist = reinterpret_cast<BaryGroup *>(sval + 32 * VS);
+    constexpr int NO = NS - dV, CS = bary_coef<DIM>();
+    __shared__ __align__(16) float s_coef[CK ? MAXQ * CS : 4];
+    if (CK) {
+        for (int k = threadIdx.x; k < nPx; k += BARY_THREADS) {
+            int t = dV;
+            for (int r = 0; r < dV; r++) {
+                s_coef[CS * k + r] = pr.cx[dV * k + r];
+                for (int c = r + 1; c < dV; c++) s_coef[CS * k + t++] = pr.cxx[NS * k + sym_idx<dV>(r, c)];
+            }
+            for (; t < CS; t++) s_coef[CS * k + t] = 0.f;
+        }
+        __syncthreads();
+    }
     long long *vals = reinterpret_cast<long long *>(a.vals);
     int *ovf = &a.err[5];
     bool bad = false;   // a contribution outside the fixed-point range (reported at the end)
@@ -228,31 +251,38 @@ __global__ void __launch_bounds__(BARY_THREADS) k_pass_bary(MixArgs ma, Rule rul
 #pragma unroll
                 for (int i = 0; i < dV * dV; i++) N[i] = 0.f;
                 if (CK) {   // every item's sums are inv: the folds are inv times the mask's rule sums
-                    float sx[NS], cxs[dV];
+                    float m[dV + NO];   // dx psi_r, then off-diagonal dx psi_r psi_c
                     if (inm == (nPx == 32 ? 0xffffffffu : (1u << nPx) - 1u)) {
+                        int t = dV;
 #pragma unroll
-                        for (int i = 0; i < NS; i++) sx[i] = pr.xsum[i];
+                        for (int r = 0; r < dV; r++) {
+                            m[r] = pr.xsum[NS + r];
 #pragma unroll
-                        for (int r = 0; r < dV; r++) cxs[r] = pr.xsum[NS + r];
+                            for (int c = r + 1; c < dV; c++) m[t++] = pr.xsum[sym_idx<dV>(r, c)];
+                        }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < NS; i++) sx[i] = 0.f;
-#pragma unroll
-                        for (int r = 0; r < dV; r++) cxs[r] = 0.f;
+                        for (int q = 0; q < dV + NO; q++) m[q] = 0.f;
                         for (unsigned mm = inm; mm; mm &= mm - 1) {
-                            const int k = __ffs(mm) - 1;
+                            const float4 *cf = reinterpret_cast<const float4 *>(&s_coef[CS * (__ffs(mm) - 1)]);
+                            float v[CS];
 #pragma unroll
-                            for (int i = 0; i < NS; i++) sx[i] += pr.cxx[NS * k + i];
+                            for (int q = 0; q < CS / 4; q++) {
+                                const float4 f = cf[q];
+                                v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
+                            }
 #pragma unroll
-                            for (int r = 0; r < dV; r++) cxs[r] += pr.cx[dV * k + r];
+                            for (int q = 0; q < dV + NO; q++) m[q] += v[q];
                         }
                     }
+                    int t = dV;
 #pragma unroll
-                    for (int i = 0; i < NS; i++) L[i] = sx[i] * inv[0];
+                    for (int r = 0; r < dV; r++) {
 #pragma unroll
-                    for (int r = 0; r < dV; r++)
+                        for (int c = r + 1; c < dV; c++) L[sym_idx<dV>(r, c)] = m[t++] * inv[0];
 #pragma unroll
-                        for (int t = 0; t < dV; t++) N[dV * r + t] = cxs[r] * inv[1 + t];
+                        for (int c = 0; c < dV; c++) N[dV * r + c] = m[r] * inv[1 + c];
+                    }
                 }
                 for (int k = 0; k < (CK ? 0 : nPx); k++) {
                     const float *rr = &res[(lane * nPx + k) * RN];
@@ -278,47 +308,27 @@ __global__ void __launch_bounds__(BARY_THREADS) k_pass_bary(MixArgs ma, Rule rul
 #pragma unroll
                 for (int i = 0; i < dV * dV; i++) nx[i] = fx64(2.f * N[i] * rTT, P.fx_mul, bad);
             }
-            // termNonloc into A[T, b] (minus sign): group sums per partner vertex, shared lookups
+            // termNonloc into A[T, b] (minus sign): the lanes' integers go to shared memory; per local
+            // vertex, lanes sharing a partner vertex form a group, and all lanes share the work of the
+            // (group, row) sums, slot lookups and reductions. (Summing the groups by shuffles runs the
+            // longest group's chain, up to 24 tetrahedra at a vertex, on all lanes: 13.4 against 10.2 ms
+            // at 6 * 32^3. The 2D passes keep the shuffles: with 6 triangles at a vertex the two are equal
+            // for constant kernels and shuffles 2 to 5% better for the others.)
             __syncwarp();
+#pragma unroll
+            for (int i = 0; i < dV * dV; i++) sval[lane * VS + i] = nx[i];
             int nent = 0;
-#pragma unroll 1
+#pragma unroll
             for (int c = 0; c < dV; c++) {
-                int col = -1;
-                if (act) {
-#pragma unroll
-                    for (int t = 0; t < dV; t++)
-                        if (t == c) col = a.T32[(long long)part * dV + t];
-                }
+                const int col = act ? a.T32[(long long)part * dV + c] : -1;
                 const unsigned grp = __match_any_sync(FULL, col);
-                const bool leader = (__ffs(grp) - 1) == lane;
-                const int maxn = __reduce_max_sync(FULL, (unsigned)__popc(grp));
-                long long own[dV], sn[dV];
-#pragma unroll
-                for (int r = 0; r < dV; r++) {
-                    long long v = 0;
-#pragma unroll
-                    for (int t = 0; t < dV; t++)
-                        if (t == c) v = nx[dV * r + t];
-                    own[r] = sn[r] = v;
-                }
-                unsigned rest = grp & ~(1u << lane);
-                for (int it = 1; it < maxn; it++) {
-                    const int src = rest ? __ffs(rest) - 1 : lane;
-                    const bool use = rest != 0;
-                    if (rest) rest &= rest - 1;
-#pragma unroll
-                    for (int r = 0; r < dV; r++) {
-                        const long long t = shfl64(own[r], src);
-                        if (use) sn[r] += t;
-                    }
-                }
-                const bool put = leader && col >= 0;
+                const bool put = (__ffs(grp) - 1) == lane && col >= 0;
                 const unsigned m = __ballot_sync(FULL, put);
                 if (put) {
-                    BaryEntry<DIM> &e = slist[nent + __popc(m & lanemask_lt())];
+                    BaryGroup &e = slist[nent + __popc(m & lanemask_lt())];
                     e.col = col;
-#pragma unroll
-                    for (int r = 0; r < dV; r++) e.v[r] = sn[r];
+                    e.c = c;
+                    e.lanes = grp;
                 }
                 nent += __popc(m);
             }
@@ -327,11 +337,15 @@ __global__ void __launch_bounds__(BARY_THREADS) k_pass_bary(MixArgs ma, Rule rul
                 const int e = w / dV, r = w - dV * e;
                 RowHash h;
                 h.hb = W.rhb[r]; h.rb = W.rrb[r]; h.mask = W.rmask[r]; h.lo = W.rlo[r];
-                if (h.mask == 0xffffffffu) continue;   // T's vertex r has no row
-                if (slist[e].col == W.tvs[r]) continue;   // the matrix diagonal: from the row sum
-                const long long s = slot_find_row(sm, h, slist[e].col);
+                const int col = slist[e].col;
+                if (h.mask == 0xffffffffu || col == W.tvs[r]) continue;   // no row; the matrix diagonal: from the row sum
+                const SlotProbe pb = slot_probe_begin(sm, h, col);   // in flight while the members are summed
+                const long long *v = &sval[dV * r + slist[e].c];
+                long long sn = 0;
+                for (unsigned mm = slist[e].lanes; mm; mm &= mm - 1) sn += v[(__ffs(mm) - 1) * VS];
+                const long long s = slot_probe_end(sm, h, col, pb);
                 if (s < 0) miss = true;
-                else red_add(vals, s, -slist[e].v[r]);
+                else red_add(vals, s, -sn);
             }
             __syncwarp();
         }

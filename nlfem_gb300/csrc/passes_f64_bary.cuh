@@ -21,7 +21,8 @@ struct F64BaryWarp {
     long long rhb[DIM + 1], rrb[DIM + 1];   // T's rows (see MixWarp)
     unsigned rmask[DIM + 1];
     int rlo[DIM + 1], tvs[DIM + 1], te[DIM + 1];
-    BaryEntry<DIM> list[32 * (DIM + 1)];    // partner vertices of a batch
+    long long val[32 * bary_vals(DIM)];     // a batch's integers, and the groups of its partner vertices
+    BaryGroup list[32 * (DIM + 1)];         // (see k_pass_bary)
 };
 // outer sums per mask: psi_r, then psi_r psi_c off the diagonal; an odd stride keeps the banks apart
 template <int DIM>
@@ -33,7 +34,7 @@ __host__ __device__ constexpr size_t f64_bary_smem(int nPx) {
 
 template <int DIM>
 __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Rule rule, PassRuleT<double> pr) {
-    constexpr int dV = DIM + 1, NO = dV * (dV - 1) / 2, TS = f64_bary_tab<DIM>();
+    constexpr int dV = DIM + 1, NO = dV * (dV - 1) / 2, TS = f64_bary_tab<DIM>(), VS = bary_vals(DIM);
     extern __shared__ __align__(16) unsigned char s_raw[];
     const PassArgs &a = fa.m.p;
     const SlotMap &sm = fa.m.m;
@@ -148,46 +149,21 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
 #pragma unroll
                 for (int q = 0; q < NO; q++) D[q] += m[dV + q] * kl;
             }
-            // termNonloc into T's rows: group sums per partner vertex, shared lookups
+            // termNonloc into T's rows: sums per partner vertex and lookups shared by the lanes
+#pragma unroll
+            for (int i = 0; i < dV * dV; i++) W.val[lane * VS + i] = nx[i];
             int nent = 0;
-#pragma unroll 1
+#pragma unroll
             for (int c = 0; c < dV; c++) {
-                int col = -1;
-                if (act) {
-#pragma unroll
-                    for (int t = 0; t < dV; t++)
-                        if (t == c) col = pv[t];
-                }
+                const int col = act ? pv[c] : -1;
                 const unsigned grp = __match_any_sync(FULL, col);
-                const bool leader = (__ffs(grp) - 1) == lane;
-                const int maxn = __reduce_max_sync(FULL, (unsigned)__popc(grp));
-                long long own[dV], sn[dV];
-#pragma unroll
-                for (int r = 0; r < dV; r++) {
-                    long long v = 0;
-#pragma unroll
-                    for (int t = 0; t < dV; t++)
-                        if (t == c) v = nx[dV * r + t];
-                    own[r] = sn[r] = v;
-                }
-                unsigned rest = grp & ~(1u << lane);
-                for (int it = 1; it < maxn; it++) {
-                    const int src = rest ? __ffs(rest) - 1 : lane;
-                    const bool use = rest != 0;
-                    if (rest) rest &= rest - 1;
-#pragma unroll
-                    for (int r = 0; r < dV; r++) {
-                        const long long t = shfl64(own[r], src);
-                        if (use) sn[r] += t;
-                    }
-                }
-                const bool put = leader && col >= 0;
+                const bool put = (__ffs(grp) - 1) == lane && col >= 0;
                 const unsigned m = __ballot_sync(FULL, put);
                 if (put) {
-                    BaryEntry<DIM> &e = W.list[nent + __popc(m & lanemask_lt())];
+                    BaryGroup &e = W.list[nent + __popc(m & lanemask_lt())];
                     e.col = col;
-#pragma unroll
-                    for (int r = 0; r < dV; r++) e.v[r] = sn[r];
+                    e.c = c;
+                    e.lanes = grp;
                 }
                 nent += __popc(m);
             }
@@ -196,11 +172,15 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                 const int e = w / dV, r = w - dV * e;
                 RowHash h;
                 h.hb = W.rhb[r]; h.rb = W.rrb[r]; h.mask = W.rmask[r]; h.lo = W.rlo[r];
-                if (h.mask == 0xffffffffu) continue;   // T's vertex r has no row
-                if (W.list[e].col == W.tvs[r]) continue;   // the matrix diagonal: from the row sum
-                const long long s = slot_find_row(sm, h, W.list[e].col);
+                const int col = W.list[e].col;
+                if (h.mask == 0xffffffffu || col == W.tvs[r]) continue;   // no row; the matrix diagonal: from the row sum
+                const SlotProbe pb = slot_probe_begin(sm, h, col);
+                const long long *v = &W.val[dV * r + W.list[e].c];
+                long long sn = 0;
+                for (unsigned mm = W.list[e].lanes; mm; mm &= mm - 1) sn += v[(__ffs(mm) - 1) * VS];
+                const long long s = slot_probe_end(sm, h, col, pb);
                 if (s < 0) miss = true;
-                else red_add(fa.m.valsN, s, W.list[e].v[r]);
+                else red_add(fa.m.valsN, s, sn);
             }
             __syncwarp();
         }
