@@ -250,17 +250,24 @@ __device__ __forceinline__ bool interacts_exact(const ProbParams &P, int method,
 // barycenter offset bf; the exact FP64 test decides the points within the squared-distance margin.
 // oc holds the outer points' centroid and the radius ro of a sphere around it holding them all: a
 // barycenter farther than delta + ro from the centroid is outside every ball (checked with the
-// squared-distance margin, ro inflated by 8u).
+// squared-distance margin, ro inflated by 8u), one nearer than delta - ro inside all of them.
+// HIT_NEAR: a pair that interacts, and every outer point's ball is certain to hold the partner (its
+// barycenter, for the barycenter rule). The radius it is judged by is at least delta / 2, where the
+// margin (relative to that radius) is still 64 u delta in length, above the 37 u delta that the
+// offsets may be off by at h = 16 delta.
+enum { HIT_NONE = 0, HIT = 1, HIT_NEAR = 2 };
+
 template <int DIM>
-__device__ __forceinline__ bool bary_filtered(const ProbParams &P, const double *xs, const float *xsf, int nPx,
+__device__ __forceinline__ int bary_filtered(const ProbParams &P, const double *xs, const float *xsf, int nPx,
                                               const double *Eb, const float *bf, const float *oc, unsigned &namb) {
     const float sqlo = P.sqdelta_f * (1.f - MARG_D), sqhi = P.sqdelta_f * (1.f + MARG_D);
     {
         float dc = 0.f;
 #pragma unroll
         for (int j = 0; j < DIM; j++) { const float d = bf[j] - oc[j]; dc = fmaf(d, d, dc); }
-        const float R = sqrtf(P.sqdelta_f) + oc[3];
-        if (dc > R * R * (1.f + MARG_D)) return false;
+        const float dl = sqrtf(P.sqdelta_f), R = dl + oc[3], r = dl - oc[3];
+        if (dc > R * R * (1.f + MARG_D)) return HIT_NONE;
+        if (r > 0.5f * dl && dc < r * r * (1.f - MARG_D)) return HIT_NEAR;
     }
     double b64[DIM];
     bool have_b64 = false;
@@ -268,25 +275,25 @@ __device__ __forceinline__ bool bary_filtered(const ProbParams &P, const double 
         float d2 = 0.f;
 #pragma unroll
         for (int j = 0; j < DIM; j++) { float d = xsf[DIM * k + j] - bf[j]; d2 = fmaf(d, d, d2); }
-        if (d2 < sqlo) return true;
+        if (d2 < sqlo) return HIT;
         if (d2 > sqhi) continue;
         namb++;
         if (!have_b64) { xbary<DIM>(Eb, b64); have_b64 = true; }
-        if (xbaryInside<DIM>(&xs[DIM * k], b64, P.sqdelta)) return true;
+        if (xbaryInside<DIM>(&xs[DIM * k], b64, P.sqdelta)) return HIT;
     }
-    return false;
+    return HIT_NONE;
 }
 
 // The same predicate with the certified FP32 geometry (certified.cuh); the exact FP64 routine
 // runs only for outer points whose FP32 decisions are within their margins.
 template <int DIM>
-__device__ __forceinline__ bool interacts_filtered(const ProbParams &P, int method, const double *xs,
+__device__ __forceinline__ int interacts_filtered(const ProbParams &P, int method, const double *xs,
                                                    const float *xsf, int nPx, const double *Eb,
-                                                   const float *pb, unsigned &namb) {
-    if (P.full_search) return true;
-    if (method == MTH_FRACTIONAL || method == MTH_WEAKSING) return true;   // close rules: every candidate
+                                                   const float *pb, const float *oc, unsigned &namb) {
+    if (P.full_search) return HIT;
+    if (method == MTH_FRACTIONAL || method == MTH_WEAKSING) return HIT;   // close rules: every candidate
     const float sqlo = P.sqdelta_f * (1.f - MARG_D), sqhi = P.sqdelta_f * (1.f + MARG_D);
-    if (DIM != 2) return false;
+    if (DIM != 2) return HIT_NONE;
     const F2 p[3] = {f2(pb[0], pb[1]), f2(pb[2], pb[3]), f2(pb[4], pb[5])};
     // First, per outer point, the disc around the triangle's centroid through its farthest vertex:
     // a ball holding that disc holds the triangle (the polygon is the triangle itself: three
@@ -296,6 +303,11 @@ __device__ __forceinline__ bool interacts_filtered(const ProbParams &P, int meth
 #pragma unroll
     for (int i = 0; i < 3; i++) { const F2 w = p[i] - cen; rb2 = fmaxf(rb2, dot(w, w)); }
     const float rb = sqrtf(rb2) * (1.f + 8.f * U32), dl = sqrtf(P.sqdelta_f);
+    {   // the disc inside every outer point's ball: judged from their centroid and enclosing radius
+        const F2 q = cen - f2(oc[0], oc[1]);
+        const float r = dl - rb - oc[3];
+        if (r > 0.5f * dl && dot(q, q) < r * r * (1.f - MARG_D)) return HIT_NEAR;
+    }
     const float din = dl - rb;
     const float sq_in = din > 0.f ? din * din * (1.f - MARG_D) : -1.f;
     const float sq_out = (dl + rb) * (dl + rb) * (1.f + MARG_D);
@@ -305,12 +317,12 @@ __device__ __forceinline__ bool interacts_filtered(const ProbParams &P, int meth
     for (int k = 0; k < nPx; k++) {
         const F2 q = cen - f2(xsf[2 * k], xsf[2 * k + 1]);
         const float dc = dot(q, q);
-        if (dc < sq_in) return true;
+        if (dc < sq_in) return HIT;
         if (dc > sq_out) continue;
         und |= 1u << k;
         if (dc < dn) { dn = dc; kn = k; }
     }
-    if (!und) return false;
+    if (!und) return HIT_NONE;
     // Then the cheap certain answer, nearest point first: one vertex strictly inside and none on
     // the sphere means both edges through it cross once, so the polygon has at least three
     // points. Only when no point gives it does any point need its polygon.
@@ -322,7 +334,7 @@ __device__ __forceinline__ bool interacts_filtered(const ProbParams &P, int meth
         const F2 Q[3] = {p[0] - x, p[1] - x, p[2] - x};
         const float d0 = dot(Q[0], Q[0]), d1 = dot(Q[1], Q[1]), d2 = dot(Q[2], Q[2]);
         const bool clear = (d0 < sqlo || d0 > sqhi) && (d1 < sqlo || d1 > sqhi) && (d2 < sqlo || d2 > sqhi);
-        if (clear && (d0 < sqlo || d1 < sqlo || d2 < sqlo)) return true;
+        if (clear && (d0 < sqlo || d1 < sqlo || d2 < sqlo)) return HIT;
         if (fclassify(Q, P.sqdelta_f) != CLS_OUT) cut |= 1u << k;
     }
     for (; cut; cut &= cut - 1) {
@@ -332,14 +344,14 @@ __device__ __forceinline__ bool interacts_filtered(const ProbParams &P, int meth
         bool amb = false;
         const int n = fretriangulate(Q, P.sqdelta_f, P.caps, nullptr, amb);   // the count only
         if (!amb) {
-            if (n >= 3) return true;
+            if (n >= 3) return HIT;
             continue;
         }
         namb++;
         double R64[18];
-        if (xretriangulate(&xs[2 * k], Eb, P.sqdelta, P.caps, R64) >= 3) return true;
+        if (xretriangulate(&xs[2 * k], Eb, P.sqdelta, P.caps, R64) >= 3) return HIT;
     }
-    return false;
+    return HIT_NONE;
 }
 
 // Appends val for every lane with push, in lane order.
@@ -357,39 +369,53 @@ __device__ __forceinline__ void queue_push(bool push, int val, int *queue, long 
 // Interaction test of candidate b against the outer element's points (doesInteract of the
 // integrate routines, integration.cpp:539,1017).
 template <int DIM, int PREC>
-__device__ __forceinline__ bool bfs_test(const BfsArgs &a, const ProbParams &P, int method, const double *xs,
+__device__ __forceinline__ int bfs_test(const BfsArgs &a, const ProbParams &P, int method, const double *xs,
                                          const float *xsf, int nPx, const float *ohi, const float *olo,
                                          const double *Ea, int b, const float *oc, unsigned &namb) {
     constexpr int dV = DIM + 1;
     const double *Eb = &a.EC[(long long)b * DIM * dV];
-    if (PREC == PREC_F64) return interacts_exact<DIM>(P, method, xs, nPx, Ea, Eb);
+    if (PREC == PREC_F64) return interacts_exact<DIM>(P, method, xs, nPx, Ea, Eb) ? HIT : HIT_NONE;
     if (method == MTH_BARYCENTER && !P.full_search) {
         float bf[DIM];
         bary_offset<DIM>(a.BCf, b, ohi, olo, bf);
         return bary_filtered<DIM>(P, xs, xsf, nPx, Eb, bf, oc, namb);
     }
-    if (DIM != 2) return P.full_search || method == MTH_FRACTIONAL || method == MTH_WEAKSING;
+    if (DIM != 2) return P.full_search || method == MTH_FRACTIONAL || method == MTH_WEAKSING ? HIT : HIT_NONE;
     float pb[DIM * dV];
 #pragma unroll
     for (int j = 0; j < DIM * dV; j++)
         pb[j] = (a.EChi[(long long)b * DIM * dV + j] - ohi[j % DIM]) + (a.EClo[(long long)b * DIM * dV + j] - olo[j % DIM]);
-    return interacts_filtered<DIM>(P, method, xs, xsf, nPx, Eb, pb, namb);
+    return interacts_filtered<DIM>(P, method, xs, xsf, nPx, Eb, pb, oc, namb);
 }
 
 // One warp per outer element aT: breadth-first search over the vertex-sharing element graph from
 // aT, through the elements that interact with aT (Cassemble.cpp:597-660).
-//   * A group of up to 32 queued elements loads all its vertices at once; each vertex is
-//     expanded the first time the search meets it (per-warp vertex stamps).
-//   * Each fresh vertex lists its incident elements, BFS_UNROLL entries per lane loaded together;
-//     they are then checked one step at a time against the per-warp element stamps (a plain load
+// Three stages, each with a buffer in shared memory (the queue for the first), take turns, a stage
+// running when it has 32 items or when nobody has and it has the most:
+//   * dequeue: 32 queued elements load all their vertices; those that the search meets for the
+//     first time (per-warp vertex stamps) are buffered. Most are old: the stamps are looked at before
+//     the lanes compare theirs.
+//   * expand: buffered vertices list their incident elements, BFS_UNROLL steps loaded together; the
+//     elements are then checked one step at a time against the per-warp element stamps (a plain load
 //     and store: an element is met from each of its vertices in quick succession, so the stamp is
-//     usually in L1). Lanes holding the same element in a step keep only the lowest.
-//   * Fresh candidates collect in a per-warp buffer and are tested 32 at a time.
+//     usually in L1). 2D: one vertex per lane, and lanes holding the same element in a step keep only
+//     the lowest. 3D: one vertex per step, its elements one per lane.
+//   * test: 32 candidates meet the interaction test; pairs go to the queue.
+// The walk is bound by the chain of its loads and votes, so the full warp per stage counts: with the
+// vertices of each queue group expanded at once (about 16 fresh ones of 32 elements, half the lanes
+// idle) the search took 46.9 ms at n = 256, delta = 0.1 and takes 42.1; in 3D, with one vertex per
+// lane, 18.8 ms at 6 * 32^3, delta = 0.1, now 15.0. Vertices are taken last in, first out: the walk
+// then stays among near elements whose stamps are in cache (first in, first out: 43.1 ms).
 // Without a singular kernel the walk order does not change the result (the connected component
-// of aT among interacting elements and label-0 bridges), so the queue is consumed in groups of
-// 32 with no level barrier. With one, the candidates found from aT itself (the elements sharing a
-// vertex with it) take the close rule and are all tested before the walk goes on.
+// of aT among interacting elements and label-0 bridges), so there is no level barrier. With one, the
+// candidates found from aT itself (the elements sharing a vertex with it) take the close rule; they
+// are all tested before the walk goes on.
+// An element's list holds the near pairs (HIT_NEAR) first, then the others in the walk's order: the
+// passes take pairs in batches of a warp, and a batch of near pairs has no cut item to wait for
+// (n = 256 mixed: 65.9 -> 60.0 ms in the pass; FP64, n = 128: 21.4 -> 20.0 ms).
 constexpr int BFS_UNROLL = 4;
+// Mark of a near pair in the queue. Elements lie below it: the stamps alone of 2^30 elements take 5 TB.
+constexpr int NEAR = 1 << 30;
 // Outer elements are handed out in chunks of consecutive indices (at most BFS_CHUNK, fewer near
 // the end): neighbouring elements (in a mesh numbered with any locality) meet largely the same
 // candidates, so the warp's stamps of the previous element are still in cache for the next one.
@@ -405,7 +431,7 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
     __shared__ float s_xf[BFS_WARPS][MAXQ * DIM];
     __shared__ float s_oc[BFS_WARPS][4];                // outer points' centroid and enclosing radius
     __shared__ int s_buf[BFS_WARPS][32 * U + 32];       // candidates waiting for the interaction test
-    __shared__ int s_vbuf[BFS_WARPS][32 * (DIM + 1)];   // fresh vertices of a queue group
+    __shared__ int s_vbuf[BFS_WARPS][32 * (DIM + 2)];   // vertices waiting to be expanded: fewer than 32 and a queue group's
     unsigned namb = 0;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;   // at most BFS_WARPS
@@ -505,82 +531,128 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
             __syncwarp();   // read before later appends reuse the slots
             nbuf -= cnt;
             const int method = (P.singular && lvl0) ? P.close : P.remote;
-            bool pair = false;
+            int hit = HIT_NONE;
             if (b >= 0) {
-                pair = bfs_test<DIM, PREC>(a, P, method, xs, xsf, rule.nPx, ohi, olo, Ea, b, s_oc[wib], namb);
+                hit = bfs_test<DIM, PREC>(a, P, method, xs, xsf, rule.nPx, ohi, olo, Ea, b, s_oc[wib], namb);
                 cand_local++;
             }
-            queue_push(pair, b, queue, a.qcap, qtail, overflow);
+            queue_push(hit != HIT_NONE, hit == HIT_NEAR ? b | NEAR : b, queue, a.qcap, qtail, overflow);
         };
-        for (;;) {
-            const long long avail = qtail - qhead;
-            if (avail > 0 && (avail >= 32 || nbuf == 0 || lvl0)) {
-                const int gn = (int)(avail < 32 ? avail : 32);
-                int sn = lane < gn ? queue[qhead + lane] : -1;
-                qhead += gn;
-                if (sn < -1) sn = -sn - 2;   // label-0 bridge stored as -(e+2)
-                int vv[dV];
+        // 3D: one candidate per lane (or -1), no element twice: the unvisited ones are stamped and buffered
+        auto step = [&](int c) {
+            bool fresh = false;
+            if (c >= 0) {
+                fresh = visited[c - eoff] != stamp;
+                if (fresh) visited[c - eoff] = stamp;
+            }
+            if (P.bridges) {   // label-0 elements are searched through, not paired
+                const bool bridge = fresh && a.labT[c] == 0;
+                queue_push(bridge, -(c + 2), queue, a.qcap, qtail, overflow);
+                fresh = fresh && !bridge;
+            }
+            const unsigned m = __ballot_sync(FULL, fresh);
+            if (fresh) buf[nbuf + __popc(m & lanemask_lt())] = c;
+            nbuf += __popc(m);
+            __syncwarp();   // this step's stamps before the next step's loads
+        };
+        // lists the elements at the last cnt (<= 32) buffered vertices
+        int nvb = 0;
+        auto expand = [&](int cnt) {
+            nvb -= cnt;
+            if (DIM == 3) {
+                // about 24 tetrahedra meet at a vertex: one vertex per step, its elements one per lane.
+                // They are distinct, so a step needs no match for lanes with the same element, and
+                // the reads of the list are coalesced.
+                for (int c0 = 0; c0 < cnt; c0 += U) {
+                    int cand[U], more = 0;
+                    long long beg[U];
+                    int deg[U];
 #pragma unroll
-                for (int r = 0; r < dV; r++) vv[r] = sn >= 0 ? a.T32[(long long)sn * dV + r] : -1;
-                int nv = 0;
-#pragma unroll
-                for (int r = 0; r < dV; r++) {
-                    int v = vv[r];
-                    const unsigned same = __match_any_sync(FULL, v);
-                    if ((__ffs(same) - 1) != lane) v = -1;
-                    bool fresh = false;
-                    if (v >= 0) {
-                        fresh = vvis[v - voff] != stamp;
-                        if (fresh) vvis[v - voff] = stamp;
+                    for (int u = 0; u < U; u++) {
+                        const int v = c0 + u < cnt ? vbuf[nvb + c0 + u] : -1;
+                        beg[u] = v >= 0 ? a.vptr[v] : 0;
+                        deg[u] = v >= 0 ? (int)(a.vptr[v + 1] - beg[u]) : 0;
+                        more = max(more, deg[u]);
                     }
-                    const unsigned m = __ballot_sync(FULL, fresh);
-                    if (fresh) vbuf[nv + __popc(m & lanemask_lt())] = v;
-                    nv += __popc(m);
-                    __syncwarp();   // the stamps of this round before the next round's loads
-                }
-                for (int c0 = 0; c0 < nv; c0 += 32) {
-                    const int v = c0 + lane < nv ? vbuf[c0 + lane] : -1;
-                    long long beg = 0;
-                    int deg = 0;
-                    if (v >= 0) { beg = a.vptr[v]; deg = (int)(a.vptr[v + 1] - beg); }
-                    const int maxdeg = (int)__reduce_max_sync(FULL, (unsigned)deg);
-                    for (int j0 = 0; j0 < maxdeg; j0 += U) {
-                        int cand[U];
+                    for (int j0 = 0; j0 < more; j0 += 32) {
 #pragma unroll
-                        for (int u = 0; u < U; u++) cand[u] = j0 + u < deg ? a.vel[beg + j0 + u] : -1;
+                        for (int u = 0; u < U; u++) cand[u] = j0 + lane < deg[u] ? a.vel[beg[u] + j0 + lane] : -1;
 #pragma unroll
-                        for (int u = 0; u < U; u++) {
-                            int c = cand[u];
-                            const int lb = (P.bridges && c >= 0) ? a.labT[c] : 1;
-                            // lanes holding the same element: the lowest takes it
-                            const unsigned same = __match_any_sync(FULL, c);
-                            if ((__ffs(same) - 1) != lane) c = -1;
-                            bool fresh = false;
-                            if (c >= 0) {
-                                fresh = visited[c - eoff] != stamp;
-                                if (fresh) visited[c - eoff] = stamp;
-                            }
-                            const bool bridge = fresh && lb == 0;
-                            queue_push(bridge, -(c + 2), queue, a.qcap, qtail, overflow);
-                            const bool totest = fresh && !bridge;
-                            const unsigned m = __ballot_sync(FULL, totest);
-                            if (totest) buf[nbuf + __popc(m & lanemask_lt())] = c;
-                            nbuf += __popc(m);
-                            __syncwarp();   // this step's stamps before the next step's loads
-                        }
+                        for (int u = 0; u < U; u++) step(cand[u]);
                         while (nbuf >= 32) test_batch(32);
                     }
                 }
-                if (lvl0) {   // the close candidates are tested before the walk goes on
-                    while (nbuf > 0) test_batch(nbuf < 32 ? nbuf : 32);
-                    lvl0 = false;
-                }
-            } else if (nbuf > 0) {
-                test_batch(nbuf < 32 ? nbuf : 32);
             } else {
-                break;
+                const int v = lane < cnt ? vbuf[nvb + lane] : -1;
+                long long beg = 0;
+                int deg = 0;
+                if (v >= 0) { beg = a.vptr[v]; deg = (int)(a.vptr[v + 1] - beg); }
+                const int maxdeg = (int)__reduce_max_sync(FULL, (unsigned)deg);
+                for (int j0 = 0; j0 < maxdeg; j0 += U) {
+                    int cand[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) cand[u] = j0 + u < deg ? a.vel[beg + j0 + u] : -1;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        int c = cand[u];
+                        const int lb = (P.bridges && c >= 0) ? a.labT[c] : 1;
+                        // lanes holding the same element: the lowest takes it
+                        const unsigned same = __match_any_sync(FULL, c);
+                        if ((__ffs(same) - 1) != lane) c = -1;
+                        bool fresh = false;
+                        if (c >= 0) {
+                            fresh = visited[c - eoff] != stamp;
+                            if (fresh) visited[c - eoff] = stamp;
+                        }
+                        const bool bridge = fresh && lb == 0;
+                        queue_push(bridge, -(c + 2), queue, a.qcap, qtail, overflow);
+                        const bool totest = fresh && !bridge;
+                        const unsigned m = __ballot_sync(FULL, totest);
+                        if (totest) buf[nbuf + __popc(m & lanemask_lt())] = c;
+                        nbuf += __popc(m);
+                        __syncwarp();   // this step's stamps before the next step's loads
+                    }
+                    while (nbuf >= 32) test_batch(32);
+                }
             }
-            if (__any_sync(FULL, overflow)) break;
+        };
+        // the vertices of the next gn (<= 32) queued elements that the search meets for the first time
+        auto dequeue = [&](int gn) {
+            int sn = lane < gn ? queue[qhead + lane] : -1;
+            qhead += gn;
+            sn = sn < -1 ? -sn - 2 : (sn >= 0 ? sn & ~NEAR : sn);   // label-0 bridge stored as -(e+2)
+            int vv[dV];
+#pragma unroll
+            for (int r = 0; r < dV; r++) vv[r] = sn >= 0 ? a.T32[(long long)sn * dV + r] : -1;
+#pragma unroll
+            for (int r = 0; r < dV; r++) {
+                const int v = vv[r];
+                bool fresh = v >= 0 && vvis[v - voff] != stamp;
+                if (!__any_sync(FULL, fresh)) continue;
+                const unsigned same = __match_any_sync(FULL, v);
+                fresh = fresh && (__ffs(same) - 1) == lane;
+                if (fresh) vvis[v - voff] = stamp;
+                const unsigned m = __ballot_sync(FULL, fresh);
+                if (fresh) vbuf[nvb + __popc(m & lanemask_lt())] = v;
+                nvb += __popc(m);
+                __syncwarp();   // the stamps of this round before the next round's loads
+            }
+        };
+        // aT first: its neighbours are tested before the walk goes on (with the close rule where the
+        // kernel is singular). Then the three stages (queued elements to vertices, vertices to
+        // candidates, candidates to tests) each wait for 32 items; when none has them, the fullest goes.
+        dequeue(1);
+        __syncwarp();
+        expand(nvb);
+        while (nbuf > 0) test_batch(nbuf < 32 ? nbuf : 32);
+        lvl0 = false;
+        while (!__any_sync(FULL, overflow)) {
+            const int avail = (int)min(qtail - qhead, (long long)32);
+            if (max(avail, max(nvb, nbuf)) == 0) break;
+            __syncwarp();   // buffers and queue entries written before they are read
+            if (nvb >= 32 || (nvb > 0 && avail < 32 && nvb >= avail && nvb >= nbuf)) expand(min(nvb, 32));
+            else if (avail >= 32 || (avail > 0 && avail >= nbuf)) dequeue(avail);
+            else test_batch(nbuf);
         }
         overflow = __any_sync(FULL, overflow);
         if (overflow) {
@@ -592,16 +664,14 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
             }
             continue;
         }
-        // pairs: queue entries that interacted (queue[0] = aT only if (aT, aT) interacts)
-        int npairs = 0;
+        // pairs: queue entries that interacted (queue[0] = aT only if (aT, aT) interacts), the near ones
+        // first: a batch of the passes then holds pairs of one kind (all inside, or mostly cut)
+        int npairs = 0, nnear = 0;
         for (long long g = 0; g < qtail; g += 32) {
-            long long gi = g + lane;
-            bool isp = false;
-            if (gi < qtail) {
-                int s = queue[gi];
-                isp = (gi == 0) ? self_pair : (s >= 0);
-            }
-            npairs += __popc(__ballot_sync(FULL, isp));
+            const long long gi = g + lane;
+            const int s = gi < qtail ? queue[gi] : -1;
+            npairs += __popc(__ballot_sync(FULL, gi == 0 ? self_pair : s >= 0));
+            nnear += __popc(__ballot_sync(FULL, s >= 0 && (s & NEAR)));
         }
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(a.pool_cursor, (unsigned long long)npairs);
@@ -613,18 +683,16 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
             if (!fits) atomicOr(&a.err[1], 1);
         }
         if (fits) {
-            int w = 0;
+            int w = 0, wf = nnear;
             for (long long g = 0; g < qtail; g += 32) {
-                long long gi = g + lane;
-                bool isp = false;
-                int s = -1;
-                if (gi < qtail) {
-                    s = queue[gi];
-                    isp = (gi == 0) ? self_pair : (s >= 0);
-                }
-                const unsigned m = __ballot_sync(FULL, isp);
-                if (isp) a.pool[base + w + __popc(m & lanemask_lt())] = s;
-                w += __popc(m);
+                const long long gi = g + lane;
+                const int s = gi < qtail ? queue[gi] : -1;
+                const bool near = s >= 0 && (s & NEAR), far = !near && (gi == 0 ? self_pair : s >= 0);
+                const unsigned mn = __ballot_sync(FULL, near), mf = __ballot_sync(FULL, far);
+                if (near) a.pool[base + w + __popc(mn & lanemask_lt())] = s & ~NEAR;
+                if (far) a.pool[base + wf + __popc(mf & lanemask_lt())] = s;
+                w += __popc(mn);
+                wf += __popc(mf);
             }
         }
     }

@@ -1257,3 +1257,33 @@ def test_fp64_pass_keeps_vanishing_entries(nl, orc):
     assert same_pattern(A, B)
     fro, mx = rel_errors(A, B)
     assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+
+
+def _shell_mesh(dim, deg, seed):
+    """A vertex with deg neighbours on a circle or sphere around it, and a second shell outside."""
+    from scipy.spatial import Delaunay
+    from nlfem_gb300 import meshes
+    rng = np.random.Generator(np.random.PCG64(seed))
+    d = rng.normal(size=(2 * deg, dim))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    r = np.where(np.arange(2 * deg) < deg, 0.5, 1.0) * rng.uniform(0.98, 1.02, 2 * deg)
+    v = np.vstack([np.zeros((1, dim)), d * r[:, None]])
+    e = Delaunay(v).simplices.astype(np.int64)
+    vol = np.abs(np.linalg.det(v[e[:, 1:]] - v[e[:, :1]]))
+    e = e[vol > 1e-6]
+    return meshes.mesh_dict(v, e, np.where(np.arange(len(e)) % 7, 1, -1))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("dim,deg", [(2, 8), (2, 45), (3, 14), (3, 70)])
+@pytest.mark.parametrize("delta", [0.12, 0.45, 1.1, 6.0])
+def test_search_shells(nl, orc, dim, deg, delta, prec):
+    """The pair search on vertices of 8 to more than 64 elements (one and several steps of a warp, with
+    and without remainders), at horizons from below the elements' size (no pair near) to far above the
+    mesh (every pair near): the pair set is the oracle's, exactly."""
+    m = _shell_mesh(dim, deg, 7 * deg + dim)
+    k = {"function": "constant" if dim == 2 else "constant3D", "horizon": delta, "outputdim": 1}
+    conf = conf2d if dim == 2 else conf3d
+    ref = orc.assemble(m, k, conf(), want_pairs=True)["pairs"]
+    got = nl.pair_list(m, k, conf(precision=prec))
+    np.testing.assert_array_equal(got, ref[np.lexsort((ref[:, 1], ref[:, 0]))])
