@@ -203,7 +203,7 @@ struct BfsArgs {
     long long pool_cap;
     unsigned long long *pool_cursor;
     long long *seg_start;
-    int *seg_cnt;
+    int *seg_cnt, *seg_near; // pairs of a segment; the first seg_near of them are near (HIT_NEAR)
     unsigned long long *n_cand;
     unsigned long long *work;   // next outer element to hand out (chunks of BFS_CHUNK)
     int *err;                // [0] queue overflow, [1] pool overflow, [2] bad method
@@ -252,9 +252,10 @@ __device__ __forceinline__ bool interacts_exact(const ProbParams &P, int method,
 // barycenter farther than delta + ro from the centroid is outside every ball (checked with the
 // squared-distance margin, ro inflated by 8u), one nearer than delta - ro inside all of them.
 // HIT_NEAR: a pair that interacts, and every outer point's ball is certain to hold the partner (its
-// barycenter, for the barycenter rule). The radius it is judged by is at least delta / 2, where the
-// margin (relative to that radius) is still 64 u delta in length, above the 37 u delta that the
-// offsets may be off by at h = 16 delta.
+// barycenter, for the barycenter rule). The radius r it is judged by is at least delta / 2 and its
+// margin 4 MARG_D r^2, 2 MARG_D r >= MARG_D delta = 256 u delta in length: the offsets may be off by
+// 37 u delta at h = 16 delta, and the rest, 219 u delta, keeps every vertex's squared distance below
+// (1 - MARG_D) delta^2 (a margin of 128 u delta), so that the passes' own class test finds the same.
 enum { HIT_NONE = 0, HIT = 1, HIT_NEAR = 2 };
 
 template <int DIM>
@@ -267,7 +268,7 @@ __device__ __forceinline__ int bary_filtered(const ProbParams &P, const double *
         for (int j = 0; j < DIM; j++) { const float d = bf[j] - oc[j]; dc = fmaf(d, d, dc); }
         const float dl = sqrtf(P.sqdelta_f), R = dl + oc[3], r = dl - oc[3];
         if (dc > R * R * (1.f + MARG_D)) return HIT_NONE;
-        if (r > 0.5f * dl && dc < r * r * (1.f - MARG_D)) return HIT_NEAR;
+        if (r > 0.5f * dl && dc < r * r * (1.f - 4.f * MARG_D)) return HIT_NEAR;
     }
     double b64[DIM];
     bool have_b64 = false;
@@ -306,7 +307,7 @@ __device__ __forceinline__ int interacts_filtered(const ProbParams &P, int metho
     {   // the disc inside every outer point's ball: judged from their centroid and enclosing radius
         const F2 q = cen - f2(oc[0], oc[1]);
         const float r = dl - rb - oc[3];
-        if (r > 0.5f * dl && dot(q, q) < r * r * (1.f - MARG_D)) return HIT_NEAR;
+        if (r > 0.5f * dl && dot(q, q) < r * r * (1.f - 4.f * MARG_D)) return HIT_NEAR;
     }
     const float din = dl - rb;
     const float sq_in = din > 0.f ? din * din * (1.f - MARG_D) : -1.f;
@@ -410,12 +411,21 @@ __device__ __forceinline__ int bfs_test(const BfsArgs &a, const ProbParams &P, i
 // of aT among interacting elements and label-0 bridges), so there is no level barrier. With one, the
 // candidates found from aT itself (the elements sharing a vertex with it) take the close rule; they
 // are all tested before the walk goes on.
-// An element's list holds the near pairs (HIT_NEAR) first, then the others in the walk's order: the
-// passes take pairs in batches of a warp, and a batch of near pairs has no cut item to wait for
-// (n = 256 mixed: 65.9 -> 60.0 ms in the pass; FP64, n = 128: 21.4 -> 20.0 ms).
+// An element's list holds the near pairs (HIT_NEAR) first, then the others: the passes take pairs in
+// batches of a warp, and a batch of near pairs has no class to find and no cut item to wait for. In 2D
+// both are in element order, by two bitmaps over a window of elements: the walk tests one element of
+// each of 32 vertices at a time, so that a batch of its order has about 69 distinct vertices (of 96) to
+// look up, one of neighbouring elements 34 where the numbering has any locality. At n = 256, delta = 0.1
+// the search takes 1.8 ms more for it, the mixed pass 37.1 instead of 47.2 ms (FP64, n = 128: 18.8
+// instead of 19.8). A list that spans more than BFS_WINDOWS windows (a numbering without locality, where
+// the order gives nothing and every window costs a pass over the queue) keeps the walk's order. 3D too:
+// there a step holds the tetrahedra of a few vertices already (element order: pass 8.7 -> 8.5 ms, search
+// 15.0 -> 16.6 at 6 * 32^3).
 constexpr int BFS_UNROLL = 4;
 // Mark of a near pair in the queue. Elements lie below it: the stamps alone of 2^30 elements take 5 TB.
 constexpr int NEAR = 1 << 30;
+constexpr int BFS_BITS = 256;     // words of an ordering bitmap: a window of 8192 elements
+constexpr int BFS_WINDOWS = 16;   // lists over more windows keep the walk's order
 // Outer elements are handed out in chunks of consecutive indices (at most BFS_CHUNK, fewer near
 // the end): neighbouring elements (in a mesh numbered with any locality) meet largely the same
 // candidates, so the warp's stamps of the previous element are still in cache for the next one.
@@ -430,8 +440,11 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
     __shared__ double s_x[BFS_WARPS][MAXQ * DIM];
     __shared__ float s_xf[BFS_WARPS][MAXQ * DIM];
     __shared__ float s_oc[BFS_WARPS][4];                // outer points' centroid and enclosing radius
-    __shared__ int s_buf[BFS_WARPS][32 * U + 32];       // candidates waiting for the interaction test
-    __shared__ int s_vbuf[BFS_WARPS][32 * (DIM + 2)];   // vertices waiting to be expanded: fewer than 32 and a queue group's
+    // candidates waiting for the interaction test; vertices waiting to be expanded (fewer than 32 and a
+    // queue group's); in 2D, after the walk, the bitmaps that order the pairs
+    constexpr int NBUF = 32 * U + 32, NVBUF = 32 * (DIM + 2);
+    constexpr int NW = DIM == 2 && 2 * BFS_BITS > NBUF + NVBUF ? 2 * BFS_BITS : NBUF + NVBUF;
+    __shared__ unsigned s_buf[BFS_WARPS][NW];
     unsigned namb = 0;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;   // at most BFS_WARPS
@@ -439,8 +452,7 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
     unsigned short *visited = a.visited + gw * a.vstride;
     unsigned short *vvis = a.vvisited + gw * a.vvstride;
     unsigned ep = a.epoch[gw];
-    int *vbuf = s_vbuf[wib];
-    int *buf = s_buf[wib];
+    int *buf = reinterpret_cast<int *>(s_buf[wib]), *vbuf = buf + NBUF;
     int *queue = a.queue + gw * a.qcap;
     double *xs = s_x[wib];
     unsigned long long cand_local = 0;
@@ -468,7 +480,7 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
         const long long aT = cnext++;
         const int lab = a.labT[aT];
         if (lab == 0) {
-            if (lane == 0) { a.seg_cnt[aT] = 0; a.seg_start[aT] = 0; }
+            if (lane == 0) { a.seg_cnt[aT] = a.seg_near[aT] = 0; a.seg_start[aT] = 0; }
             continue;
         }
         const ProbParams P = a.probs[a.eprob[aT]];
@@ -536,7 +548,8 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
                 hit = bfs_test<DIM, PREC>(a, P, method, xs, xsf, rule.nPx, ohi, olo, Ea, b, s_oc[wib], namb);
                 cand_local++;
             }
-            queue_push(hit != HIT_NONE, hit == HIT_NEAR ? b | NEAR : b, queue, a.qcap, qtail, overflow);
+            // near by the remote rule's test only: that is what the passes integrate by
+            queue_push(hit != HIT_NONE, hit == HIT_NEAR && method == P.remote ? b | NEAR : b, queue, a.qcap, qtail, overflow);
         };
         // 3D: one candidate per lane (or -1), no element twice: the unvisited ones are stamped and buffered
         auto step = [&](int c) {
@@ -659,30 +672,72 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
             if (lane == 0) {
                 atomicOr(&a.err[0], 1);
                 atomicMax((unsigned long long *)a.qneed, (unsigned long long)(qtail + 1));
-                a.seg_cnt[aT] = 0;
+                a.seg_cnt[aT] = a.seg_near[aT] = 0;
                 a.seg_start[aT] = 0;
             }
             continue;
         }
-        // pairs: queue entries that interacted (queue[0] = aT only if (aT, aT) interacts), the near ones
-        // first: a batch of the passes then holds pairs of one kind (all inside, or mostly cut)
-        int npairs = 0, nnear = 0;
+        // pairs: queue entries that interacted (queue[0] = aT only if (aT, aT) interacts), the near ones first
+        int npairs = 0, nnear = 0, bmin = NEAR - 1, bmax = 0;
         for (long long g = 0; g < qtail; g += 32) {
             const long long gi = g + lane;
             const int s = gi < qtail ? queue[gi] : -1;
-            npairs += __popc(__ballot_sync(FULL, gi == 0 ? self_pair : s >= 0));
+            const bool pair = gi == 0 ? self_pair : s >= 0;
+            if (pair) {
+                bmin = min(bmin, s & ~NEAR);
+                bmax = max(bmax, s & ~NEAR);
+            }
+            npairs += __popc(__ballot_sync(FULL, pair));
             nnear += __popc(__ballot_sync(FULL, s >= 0 && (s & NEAR)));
         }
+        bmin = __reduce_min_sync(FULL, bmin);
+        bmax = __reduce_max_sync(FULL, bmax);
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(a.pool_cursor, (unsigned long long)npairs);
         base = __shfl_sync(FULL, base, 0);
         const bool fits = base + npairs <= (unsigned long long)a.pool_cap;
         if (lane == 0) {
             a.seg_cnt[aT] = npairs;
+            a.seg_near[aT] = nnear;
             a.seg_start[aT] = (long long)base;
             if (!fits) atomicOr(&a.err[1], 1);
         }
-        if (fits) {
+        if (!fits) continue;
+        const int e00 = bmin & ~31;
+        if (DIM == 2 && npairs > 0 && (bmax - e00) / (32 * BFS_BITS) < BFS_WINDOWS) {   // in element order
+            unsigned *bm = s_buf[wib];   // bits of the near pairs, then of the others
+            long long wn = (long long)base, wf = wn + nnear;
+            for (int e0 = e00; e0 <= bmax; e0 += 32 * BFS_BITS) {
+                __syncwarp();
+                for (int i = lane; i < 2 * BFS_BITS; i += 32) bm[i] = 0;
+                __syncwarp();
+                for (long long g = lane; g < qtail; g += 32 * U) {
+                    int s[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) s[u] = g + 32 * u < qtail ? queue[g + 32 * u] : -1;
+                    if (g == 0 && !self_pair) s[0] = -1;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int rel = (s[u] & ~NEAR) - e0;
+                        if (s[u] >= 0 && rel >= 0 && rel < 32 * BFS_BITS)
+                            atomicOr(&bm[(s[u] & NEAR ? 0 : BFS_BITS) + (rel >> 5)], 1u << (rel & 31));
+                    }
+                }
+                __syncwarp();
+                for (int i0 = 0; i0 < 2 * BFS_BITS; i0 += 32) {
+                    const unsigned word = bm[i0 + lane];
+                    const int first = e0 + 32 * (i0 & (BFS_BITS - 1)) + lane;
+                    long long &w = i0 < BFS_BITS ? wn : wf;
+                    for (unsigned nz = __ballot_sync(FULL, word != 0); nz; nz &= nz - 1) {
+                        const int j = __ffs(nz) - 1;
+                        const unsigned wd = __shfl_sync(FULL, word, j);
+                        if ((wd >> lane) & 1u) a.pool[w + __popc(wd & lanemask_lt())] = first + 32 * j;
+                        w += __popc(wd);
+                    }
+                }
+            }
+            __syncwarp();   // the bitmap read before the next walk's buffers
+        } else {   // in the walk's order
             int w = 0, wf = nnear;
             for (long long g = 0; g < qtail; g += 32) {
                 const long long gi = g + lane;

@@ -129,6 +129,8 @@ struct PassArgs {
     const long long *out_ptr, *in_ptr;
     const int *out_cnt;         // out-pair counts when the out-lists are the search's pool segments
                                 // (out_ptr = segment starts, pB = the pool); null: out_ptr[T + 1] ends
+    const int *near_cnt;        // one-sided passes: the first near_cnt[T] pairs of T are near (k_bfs): every
+                                // outer point's ball holds the partner. null: not known
     const int *pB, *inA;
     const long long *rowptr;
     const int *cols;

@@ -32,17 +32,13 @@ struct BaryWarp {
     int rlo[DIM + 1];                   // T's rows: first window word (window-rank map)
     int tvs[DIM + 1];                   // T's vertices
 };
-struct BaryGroup {   // lanes of a batch whose partners share a vertex (as local vertex c)
-    int col, c;
-    unsigned lanes;
-};
 // integers of a lane's pair, padded to an odd count so that the lanes' words fall in different banks
 __host__ __device__ constexpr int bary_vals(int dim) { return (dim + 1) * (dim + 1) + (dim == 3); }
 template <int DIM>
 __host__ __device__ constexpr size_t bary_res_bytes(int nPx) {
-    return (size_t)32 * nPx * (DIM + 2) * 4 > 32 * (bary_vals(DIM) * 8 + (DIM + 1) * sizeof(BaryGroup))
+    return (size_t)32 * nPx * (DIM + 2) * 4 > 32 * (bary_vals(DIM) * 8 + (DIM + 1) * sizeof(VertexGroup))
                ? (size_t)32 * nPx * (DIM + 2) * 4
-               : 32 * (bary_vals(DIM) * 8 + (DIM + 1) * sizeof(BaryGroup));
+               : 32 * (bary_vals(DIM) * 8 + (DIM + 1) * sizeof(VertexGroup));
 }
 // outer rule coefficients per point, read at lane-dependent points: dx psi_r, then dx psi_r psi_c (r < c)
 template <int DIM>
@@ -82,7 +78,7 @@ __global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs 
     unsigned short *lst = reinterpret_cast<unsigned short *>(reinterpret_cast<unsigned char *>(res) + bary_res_bytes<DIM>(nPx));
     constexpr int VS = bary_vals(DIM);
     long long *sval = reinterpret_cast<long long *>(res);                  // [32][VS], after the fold
-    BaryGroup *slist = reinterpret_cast<BaryGroup *>(sval + 32 * VS);
+    VertexGroup *slist = reinterpret_cast<VertexGroup *>(sval + 32 * VS);
     constexpr int NO = NS - dV, CS = bary_coef<DIM>();
     __shared__ __align__(16) float s_coef[CK ? MAXQ * CS : 4];
     if (CK) {
@@ -109,6 +105,7 @@ __global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs 
         if (idx >= a.count) break;
         const int T = a.list ? a.list[idx] : idx;
         const long long lb = a.out_ptr[T], le = a.out_cnt ? lb + a.out_cnt[T] : a.out_ptr[T + 1];
+        const long long ln = lb + (a.near_cnt ? a.near_cnt[T] : 0);   // near pairs come first
         if (lb == le || a.labT[T] == 0) continue;
         int tv[dV];
         unsigned keepmask = 0;
@@ -152,6 +149,7 @@ __global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs 
         for (long long p0 = lb; p0 < le; p0 += 32) {
             const long long p = p0 + lane;
             const bool act = p < le;
+            const bool near = min(p0 + 32, le) <= ln;   // the whole batch: no classes to find
             const int part = part_next;
             part_next = p + 32 < le ? a.pB[p + 32] : T;
             if (!CK) {   // the inner quadrature needs the partner's vertices
@@ -162,18 +160,20 @@ __global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs 
             }
             W.prt[lane] = a.adetf[part];
             float bf[DIM];
-            bary_offset<DIM>(a.BCf, part, ohi, olo, bf);
+            if (!(CK && near)) bary_offset<DIM>(a.BCf, part, ohi, olo, bf);
             // owner: which outer points see the partner's barycenter inside the ball
             bool have_b64 = false;
             double b64[DIM];
             float inv[RN];   // constant kernel: an item's sums
-            unsigned inm = 0;   // constant kernel: outer points whose ball holds the barycenter
+            // constant kernel: outer points whose ball holds the barycenter
+            unsigned inm = CK && near && act ? (nPx == 32 ? 0xffffffffu : (1u << nPx) - 1u) : 0;
             if (CK) {
                 const float kr = P.kc_f * W.prt[lane];
 #pragma unroll
                 for (int q = 0; q < RN; q++) inv[q] = kr * pr.insum[q];
             }
-            for (int k = 0; k < nPx; k++) {
+            if (CK && near) { nitin += __popc(inm); nsub += __popc(inm); }
+            for (int k = 0; k < (CK && near ? 0 : nPx); k++) {
                 unsigned char c = 0;
                 if (act) {
                     float d2 = 0.f;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs 
                 const bool put = (__ffs(grp) - 1) == lane && col >= 0;
                 const unsigned m = __ballot_sync(FULL, put);
                 if (put) {
-                    BaryGroup &e = slist[nent + __popc(m & lanemask_lt())];
+                    VertexGroup &e = slist[nent + __popc(m & lanemask_lt())];
                     e.col = col;
                     e.c = c;
                     e.lanes = grp;

@@ -556,6 +556,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
         if (idx >= a.count) break;
         const int T = a.list ? a.list[idx] : idx;
         const long long lb = a.out_ptr[T], le = a.out_cnt ? lb + a.out_cnt[T] : a.out_ptr[T + 1];
+        const long long ln = lb + (a.near_cnt ? a.near_cnt[T] : 0);   // near pairs come first
         if (lb == le || a.labT[T] == 0) continue;
         int tv[3];
         unsigned keepmask = 0;   // bit r: the row of T's vertex r exists
@@ -603,6 +604,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
         for (long long p0 = lb; p0 < le; p0 += 32) {
             const long long p = p0 + lane;
             const bool act = p < le;
+            const bool near = min(p0 + 32, le) <= ln;   // the whole batch: no classes to find
             const int part = part_next;
             part_next = p + 32 < le ? a.pB[p + 32] : T;
             int pv[3];
@@ -626,14 +628,15 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
 #pragma unroll
             for (int c = 0; c < 3; c++) W.pve[lane][c] = ve[c];
             unsigned inm = 0, cutm = 0;
-            if (act && !close) {
+            if (act && near) inm = nPx >= 32 ? 0xffffffffu : (1u << nPx) - 1u;
+            if (act && !close && !(CK && near)) {
                 float pc[6];
 #pragma unroll
                 for (int j = 0; j < 6; j++)
                     pc[j] = (a.EChi[(long long)part * 6 + j] - ((j & 1) ? ohi1 : ohi0)) + (a.EClo[(long long)part * 6 + j] - ((j & 1) ? olo1 : olo0));
 #pragma unroll
                 for (int j = 0; j < 3; j++) W.pc[lane][j] = f2(pc[2 * j], pc[2 * j + 1]);
-                for (int k = 0; k < nPx; k++) {
+                for (int k = 0; k < (near ? 0 : nPx); k++) {
                     const F2 x = xf[k];
                     const F2 Q[3] = {f2(pc[0] - x.x, pc[1] - x.y), f2(pc[2] - x.x, pc[3] - x.y), f2(pc[4] - x.x, pc[5] - x.y)};
                     const int c = fclassify(Q, P.sqdelta_f);

@@ -22,7 +22,7 @@ struct F64BaryWarp {
     unsigned rmask[DIM + 1];
     int rlo[DIM + 1], tvs[DIM + 1], te[DIM + 1];
     long long val[32 * bary_vals(DIM)];     // a batch's integers, and the groups of its partner vertices
-    BaryGroup list[32 * (DIM + 1)];         // (see k_pass_bary)
+    VertexGroup list[32 * (DIM + 1)];         // (see k_pass_bary)
 };
 // outer sums per mask: psi_r, then psi_r psi_c off the diagonal; an odd stride keeps the banks apart
 template <int DIM>
@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
         if (idx >= a.count) break;
         const int T = a.list ? a.list[idx] : idx;
         const long long lb = a.out_ptr[T], le = a.out_cnt ? lb + a.out_cnt[T] : a.out_ptr[T + 1];
+        const long long ln = lb + (a.near_cnt ? a.near_cnt[T] : 0);   // near pairs come first
         if (lb == le || a.labT[T] == 0) continue;
         if (lane < dV) {
             const int u = a.T32[(long long)T * dV + lane];
@@ -96,16 +97,18 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
         for (long long p0 = lb; p0 < le; p0 += 32) {
             const long long p = p0 + lane;
             const bool act = p < le;
+            const bool near = min(p0 + 32, le) <= ln;   // the whole batch: no classes to find
             const int part = part_next;
             part_next = p + 32 < le ? a.pB[p + 32] : T;
             int pv[dV];
 #pragma unroll
             for (int c = 0; c < dV; c++) pv[c] = a.T32[(long long)part * dV + c];
             unsigned inm = 0;
-            if (act) {
+            if (act && near) inm = nPx == 32 ? 0xffffffffu : (1u << nPx) - 1u;
+            else if (act) {
                 float bf[DIM];
                 bary_offset<DIM>(a.BCf, part, ohi, olo, bf);
-                unsigned near = 0;
+                unsigned und = 0;
                 for (int k = 0; k < nPx; k++) {
                     float d2 = 0.f;
 #pragma unroll
@@ -114,14 +117,14 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                         d2 = fmaf(d, d, d2);
                     }
                     inm |= (unsigned)(d2 < sqlo) << k;
-                    near |= (unsigned)(d2 >= sqlo && d2 <= sqhi) << k;
+                    und |= (unsigned)(d2 >= sqlo && d2 <= sqhi) << k;
                 }
-                if (near) {   // inside the margin: the exact test decides
+                if (und) {   // inside the margin: the exact test decides
                     double b64[DIM];
                     xbary<DIM>(&a.EC[(long long)part * DIM * dV], b64);
-                    namb += __popc(near);
-                    for (; near; near &= near - 1) {
-                        const int k = __ffs(near) - 1;
+                    namb += __popc(und);
+                    for (; und; und &= und - 1) {
+                        const int k = __ffs(und) - 1;
                         if (xbaryInside<DIM>(&W.x64[DIM * k], b64, P.sqdelta)) inm |= 1u << k;
                     }
                 }
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                 const bool put = (__ffs(grp) - 1) == lane && col >= 0;
                 const unsigned m = __ballot_sync(FULL, put);
                 if (put) {
-                    BaryGroup &e = W.list[nent + __popc(m & lanemask_lt())];
+                    VertexGroup &e = W.list[nent + __popc(m & lanemask_lt())];
                     e.col = col;
                     e.c = c;
                     e.lanes = grp;

@@ -536,7 +536,7 @@ struct Session {
     DevBuf vcnt, vptr, vel, adjcnt, xadj, adj;
     DevBuf stamp_epoch;   // per-warp stamp epochs of the search
     long long stamp_layout[3] = {0, 0, 0};   // warps, element and vertex stride the stamps were laid out for
-    DevBuf visited, vvisited, queue, pool, seg_start, seg_cnt, out_ptr, pA, pB, incnt, in_ptr, inA;
+    DevBuf visited, vvisited, queue, pool, seg_start, seg_cnt, seg_near, out_ptr, pA, pB, incnt, in_ptr, inA;
     DevBuf marks, rowcnt, rowptr, cols, acc, tiny, vals, keepcnt, fptr, fcols, fvals;
     DevBuf closelist, scan_tmp, counters, err, facc, ftiny, fd;
     DevBuf out64a, out64b;
@@ -587,7 +587,7 @@ struct Session {
     std::vector<DevBuf *> buffers() {
         return {&T64, &labT64, &V, &labV64, &eoffd, &voffd, &prm, &duffy, &duffyf, &T32, &labT, &eprob,
                 &EC, &adet, &labV, &vprob, &vcnt, &vptr, &vel, &adjcnt, &xadj, &adj, &visited, &vvisited, &stamp_epoch,
-                &queue, &pool, &seg_start, &seg_cnt, &out_ptr, &pA, &pB, &incnt, &in_ptr, &inA,
+                &queue, &pool, &seg_start, &seg_cnt, &seg_near, &out_ptr, &pA, &pB, &incnt, &in_ptr, &inA,
                 &marks, &rowcnt, &rowptr, &cols, &acc, &tiny, &vals, &keepcnt, &fptr, &fcols,
                 &fvals, &closelist, &scan_tmp, &counters, &err, &facc, &ftiny, &fd, &out64a, &out64b,
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
@@ -1054,6 +1054,7 @@ static int run_bfs(Session &S) {
     }
     ENS(S.seg_start, sizeof(long long) * (nE + 1));
     ENS(S.seg_cnt, sizeof(int) * (nE + 1));
+    ENS(S.seg_near, sizeof(int) * (nE + 1));
     for (int attempt = 0; attempt < 8; attempt++) {
         ENS(S.queue, sizeof(int) * (size_t)nwarps * S.qcap);
         ENS(S.pool, sizeof(int) * (size_t)S.pool_cap);
@@ -1074,6 +1075,7 @@ static int run_bfs(Session &S) {
         unsigned long long *cnt = S.counters.get<unsigned long long>();
         a.pool_cursor = cnt + 0; a.n_cand = cnt + 1; a.qneed = (long long *)(cnt + 2);
         a.seg_start = S.seg_start.get<long long>(); a.seg_cnt = S.seg_cnt.get<int>();
+        a.seg_near = S.seg_near.get<int>();
         a.err = S.err.get<int>();
         a.n_amb = cnt + 7;
         a.work = cnt + 3;
@@ -1764,6 +1766,10 @@ static int run_pass_one_sided(Session &S, const PassArgs &pa, const PassRule &pr
             if (L[i].count == 0) continue;
             ma.p.list = L[i].list;
             ma.p.count = L[i].count;
+            if (retri && L[i].cls == MIX_CONST && ma.p.near_cnt) {
+                CK(cudaMemsetAsync(ma.work, 0, sizeof(int), S.st));
+                k_pass_near2d<<<(unsigned)(S.nSM * NEAR_BLOCKS), MIX_THREADS, 0, S.st>>>(ma, pr, S.rule.nPx); ++S.nlaunch;
+            }
             CK(cudaMemsetAsync(ma.work, 0, sizeof(int), S.st));
             kfn[L[i].cls]<<<(unsigned)(S.nSM * per_sm[i]), threads, smem, S.st>>>(ma, S.rule, pr); ++S.nlaunch;
             CK(cudaGetLastError());
@@ -1958,6 +1964,7 @@ static int run_passes(Session &S) {
     a.closebuf = S.closebuf.get<double>(); a.err = S.err.get<int>();
     a.zptr = S.zptr.get<long long>(); a.zidx = S.zidx.get<long long>();
     a.n_subtri = cnt + 5; a.n_amb = cnt + 6; a.n_close = cnt + 4; a.n_in = cnt + 12; a.n_cut = cnt + 13;
+    a.near_cnt = S.pmode == PM_BARY || S.pmode == PM_RETRI ? S.seg_near.get<int>() : nullptr;
     a.touched = S.prec == PREC_MIX && S.pmode == PM_COLORED ? S.touched.get<unsigned char>() : nullptr;
     if (S.pmode == PM_VEC) return run_pass_vec<DIM>(S);
     const PassRule pr = make_pass_rule<float>(S.rule, DIM);

@@ -161,9 +161,14 @@ __device__ __forceinline__ long long fx64(float v, float mul, int *ovf) {
 // The same with the overflow recorded in a flag of the caller (reported once, not per value).
 __device__ __forceinline__ long long fx64(float v, float mul, bool &bad) {
     const float t = v * mul;
-    const bool ok = fabsf(t) < 4.0e18f;
-    bad |= !ok;
-    return ok ? __float2ll_rn(t) : 0;
+    bad |= !(fabsf(t) < 4.0e18f);
+    return __float2ll_rn(t);   // saturates; the pass is redone
+}
+// The same with the largest magnitude (NaN stays) in a variable of the caller, checked once.
+__device__ __forceinline__ long long fx64(float v, float mul, float &most) {
+    const float t = v * mul;
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(most) : "f"(fabsf(t)));
+    return __float2ll_rn(t);
 }
 __device__ __forceinline__ long long fx64d(double v, double mul, bool &bad) {
     const double t = v * mul;

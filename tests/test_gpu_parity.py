@@ -1287,3 +1287,26 @@ def test_search_shells(nl, orc, dim, deg, delta, prec):
     ref = orc.assemble(m, k, conf(), want_pairs=True)["pairs"]
     got = nl.pair_list(m, k, conf(precision=prec))
     np.testing.assert_array_equal(got, ref[np.lexsort((ref[:, 1], ref[:, 0]))])
+
+
+@pytest.mark.parametrize("n,delta", [(260, 0.02), (40, 0.3)])
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+def test_numbering_does_not_change_the_matrix(nl, n, delta, prec):
+    """Pair lists are ordered by element (near pairs apart) where an element's partners span a few thousand
+    numbers, and by the walk where they span more than 131072 (n = 260 renumbered: 1.35e5 elements). Every sum
+    over pairs is an integer one in the mixed path, so a renumbered mesh gives the renumbered matrix bit for
+    bit; FP64 forms an element's own block in floating point (its pairs' order) and agrees to rounding."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(n, delta, jitter=0.2, seed=5)
+    rng = np.random.Generator(np.random.PCG64(n))
+    pv, pe = rng.permutation(len(v)), rng.permutation(len(e))   # new vertex i is the old pv[i]
+    inv = np.argsort(pv)
+    k = {"function": "constant", "horizon": delta, "outputdim": 1}
+    A = nl.stiffnessMatrix(meshes.mesh_dict(v, e, l), k, conf2d(precision=prec)).tocsr()
+    B = nl.stiffnessMatrix(meshes.mesh_dict(v[pv], inv[e[pe]], l[pe]), k, conf2d(precision=prec)).tocsr()
+    C = B[inv][:, inv].tocsr()
+    assert same_pattern(A, C)
+    if prec == "mixed":
+        assert np.array_equal(A.data, C.data)
+    else:
+        assert abs(A.data - C.data).max() < FP64_TOL * abs(A.data).max()
