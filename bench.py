@@ -460,8 +460,8 @@ def run_gpu(args, rank=0, world=1, dist=None):
             "roofline": {"bound": "fp64", "achieved": a1, "peak": peak64, "unit": "TFLOP/s", "frac": a1 / peak64,
                          "note": "the mixed path's FLOP model over the FP64 instance's quadrature phase"},
             "note": "precision \"fp64-onesided\": the headline's one-sided pass, closed forms and fixed-point sums "
-                    "in FP64 arithmetic (FP64 class tests, the exact FP64 polygon routine); the plain FP64 arm "
-                    "beside it is the reference's two-sided algorithm on the GPU",
+                    "in FP64 arithmetic (classes and polygon structure by the certified FP32 geometry), every "
+                    "structural slot kept; the FP64 arm beside it takes the same pass where it applies",
             "clocks": clk1}
     dg = reference_digest(args)
     if dg is not None:
