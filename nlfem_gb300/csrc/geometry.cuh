@@ -338,6 +338,8 @@ struct ProbParams {
     int f64ok;        // the one-sided FP64 pass takes this problem (passes_f64.cuh)
     int xN, xD, xS;   // its fixed-point bounds: 2^(xN / 8) above a pair's termNonloc per |T| |b|, 2^xD above
                       // its diagonal blocks times the mesh's |det| sum, 2^xS above the outer weights' sum times that
+    int limN, limE, limD; // bits of the largest single contribution to a termNonloc slot, to an element's
+                      // termLocalPrime sums, to a diagonal-block slot (f64_fix)
 };
 
 // Close pairs of a singular kernel take a Duffy rule: fractional or weakSingular.

@@ -108,10 +108,11 @@ __device__ __forceinline__ int exp_above(double x) {
     const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1022;
     return e < -900 ? -900 : e;
 }
-// q rounded to an integer (a nonzero one never to zero); |q| >= 2^62 or NaN sets bad
-__device__ __forceinline__ long long f64_fix(double q, bool &bad) {
+// q rounded to an integer (a nonzero one never to zero); |q| >= 2^lim or NaN sets bad. Rigorous bounds
+// (all but singular kernels) leave a sum its 62 bits; without one lim is what keeps the sum from wrapping.
+__device__ __forceinline__ long long f64_fix(double q, int lim, bool &bad) {
     const long long b = __double_as_longlong(q);
-    bad |= ((int)(b >> 52) & 0x7ff) >= 1023 + F64_BITS;
+    bad |= ((int)(b >> 52) & 0x7ff) >= 1023 + lim;
     const long long i = __double2ll_rn(q);
     return (i == 0 && (b << 1) != 0) ? (b < 0 ? -1LL : 1LL) : i;
 }
@@ -598,6 +599,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
 #pragma unroll
         for (int r = 0; r < 3; r++) et[r] = 8 * F64_BITS - P.xN - W.te[r];
         const double dTs = scale2(dT, F64_BITS - P.xS);
+        const int limN = CK ? F64_BITS : P.limN, limE = CK ? F64_BITS : P.limE;
         double D[3] = {0, 0, 0};   // termLocal of T's pairs, off-diagonal
         const bool frac_close = KIND == MIX_SINGULAR && duffy_close(P);
         int part_next = lb + lane < le ? a.pB[lb + lane] : T;   // partners one batch ahead
@@ -705,7 +707,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                     } else {
                         const int ex = o < 9 ? (8 * F64_BITS - P.xN - W.te[o / 3] - W.pve[pl][o % 3]) >> 3 : F64_BITS - P.xD - W.pe[pl];
                         const double q = scale2(v, ex);
-                        const long long iv = f64_fix(q, bad);
+                        const long long iv = f64_fix(q, o < 9 ? limN : limE, bad);
                         A[o] = iv;
                         if (o >= 12) A[o + 3] = f64_fix_lo(q, iv);
                         else if (NW == 2) A[F64_OUT + 3 + o] = f64_fix_lo(q, iv);
@@ -732,13 +734,13 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                 for (int c = 0; c < 3; c++) {
                     const double iN = kr * pr.insum[1 + c];
 #pragma unroll
-                    for (int r = 0; r < 3; r++) nx[3 * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve[c]) >> 3), bad);
+                    for (int r = 0; r < 3; r++) nx[3 * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve[c]) >> 3), limN, bad);
                 }
                 const double kl = kr * pr.insum[0];
 #pragma unroll
                 for (int q = 0; q < 3; q++) D[q] += m[3 + q] * kl;
                 const double q = m[6] * dTs;
-                const long long iv = f64_fix(q, bad);
+                const long long iv = f64_fix(q, limE, bad);
                 red_add(ep, 0, iv);
                 red_add(ep, 1, f64_fix_lo(q, iv));
             }
@@ -765,14 +767,14 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
 #pragma unroll
                     for (int q = 0; q < 3; q++) {
                         const double v = scale2(cb[q == 2 ? 23 : 19 + q], F64_BITS - P.xD - eb);
-                        const long long iv = f64_fix(v, bad);
+                        const long long iv = f64_fix(v, limE, bad);
                         red_add(ep, 2 + q, iv);
                         red_add(ep, 5 + q, f64_fix_lo(v, iv));
                     }
 #pragma unroll
                     for (int i = 0; i < 9; i++) {
                         const double q = scale2(cb[9 + i], (et[i / 3] - ve[i % 3]) >> 3);
-                        nx[i] = f64_fix(q, bad);
+                        nx[i] = f64_fix(q, limN, bad);
                         if (NW == 2) nx[NW == 2 ? 9 + i : 0] = f64_fix_lo(q, nx[i]);
                     }
                 }
@@ -837,7 +839,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
             const double d = r + c == 1 ? D[0] : (r + c == 2 ? D[1] : D[2]);
             if (s >= 0) {
                 const double q = scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3));
-                const long long iv = f64_fix(q, bad);
+                const long long iv = f64_fix(q, CK ? F64_BITS : P.limD, bad);
                 red_add(vals, s, iv);
                 red_add(fa.valslo, s, f64_fix_lo(q, iv));
             } else if (keepmask & (1u << r)) miss = true;
@@ -898,7 +900,7 @@ __global__ void k_elem_blocks_f64(const long long *__restrict__ elp, const doubl
             const int v = T32[e * 3 + r], s = dslot[e * 9 + 3 * r + c];
             if (s >= 0) {
                 const double q = scale2(b[r + c - 1], F64_BITS - P.xD - ((vexp[v] + 7) >> 3));
-                const long long iv = f64_fix(q, bad);
+                const long long iv = f64_fix(q, P.limD, bad);
                 red_add(vals, s, iv);
                 red_add(valslo, s, f64_fix_lo(q, iv));
             } else if (labV[v] > 0) {

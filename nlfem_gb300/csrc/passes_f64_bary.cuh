@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                     const int ve = fa.vexp[pv[c]];
                     const double iN = kr * pr.insum[1 + c];
 #pragma unroll
-                    for (int r = 0; r < dV; r++) nx[dV * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve) >> 3), bad);
+                    for (int r = 0; r < dV; r++) nx[dV * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve) >> 3), F64_BITS, bad);
                 }
                 const double kl = kr * pr.insum[0];
 #pragma unroll
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                     miss = true;
                 } else {
                     const double q = scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3));
-                    const long long iv = f64_fix(q, bad);
+                    const long long iv = f64_fix(q, F64_BITS, bad);
                     red_add(vals, s, iv);
                     red_add(fa.valslo, s, f64_fix_lo(q, iv));
                 }

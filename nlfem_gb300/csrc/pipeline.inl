@@ -241,8 +241,13 @@ static MeshScan scan_mesh(const nlfem_problem &p) {
 // passes_f64_bary.cuh, the barycenter rule with a constant kernel), and the bounds its units follow
 // from. A pair's blocks are at most kbound |T| |b| times the rules' absolute sums (CN, CD: basis
 // functions at inner points of polygons inside the element are at most the largest absolute row
-// sum of the rule's own); for singular kernels kbound is the value at the mean element size times
-// 2^20, and contributions beyond it are detected. Elements near degenerate (where the reference's
+// sum of the rule's own). For singular kernels kbound is no bound but the value at the mean element size
+// times 2^20; there every contribution is held to its share of the 62 bits instead, by the largest
+// number of contributions that a sum can have: a pair of vertices shares at most (largest valence)^2
+// element pairs, each seen from its own and from the mirrored side; an element has at most nE partners;
+// a diagonal-block slot takes two contributions per element at the vertex. A contribution above its share
+// (elements about 140 times smaller than the mean at s = 0.4) hands the call to the general pass.
+// Elements near degenerate (where the reference's
 // solve2x2 may abort; the barycenter rule never calls it), bounds far outside the exponent range
 // and options that need the general pass go there. fp64-onesided, which has no such pass to match,
 // is bound only by the range.
@@ -279,6 +284,15 @@ static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, const MeshScan
     P.xN = (int)ceil(8.0 * log2(CN) + 1e-3);
     P.xD = exact_ceil_log2(CD);
     P.xS = exact_ceil_log2(sx * atot);
+    P.limN = P.limE = P.limD = F64_BITS;
+    if (P.singular) {
+        std::vector<int> valence(p.nV, 0);
+        int most = 1;
+        for (long i = 0; i < (long)dV * p.nE; i++) most = std::max(most, ++valence[p.elements[i]]);
+        P.limN -= exact_ceil_log2(2.0 * most * most);
+        P.limE -= exact_ceil_log2((double)p.nE);
+        P.limD -= exact_ceil_log2(2.0 * most);
+    }
     if (p.precision == NLFEM_PREC_FP64)
         P.f64ok = m.sound && m.amin > (bary ? -1.0 : 1e-60) && !P.full_search && !P.zeta && (!P.singular || duffy_close(P));
     else

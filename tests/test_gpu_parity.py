@@ -1310,3 +1310,43 @@ def test_numbering_does_not_change_the_matrix(nl, n, delta, prec):
         assert np.array_equal(A.data, C.data)
     else:
         assert abs(A.data - C.data).max() < FP64_TOL * abs(A.data).max()
+
+
+def _graded_mesh(n, delta, p, seed):
+    """regular_square with its distances from the centre raised to the power p: elements shrink towards the centre."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(n, delta, jitter=0.1, seed=seed)
+    d = v - 0.5
+    r = np.linalg.norm(d, axis=1)
+    return meshes.mesh_dict(0.5 + d * ((r / r.max()) ** (p - 1))[:, None], e, l)
+
+
+@pytest.mark.parametrize("n,s,p,seed,onesided", [(16, 0.4, 4.25, 3, False), (16, 0.6, 3.75, 3, False), (10, 0.4, 5.25, 3, False),
+                                                 (8, 0.5, 5.5, 5, False), (16, 0.4, 5.5, 3, False), (16, 0.4, 2.0, 3, True)])
+def test_fp64_singular_sums_on_graded_meshes(nl, orc, n, s, p, seed, onesided):
+    """Singular kernels have no rigorous bound for the one-sided FP64 pass's integer sums. On meshes graded
+    so far that a sum of contributions, or one of them, could leave the integers' range, the call is handed
+    to the general pass (slot_map 0 in the stats), in a one-shot call, in a session and in a graph session;
+    moderate grading stays on the one-sided pass. All meet the FP64 bar against the oracle."""
+    from nlfem_gb300 import _lib
+    m = _graded_mesh(n, 0.3, p, seed)
+    k = {"function": "fractional", "horizon": 0.3, "outputdim": 1, "fractional_s": s}
+    c = conf2d(rule="7", close="fractional", deg=3)
+    B = orc.assemble(m, k, c)["A"]
+
+    def check(A, st):
+        assert (st["slot_map"] != 0) == onesided
+        assert same_pattern(A, B)
+        fro, mx = rel_errors(A, B)
+        assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+
+    A = nl.stiffnessMatrix(dict(m), k, c)
+    check(A, _lib.stats())
+    for graph in (False, True):
+        sess = nl.Session([(dict(m), k, c)])
+        try:
+            for _ in range(2):
+                st = sess.assemble(graph=graph)
+                check(sess.download(0), st)
+        finally:
+            sess.close()
