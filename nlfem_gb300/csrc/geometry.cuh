@@ -339,7 +339,7 @@ struct ProbParams {
     int xN, xD, xS;   // its fixed-point bounds: 2^(xN / 8) above a pair's termNonloc per |T| |b|, 2^xD above
                       // its diagonal blocks times the mesh's |det| sum, 2^xS above the outer weights' sum times that
     int limN, limE, limD; // bits of the largest single contribution to a termNonloc slot, to an element's
-                      // termLocalPrime sums, to a diagonal-block slot (f64_fix)
+                      // termLocalPrime sums, to a diagonal-block slot (f64_split)
 };
 
 // Close pairs of a singular kernel take a Duffy rule: fractional or weakSingular.

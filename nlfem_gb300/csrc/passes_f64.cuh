@@ -20,19 +20,22 @@
 // triangles: 0.52 against 66.6 ms; parabola, 2 * 57^2: 5.4 against 257 ms; fractional, 2 * 40^2:
 // 9.6 against about 540 ms. The FP64 pipe is 70 to 89% busy in these.
 //
-// Sums. Every contribution is rounded once to a 64-bit integer and added with an integer atomic,
-// so the result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
+// Sums. Every contribution is cut into 64-bit integers that are added with integer atomics, so the
+// result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
 // follows from a bound of that slot: the blocks' sum over the elements at t and at v is at most
 // 2^xN |patch t| |patch v|, with |patch| the elements' |det| sum at a vertex. Exponents are kept
 // in eighths of a bit (vexp = 8 log2 |patch|, rounded up), so that only their sum is rounded to a
 // whole power: the unit 2^((xN + vexp[t] + vexp[v]) / 8 - 62) is near 2^-55 of a pair that fills the
-// ball, whatever the mesh grading. The sums with many more terms keep a second integer 40 bits below
-// the first: termLocal in the diagonal-block slots (unit 2^(xD + vexp[t] - 62)), and per partner
-// element its termLocalPrime, of which a constant kernel's inside part is one number, the |T|
-// weighted sum of the outer rule over the inside masks. So do all sums of singular kernels, whose
-// bound is loose and whose near pairs are far above their far ones. A nonzero contribution that
-// rounds to zero counts one unit, so a slot is zero only when all its contributions are (the
-// reference drops exact zeros).
+// ball, whatever the mesh grading. A contribution near the bound is a whole number of units; of a
+// smaller one a second integer, 40 bits below the first, holds what is left, and of one below about
+// 2^-50 of the bound (a sliver that the sphere cuts off) a third, 40 bits lower again. So a slot holds
+// all bits of its contributions however small they are against the bound: the smallest entries of a matrix
+// are 1e-24 of the largest. Most batches have no second and almost all no third parts, and skip them.
+// The sums with many more terms have two integers: termLocal in the diagonal-block slots (unit
+// 2^(xD + vexp[t] - 62)), and per partner element its termLocalPrime, of which a constant kernel's
+// inside part is one number, the |T| weighted sum of the outer rule over the inside masks. A nonzero
+// contribution counts at least one of the last units, so a slot is zero only when all its
+// contributions are (the reference drops exact zeros).
 #pragma once
 #include "passes_mix.cuh"
 
@@ -44,14 +47,15 @@ constexpr int F64_CAP = 128;   // items integrated before their pairs are folded
 constexpr int F64_RN = 7;      // per item: innerLocal, innerNonloc[3], off-diagonal termLocalPrime sums[3]
 constexpr int F64_OUT = 15;    // per pair: termNonloc[9], off-diagonal termLocal[3] and termLocalPrime[3]
 constexpr int F64_BITS = 62;   // a bound of 2^x has the unit 2^(x - 62)
-constexpr int F64_WIDE = 40;   // bits of a second integer
+constexpr int F64_WIDE = 40;   // bits from one integer of a sum to the next
+constexpr int F64_ERR_THIRD = 12;   // err[]: some slot has a third integer
 constexpr int F64_ELP = 8;     // per element: inside sum (two integers), cut termLocalPrime[3], second integers[3]
 
 struct F64Args {
     MixArgs m;                  // m.elp: F64_ELP integers per element
     const int *vexp;            // per vertex, 8 log2 of its elements' |det| sum, rounded up
     long long *valslo;          // second integers of vals
-    long long *valsNlo;         // second integers of valsN (singular kernels)
+    long long *valsNt;          // third integers of valsN (m.valsN: two integers per slot)
     const double *idet;         // per element, 1 / det (signed)
     const double *mtab;         // constant kernels: the mask table (k_mask_table)
     const double *pw;           // singular kernels: power tables (primitives.cuh)
@@ -71,28 +75,23 @@ struct F64Warp {
     unsigned char order[F64_CAP];           // the inside items, then the cut items (kernels that list both)
     unsigned char pl[32], ps[32], pn[32];   // chunk's pairs: owner lane, first item, item count
 };
-template <int NW>
 struct F64Entry {   // one partner vertex of a batch and its integer sums over T's rows
     int col, pad;
-    long long v[3 * NW];
+    long long v[6];   // first integers, second integers
 };
-__host__ __device__ constexpr int f64_words(int kind) { return kind == MIX_SINGULAR ? 2 : 1; }
-// per-pair sums of the folded items (15, and second integers: termLocalPrime[3], termNonloc[9]), then the item results; the scatter
-// list lies over both
-__host__ __device__ constexpr int f64_acc(int kind) { return F64_OUT + (kind == MIX_SINGULAR ? 12 : 3); }
-__host__ __device__ constexpr size_t f64_work_bytes(int kind) {
-    return (size_t)(32 * f64_acc(kind) + F64_CAP * F64_RN) * 8 > 96 * (8 + 24 * (size_t)f64_words(kind))
-               ? (size_t)(32 * f64_acc(kind) + F64_CAP * F64_RN) * 8
-               : 96 * (8 + 24 * (size_t)f64_words(kind));
-}
-__host__ __device__ constexpr size_t f64_warp_bytes(int kind, int nPx) {
-    return (sizeof(F64Warp) + 15) / 16 * 16 + (size_t)nPx * (24 + 56) + f64_work_bytes(kind) + 16;
+// per-pair sums of the folded items (15, and termLocalPrime's second integers), then the item results;
+// the scatter list lies over both
+constexpr int F64_ACC = F64_OUT + 3;
+constexpr size_t F64_WORK_BYTES = (size_t)(32 * F64_ACC + F64_CAP * F64_RN) * 8;
+static_assert(F64_WORK_BYTES >= 96 * sizeof(F64Entry), "the scatter list lies over the item results");
+__host__ __device__ constexpr size_t f64_warp_bytes(int nPx) {
+    return (sizeof(F64Warp) + 15) / 16 * 16 + (size_t)nPx * (24 + 56) + F64_WORK_BYTES + 16;
 }
 // mask sums of the outer rule: one table of up to 256 entries per 8 outer points
-__host__ __device__ constexpr int f64_tab_entries(int nPx) { return nPx <= 8 ? 1 << nPx : 256 * ((nPx + 7) / 8); }
+__host__ __device__ constexpr int f64_tab_entries(int nPx) { return 256 * (nPx / 8) + (nPx % 8 ? 1 << (nPx % 8) : 0); }
 __host__ __device__ constexpr size_t f64_smem_bytes(int kind, int nPx) {
     return (kind == MIX_CONST ? (size_t)f64_tab_entries(nPx) * 7 * 8 : 0) +
-           F64_WARPS * ((f64_warp_bytes(kind, nPx) + 15) / 16 * 16) + 16;
+           F64_WARPS * ((f64_warp_bytes(nPx) + 15) / 16 * 16) + 16;
 }
 
 // 2^e, e in [-1022, 1023]
@@ -108,20 +107,50 @@ __device__ __forceinline__ int exp_above(double x) {
     const int e = ((__double2hiint(x) >> 20) & 0x7ff) - 1022;
     return e < -900 ? -900 : e;
 }
-// q rounded to an integer (a nonzero one never to zero); |q| >= 2^lim or NaN sets bad. Rigorous bounds
-// (all but singular kernels) leave a sum its 62 bits; without one lim is what keeps the sum from wrapping.
-__device__ __forceinline__ long long f64_fix(double q, int lim, bool &bad) {
+// q (a number of units) = hi + lo 2^-40 + rest, all of q's sign, by its bits: the conversions of the FP64
+// pipe are as slow as its arithmetic. rest is set where bits are left over (|q| < 2^12); f64_third holds
+// those. |q| >= 2^lim or NaN sets bad: rigorous bounds (all but singular kernels) leave a sum its 62 bits;
+// without one lim is what keeps the sum from wrapping.
+__device__ __forceinline__ void f64_split(double q, int lim, bool &bad, long long &hi, long long &lo, bool &rest) {
     const long long b = __double_as_longlong(q);
-    bad |= ((int)(b >> 52) & 0x7ff) >= 1023 + lim;
-    const long long i = __double2ll_rn(q);
-    return (i == 0 && (b << 1) != 0) ? (b < 0 ? -1LL : 1LL) : i;
+    const int x = (int)(b >> 52) & 0x7ff, n = 1075 - x;   // |q| = m 2^-n
+    const long long m = x ? (b & 0xfffffffffffffLL) | 1LL << 52 : 0;
+    bad |= x >= 1023 + lim;
+    long long h, l = 0;
+    if (n <= 0) {
+        h = m << min(-n, 63);
+    } else {
+        h = m >> min(n, 63);
+        const long long f = m - (h << min(n, 63));
+        const int k = min(n - F64_WIDE, 63);
+        l = k <= 0 ? f << -k : f >> k;
+        rest |= k > 0 && (l << k) != f;
+    }
+    hi = b < 0 ? -h : h;
+    lo = b < 0 ? -l : l;
 }
-// the second integer: what the first one's rounding left, 2^40 times finer
-__device__ __forceinline__ long long f64_fix_lo(double q, long long i) {
-    return __double2ll_rn((q - (double)i) * (double)(1LL << F64_WIDE));
+// The third integer: the bits of |q| < 2^13 below 2^-40, in units of 2^-80 (a nonzero rest never to zero).
+__device__ __forceinline__ long long f64_third(double q) {
+    const long long b = __double_as_longlong(q);
+    const int n = 1075 - ((int)(b >> 52) & 0x7ff), k = min(n - F64_WIDE, 63);
+    const long long a = (b & 0xfffffffffffffLL) | 1LL << 52, g = a - ((a >> k) << k);
+    const long long t = n <= 2 * F64_WIDE ? g << (2 * F64_WIDE - n) : max(g >> min(n - 2 * F64_WIDE, 63), 1LL);
+    return b < 0 ? -t : t;
 }
-__device__ __forceinline__ double f64_join(long long hi, long long lo) {
-    return (double)hi + (double)lo * (1.0 / (double)(1LL << F64_WIDE));
+// The sums of two integers: a nonzero contribution counts at least one of the second's units.
+__device__ __forceinline__ void f64_split2(double q, int lim, bool &bad, long long &hi, long long &lo) {
+    bool rest = false;
+    f64_split(q, lim, bad, hi, lo, rest);
+    if (rest && (hi | lo) == 0) lo = __double2hiint(q) < 0 ? -1 : 1;
+}
+// Their value: the lower integers' carries go up first, so that no cancellation is left between them.
+__device__ __forceinline__ double f64_join(long long hi, long long lo, long long third = 0) {
+    constexpr double W = 1.0 / (double)(1LL << F64_WIDE);
+    lo += (third + (1LL << (F64_WIDE - 1))) >> F64_WIDE;
+    third -= (third + (1LL << (F64_WIDE - 1))) >> F64_WIDE << F64_WIDE;
+    hi += (lo + (1LL << (F64_WIDE - 1))) >> F64_WIDE;
+    lo -= (lo + (1LL << (F64_WIDE - 1))) >> F64_WIDE << F64_WIDE;
+    return (double)hi + W * ((double)lo + W * (double)third);
 }
 
 // s + c += x y, c the low part of the sum (product and sum without loss to second order)
@@ -248,7 +277,6 @@ __device__ __forceinline__ void f64_item_exact(const ProbParams &P, const Rule &
 struct F64Poly {
     double R[18], L[18];
     int n;
-    unsigned seg;   // bit j: the side from point j - 1 (cyclic) to j may lie off the two edges through vertex 0
 };
 
 // The polygon of B(x) and the triangle Q (relative to x), e1, e2 its edges from Q0. The certified FP32
@@ -256,7 +284,7 @@ struct F64Poly {
 // reference's branches); only the points themselves are FP64: per crossing a square root and a
 // quotient, per cap a reciprocal square root. In reference coordinates vertices are constants and
 // a crossing is its root. Against the exact routine, which takes both roots of all three edges with
-// their divisions for every item, that is about a third of the FP64 instructions: with the boundary
+// their divisions for every item, that is about a third of the FP64 instructions: with the closed
 // moments of f64_item 51.5 -> 20.5 ms on 2 * 128^2 triangles (constant kernel). False where a decision
 // is within its margin. LATE takes such an item's polygon from the exact routine instead, and is false
 // where that holds less than 1e-5 of the partner (f64_item_exact then; above, every sum of the item is
@@ -279,7 +307,6 @@ __device__ __forceinline__ bool f64_polygon(const ProbParams &P, const double *x
             if (j >= 2)
                 area += fabs((Y.R[2 * j - 2] - Y.R[0]) * (Y.R[2 * j + 1] - Y.R[1]) - (Y.R[2 * j - 1] - Y.R[1]) * (Y.R[2 * j] - Y.R[0]));
         }
-        Y.seg = (1u << Y.n) - 1u;
         return Y.n < 3 || area >= 1e-5 * adet;
     }
     bool amb = false;
@@ -287,15 +314,8 @@ __device__ __forceinline__ bool f64_polygon(const ProbParams &P, const double *x
     Y.n = fretriangulate<true>(Qf, P.sqdelta_f, P.caps, nullptr, amb, nullptr, &codes);
     if (amb) return false;
     unsigned xm = 0, cm = 0;
-    // by code, whether the point lies on edge 0 (bit c) and edge 2 (bit c + 16): vertices 0, 1 and the
-    // roots 3, 4 of edge 0; vertices 0, 2 and the roots 7, 8 of edge 2
-    constexpr unsigned ON = 0x0000001bu | 0x01850000u;
-    Y.seg = 0;
-    int cp = Y.n ? (int)(codes >> (4 * Y.n - 4)) & 15 : 0;
     for (int j = 0; j < Y.n; j++) {
         const int c = (int)(codes >> (4 * j)) & 15;
-        Y.seg |= (unsigned)(((ON >> c) & (ON >> cp) & 0x10001u) == 0) << j;
-        cp = c;
         xm |= (unsigned)(c >= FCODE_X && c < FCODE_CAP) << j;
         cm |= (unsigned)(c == FCODE_CAP) << j;
         if (c < 3) {
@@ -343,10 +363,13 @@ __device__ __forceinline__ bool f64_polygon(const ProbParams &P, const double *x
 // Polynomial kernels need no inner points. An inside item of the parabola kernel is a combination of
 // the rule's moments to degree four. Where the inner rule integrates the polynomials exactly (degree two
 // for constant kernels, four for the parabola), the sums over the fan are the polygon's integrals,
-// taken from its boundary in reference coordinates (Green's theorem with the origin in vertex 0, so that
-// sides on the two edges through it add nothing): closed forms per side for constant kernels; for
-// the parabola the integral over the triangle (0, P0, P1) of a monomial of degree d is
-// (P0 x P1) / (d + 2) times its mean over the side, by the 3-point Gauss rule (exact to degree five).
+// taken from its sides in reference coordinates about its first point: closed forms per side for constant
+// kernels; for the parabola the integral over the triangle (0, P0, P1) of a monomial of degree d is
+// (P0 x P1) / (d + 2) times its mean over the side, by the 3-point Gauss rule (exact to degree five). The
+// polygon's own point as the origin keeps the digits of a small one, whose sides are short against their
+// distance from any other origin (taken from the partner's vertex 0, the smallest entries of a parabola
+// matrix were off by 1e-5 of themselves; the sides that lie on the edges through that vertex and add
+// nothing are about as many as the two through the first point).
 // Returns false for a cut item whose polygon the certified run leaves open, which takes LATE.
 template <int KIND, bool LATE>
 __device__ __forceinline__ bool f64_item(const ProbParams &P, const Rule &rule, const PassRuleT<double> &pr, bool inside,
@@ -356,20 +379,29 @@ __device__ __forceinline__ bool f64_item(const ProbParams &P, const Rule &rule, 
     const double e[4] = {Eb[2] - Eb[0], Eb[3] - Eb[1], Eb[4] - Eb[0], Eb[5] - Eb[1]};
     double S0 = 0, S1[3] = {0, 0, 0}, S2[3] = {0, 0, 0};
     const bool parab = KIND == MIX_REGULAR && P.kernel == KER_PARABOLA;
-    // parabola: kernel kc (k0 - k1 . r - (ka r1^2 + 2 kb r1 r2 + kd r2^2)) in reference coordinates r
+    // parabola: kernel kc (k0 - k1 . u - (ka u1^2 + 2 kb u1 u2 + kd u2^2)) in reference coordinates u about the
+    // point that lies at (yx, yy) from x
     double k0 = 0, k1x = 0, k1y = 0, ka = 0, kb2 = 0, kd = 0;
-    if (parab) {
-        k0 = P.sqdelta - (Q[0] * Q[0] + Q[1] * Q[1]);
-        k1x = 2.0 * (Q[0] * e[0] + Q[1] * e[1]);
-        k1y = 2.0 * (Q[0] * e[2] + Q[1] * e[3]);
+    auto parab_at = [&](double yx, double yy) {
+        k0 = P.sqdelta - (yx * yx + yy * yy);
+        k1x = 2.0 * (yx * e[0] + yy * e[1]);
+        k1y = 2.0 * (yx * e[2] + yy * e[3]);
         ka = e[0] * e[0] + e[1] * e[1];
         kb2 = 2.0 * (e[0] * e[2] + e[1] * e[3]);
         kd = e[2] * e[2] + e[3] * e[3];
-    }
+    };
     auto from_moments = [&](double f, const double *I) {   // I: integrals of the kernel times 1, r1, r2, r1^2, r1 r2, r2^2
         S0 = f * I[0];
         S1[0] = f * (I[0] - I[1] - I[2]); S1[1] = f * I[1]; S1[2] = f * I[2];
         S2[0] = f * (I[1] - I[3] - I[4]); S2[1] = f * (I[2] - I[4] - I[5]); S2[2] = f * I[4];
+    };
+    auto from_moments_at = [&](double o1, double o2, const double *I) {   // the same of u = r - (o1, o2)
+        const double o0 = 1.0 - o1 - o2, i12 = I[1] + I[2];
+        S0 = I[0];
+        S1[0] = o0 * I[0] - i12; S1[1] = o1 * I[0] + I[1]; S1[2] = o2 * I[0] + I[2];
+        S2[0] = o0 * S1[1] - o1 * i12 - (I[3] + I[4]);
+        S2[1] = o0 * S1[2] - o2 * i12 - (I[4] + I[5]);
+        S2[2] = o1 * S1[2] + (o2 * I[1] + I[4]);
     };
     auto sum_point = [&](double k, int i, double *I) {   // inner point i with kernel value k
         I[0] += k * rule.dy[i];
@@ -381,6 +413,7 @@ __device__ __forceinline__ bool f64_item(const ProbParams &P, const Rule &rule, 
     };
     if (KIND == MIX_REGULAR && parab && inside) {
         nsub++;
+        parab_at(Q[0], Q[1]);
         const double *m = pr.mom, *h = pr.mom4;
         auto sum = [&](double c, double cx, double cy, double cxx, double cxy, double cyy) {
             return k0 * c - (k1x * cx + k1y * cy) - (ka * cxx + kb2 * cxy + kd * cyy);
@@ -405,57 +438,49 @@ __device__ __forceinline__ bool f64_item(const ProbParams &P, const Rule &rule, 
             return LATE;
         }
         if (Y.n >= 3) nsub += Y.n - 2;
-        if (KIND == MIX_CONST && (exact & 1)) {
-            if (Y.n >= 3) {
-                double A = 0, Mx = 0, My = 0, Mxx = 0, Mxy = 0, Myy = 0;
-#pragma unroll 1
-                for (unsigned sg = Y.seg; sg; sg &= sg - 1) {   // sides through the origin's edges add nothing
-                    const int j = __ffs(sg) - 1, i = j ? j - 1 : Y.n - 1;
-                    const double x0 = Y.L[2 * i], y0 = Y.L[2 * i + 1], x1 = Y.L[2 * j], y1 = Y.L[2 * j + 1];
-                    const double c = x0 * y1 - x1 * y0, sx = x0 + x1, sy = y0 + y1;
-                    A += c;
-                    Mx = fma(c, sx, Mx);
-                    My = fma(c, sy, My);
-                    Mxx = fma(c, fma(sx, sx, -(x0 * x1)), Mxx);
-                    Myy = fma(c, fma(sy, sy, -(y0 * y1)), Myy);
-                    Mxy = fma(c, fma(sx, sy, fma(x0, y0, x1 * y1)), Mxy);
-                }
-                const double f = P.kc * adet;
-                A *= 0.5 * f;
-                Mx *= (1.0 / 6.0) * f;
-                My *= (1.0 / 6.0) * f;
-                Mxx *= (1.0 / 12.0) * f;
-                Myy *= (1.0 / 12.0) * f;
-                Mxy *= (1.0 / 24.0) * f;
-                S0 = A;
-                S1[0] = A - Mx - My; S1[1] = Mx; S1[2] = My;
-                S2[0] = Mx - Mxx - Mxy; S2[1] = My - Mxy - Myy; S2[2] = Mxy;
-            }
-        } else if (KIND == MIX_REGULAR && parab && (exact & 2)) {
+        if ((KIND == MIX_CONST && (exact & 1)) || (KIND == MIX_REGULAR && parab && (exact & 2))) {
             double I[6] = {0, 0, 0, 0, 0, 0};
+            const double o1 = Y.L[0], o2 = Y.L[1];
+            if (KIND != MIX_CONST && Y.n >= 3) parab_at(Y.R[0], Y.R[1]);
             const double k02 = 0.5 * k0, k03 = (1.0 / 3.0) * k0, k04 = 0.25 * k0;
-            if (Y.n < 3) Y.seg = 0;
+            double x1 = Y.L[2] - o1, y1 = Y.L[3] - o2;
 #pragma unroll 1
-            for (unsigned sg = Y.seg; sg; sg &= sg - 1) {
-                const int j = __ffs(sg) - 1, i = j ? j - 1 : Y.n - 1;
-                const double x0 = Y.L[2 * i], y0 = Y.L[2 * i + 1], dx = Y.L[2 * j] - x0, dy = Y.L[2 * j + 1] - y0;
-                const double c = x0 * dy - dx * y0;
+            for (int j = 2; j < Y.n; j++) {
+                const double x0 = x1, y0 = y1;
+                x1 = Y.L[2 * j] - o1;
+                y1 = Y.L[2 * j + 1] - o2;
+                const double c = fabs(x0 * y1 - x1 * y0);
+                if (KIND == MIX_CONST) {
+                    const double sx = x0 + x1, sy = y0 + y1;
+                    I[0] += c;
+                    I[1] = fma(c, sx, I[1]);
+                    I[2] = fma(c, sy, I[2]);
+                    I[3] = fma(c, fma(sx, sx, -(x0 * x1)), I[3]);
+                    I[4] = fma(c, fma(sx, sy, fma(x0, y0, x1 * y1)), I[4]);
+                    I[5] = fma(c, fma(sy, sy, -(y0 * y1)), I[5]);
+                } else {
+                    const double dx = x1 - x0, dy = y1 - y0;
 #pragma unroll
-                for (int g = 0; g < 3; g++) {
-                    const double t = g == 1 ? 0.5 : (g == 0 ? 0.11270166537925831 : 0.8872983346207417);
-                    const double zx = fma(t, dx, x0), zy = fma(t, dy, y0), cg = c * (g == 1 ? 4.0 / 9.0 : 5.0 / 18.0);
-                    const double k1 = k1x * zx + k1y * zy, k2 = zx * (ka * zx) + zy * (kb2 * zx + kd * zy);
-                    const double w0 = cg * (k02 - (1.0 / 3.0) * k1 - 0.25 * k2), w1 = cg * (k03 - 0.25 * k1 - 0.2 * k2);
-                    const double w2 = cg * (k04 - 0.2 * k1 - (1.0 / 6.0) * k2), tx = w2 * zx;
-                    I[0] += w0;
-                    I[1] += w1 * zx;
-                    I[2] += w1 * zy;
-                    I[3] += tx * zx;
-                    I[4] += tx * zy;
-                    I[5] += (w2 * zy) * zy;
+                    for (int g = 0; g < 3; g++) {
+                        const double t = g == 1 ? 0.5 : (g == 0 ? 0.11270166537925831 : 0.8872983346207417);
+                        const double zx = fma(t, dx, x0), zy = fma(t, dy, y0), cg = c * (g == 1 ? 4.0 / 9.0 : 5.0 / 18.0);
+                        const double k1 = k1x * zx + k1y * zy, k2 = zx * (ka * zx) + zy * (kb2 * zx + kd * zy);
+                        const double w0 = cg * (k02 - (1.0 / 3.0) * k1 - 0.25 * k2), w1 = cg * (k03 - 0.25 * k1 - 0.2 * k2);
+                        const double w2 = cg * (k04 - 0.2 * k1 - (1.0 / 6.0) * k2), tx = w2 * zx;
+                        I[0] += w0;
+                        I[1] += w1 * zx;
+                        I[2] += w1 * zy;
+                        I[3] += tx * zx;
+                        I[4] += tx * zy;
+                        I[5] += (w2 * zy) * zy;
+                    }
                 }
             }
-            from_moments(P.kc * adet, I);
+            const double f = P.kc * adet;
+            I[0] *= KIND == MIX_CONST ? 0.5 * f : f;
+#pragma unroll
+            for (int q = 1; q < 6; q++) I[q] *= KIND != MIX_CONST ? f : (q < 3 ? (1.0 / 6.0) * f : (q == 4 ? (1.0 / 24.0) * f : (1.0 / 12.0) * f));
+            if (Y.n >= 3) from_moments_at(o1, o2, I);
         } else if (KIND == MIX_CONST) {   // the rule's moments on each fan triangle (see item_cut_const)
             const double m0 = pr.mom[0], mx = pr.mom[1], my = pr.mom[2], mxx = pr.mom[3], mxy = pr.mom[4], myy = pr.mom[5];
             const double la[3] = {1.0 - Y.L[0] - Y.L[1], Y.L[0], Y.L[1]};
@@ -525,7 +550,6 @@ __device__ __noinline__ unsigned f64_item_late(const ProbParams *P, const Rule &
 template <int KIND>
 __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule rule, PassRuleT<double> pr) {
     constexpr bool CK = KIND == MIX_CONST;
-    constexpr int NW = f64_words(KIND);
     extern __shared__ __align__(16) unsigned char s_raw[];
     const PassArgs &a = fa.m.p;
     const SlotMap &sm = fa.m.m;
@@ -533,15 +557,15 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
     const int nPx = rule.nPx;
     double *tab = reinterpret_cast<double *>(s_raw);   // mask sums (constant kernels)
     unsigned char *wbase = reinterpret_cast<unsigned char *>(tab + (CK ? 7 * f64_tab_entries(nPx) : 0));
-    wbase = s_raw + ((wbase - s_raw) + 15) / 16 * 16 + (size_t)wib * ((f64_warp_bytes(KIND, nPx) + 15) / 16 * 16);
+    wbase = s_raw + ((wbase - s_raw) + 15) / 16 * 16 + (size_t)wib * ((f64_warp_bytes(nPx) + 15) / 16 * 16);
     F64Warp &W = *reinterpret_cast<F64Warp *>(wbase);
     double *x64 = reinterpret_cast<double *>(wbase + (sizeof(F64Warp) + 15) / 16 * 16);   // [nPx][2]
     F2 *xf = reinterpret_cast<F2 *>(x64 + 2 * nPx);                                       // [nPx]
     double *coef = reinterpret_cast<double *>(xf + nPx);   // [nPx][7]: |T| dx times psi_r, psi_r psi_c (r < c), 1
     unsigned char *work = reinterpret_cast<unsigned char *>(coef + 7 * nPx);
-    long long *acc = reinterpret_cast<long long *>(work);                                 // [32][f64_acc]
-    double *res = reinterpret_cast<double *>(acc + 32 * f64_acc(KIND));                   // [F64_CAP][F64_RN]
-    F64Entry<NW> *slist = reinterpret_cast<F64Entry<NW> *>(work);
+    long long *acc = reinterpret_cast<long long *>(work);                                 // [32][F64_ACC]
+    double *res = reinterpret_cast<double *>(acc + 32 * F64_ACC);                   // [F64_CAP][F64_RN]
+    F64Entry *slist = reinterpret_cast<F64Entry *>(work);
     if (CK) {
         for (int i = threadIdx.x; i < 7 * f64_tab_entries(nPx); i += F64_THREADS) tab[i] = fa.mtab[i];
         __syncthreads();
@@ -701,26 +725,19 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                     const int ri = o < 9 ? 1 + o % 3 : (o < 12 ? 0 : o - 8);
                     double v = 0;
                     for (int i = W.ps[r], e = i + W.pn[r]; i < e; i++) v += coef[7 * (W.list[i] & 31) + ci] * res[i * F64_RN + ri];
-                    long long *A = &acc[pl * f64_acc(KIND)];
-                    if (o >= 9 && o < 12) {
-                        A[o] = __double_as_longlong(v);
-                    } else {
-                        const int ex = o < 9 ? (8 * F64_BITS - P.xN - W.te[o / 3] - W.pve[pl][o % 3]) >> 3 : F64_BITS - P.xD - W.pe[pl];
-                        const double q = scale2(v, ex);
-                        const long long iv = f64_fix(q, o < 9 ? limN : limE, bad);
-                        A[o] = iv;
-                        if (o >= 12) A[o + 3] = f64_fix_lo(q, iv);
-                        else if (NW == 2) A[F64_OUT + 3 + o] = f64_fix_lo(q, iv);
-                    }
+                    long long *A = &acc[pl * F64_ACC];
+                    if (o < 12) A[o] = __double_as_longlong(v);
+                    else f64_split2(scale2(v, F64_BITS - P.xD - W.pe[pl]), limE, bad, A[o], A[o + 3]);
                 }
                 __syncwarp();
                 base = end;
                 basein = endin;
             }
-            // owner: the pair's blocks as integers (termLocal stays FP64, summed per lane)
-            long long nx[9 * NW];
+            // owner: the pair's termNonloc (termLocal is summed per lane)
+            const long long *A = &acc[lane * F64_ACC];
+            double nx[9];
 #pragma unroll
-            for (int i = 0; i < 9 * NW; i++) nx[i] = 0;
+            for (int i = 0; i < 9; i++) nx[i] = cnt ? __longlong_as_double(A[i]) : 0.0;
             long long *ep = &fa.m.elp[(long long)part * F64_ELP];
             if (CK && inm) {   // inside items: kc |T| |b| times the rule's sums
                 double m[7];
@@ -734,23 +751,17 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                 for (int c = 0; c < 3; c++) {
                     const double iN = kr * pr.insum[1 + c];
 #pragma unroll
-                    for (int r = 0; r < 3; r++) nx[3 * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve[c]) >> 3), limN, bad);
+                    for (int r = 0; r < 3; r++) nx[3 * r + c] = fma(m[r], iN, nx[3 * r + c]);
                 }
                 const double kl = kr * pr.insum[0];
 #pragma unroll
                 for (int q = 0; q < 3; q++) D[q] += m[3 + q] * kl;
-                const double q = m[6] * dTs;
-                const long long iv = f64_fix(q, limE, bad);
-                red_add(ep, 0, iv);
-                red_add(ep, 1, f64_fix_lo(q, iv));
+                long long hi, lo;
+                f64_split2(m[6] * dTs, limE, bad, hi, lo);
+                red_add(ep, 0, hi);
+                if (lo) red_add(ep, 1, lo);
             }
             if (cnt) {
-                const long long *A = &acc[lane * f64_acc(KIND)];
-#pragma unroll
-                for (int i = 0; i < 9; i++) {
-                    nx[i] += A[i];
-                    if (NW == 2) nx[NW == 2 ? 9 + i : 0] += A[F64_OUT + 3 + i];
-                }
 #pragma unroll
                 for (int q = 0; q < 3; q++) D[q] += __longlong_as_double(A[9 + q]);
 #pragma unroll
@@ -766,67 +777,89 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                     D[0] += cb[1]; D[1] += cb[2]; D[2] += cb[5];
 #pragma unroll
                     for (int q = 0; q < 3; q++) {
-                        const double v = scale2(cb[q == 2 ? 23 : 19 + q], F64_BITS - P.xD - eb);
-                        const long long iv = f64_fix(v, limE, bad);
-                        red_add(ep, 2 + q, iv);
-                        red_add(ep, 5 + q, f64_fix_lo(v, iv));
+                        long long hi, lo;
+                        f64_split2(scale2(cb[q == 2 ? 23 : 19 + q], F64_BITS - P.xD - eb), limE, bad, hi, lo);
+                        red_add(ep, 2 + q, hi);
+                        red_add(ep, 5 + q, lo);
                     }
 #pragma unroll
-                    for (int i = 0; i < 9; i++) {
-                        const double q = scale2(cb[9 + i], (et[i / 3] - ve[i % 3]) >> 3);
-                        nx[i] = f64_fix(q, limN, bad);
-                        if (NW == 2) nx[NW == 2 ? 9 + i : 0] = f64_fix_lo(q, nx[i]);
-                    }
+                    for (int i = 0; i < 9; i++) nx[i] = cb[9 + i];
                 }
             }
             // termNonloc into T's own rows: lanes sharing a partner vertex add their integers, all
             // lanes share the (vertex, row) lookups; the mirrored entries come from k_sym_add_f64
             __syncwarp();
             int nent = 0;
+            auto slot_of = [&](int r, int col) {   // of T's row r; -2: no such entry is kept
+                RowHash h;
+                h.hb = W.rhb[r]; h.rb = W.rrb[r]; h.mask = W.rmask[r]; h.lo = W.rlo[r];
+                if (col == W.tvs[r]) return -2LL;   // the matrix diagonal: from the row sum
+                if (h.mask != 0xffffffffu) return slot_find_row(sm, h, col);
+                if (a.labV[col] > 0) return slot_find(sm, col, W.tvs[r]);   // T's vertex has no row: the mirror
+                return -2LL;
+            };
 #pragma unroll 1
             for (int c = 0; c < 3; c++) {
                 const int col = act ? sel3(pv, c) : -1;
+                long long o[3], ol[3], s[3], sl[3];
+                double q[3];
+                unsigned rests = 0;
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    bool rest = false;
+                    q[r] = scale2(sel3(&nx[3 * r], c), (et[r] - sel3(ve, c)) >> 3);
+                    f64_split(q[r], limN, bad, o[r], ol[r], rest);
+                    rests |= (unsigned)rest << r;
+                    s[r] = o[r];
+                    sl[r] = ol[r];
+                }
+                if (__any_sync(FULL, rests)) {   // slivers (about one cut item in 1000): third integers
+#pragma unroll
+                    for (int r = 0; r < 3; r++) {
+                        const long long st = (rests >> r) & 1u ? slot_of(r, col) : -1;
+                        if (st < 0) continue;   // the scatter below reports what is missing
+                        red_add(fa.valsNt, st, f64_third(q[r]));
+                        a.err[F64_ERR_THIRD] = 1;
+                    }
+                }
+                const bool wide = __any_sync(FULL, ol[0] | ol[1] | ol[2]);
                 const unsigned grp = __match_any_sync(FULL, col);
                 const bool leader = (__ffs(grp) - 1) == lane;
                 const int maxn = __reduce_max_sync(FULL, (unsigned)__popc(grp));
-                long long o[3 * NW], s[3 * NW];
-#pragma unroll
-                for (int r = 0; r < 3 * NW; r++) o[r] = s[r] = sel3(&nx[3 * r], c);
                 unsigned rest = grp & ~(1u << lane);
                 for (int it = 1; it < maxn; it++) {
                     const int src = rest ? __ffs(rest) - 1 : lane;
                     const bool use = rest != 0;
                     if (rest) rest &= rest - 1;
 #pragma unroll
-                    for (int r = 0; r < 3 * NW; r++) {
+                    for (int r = 0; r < 3; r++) {
                         const long long t = shfl64(o[r], src);
                         if (use) s[r] += t;
+                    }
+                    if (!wide) continue;
+#pragma unroll
+                    for (int r = 0; r < 3; r++) {
+                        const long long t = shfl64(ol[r], src);
+                        if (use) sl[r] += t;
                     }
                 }
                 const bool put = leader && col >= 0;
                 const unsigned m = __ballot_sync(FULL, put);
                 if (put) {
-                    F64Entry<NW> &e = slist[nent + __popc(m & lanemask_lt())];
+                    F64Entry &e = slist[nent + __popc(m & lanemask_lt())];
                     e.col = col;
 #pragma unroll
-                    for (int r = 0; r < 3 * NW; r++) e.v[r] = s[r];
+                    for (int r = 0; r < 3; r++) { e.v[r] = s[r]; e.v[3 + r] = sl[r]; }
                 }
                 nent += __popc(m);
             }
             __syncwarp();
             for (int w = lane; w < 3 * nent; w += 32) {
                 const int e = w / 3, r = w - 3 * e;
-                const int col = slist[e].col;
-                if (col == W.tvs[r]) continue;   // the matrix diagonal: from the row sum
-                RowHash h;
-                h.hb = W.rhb[r]; h.rb = W.rrb[r]; h.mask = W.rmask[r]; h.lo = W.rlo[r];
-                long long s;
-                if (h.mask != 0xffffffffu) s = slot_find_row(sm, h, col);
-                else if (a.labV[col] > 0) s = slot_find(sm, col, W.tvs[r]);   // T's vertex has no row: the mirror
-                else continue;
-                if (s < 0) { miss = true; continue; }
-                red_add(fa.m.valsN, s, slist[e].v[r]);
-                if (NW == 2) red_add(fa.valsNlo, s, slist[e].v[3 + r]);
+                const long long st = slot_of(r, slist[e].col);
+                if (st < 0) { miss |= st == -1; continue; }
+                red_add(fa.m.valsN, 2 * st, slist[e].v[r]);
+                if (slist[e].v[3 + r]) red_add(fa.m.valsN, 2 * st + 1, slist[e].v[3 + r]);
             }
             __syncwarp();
         }
@@ -838,10 +871,10 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
             const int s = sm.dslot[(long long)T * 9 + lane];
             const double d = r + c == 1 ? D[0] : (r + c == 2 ? D[1] : D[2]);
             if (s >= 0) {
-                const double q = scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3));
-                const long long iv = f64_fix(q, CK ? F64_BITS : P.limD, bad);
-                red_add(vals, s, iv);
-                red_add(fa.valslo, s, f64_fix_lo(q, iv));
+                long long hi, lo;
+                f64_split2(scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3)), CK ? F64_BITS : P.limD, bad, hi, lo);
+                red_add(vals, s, hi);
+                red_add(fa.valslo, s, lo);
             } else if (keepmask & (1u << r)) miss = true;
         }
         __syncwarp();
@@ -899,10 +932,10 @@ __global__ void k_elem_blocks_f64(const long long *__restrict__ elp, const doubl
             if (r == c) continue;   // the diagonal comes from the row sum (k_sym_add_f64)
             const int v = T32[e * 3 + r], s = dslot[e * 9 + 3 * r + c];
             if (s >= 0) {
-                const double q = scale2(b[r + c - 1], F64_BITS - P.xD - ((vexp[v] + 7) >> 3));
-                const long long iv = f64_fix(q, P.limD, bad);
-                red_add(vals, s, iv);
-                red_add(valslo, s, f64_fix_lo(q, iv));
+                long long hi, lo;
+                f64_split2(scale2(b[r + c - 1], F64_BITS - P.xD - ((vexp[v] + 7) >> 3)), P.limD, bad, hi, lo);
+                red_add(vals, s, hi);
+                red_add(valslo, s, lo);
             } else if (labV[v] > 0) {
                 atomicOr(&err[3], 1);
             }
@@ -916,12 +949,19 @@ __global__ void k_elem_blocks_f64(const long long *__restrict__ elp, const doubl
 // twice).
 __global__ void k_sym_add_f64(const long long *__restrict__ rowptr, const int *__restrict__ cols,
                               const int *__restrict__ tpos, const long long *__restrict__ valsN,
-                              const long long *__restrict__ valsNlo, const long long *__restrict__ valslo,
+                              const long long *__restrict__ valsNt, const long long *__restrict__ valslo,
                               const int *__restrict__ vexp, const int *__restrict__ vprob,
-                              const ProbParams *__restrict__ probs, long long nrows, double *__restrict__ vals) {
+                              const ProbParams *__restrict__ probs, long long nrows, const int *__restrict__ err,
+                              double *__restrict__ vals) {
     const int lane = threadIdx.x & 31;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    const bool third = err[F64_ERR_THIRD] != 0;
+    const longlong2 *N = reinterpret_cast<const longlong2 *>(valsN);
+    auto sum_of = [&](long long s) {
+        const longlong2 q = N[s];
+        return f64_join(q.x, q.y, third ? valsNt[s] : 0);
+    };
     for (long long t = gw; t < nrows; t += nw) {
         const long long b = rowptr[t], e = rowptr[t + 1];
         if (b == e) continue;
@@ -934,11 +974,11 @@ __global__ void k_sym_add_f64(const long long *__restrict__ rowptr, const int *_
             if (v == (int)t) { dslot = s; continue; }
             const int tp = tpos ? tpos[s] : -1;
             const long long ts = tp >= 0 ? rowptr[v] + tp : -1;
-            double q = valsNlo ? f64_join(valsN[s], valsNlo[s]) : (double)valsN[s];
-            if (ts >= 0) q += valsNlo ? f64_join(valsN[ts], valsNlo[ts]) : (double)valsN[ts];
+            double q = sum_of(s);
+            if (ts >= 0) q += sum_of(ts);
             const long long dh = reinterpret_cast<const long long *>(vals)[s];
             double x = -scale2(q, -((eN - vexp[v]) >> 3));
-            if (dh) x += scale2(f64_join(dh, valslo[s]), eD);   // a slot of a diagonal block
+            if (dh | valslo[s]) x += scale2(f64_join(dh, valslo[s]), eD);   // a slot of a diagonal block
             vals[s] = x;
             off += x;
         }

@@ -7,8 +7,8 @@
 // distance (the exact FP64 test inside its margin). That leaves about 45 FP64 instructions per 3D
 // pair: products and conversions of its (dim + 1)^2 termNonloc entries. The general pass runs the
 // outer x inner point loop (121 kernel values per pair with 11-point rules) on the FP64 pipe instead.
-// Sums and their units are those of passes_f64.cuh (termNonloc per slot, termLocal with second
-// integers in the diagonal-block slots); k_sym_add_f64 without transposed slots completes the rows.
+// Sums and their units are those of passes_f64.cuh (two integers per sum, third ones for what is far
+// below the units); k_sym_add_f64 without transposed slots completes the rows.
 #pragma once
 #include "passes_f64.cuh"
 
@@ -21,7 +21,8 @@ struct F64BaryWarp {
     long long rhb[DIM + 1], rrb[DIM + 1];   // T's rows (see MixWarp)
     unsigned rmask[DIM + 1];
     int rlo[DIM + 1], tvs[DIM + 1], te[DIM + 1];
-    long long val[32 * bary_vals(DIM)];     // a batch's integers, and the groups of its partner vertices
+    long long val[32 * bary_vals(DIM)];     // a batch's integers,
+    long long low[32 * bary_vals(DIM)];     // their second integers, and the groups of its partner vertices
     VertexGroup list[32 * (DIM + 1)];         // (see k_pass_bary)
 };
 // outer sums per mask: psi_r, then psi_r psi_c off the diagonal; an odd stride keeps the banks apart
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                 }
             }
             nitin += __popc(inm);
-            long long nx[dV * dV];
+            double nx[dV * dV];
 #pragma unroll
             for (int i = 0; i < dV * dV; i++) nx[i] = 0;
             if (inm) {
@@ -146,15 +147,39 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                     const int ve = fa.vexp[pv[c]];
                     const double iN = kr * pr.insum[1 + c];
 #pragma unroll
-                    for (int r = 0; r < dV; r++) nx[dV * r + c] = f64_fix(scale2(m[r] * iN, (et[r] - ve) >> 3), F64_BITS, bad);
+                    for (int r = 0; r < dV; r++) nx[dV * r + c] = scale2(m[r] * iN, (et[r] - ve) >> 3);
                 }
                 const double kl = kr * pr.insum[0];
 #pragma unroll
                 for (int q = 0; q < NO; q++) D[q] += m[dV + q] * kl;
             }
             // termNonloc into T's rows: sums per partner vertex and lookups shared by the lanes
+            bool rest = false, low = false;
 #pragma unroll
-            for (int i = 0; i < dV * dV; i++) W.val[lane * VS + i] = nx[i];
+            for (int i = 0; i < dV * dV; i++) {
+                f64_split(nx[i], F64_BITS, bad, W.val[lane * VS + i], W.low[lane * VS + i], rest);
+                low |= W.low[lane * VS + i] != 0;
+            }
+            low = __any_sync(FULL, low);
+            if (__any_sync(FULL, rest)) {   // elements far smaller than their neighbours
+                for (int i = 0; rest && i < dV * dV; i++) {
+                    const int r = i / dV, c = i - dV * r, col = a.T32[(long long)part * dV + c];
+                    double q = 0;
+#pragma unroll
+                    for (int j = 0; j < dV * dV; j++) q = j == i ? nx[j] : q;
+                    long long hi, lo;
+                    bool third = false, dummy = false;
+                    f64_split(q, F64_BITS, dummy, hi, lo, third);
+                    RowHash h;
+                    h.hb = W.rhb[r]; h.rb = W.rrb[r]; h.mask = W.rmask[r]; h.lo = W.rlo[r];
+                    if (!third || h.mask == 0xffffffffu || col == W.tvs[r]) continue;
+                    const long long s = slot_find_row(sm, h, col);
+                    if (s < 0) continue;   // the scatter below reports it
+                    red_add(fa.valsNt, s, f64_third(q));
+                    a.err[F64_ERR_THIRD] = 1;
+                }
+                __syncwarp();
+            }
             int nent = 0;
 #pragma unroll
             for (int c = 0; c < dV; c++) {
@@ -178,12 +203,18 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                 const int col = W.list[e].col;
                 if (h.mask == 0xffffffffu || col == W.tvs[r]) continue;   // no row; the matrix diagonal: from the row sum
                 const SlotProbe pb = slot_probe_begin(sm, h, col);
-                const long long *v = &W.val[dV * r + W.list[e].c];
-                long long sn = 0;
+                const long long *v = &W.val[dV * r + W.list[e].c], *vl = &W.low[dV * r + W.list[e].c];
+                long long sn = 0, sl = 0;
                 for (unsigned mm = W.list[e].lanes; mm; mm &= mm - 1) sn += v[(__ffs(mm) - 1) * VS];
+                if (low)
+                    for (unsigned mm = W.list[e].lanes; mm; mm &= mm - 1) sl += vl[(__ffs(mm) - 1) * VS];
                 const long long s = slot_probe_end(sm, h, col, pb);
-                if (s < 0) miss = true;
-                else red_add(fa.m.valsN, s, sn);
+                if (s < 0) {
+                    miss = true;
+                } else {
+                    red_add(fa.m.valsN, 2 * s, sn);
+                    if (sl) red_add(fa.m.valsN, 2 * s + 1, sl);
+                }
             }
             __syncwarp();
         }
@@ -204,10 +235,10 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_bary_f64(F64Args fa, Ru
                 if (s < 0) {
                     miss = true;
                 } else {
-                    const double q = scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3));
-                    const long long iv = f64_fix(q, F64_BITS, bad);
-                    red_add(vals, s, iv);
-                    red_add(fa.valslo, s, f64_fix_lo(q, iv));
+                    long long hi, lo;
+                    f64_split2(scale2(d, F64_BITS - P.xD - ((W.te[r] + 7) >> 3)), F64_BITS, bad, hi, lo);
+                    red_add(vals, s, hi);
+                    red_add(fa.valslo, s, lo);
                 }
             }
         }

@@ -279,7 +279,20 @@ static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, const MeshScan
     if (bary) kbound *= 2.0;   // the rule's weight 2
     if (P.kernel == KER_PARABOLA) kbound *= cy * cy;   // inner points outside the polygon
     if (P.singular) kbound *= 1048576.0;
-    const double CN = kbound * *std::max_element(px, px + 4) * sy * cy, CD = 2 * kbound * sx * cx * cx * sy * cy * cy * atot;
+    // the inner sum of |psi_c|: a rule of nonnegative weights and inner points that is exact for linear functions
+    // gives a part of the element at most the whole's integral (the 7- and 16-point rules: 1/6 instead of 1/2)
+    double in1 = 0;
+    bool linear = cy <= 1.0 + 1e-12;
+    for (int j = 0; j < dim; j++) {
+        double first = 0;
+        for (int k = 0; k < p.nPy; k++) {
+            linear = linear && p.dy[k] >= 0;
+            first += p.dy[k] * p.Py[dim * k + j];
+        }
+        linear = linear && fabs(first * (dim + 1) - sy) <= 1e-13 * sy;
+        in1 = std::max(in1, first * (1 + 1e-9));
+    }
+    const double CN = kbound * *std::max_element(px, px + 4) * (linear ? in1 : sy * cy), CD = 2 * kbound * sx * cx * cx * sy * cy * cy * atot;
     if (!(CN > 1e-120 && CN < 1e120 && CD > 1e-120 && CD < 1e120 && sx > 1e-30 && atot > 1e-60 && atot < 1e60 && m.amax < 1e60)) return;
     P.xN = (int)ceil(8.0 * log2(CN) + 1e-3);
     P.xD = exact_ceil_log2(CD);
@@ -546,7 +559,7 @@ struct Session {
     bool cert = false;         // the pair search takes the certified FP32 geometry
     DevBuf pw;                 // power tables of the singular kernels (FP64), PW_N numbers per problem
     DevBuf idet;               // 1 / det per element (FP64 retriangulate pass)
-    DevBuf vexp, valsNlo, valslo, mtab;   // FP64 one-sided passes: vertex exponents, second integers, mask table
+    DevBuf vexp, valsNt, valslo, mtab;   // FP64 one-sided passes: vertex exponents, lower integers, mask table
     DevBuf vcnt, vptr, vel, adjcnt, xadj, adj;
     DevBuf stamp_epoch;   // per-warp stamp epochs of the search
     long long stamp_layout[3] = {0, 0, 0};   // warps, element and vertex stride the stamps were laid out for
@@ -607,7 +620,7 @@ struct Session {
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
                 &hcap, &hptr, &htab, &tpos, &dslot, &rwords, &rbase, &rlo, &rankmap, &eid_ptr, &eid, &vp_cnt, &vp_off, &vp_ptr, &vp_scratch, &pscratch, &rowoff, &kclist, &valsN, &elp,
                 &po_cnt, &po_off, &po_ptr, &po_scratch, &tcnt, &tptr, &tcols, &sv_vec, &sv_part, &zptr, &zidx, &vacc, &vtiny,
-                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNlo, &valslo, &mtab, &pw, &idet};
+                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNt, &valslo, &mtab, &pw, &idet};
     }
     ~Session() {
         for (DevBuf *b : buffers()) b->release();
@@ -1828,19 +1841,17 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     int nl = 0;
     int r = class_launches(S, L, &nl);
     if (r) return r;
-    bool wide = false;
-    for (int i = 0; i < nl; i++) wide = wide || L[i].cls == MIX_SINGULAR;
     ENS(S.vexp, sizeof(int) * (S.nV + 1));
-    ENS(S.valsN, sizeof(long long) * (nnz + 1));
+    ENS(S.valsN, 2 * sizeof(long long) * (nnz + 1));
+    ENS(S.valsNt, sizeof(long long) * (nnz + 1));
     const size_t elp_bytes = sizeof(long long) * F64_ELP * (S.nE + 1);
     if (retri) ENS(S.elp, elp_bytes);
     ENS(S.valslo, sizeof(long long) * (nnz + 1));
-    if (wide) ENS(S.valsNlo, sizeof(long long) * (nnz + 1));
     k_vexp<<<grid_for(S.nV, 256), 256, 0, S.st>>>(S.vptr.get<long long>(), S.vel.get<int>(), S.adet.get<double>(), S.nV, S.vexp.get<int>()); ++S.nlaunch;
-    CK(cudaMemsetAsync(S.valsN.p, 0, sizeof(long long) * (nnz + 1), S.st));
+    CK(cudaMemsetAsync(S.valsN.p, 0, 2 * sizeof(long long) * (nnz + 1), S.st));
+    CK(cudaMemsetAsync(S.valsNt.p, 0, sizeof(long long) * (nnz + 1), S.st));
     if (retri) CK(cudaMemsetAsync(S.elp.p, 0, elp_bytes, S.st));
     CK(cudaMemsetAsync(S.valslo.p, 0, sizeof(long long) * (nnz + 1), S.st));
-    if (wide) CK(cudaMemsetAsync(S.valsNlo.p, 0, sizeof(long long) * (nnz + 1), S.st));
     CK(cudaMemsetAsync(S.err.get<int>() + 5, 0, sizeof(int), S.st));
     const int tab_n = f64_tab_entries(S.rule.nPx), tab_ts = retri ? 7 : f64_bary_tab<DIM>();
     ENS(S.mtab, sizeof(double) * tab_n * tab_ts);
@@ -1870,7 +1881,7 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     fa.m.elp = S.elp.get<long long>();
     fa.vexp = S.vexp.get<int>();
     fa.idet = S.idet.get<double>();
-    fa.valsNlo = wide ? S.valsNlo.get<long long>() : nullptr;
+    fa.valsNt = S.valsNt.get<long long>();
     fa.valslo = S.valslo.get<long long>();
     for (int i = 0; i < nl; i++) {
         if (L[i].count == 0) continue;
@@ -1889,7 +1900,7 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
     }
     if (retri) k_elem_blocks_f64<<<grid_for(S.nE, 256), 256, 0, S.st>>>(fa.m.elp, S.adet.get<double>(), fa.vexp, S.dslot.get<int>(), S.T32.get<int>(), S.labV.get<int>(), S.eprob.get<int>(), S.prm.get<ProbParams>(), pr.insum[5], pr.insum[6], pr.insum[8], S.nE, S.vals.get<long long>(), fa.valslo, S.err.get<int>());
     S.nlaunch += retri;
-    k_sym_add_f64<<<S.nSM * 16, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.cols.get<int>(), retri ? S.tpos.get<int>() : nullptr, fa.m.valsN, fa.valsNlo, fa.valslo, fa.vexp, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.nV, S.vals.get<double>()); ++S.nlaunch;
+    k_sym_add_f64<<<S.nSM * 16, 256, 0, S.st>>>(S.rowptr.get<long long>(), S.cols.get<int>(), retri ? S.tpos.get<int>() : nullptr, fa.m.valsN, fa.valsNt, fa.valslo, fa.vexp, S.vprob.get<int>(), S.prm.get<ProbParams>(), S.nV, S.err.get<int>(), S.vals.get<double>()); ++S.nlaunch;
     CK(cudaGetLastError());
     return NLFEM_OK;   // the range flag (err[5]) is read with the number of entries (run_finish)
 }

@@ -1350,3 +1350,50 @@ def test_fp64_singular_sums_on_graded_meshes(nl, orc, n, s, p, seed, onesided):
                 check(sess.download(0), st)
         finally:
             sess.close()
+
+
+def _tiny_elements_mesh():
+    """Vertices moved to within 1e-7 cells of a neighbour: elements 1e-7 of the others beside them."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(14, 0.1, jitter=0.2, seed=91)
+    for i in (52, 97, 130, 171):
+        v[i] = v[i + 1] + 1e-7 / 14 * np.array([-1.0, 0.3])
+    return meshes.mesh_dict(v, e, l)
+
+
+@pytest.mark.parametrize("case", ["constant", "parabola", "parabola_nocaps", "constant16", "graded", "vanishing", "tiny_bary", "cube"])
+def test_fp64_every_entry(nl, orc, case):
+    """Every matrix entry of the one-sided FP64 passes to eight digits, not only the large ones: entries from
+    slivers that a sphere cuts off are down to 1e-24 of the largest. The bound is the rounding of the
+    coordinates (2^-53 of about 1.5) over the least depth of a polygon that the certified structure leaves to
+    the pass's own formulas (2^-18 of the horizon, 0.1), times eight."""
+    from nlfem_gb300 import meshes, _lib
+    c, delta, kern = conf2d(), 0.1, "parabola"
+    if case == "vanishing":   # the mesh of test_fp64_pass_keeps_vanishing_entries
+        delta = 0.1099
+        v, e, l = meshes.regular_square(26, delta, jitter=0.2, seed=26)
+        rng = np.random.Generator(np.random.PCG64(475299725))
+        s, t = int(rng.integers(1, len(v))), int(rng.integers(1, len(e)))
+        v = v + rng.uniform(-0.5, 0.5, 2)
+        m = meshes.mesh_dict(np.roll(v, s, axis=0), np.roll((e + s) % len(v), t, axis=0), np.roll(l, t))
+    elif case == "graded":
+        delta, m = 0.3, _graded_mesh(16, 0.3, 3.0, 3)
+    elif case == "tiny_bary":
+        delta, kern, m, c = 0.15, "constant", _tiny_elements_mesh(), conf2d(method="baryCenter")
+    elif case == "cube":
+        delta, kern, m, c = 0.2, "constant3D", cube_mesh(8, 0.1, jitter=0.2, seed=1), conf3d()
+    else:
+        m = square_mesh(32, delta, jitter=0.2, seed=1)
+        if case.startswith("constant"):
+            kern = "constant"
+        if case == "constant16":
+            c = conf2d(rule="16")
+        if case == "parabola_nocaps":
+            c = conf2d(caps=0)
+    k = {"function": kern, "horizon": delta, "outputdim": 1}
+    A = nl.stiffnessMatrix(m, k, c).tocsr()
+    assert _lib.stats()["slot_map"] != 0
+    B = orc.assemble(m, k, c)["A"].tocsr()
+    assert same_pattern(A, B)
+    off = np.abs(A.data - B.data) / np.abs(B.data)
+    assert off.max() < 1e-8, (off.max(), np.abs(B.data)[off.argmax()] / np.abs(B.data).max())
