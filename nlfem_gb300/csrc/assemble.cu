@@ -413,19 +413,25 @@ __device__ __forceinline__ int bfs_test(const BfsArgs &a, const ProbParams &P, i
 // are all tested before the walk goes on.
 // An element's list holds the near pairs (HIT_NEAR) first, then the others: the passes take pairs in
 // batches of a warp, and a batch of near pairs has no class to find and no cut item to wait for. In 2D
-// both are in element order, by two bitmaps over a window of elements: the walk tests one element of
-// each of 32 vertices at a time, so that a batch of its order has about 69 distinct vertices (of 96) to
-// look up, one of neighbouring elements 34 where the numbering has any locality. At n = 256, delta = 0.1
-// the search takes 1.8 ms more for it, the mixed pass 37.1 instead of 47.2 ms (FP64, n = 128: 18.8
-// instead of 19.8). A list that spans more than BFS_WINDOWS windows (a numbering without locality, where
-// the order gives nothing and every window costs a pass over the queue) keeps the walk's order. 3D too:
-// there a step holds the tetrahedra of a few vertices already (element order: pass 8.7 -> 8.5 ms, search
-// 15.0 -> 16.6 at 6 * 32^3).
+// both can be put in element order, by two bitmaps over a window of elements: the walk tests one element
+// of each of 32 vertices at a time, so that a batch of its order has about 69 distinct vertices (of 96) to
+// look up; a batch in element order has 34 of them in a row-major mesh, 81 in a shuffled one. Two
+// conditions, by times of whole assemblies (mixed, constant kernel):
+//   * The problem's numbering is local (ProbParams::local): few distinct vertices in 32 consecutive elements.
+//     Element order against the walk's, n = 256, delta = 0.1, the mesh's elements shuffled in blocks of
+//     B: 0.97 of the time for B = 64 (34 vertices), 0.99 for 8 (40), 1.00 for 6 (44), 1.01 for 4 (48), 1.09 for
+//     2 (64), 1.27 for 1 (96); n = 128: 0.985, 1.00, 1.00, 1.02, 1.06, 1.14. In Morton order (26) 0.89.
+//   * The list has BFS_FILL pairs per window, since every window costs a pass over the queue and its bitmaps:
+//     n = 256 in blocks of 64 with 180 pairs per window 0.97, 80: 1.00, 25: 1.07, 8: 1.12; row-major with 640
+//     (delta = 0.06): 0.93, 200: 0.99, 90: 1.00, 49: 1.02.
+// The lists' order is that of the problem alone (windows are laid from its first element), so a batch
+// gives every problem the sums of its single assembly. 3D keeps the walk's order: there a step holds the
+// tetrahedra of a few vertices already (element order: pass 8.7 -> 8.5 ms, search 15.0 -> 16.6 at 6 * 32^3).
 constexpr int BFS_UNROLL = 4;
 // Mark of a near pair in the queue. Elements lie below it: the stamps alone of 2^30 elements take 5 TB.
 constexpr int NEAR = 1 << 30;
 constexpr int BFS_BITS = 256;     // words of an ordering bitmap: a window of 8192 elements
-constexpr int BFS_WINDOWS = 16;   // lists over more windows keep the walk's order
+constexpr int BFS_FILL = 96;      // least pairs per window of a list in element order
 // Outer elements are handed out in chunks of consecutive indices (at most BFS_CHUNK, fewer near
 // the end): neighbouring elements (in a mesh numbered with any locality) meet largely the same
 // candidates, so the warp's stamps of the previous element are still in cache for the next one.
@@ -703,8 +709,8 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
             if (!fits) atomicOr(&a.err[1], 1);
         }
         if (!fits) continue;
-        const int e00 = bmin & ~31;
-        if (DIM == 2 && npairs > 0 && (bmax - e00) / (32 * BFS_BITS) < BFS_WINDOWS) {   // in element order
+        const int e00 = (int)eoff + ((bmin - (int)eoff) & ~31);
+        if (DIM == 2 && P.local && npairs >= ((bmax - e00) / (32 * BFS_BITS) + 1) * BFS_FILL) {   // in element order
             unsigned *bm = s_buf[wib];   // bits of the near pairs, then of the others
             long long wn = (long long)base, wf = wn + nnear;
             for (int e0 = e00; e0 <= bmax; e0 += 32 * BFS_BITS) {

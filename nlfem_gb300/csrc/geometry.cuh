@@ -335,6 +335,7 @@ struct ProbParams {
     double el;        // mean element measure (bounding box / nE), for capacity estimates
     int cert;         // the certified FP32 geometry may decide the search and the classes (certified.cuh):
                       // element sizes, horizon and coordinates in its range
+    int local;        // consecutive elements share vertices: pair lists may be put in element order (k_bfs)
     int f64ok;        // the one-sided FP64 pass takes this problem (passes_f64.cuh)
     int xN, xD, xS;   // its fixed-point bounds: 2^(xN / 8) above a pair's termNonloc per |T| |b|, 2^xD above
                       // its diagonal blocks times the mesh's |det| sum, 2^xS above the outer weights' sum times that

@@ -237,6 +237,21 @@ static MeshScan scan_mesh(const nlfem_problem &p) {
     return m;
 }
 
+// Whether the numbering is local: 32 consecutive elements have at most 42 distinct vertices (of 96 in 2D;
+// row-major 34, no locality 96; the line by measurement, see k_bfs), by 16 groups spread over the mesh.
+static bool local_numbering(const nlfem_problem &p) {
+    const long dV = p.dim + 1, len = std::min<long>(p.nE, 32), groups = std::min<long>(16, p.nE / len);
+    std::vector<long> v(dV * len);
+    long distinct = 0;
+    for (long g = 0; g < groups; g++) {
+        const long *t = &p.elements[dV * (g * ((p.nE - len) / std::max<long>(groups - 1, 1)))];
+        std::copy(t, t + dV * len, v.begin());
+        std::sort(v.begin(), v.end());
+        distinct += std::unique(v.begin(), v.end()) - v.begin();
+    }
+    return 32 * distinct <= 42 * groups * len;
+}
+
 // Whether a one-sided FP64 pass takes the problem (passes_f64.cuh, the 2D retriangulate rule;
 // passes_f64_bary.cuh, the barycenter rule with a constant kernel), and the bounds its units follow
 // from. A pair's blocks are at most kbound |T| |b| times the rules' absolute sums (CN, CD: basis
@@ -460,6 +475,7 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
     MeshScan scan;
     if (system) {
         scan = p.dim == 2 ? scan_mesh<2>(p) : scan_mesh<3>(p);
+        P.local = p.dim == 2 && local_numbering(p);
         const double lim = p.precision == NLFEM_PREC_MIXED ? MIX_MAX_H_OVER_DELTA : 512.0;
         if (p.precision != NLFEM_PREC_FP64 && scan.hmax2 > lim * lim * p.sqdelta)
             return fail(NLFEM_ERR_UNSUPPORTED, std::string("precision \"") + (p.precision == NLFEM_PREC_MIXED ? "mixed" : "fp64-onesided") +

@@ -1397,3 +1397,21 @@ def test_fp64_every_entry(nl, orc, case):
     assert same_pattern(A, B)
     off = np.abs(A.data - B.data) / np.abs(B.data)
     assert off.max() < 1e-8, (off.max(), np.abs(B.data)[off.argmax()] / np.abs(B.data).max())
+
+
+@pytest.mark.parametrize("n,delta,shuffled", [(260, 0.02, True), (260, 0.02, False), (200, 0.012, False), (60, 0.1, False)])
+def test_fp64_batch_keeps_the_pair_order(nl, n, delta, shuffled):
+    """FP64 forms an element's own block in floating point, in the order of its pair list. That order is the
+    problem's alone (element order or the walk's, at any span of the list's element numbers), so a problem behind
+    another one in a batch gives the bits of its single assembly."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(n, delta, jitter=0.2, seed=5)
+    if shuffled:
+        pe = np.random.default_rng(n).permutation(len(e))
+        e, l = e[pe], l[pe]
+    k = {"function": "constant", "horizon": delta, "outputdim": 1}
+    m, c = meshes.mesh_dict(v, e, l), conf2d()
+    A = nl.stiffnessMatrix(m, k, c).tocsr()
+    first = square_mesh(3, 0.1)   # 18 elements: no multiple of a bitmap word
+    B = nl.stiffnessMatrix_batch([(first, KC, c), (m, k, c)])[1].tocsr()
+    assert same_pattern(A, B) and np.array_equal(A.data, B.data)
