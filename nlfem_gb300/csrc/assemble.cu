@@ -206,7 +206,7 @@ struct BfsArgs {
     int *seg_cnt, *seg_near; // pairs of a segment; the first seg_near of them are near (HIT_NEAR)
     unsigned long long *n_cand;
     unsigned long long *work;   // next outer element to hand out (chunks of BFS_CHUNK)
-    int *err;                // [0] queue overflow, [1] pool overflow, [2] bad method
+    int *err;                // [0] queue overflow, [1] pool overflow, [2] some element has no pair
     long long *qneed;
 };
 
@@ -707,6 +707,7 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
             a.seg_near[aT] = nnear;
             a.seg_start[aT] = (long long)base;
             if (!fits) atomicOr(&a.err[1], 1);
+            if (npairs == 0) a.err[2] = 1;
         }
         if (!fits) continue;
         const int e00 = (int)eoff + ((bmin - (int)eoff) & ~31);
@@ -818,6 +819,8 @@ struct RowArgs {
     // rows' elements' vertex lists (vpool / vseg_start / vseg_cnt: mode 0 run over elements, each
     // element its own row, lists its partners' vertices and its own)
     int mode, all_rows;
+    const int *lone;           // elements without out-pairs that are partners (null: there are none): their
+                               // lists hold their own vertices, for the blocks that their pairs add to them
     const int *vpool;
     const long long *vseg_start;
     const int *vseg_cnt;
@@ -877,6 +880,18 @@ __global__ void __launch_bounds__(256) k_row_pattern(RowArgs a, int pass) {
     }
 }
 
+// Marks the partners that have no out-pairs themselves (RowArgs::lone). One warp per element.
+__global__ void k_lone_partners(RowArgs a, long long nE, int *__restrict__ lone) {
+    const int lane = threadIdx.x & 31;
+    const long long T = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (T >= nE) return;
+    const long long ob = a.out_ptr[T], oe = a.out_cnt ? ob + a.out_cnt[T] : a.out_ptr[T + 1];
+    for (long long i = ob + lane; i < oe; i += 32) {
+        const int b = a.pB[i];
+        if ((a.out_cnt ? (long long)a.out_cnt[b] : a.out_ptr[b + 1] - a.out_ptr[b]) == 0) lone[b] = 1;
+    }
+}
+
 // Same row sets with the marks as a bitmap over the problem's vertices in shared memory (words
 // 32-bit words per warp): a shared-memory atomicOr replaces the global exchange, and the set
 // bits come out in increasing order, so the rows need no sort. pass 0 counts, pass 1 writes.
@@ -933,7 +948,7 @@ __global__ void __launch_bounds__(256) k_row_pattern_bm(RowArgs a, int pass, int
             const int T = a.vel[t];
             const long long ob = a.out_ptr[T], oe = a.out_cnt ? ob + a.out_cnt[T] : a.out_ptr[T + 1];
             const long long ib = a.in_ptr ? a.in_ptr[T] : 0, ie = a.in_ptr ? a.in_ptr[T + 1] : 0;
-            if (oe == ob && ie == ib) continue;
+            if (oe == ob && ie == ib && !(a.lone && a.lone[T])) continue;
             const int nout = (int)(oe - ob), nEl = 1 + nout + (int)(ie - ib);
             for (int el_i = lane; el_i < nEl; el_i += 32) {   // one partner element per lane
                 int el;

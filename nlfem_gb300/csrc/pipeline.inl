@@ -586,6 +586,8 @@ struct Session {
     DevBuf hcap, hptr, htab, tpos, dslot;   // slot maps of the one-sided passes
     DevBuf rwords, rbase, rlo, rankmap;      // window-rank slot map (slots.cuh)
     // one-sided passes: per element, the vertices of its partners and its own (row patterns)
+    bool lone_elements = false;             // the search found elements without a pair
+    DevBuf lone;                            // those of them that are partners (2D retriangulate pattern)
     DevBuf eid_ptr, eid, vp_cnt, vp_off, vp_ptr, vp_scratch;
     long long vp_cap = 0;
     bool vlists = false;
@@ -636,7 +638,7 @@ struct Session {
                 &EChi, &EClo, &adetf, &BCf, &color, &color2, &colorlist, &closeA, &closeB, &closebuf, &touched,
                 &hcap, &hptr, &htab, &tpos, &dslot, &rwords, &rbase, &rlo, &rankmap, &eid_ptr, &eid, &vp_cnt, &vp_off, &vp_ptr, &vp_scratch, &pscratch, &rowoff, &kclist, &valsN, &elp,
                 &po_cnt, &po_off, &po_ptr, &po_scratch, &tcnt, &tptr, &tcols, &sv_vec, &sv_part, &zptr, &zidx, &vacc, &vtiny,
-                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNt, &valslo, &mtab, &pw, &idet};
+                &dgT32, &dglabV, &dgvprob, &dgvptr, &dgvel, &vexp, &valsNt, &valslo, &mtab, &pw, &idet, &lone};
     }
     ~Session() {
         for (DevBuf *b : buffers()) b->release();
@@ -1127,12 +1129,13 @@ static int run_bfs(Session &S) {
         CK(cudaGetLastError());
         if (S.replay) return NLFEM_OK;   // overflow flags are checked after the replay
         unsigned long long hc[3];
-        int he[2];
-        int r = d2h2(S, hc, cnt, 3, he, S.err.get<int>(), 2);
+        int he[3];
+        int r = d2h2(S, hc, cnt, 3, he, S.err.get<int>(), 3);
         if (r) return r;
         S.P = (long long)hc[0];   // pool cursor: the pairs found
         if (he[0]) { S.qcap = std::max<long long>((long long)hc[2] * 3 / 2, S.qcap * 2); continue; }
         if (he[1]) { S.pool_cap = (long long)hc[0] + (long long)hc[0] / 8 + 1024; continue; }
+        S.lone_elements = he[2] != 0;
         S.stats.n_candidates = (long)hc[1];
         return NLFEM_OK;
     }
@@ -1352,7 +1355,7 @@ static int run_rows_direct(Session &S, RowArgs o, long long nrows, DevBuf &cnt, 
     return NLFEM_OK;
 }
 
-// Per element, the vertices of its partners and its own (none without a partner): the bitmap
+// Per element, the vertices of its partners and its own (none where it is in no pair): the bitmap
 // kernel in mode 0 over elements, each element the only member of its own row. The one-sided
 // passes' row patterns are then unions of these lists (mode 2).
 template <int DIM>
@@ -1365,6 +1368,12 @@ static int run_elem_vlists(Session &S, const RowArgs &a, int words, int threads,
     o.in_ptr = nullptr;
     o.all_rows = 1;
     o.mode = 0;
+    if (S.pmode == PM_RETRI && S.lone_elements) {   // two-sided blocks: partners without out-pairs have lists too
+        ENS(S.lone, sizeof(int) * (nE + 1));
+        CK(cudaMemsetAsync(S.lone.p, 0, sizeof(int) * (nE + 1), S.st));
+        k_lone_partners<<<grid_for(nE * 32, 256), 256, 0, S.st>>>(a, nE, S.lone.get<int>()); ++S.nlaunch;
+        o.lone = S.lone.get<int>();
+    }
     o.vptr = S.eid_ptr.get<long long>(); o.vel = S.eid.get<int>(); o.vprob = S.eprob.get<int>(); o.nV = nE;
     int r = run_rows_direct<DIM>(S, o, nE, S.vp_cnt, S.vp_off, S.vp_ptr, S.vp_scratch, S.vp_cap, 15, 11,
                                  words, threads, grid, smem);

@@ -1415,3 +1415,34 @@ def test_fp64_batch_keeps_the_pair_order(nl, n, delta, shuffled):
     first = square_mesh(3, 0.1)   # 18 elements: no multiple of a bitmap word
     B = nl.stiffnessMatrix_batch([(first, KC, c), (m, k, c)])[1].tocsr()
     assert same_pattern(A, B) and np.array_equal(A.data, B.data)
+
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed", "fp64-onesided"])
+@pytest.mark.parametrize("kern,h_over_delta", [("constant", 4), ("parabola", 6), ("constant", 6), ("constant", 10)])
+def test_partners_without_pairs_of_their_own(nl, orc, kern, h_over_delta, prec):
+    """With the centroid rule and elements of 4 to 14 horizons, some elements are partners (a neighbour's ball
+    reaches into them) without any pair of their own, not even with themselves (their own ball lies inside
+    them: no polygon). Their vertices' rows hold the blocks that their pairs add to them."""
+    from nlfem_gb300 import quadrules
+    m = square_mesh(14, 0.1, jitter=0.25, seed=8)
+    k = {"function": kern, "horizon": 1.2 / 14 * np.sqrt(2.0) / h_over_delta, "outputdim": 1}
+    P, w = quadrules.centroid1()
+    c = conf2d(precision=prec)
+    c["quadrature"] = {"outer": {"points": P, "weights": w}, "inner": {"points": P, "weights": w}}
+    r = orc.assemble(m, k, c, want_pairs=True)
+    B = r["A"]
+    assert len(np.setdiff1d(r["pairs"][:, 1], r["pairs"][:, 0])) > 0
+    A = nl.stiffnessMatrix(dict(m), k, c)
+    assert same_pattern(A, B)
+    if prec != "mixed":   # (these matrices are slivers only, where FP32 has no fixed accuracy)
+        fro, mx = rel_errors(A, B)
+        assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+    s = nl.Session([(dict(m), k, c)])
+    try:
+        for _ in range(3):
+            s.assemble(graph=True)
+            C = s.download(0)
+            assert same_pattern(A, C) and np.array_equal(A.tocsr().data, C.data)
+    finally:
+        s.close()
