@@ -228,6 +228,23 @@ __device__ __forceinline__ double f64_div(double a, double b) {
     return fma(y, fma(-b, q, a), q);
 }
 
+// Classes by FP64 tests, for problems outside the certified FP32 range (precision "fp64-onesided" only;
+// "fp64" takes the general pass there): triangle Q relative to the ball's center, inside and outside with a
+// margin of 2^-40, far above the tests' rounding for elements up to 512 horizons; the rest is cut.
+constexpr double MARG_D64 = 1.0 / 1099511627776.0;
+__device__ __noinline__ int f64_class(double sq, const double *x, const double *Eb) {
+    const double sqlo = sq * (1.0 - MARG_D64), sqhi = sq * (1.0 + MARG_D64);
+    bool in = true, out = true;
+    for (int i = 0; i < 3; i++) {
+        const int j = i == 2 ? 0 : i + 1;
+        const double px = Eb[2 * i] - x[0], py = Eb[2 * i + 1] - x[1], ux = Eb[2 * j] - Eb[2 * i], uy = Eb[2 * j + 1] - Eb[2 * i + 1];
+        const double pp = px * px + py * py, pu = px * ux + py * uy, uu = ux * ux + uy * uy, cr = px * uy - py * ux;
+        in = in && pp < sqlo;
+        out = out && pp > sqhi && (!(pu < 0.0 && -pu < uu) || cr * cr > sqhi * uu);   // the end point, then the side
+    }
+    return in ? CLS_IN : (out ? CLS_OUT : CLS_CUT);
+}
+
 // Kernel value from r2 = |x - y|^2; pw the problem's power table (singular kernels).
 template <int KIND>
 __device__ __forceinline__ double f64_kernel(const ProbParams &P, const double *pw, double r2) {
@@ -665,7 +682,7 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                 for (int k = 0; k < (near ? 0 : nPx); k++) {
                     const F2 x = xf[k];
                     const F2 Q[3] = {f2(pc[0] - x.x, pc[1] - x.y), f2(pc[2] - x.x, pc[3] - x.y), f2(pc[4] - x.x, pc[5] - x.y)};
-                    const int c = fclassify(Q, P.sqdelta_f);
+                    const int c = P.cert ? fclassify(Q, P.sqdelta_f) : f64_class(P.sqdelta, &x64[2 * k], &a.EC[(long long)part * 6]);
                     inm |= (unsigned)(c == CLS_IN) << k;
                     cutm |= (unsigned)(c == CLS_CUT) << k;
                 }
@@ -706,7 +723,8 @@ __global__ void __launch_bounds__(F64_THREADS, 3) k_pass_f64(F64Args fa, Rule ru
                     for (int i0 = first + lane, r = 0; i0 < past; i0 += 32, r++) {
                         const int i = CK ? i0 : W.order[i0], it = W.list[i], k = it & 31, j = it >> 6, b = W.pid[j];
                         const F2 xk = xf[k], Qf[3] = {W.pc[j][0] - xk, W.pc[j][1] - xk, W.pc[j][2] - xk};
-                        if (!f64_item<KIND, false>(P, rule, pr, !CK && part0 == 0, fa.exact, pw, &x64[2 * k], Qf, &a.EC[(long long)b * 6],
+                        const bool inside = !CK && part0 == 0;
+                        if ((!P.cert && !inside) || !f64_item<KIND, false>(P, rule, pr, inside, fa.exact, pw, &x64[2 * k], Qf, &a.EC[(long long)b * 6],
                                                    a.adet[b], fa.idet[b], &res[i * F64_RN], nsub))
                             late |= 1u << r;
                     }

@@ -265,10 +265,10 @@ static bool local_numbering(const nlfem_problem &p) {
 // Elements near degenerate (where the reference's
 // solve2x2 may abort; the barycenter rule never calls it), bounds far outside the exponent range
 // and options that need the general pass go there. fp64-onesided, which has no such pass to match,
-// is bound only by the range.
+// is bound only by the range; outside the certified tests' range it takes FP64 ones.
 static void set_f64_bounds(const nlfem_problem &p, ProbParams &P, const MeshScan &m, double kbound) {
     P.f64ok = 0;
-    if (!P.cert || !m.known || p.outdim != 1 || p.is_dg) return;
+    if ((!P.cert && p.precision == NLFEM_PREC_FP64) || !m.known || p.outdim != 1 || p.is_dg) return;
     if (p.nPx <= 0 || p.nPx > MAXQ || p.nPy <= 0 || p.nPy > MAXQ || !p.Px || !p.dx || !p.Py || !p.dy) return;   // make_rule reports it
     const bool bary = P.remote == MTH_BARYCENTER;
     if (bary ? P.kernel != KER_CONSTANT && P.kernel != KER_CONSTANT3D

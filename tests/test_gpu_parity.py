@@ -1446,3 +1446,27 @@ def test_partners_without_pairs_of_their_own(nl, orc, kern, h_over_delta, prec):
             assert same_pattern(A, C) and np.array_equal(A.tocsr().data, C.data)
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("kern,h_over_delta,shift", [("constant", 30, 0.0), ("parabola", 52, 0.0), ("constant", 260, 0.0),
+                                                     ("fractional", 52, 0.0), ("constant", 0.3, 4e4)])
+def test_fp64_onesided_outside_the_certified_range(nl, orc, kern, h_over_delta, shift):
+    """precision "fp64-onesided" stays one-sided for elements of 16 to 512 horizons and for meshes far from the
+    origin, where its classes come from FP64 tests and every cut polygon from the exact routine."""
+    from nlfem_gb300 import meshes, _lib
+    n, delta = 24, 1.2 / 24 * np.sqrt(2.0) / h_over_delta
+    v, e, l = meshes.regular_square(n, 0.1, jitter=0.2, seed=33)
+    m = meshes.mesh_dict(v + shift, e, l)
+    k = {"function": kern, "horizon": delta, "outputdim": 1}
+    c = conf2d()
+    if kern == "fractional":
+        k["fractional_s"] = 0.4
+        c = conf2d(rule="16", close="fractional", deg=3)
+    A = nl.stiffnessMatrix(m, k, dict(c, precision="fp64-onesided"))
+    assert _lib.stats()["slot_map"] != 0
+    B = orc.assemble(m, k, c)["A"]
+    assert same_pattern(A, B)
+    if B.nnz:
+        fro, mx = rel_errors(A, B)
+        tol = FP64_TOL + 64 * 1.1e-16 * shift / 0.05   # the reference's polygon points are absolute
+        assert fro < tol and mx < tol, (fro, mx)
