@@ -423,7 +423,9 @@ __device__ __forceinline__ int bfs_test(const BfsArgs &a, const ProbParams &P, i
 //     2 (64), 1.27 for 1 (96); n = 128: 0.985, 1.00, 1.00, 1.02, 1.06, 1.14. In Morton order (26) 0.89.
 //   * The list has BFS_FILL pairs per window, since every window costs a pass over the queue and its bitmaps:
 //     n = 256 in blocks of 64 with 180 pairs per window 0.97, 80: 1.00, 25: 1.07, 8: 1.12; row-major with 640
-//     (delta = 0.06): 0.93, 200: 0.99, 90: 1.00, 49: 1.02.
+//     (delta = 0.06): 0.93, 200: 0.99, 90: 1.00, 49: 1.02. Problems of at most one list per search warp
+//     (16 on each of 152 SMs) need fewer: the windows then cost no throughput, and the passes' chains of
+//     batches get shorter (FP64, n = 32, 73 pairs: 0.95; n = 24, 44: 0.98; n = 16, 28: 1.03 for the parabola).
 // The lists' order is that of the problem alone (windows are laid from its first element), so a batch
 // gives every problem the sums of its single assembly. 3D keeps the walk's order: there a step holds the
 // tetrahedra of a few vertices already (element order: pass 8.7 -> 8.5 ms, search 15.0 -> 16.6 at 6 * 32^3).
@@ -431,7 +433,8 @@ constexpr int BFS_UNROLL = 4;
 // Mark of a near pair in the queue. Elements lie below it: the stamps alone of 2^30 elements take 5 TB.
 constexpr int NEAR = 1 << 30;
 constexpr int BFS_BITS = 256;     // words of an ordering bitmap: a window of 8192 elements
-constexpr int BFS_FILL = 96;      // least pairs per window of a list in element order
+constexpr int BFS_FILL = 96, BFS_FILL_FEW = 32, BFS_FEW = 16 * 152;   // least pairs per window of a list in element
+                                  // order, in problems of more and of at most BFS_FEW elements
 // Outer elements are handed out in chunks of consecutive indices (at most BFS_CHUNK, fewer near
 // the end): neighbouring elements (in a mesh numbered with any locality) meet largely the same
 // candidates, so the warp's stamps of the previous element are still in cache for the next one.
@@ -711,7 +714,7 @@ __global__ void __launch_bounds__(BFS_THREADS, DIM == 3 ? 4 : 2) k_bfs(BfsArgs a
         }
         if (!fits) continue;
         const int e00 = (int)eoff + ((bmin - (int)eoff) & ~31);
-        if (DIM == 2 && P.local && npairs >= ((bmax - e00) / (32 * BFS_BITS) + 1) * BFS_FILL) {   // in element order
+        if (DIM == 2 && P.local && npairs >= ((bmax - e00) / (32 * BFS_BITS) + 1) * (P.nE <= BFS_FEW ? BFS_FILL_FEW : BFS_FILL)) {   // in element order
             unsigned *bm = s_buf[wib];   // bits of the near pairs, then of the others
             long long wn = (long long)base, wf = wn + nnear;
             for (int e0 = e00; e0 <= bmax; e0 += 32 * BFS_BITS) {
