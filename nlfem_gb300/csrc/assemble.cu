@@ -117,15 +117,22 @@ __global__ void k_prep_vertices(const long long *__restrict__ lab64, const int *
 }
 
 // ------------------------------------------------------------------ dual graph
-__global__ void k_vinc_count(const int *__restrict__ T32, long long n, int *__restrict__ vcnt) {
+// Whether vertex reference i repeats one of its element (a collapsed element). Such an element is listed once
+// at the vertex: the 3D search takes the elements of a list for distinct.
+__device__ __forceinline__ bool vref_repeats(const int *__restrict__ T32, long long i, int dV) {
+    for (int r = (int)(i % dV); r > 0; r--)
+        if (T32[i - r] == T32[i]) return true;
+    return false;
+}
+__global__ void k_vinc_count(const int *__restrict__ T32, long long n, int dV, int *__restrict__ vcnt) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) atomicAdd(&vcnt[T32[i]], 1);
+    if (i < n && !vref_repeats(T32, i, dV)) atomicAdd(&vcnt[T32[i]], 1);
 }
 __global__ void k_vinc_fill(const int *__restrict__ T32, long long n, int dV,
                             const long long *__restrict__ vptr, int *__restrict__ vfill,
                             int *__restrict__ vel) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || vref_repeats(T32, i, dV)) return;
     int v = T32[i];
     long long pos = vptr[v] + atomicAdd(&vfill[v], 1);
     vel[pos] = (int)(i / dV);

@@ -1015,7 +1015,7 @@ static int run_dual(Session &S) {
     ENS(S.vptr, sizeof(long long) * (nV + 1));
     ENS(S.vel, sizeof(int) * nE * dV);
     CK(cudaMemsetAsync(S.vcnt.p, 0, sizeof(int) * (nV + 1), S.st));
-    k_vinc_count<<<grid_for(nE * dV, 256), 256, 0, S.st>>>(S.T32.get<int>(), nE * dV, S.vcnt.get<int>()); ++S.nlaunch;
+    k_vinc_count<<<grid_for(nE * dV, 256), 256, 0, S.st>>>(S.T32.get<int>(), nE * dV, dV, S.vcnt.get<int>()); ++S.nlaunch;
     int r = scan_excl<int>(S, S.vcnt.get<int>(), nV, S.vptr.get<long long>());
     if (r) return r;
     CK(cudaMemsetAsync(S.vcnt.p, 0, sizeof(int) * (nV + 1), S.st));

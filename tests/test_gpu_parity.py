@@ -1470,3 +1470,22 @@ def test_fp64_onesided_outside_the_certified_range(nl, orc, kern, h_over_delta, 
         fro, mx = rel_errors(A, B)
         tol = FP64_TOL + 64 * 1.1e-16 * shift / 0.05   # the reference's polygon points are absolute
         assert fro < tol and mx < tol, (fro, mx)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_3d_search_elements_naming_a_vertex_twice(nl, orc, prec):
+    """Collapsed tetrahedra (a vertex named twice or three times) are found once like any other element: the pair
+    list and the matrix are the oracle's."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_cube(4, 0.1, jitter=0.15, seed=6)
+    extra = np.array([[e[10][0], e[10][0], e[10][1], e[10][2]], [e[50][1], e[50][3], e[50][1], e[50][0]],
+                      [e[90][2], e[90][2], e[90][2], e[90][3]]])
+    m = meshes.mesh_dict(v, np.vstack([e, extra]), np.concatenate([l, [1, 1, 1]]))
+    k = {"function": "constant3D", "horizon": 0.4, "outputdim": 1}
+    ref = orc.assemble(m, k, conf3d(), want_pairs=True)
+    got = nl.pair_list(m, k, conf3d(precision=prec))
+    np.testing.assert_array_equal(got, ref["pairs"][np.lexsort((ref["pairs"][:, 1], ref["pairs"][:, 0]))])
+    A = nl.stiffnessMatrix(m, k, conf3d(precision=prec))
+    fro, mx = rel_errors(A, ref["A"])
+    tol = FP64_TOL if prec == "fp64" else 1e-6
+    assert fro < tol and mx < tol, (fro, mx)
