@@ -486,9 +486,16 @@ static int make_params(const nlfem_problem &p, bool system, ProbParams &P) {
         // The margins also assume that the squares and products of the tests stay normal FP32
         // numbers, and that a double-float pair holds a coordinate to far below 2^-24 delta (its own
         // rounding is 2^-48 of the coordinate). The FP64 paths check both.
-        double cmax = 0;
+        // The outer points' offsets from a vertex are FP32 numbers too, so a rule with points outside of its
+        // element counts as an element that large.
+        double cmax = 0, reach = 1;
+        for (int k = 0; p.Px && k < std::min(p.nPx, MAXQ); k++) {
+            double sum = 0;
+            for (int j = 0; j < p.dim; j++) sum += fabs(p.Px[(long)p.dim * k + j]);
+            reach = std::max(reach, sum);
+        }
         for (int j = 0; j < p.dim; j++) cmax = std::max(cmax, std::max(fabs(lo[j]), fabs(hi[j])));
-        P.cert = finite == 0 && scan.hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
+        P.cert = finite == 0 && reach * reach * scan.hmax2 <= MIX_MAX_H_OVER_DELTA * MIX_MAX_H_OVER_DELTA * p.sqdelta && cmax <= 65536.0 * P.delta &&
                  p.sqdelta < 1e14 && std::min(scan.hmin2, p.sqdelta) > 1e-24 && scan.hmin2 * p.sqdelta > 1e-28;
     }
     double mag, kbound = 0;   // kbound: bound of |kernel| inside the ball (estimate for singular kernels)

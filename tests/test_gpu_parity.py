@@ -1489,3 +1489,22 @@ def test_3d_search_elements_naming_a_vertex_twice(nl, orc, prec):
     fro, mx = rel_errors(A, ref["A"])
     tol = FP64_TOL if prec == "fp64" else 1e-6
     assert fro < tol and mx < tol, (fro, mx)
+
+
+@pytest.mark.parametrize("method", ["retriangulate", "baryCenter"])
+@pytest.mark.parametrize("h_over_delta,onesided", [(1.0, True), (10.0, False)])
+def test_fp64_outer_points_outside_the_element(nl, orc, method, h_over_delta, onesided):
+    """The FP32 tests that decide fp64's search and classes hold for offsets of at most 16 horizons. An outer rule
+    with points at 9 element sizes leaves that range with elements of 10 horizons: the FP64 routines take over."""
+    from nlfem_gb300 import _lib, quadrules
+    m = square_mesh(12, 0.1, jitter=0.2, seed=14)
+    k = {"function": "constant", "horizon": 1.2 / 12 * np.sqrt(2.0) / h_over_delta, "outputdim": 1}
+    c = conf2d(method=method)
+    c["quadrature"]["outer"] = {"points": np.array([[6.0, -3.0], [-3.0, -2.0], [-2.0, 6.0]]), "weights": np.full(3, 1 / 6)}
+    A = nl.stiffnessMatrix(m, k, c)
+    assert (_lib.stats()["slot_map"] != 0) == onesided
+    B = orc.assemble(m, k, c)["A"]
+    assert same_pattern(A, B)
+    if B.nnz:
+        fro, mx = rel_errors(A, B)
+        assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
