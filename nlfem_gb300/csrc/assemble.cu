@@ -437,7 +437,8 @@ __device__ __forceinline__ int bfs_test(const BfsArgs &a, const ProbParams &P, i
 // gives every problem the sums of its single assembly. 3D keeps the walk's order: there a step holds the
 // tetrahedra of a few vertices already (element order: pass 8.7 -> 8.5 ms, search 15.0 -> 16.6 at 6 * 32^3).
 constexpr int BFS_UNROLL = 4;
-// Mark of a near pair in the queue. Elements lie below it: the stamps alone of 2^30 elements take 5 TB.
+// Mark of a near pair in the queue. Elements lie below it (checked in session_init; 2^30 elements need about
+// 200 bytes each for the mesh and the search before the first pair, so no call that fits a GPU is refused).
 constexpr int NEAR = 1 << 30;
 constexpr int BFS_BITS = 256;     // words of an ordering bitmap: a window of 8192 elements
 constexpr int BFS_FILL = 96, BFS_FILL_FEW = 32, BFS_FEW = 16 * 152;   // least pairs per window of a list in element

@@ -740,6 +740,10 @@ static int session_init(Session &S, const nlfem_problem *probs, int n, bool syst
     S.hprm.resize(n);
     S.eoff.assign(n + 1, 0);
     S.voff.assign(n + 1, 0);
+    long long elements = 0;   // before anything walks over them
+    for (int i = 0; i < n; i++) elements += std::max<long>(probs[i].nE, 0);
+    if (system && elements >= NEAR)
+        return fail(NLFEM_ERR_UNSUPPORTED, "batch too large (2^30 elements: the pair search marks near pairs by bit 30)");
     for (int i = 0; i < n; i++) {
         const nlfem_problem &p = probs[i];
         if (p.dim != S.dim) return fail(NLFEM_ERR_INVALID, "all problems of a batch must share the dimension");

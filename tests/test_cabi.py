@@ -143,3 +143,16 @@ def test_reference_configuration_checks(lib):
         with pytest.raises(_lib.NlfemError, match="Please set fractional_s") as e:
             nlfem.stiffnessMatrix(mm, k, conf2d(close="fractional", deg=3))
         assert e.value.code == 1
+
+
+def test_batch_of_2_30_elements_refused(lib):
+    """The pair search marks near pairs by bit 30 of the element number, so a call holds fewer than 2^30 elements
+    in all its problems. Judged by the counts alone, before the arrays are walked."""
+    from nlfem_gb300 import nlfem, _lib
+    p = nlfem._Problem(square_mesh(4), {"function": "constant", "horizon": 0.1, "outputdim": 1}, conf2d(), system=True)
+    probs = (_lib.Problem * 2)(p.c, p.c)
+    for q in probs:
+        q.nE = 1 << 29
+    outs = (_lib.CSR32 * 2)()
+    assert lib.nlfem_stiffness_batch32(probs, 2, outs) == 4
+    assert b"2^30" in lib.nlfem_last_error()
