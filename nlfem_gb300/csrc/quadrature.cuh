@@ -499,6 +499,29 @@ __global__ void k_close_list(QuadArgs a, int *list, unsigned long long *count) {
     list[i] = (int)p;
 }
 
+// Power tables (pw_eval): table p for problem p's kernel kc |z|^-expo.
+__global__ void k_pw_table(const ProbParams *__restrict__ probs, int nProb, double *__restrict__ tab) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, p = i / PW_N, q = i - p * PW_N;
+    if (p >= nProb || !probs[p].singular) return;
+    const double h = -0.5 * probs[p].expo;
+    double v = 0;
+    if (q < 5) {   // binomial coefficients of (1 + t)^h
+        v = 1.0;
+        for (int n = 0; n <= q; n++) v *= (h - n) / (n + 1.0);
+    } else if (q >= PW_E && q < PW_M) {   // kc 2^(E h); zero and subnormal arguments give infinity
+        const int e = q - PW_E;
+        const double E = e - 1023.0, hi = E * h, lo = fma(E, h, -hi), I = rint(hi);
+        v = e == 0 ? __longlong_as_double(0x7ff0000000000000LL)
+                   : (e == 2047 ? __longlong_as_double(0x7ff8000000000000LL)
+                                : probs[p].kc * ldexp(exp2(hi - I) * fma(lo, 0.6931471805599453, 1.0), (int)I));
+    } else if (q >= PW_M) {
+        const int j = (q - PW_M) >> 1;
+        const double inv = rint(8192.0 / (1.0 + (j + 0.5) / PW_J)) / 8192.0;
+        v = (q & 1) ? pow(inv, -h) : inv;
+    }
+    tab[i] = v;
+}
+
 // One warp per close pair: integrate_fractional (integration.cpp:187-288) with join()
 // (:1913-1958), FP64 throughout; lanes stride over the Duffy points, warp-reduce the blocks.
 // Sum over the Duffy points of one close pair (integration.cpp:187-288) of w pxy pxy^T, upper

@@ -1508,3 +1508,47 @@ def test_fp64_outer_points_outside_the_element(nl, orc, method, h_over_delta, on
     if B.nnz:
         fro, mx = rel_errors(A, B)
         assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+
+
+def _far_triangle(m):
+    """m beside a separate triangle of 70 horizons (delta = 0.02), which no ball of m reaches."""
+    from nlfem_gb300 import meshes
+    v = np.vstack([m["vertices"], [[5.0, 5.0], [6.0, 5.1], [5.2, 6.0]]])
+    n = len(m["vertices"])
+    return meshes.mesh_dict(v, np.vstack([m["elements"], [[n, n + 1, n + 2]]]), np.append(m["elementLabels"], 1))
+
+
+@pytest.mark.parametrize("case", ["sliver", "large_element", "full_search", "label_kernel"])
+def test_fp64_general_pass_by_its_stats(nl, orc, case):
+    """Calls outside the one-sided FP64 pass take the general one, seen in the stats (slot_map 0): alone, and together
+    with an ordinary problem that takes the one-sided pass by itself."""
+    from nlfem_gb300 import meshes, _lib
+    m, k, c = square_mesh(10, 0.02, jitter=0.1, seed=73), {"function": "constant", "horizon": 0.02, "outputdim": 1}, conf2d()
+    bad, kb, cb = m, dict(k), dict(c)
+    if case == "sliver":
+        v = m["vertices"].copy()
+        v[0] = 0.5 * (v[1] + v[12]) + np.array([-3e-13, 3e-13])   # onto the opposite side of its triangle (0, 1, 12)
+        bad = meshes.mesh_dict(v, m["elements"], m["elementLabels"])
+    elif case == "large_element":
+        bad = _far_triangle(m)
+    elif case == "full_search":
+        cb["is_fullConnectedComponentSearch"] = 1
+    else:
+        kb["function"] = "labeled"
+        bad = labeled_mesh(10)
+        kb["horizon"] = 0.1
+    ref, ok = orc.assemble(bad, kb, cb)["A"], orc.assemble(m, k, c)["A"]
+
+    def check(A, B):
+        assert same_pattern(A, B)
+        fro, mx = rel_errors(A, B)
+        assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
+
+    check(nl.stiffnessMatrix(dict(m), k, c), ok)
+    assert _lib.stats()["slot_map"] != 0
+    check(nl.stiffnessMatrix(dict(bad), kb, cb), ref)
+    assert _lib.stats()["slot_map"] == 0
+    A, B = nl.stiffnessMatrix_batch([(dict(bad), kb, cb), (dict(m), k, c)])
+    assert _lib.stats()["slot_map"] == 0
+    check(A, ref)
+    check(B, ok)
