@@ -754,6 +754,7 @@ __global__ void __launch_bounds__(128) k_quad_close(QuadArgs a, Duffy d) {
     if (w >= a.nlist) return;
     const long long p = a.list[w];
     const int aT = a.pA[p], bT = a.pB[p];
+    if (aT < 0) return;   // not a close pair (k_close_pairs): a label-0 element, or a kernel without a Duffy rule
     const int prob = a.eprob[aT];
     const ProbParams P = a.probs[prob];
     const double *pw = FAST ? nullptr : a.pw + (long long)prob * PW_N;

@@ -1552,3 +1552,27 @@ def test_fp64_general_pass_by_its_stats(nl, orc, case):
     assert _lib.stats()["slot_map"] == 0
     check(A, ref)
     check(B, ok)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("close", ["fractional", "weakSingular"])
+def test_close_pair_slots_that_hold_no_pair(nl, orc, close, prec):
+    """Close-pair slots of label-0 elements, and in a batch those of a problem whose kernel has no Duffy rule,
+    hold no pair and are passed over."""
+    from nlfem_gb300 import meshes
+    v, e, l = meshes.regular_square(15, 0.1, jitter=0.2, seed=38)
+    l = np.random.default_rng(38).choice([1, 1, 1, -1, 0], size=len(e))
+    m = meshes.mesh_dict(v, e, l)
+    s = 0.4 if close == "fractional" else 0.3
+    k = {"function": "fractional", "horizon": 0.11, "outputdim": 1, "fractional_s": s}
+    c = conf2d(rule="16", close=close, deg=3, precision=prec)
+    other = (square_mesh(9, 0.1, jitter=0.1, seed=2), {"function": "constant", "horizon": 0.15, "outputdim": 1},
+             conf2d(rule="16", precision=prec))
+    tol = FP64_TOL if prec == "fp64" else 1e-6
+    A = nl.stiffnessMatrix(m, k, c)
+    As = nl.stiffnessMatrix_batch([other, (m, k, c)])
+    B, C = orc.assemble(m, k, c)["A"], orc.assemble(*other)["A"]
+    for X, Y in ((A, B), (As[0], C), (As[1], B)):
+        assert same_pattern(X, Y)
+        fro, mx = rel_errors(X, Y)
+        assert fro < tol and mx < tol, (fro, mx)
