@@ -61,6 +61,23 @@ static int ensure(DevBuf &b, size_t bytes, bool no_grow) {
 }
 #define ENS(buf, bytes) do { int r_ = ensure(buf, bytes, S.replay); if (r_) return r_; } while (0)
 
+// Lets kernel fn be launched with bytes of dynamic shared memory. The limit belongs to the function on its
+// device, for all threads, so it only ever grows: another thread's smaller need must not take it back
+// between this call and the launch.
+static cudaError_t allow_smem(const void *fn, size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limit;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> g(mu);
+    size_t &now = limit.emplace(std::make_pair(dev, fn), 0).first->second;
+    if (bytes <= now) return cudaSuccess;
+    const cudaError_t s = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (s == cudaSuccess) now = bytes;
+    return s;
+}
+
 // ---------------------------------------------------------------- configuration parsing
 static int kernel_id(const char *s) {
     std::string k(s ? s : "");
@@ -1155,7 +1172,7 @@ static int run_bfs(Session &S) {
 
 static int sort_segments(Session &S, const long long *ptr, long long nseg, int *data) {
     const int cap = 16384;
-    CK(cudaFuncSetAttribute(k_row_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, cap * (int)sizeof(int)));
+    CK(allow_smem((const void *)k_row_sort, cap * sizeof(int)));
     k_row_sort<<<S.nSM * 4, 256, cap * sizeof(int), S.st>>>(ptr, nseg, data, cap); ++S.nlaunch;
     k_row_sort_global<<<S.nSM * 4, 256, 0, S.st>>>(ptr, nseg, data, cap); ++S.nlaunch;
     CK(cudaGetLastError());
@@ -1448,7 +1465,7 @@ static int run_pattern_bm(Session &S, int words, int threads) {
     a.rowptr = nullptr; a.cols = nullptr; a.rowcnt = S.rowcnt.get<int>();
     a.scratch = nullptr; a.cap = 0; a.cursor = nullptr; a.rowoff = nullptr; a.ovf = nullptr;
     const size_t smem = (size_t)words * 4 * (threads / 32);
-    CK(cudaFuncSetAttribute(k_row_pattern_bm<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(allow_smem((const void *)k_row_pattern_bm<DIM>, smem));
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_row_pattern_bm<DIM>, threads, smem));
     const unsigned grid = (unsigned)(S.nSM * std::max(per_sm, 1));
@@ -1541,7 +1558,7 @@ static int run_pattern(Session &S) {
     a.rowptr = S.rowptr.get<long long>(); a.cols = S.cols.get<int>();
     k_row_pattern<DIM><<<S.nSM * 4, 256, 0, S.st>>>(a, 1); ++S.nlaunch;
     const int cap = 16384;
-    CK(cudaFuncSetAttribute(k_row_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, cap * (int)sizeof(int)));
+    CK(allow_smem((const void *)k_row_sort, cap * sizeof(int)));
     k_row_sort<<<S.nSM * 4, 256, cap * sizeof(int), S.st>>>(S.rowptr.get<long long>(), nV, S.cols.get<int>(), cap); ++S.nlaunch;
     k_row_sort_global<<<S.nSM * 4, 256, 0, S.st>>>(S.rowptr.get<long long>(), nV, S.cols.get<int>(), cap); ++S.nlaunch;
     CK(cudaGetLastError());
@@ -1775,7 +1792,7 @@ static int run_pass_one_sided(Session &S, const PassArgs &pa, const PassRule &pr
     int rc = class_launches(S, L, &nl);
     if (rc) return rc;
     for (int i = 0; i < nl; i++) {
-        CK(cudaFuncSetAttribute(kfn[L[i].cls], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem((const void *)kfn[L[i].cls], smem));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[i], kfn[L[i].cls], threads, smem));
         if (per_sm[i] < 1) return fail(NLFEM_ERR_UNSUPPORTED, "quadrature rule too large for the pass's shared memory");
         if (S.tune_pass > 0) per_sm[i] = std::min(per_sm[i], S.tune_pass);   // autotuned
@@ -1901,7 +1918,7 @@ static int run_pass_f64(Session &S, const PassArgs &pa) {
         if (L[i].count == 0) continue;
         const size_t smem = retri ? f64_smem_bytes(L[i].cls, S.rule.nPx) : f64_bary_smem<DIM>(S.rule.nPx);
         int per_sm = 0;
-        CK(cudaFuncSetAttribute(kfn[L[i].cls], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem((const void *)kfn[L[i].cls], smem));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn[L[i].cls], F64_THREADS, smem));
         per_sm = std::max(per_sm, 1);
         if (S.tune_pass > 0) per_sm = std::min(per_sm, S.tune_pass);   // autotuned
@@ -2017,8 +2034,8 @@ static int run_passes(Session &S) {
         return run_pass_one_sided(S, a, pr, k, BARY_THREADS, bary_warp_bytes<DIM>(S.rule.nPx) * BARY_WARPS);
     }
     const size_t smem = sizeof(int) * PASS_WARPS * dV * ROWCACHE;
-    if (S.prec == PREC_MIX) CK(cudaFuncSetAttribute(k_pass<DIM, PREC_MIX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else CK(cudaFuncSetAttribute(k_pass<DIM, PREC_F64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (S.prec == PREC_MIX) CK(allow_smem((const void *)k_pass<DIM, PREC_MIX>, smem));
+    else CK(allow_smem((const void *)k_pass<DIM, PREC_F64>, smem));
     const int ncol = (int)S.color_off.size() - 1;
     for (int c = 0; c < ncol; c++) {
         a.list = S.colorlist.get<int>() + S.color_off[c];

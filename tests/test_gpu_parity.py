@@ -1576,3 +1576,33 @@ def test_close_pair_slots_that_hold_no_pair(nl, orc, close, prec):
         assert same_pattern(X, Y)
         fro, mx = rel_errors(X, Y)
         assert fro < tol and mx < tol, (fro, mx)
+
+
+def test_threads_of_different_sizes(nl):
+    """One-shot calls of four threads at once, of different sizes, rules, kernels and precisions (different shared-memory
+    needs of the same kernels), give the bits of the same calls one after the other."""
+    import threading
+    calls = []
+    for i, (n, rule, kern, prec) in enumerate([(4, "7", "constant", "fp64"), (30, "16", "constant", "fp64"), (12, "7", "parabola", "mixed"),
+                                               (60, "7", "constant", "mixed"), (8, "16", "parabola", "fp64"), (24, "16", "parabola", "mixed"),
+                                               (40, "7", "constant", "fp64"), (10, "16", "constant", "mixed")]):
+        calls.append((square_mesh(n, 0.1, jitter=0.2, seed=i), {"function": kern, "horizon": 0.1, "outputdim": 1}, conf2d(rule=rule, precision=prec)))
+    want = [nl.stiffnessMatrix(*c).tocsr() for c in calls]
+    errors = []
+
+    def work(t):
+        try:
+            for r in range(24):
+                i = (5 * r + 3 * t) % len(calls)
+                A = nl.stiffnessMatrix(*calls[i]).tocsr()
+                if not (same_pattern(A, want[i]) and np.array_equal(A.data, want[i].data)):
+                    errors.append((t, r, i))
+        except Exception as ex:
+            errors.append((t, repr(ex)))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[:4]
