@@ -34,15 +34,16 @@ import numpy as np
 
 METRIC = "element-pair quadratures/s: mixed vs FP64 on one GB300 at <=1e-6 rel err"
 
-# DRAM traffic (read + write bytes) per pair of the quadrature pass, from an ncu capture of one
-# launch on a smaller case of the workload: k_pass_mix2d<0> on the 2D constant-kernel workload at
-# n = 128 (2.56e7 pairs: 187.7 MB read, 35.0 MB written), k_pass_bary<3> on the 3D one at n = 24
-# (2.59e7 pairs: 143.7 MB read, 8.2 MB written). The passes stream their pair lists and reuse the
-# mesh from L2, so the traffic grows with the pairs. Reported as roofline.traffic (scaled to this
-# run's pairs) with its source.
+# DRAM traffic (read + write bytes) per pair of the quadrature pass, from an ncu capture of its launches
+# on a smaller case of the workload: on the 2D constant-kernel workload at n = 128 (2.56e7 pairs)
+# k_pass_near2d 132.1 MB read, 14.8 MB written and k_pass_mix2d<0> 112.4 MB, 18.2 MB; on the 3D one at
+# n = 24 (2.60e7 pairs) k_pass_bary<3> 144.8 MB read, 8.5 MB written. The passes stream their pair
+# lists and reuse the mesh from L2, so the traffic grows with the pairs. Reported as roofline.traffic
+# (scaled to this run's pairs) with its source.
 PASS_TRAFFIC = {
-    "c2": ((187.713e6 + 35.046e6) / 25573871, "k_pass_mix2d<0> on the 2D constant-kernel workload at n=128 (2.56e7 pairs)"),
-    "c4": ((143.728e6 + 8.242e6) / 25852104, "k_pass_bary<3> on the 3D constant-kernel workload at n=24 (2.59e7 pairs)"),
+    "c2": ((132.086e6 + 14.784e6 + 112.413e6 + 18.205e6) / 25573871,
+           "k_pass_near2d and one of k_pass_mix2d<0> on the 2D constant-kernel workload at n=128 (2.56e7 pairs)"),
+    "c4": ((144.844e6 + 8.480e6) / 25955449, "k_pass_bary<3> on the 3D constant-kernel workload at n=24 (2.60e7 pairs)"),
 }
 # Algorithmic bytes of the pair search per tested candidate: its 16-bit visited stamp (2 B), its
 # incidence entry (4 B), a share of a vertex's stamp and incidence range (about 4 B) and the
@@ -211,6 +212,37 @@ def algorithmic_flops(st, conf, kernel, dim=2):
     return st["n_pairs"] * (12 + nPx * 198) + st["n_subtri"] * (11 + nPy * (51 + kf))
 
 
+def fp64_pass_flops(st, conf, kernel, dim=2):
+    """Floating-point operations on the FP64 pipe of the one-sided FP64 passes (an FMA counts 2), or None
+    where there is no model (kernels other than the constant ones). Classes and polygon structure are
+    FP32 there and the sums integers, so neither counts.
+      retriangulate (passes_f64.cuh), per pair 31 (its blocks from the mask sums) and 7 per further mask
+      byte; cut item 10 (edges) + 2 * 43 (two crossings) + 32 (a cap) + 31 (moments to basis functions) + 30
+      (fold of 15 outputs); side of its polygon 29.
+      baryCenter (passes_f64_bary.cuh), per pair 2 + dV + dV^2 products, 2 per off-diagonal entry of
+      termLocal, and the mask sums of further bytes."""
+    if kernel["function"] not in ("constant", "constant3D"):
+        return None
+    further = (len(conf["quadrature"]["outer"]["weights"]) + 7) // 8 - 1
+    if conf["approxBalls"]["method"] == "baryCenter":
+        dV = dim + 1
+        off = dV * (dV - 1) // 2
+        return st["n_pairs"] * (2 + dV + dV * dV + 2 * off + further * (dV + off))
+    return (st["n_pairs"] * (31 + 7 * further) + st["n_items_cut"] * (10 + 2 * 43 + 32 + 31 + 30)
+            + (st["n_subtri"] - st["n_items_in"]) * 29)
+
+
+def fp64_roofline(st, conf, kernel, dim, peak):
+    """The FP64 arm's quadrature phase against the FP64 peak: the one-sided pass by fp64_pass_flops, the general
+    pass (no slot map in the stats) by algorithmic_flops."""
+    flops = fp64_pass_flops(st, conf, kernel, dim) if st["slot_map"] else algorithmic_flops(st, conf, kernel, dim)
+    a = flops / (st["ms_quad"] / 1000.0) / 1e12 if flops else None
+    return {"bound": "fp64", "achieved": a, "peak": peak, "unit": "TFLOP/s", "frac": a / peak if a else None,
+            "note": ("FP64 operations of the one-sided pass that ran (bench.fp64_pass_flops; none modelled for this "
+                     "kernel where null)" if st["slot_map"] else "the reference algorithm's operations (bench.algorithmic_flops)")
+            + " / device time of the quadrature phase; peak = FP64 FMA throughput measured in this run"}
+
+
 def cpu_sample(problems, seconds, threads):
     """Oracle (CPU restatement, FP64, OpenMP) on a bounded sample of outer elements of each
     problem in turn, until about `seconds` of work; returns (pairs, seconds, elements)."""
@@ -359,11 +391,14 @@ def run_gpu(args, rank=0, world=1, dist=None):
     kernels = {k["function"] for _, k, _ in problems}
     kernel0 = problems[0][1] if len(kernels) == 1 else {"function": "mixed"}
     conf0 = problems[0][2]
+    dim0 = int(problems[0][0]["vertices"].shape[1])
     flops = algorithmic_flops(st, conf0, kernel0)
     achieved = flops / (st["ms_quad"] / 1000.0) / 1e12
     bary = conf0["approxBalls"]["method"] == "baryCenter"
     kname = ("k_pass_bary (one-sided barycenter quadrature + fixed-point scatter, one persistent launch)" if bary else
-             "k_pass_mix2d (one-sided quadrature + fixed-point scatter, one persistent launch)")
+             "k_pass_near2d and k_pass_mix2d (one-sided quadrature + fixed-point scatter: the pairs inside every ball, "
+             "then the others)" if kernels == {"constant"} else
+             "k_pass_mix2d (one-sided quadrature + fixed-point scatter, one persistent launch per kernel class)")
 
     # end to end through the public API: pinned host inputs, host CSR out
     pins = [pinned(m) for m, _, _ in problems]
@@ -414,7 +449,7 @@ def run_gpu(args, rank=0, world=1, dist=None):
                              "quadrature phase; peak = FP32 FMA throughput measured in this run (of measured); "
                              "CUDA-core bound path with no GEMM-shaped work, so neither the tensor-core nor the "
                              "HBM peak applies"},
-        "search": search_roofline(st, conf0, int(problems[0][0]["vertices"].shape[1])),
+        "search": search_roofline(st, conf0, dim0),
         "peaks_measured": {"fp32_tflops": peak32, "fp64_tflops": peak64,
                            "hbm_gbs": measured_peaks().get("hbm_gbs")},
         "e2e": {"value": e2e, "unit": "pairs/s", "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h),
@@ -432,33 +467,29 @@ def run_gpu(args, rank=0, world=1, dist=None):
         A64 = [sess64.download(i) for i in range(len(problems))]
         errs = [rel_err(A_mixed[i], A64[i]) for i in range(len(problems))]
         sess64.close()
-        a64 = algorithmic_flops(st64, problems64[0][2], kernel0) / (st64["ms_quad"] / 1000.0) / 1e12
         line["fp64"] = {"value": p64 / s64, "unit": "pairs/s", "steps": args.fp64_steps,
                         "ms_per_step": 1000.0 * s64 / args.fp64_steps, "mixed_over_fp64": value / (p64 / s64),
-                        "roofline": {"bound": "fp64", "achieved": a64, "peak": peak64, "unit": "TFLOP/s",
-                                     "frac": a64 / peak64},
+                        "roofline": fp64_roofline(st64, problems64[0][2], kernel0, dim0, peak64),
                         "clocks": clk64}
         line["rel_err_vs_fp64"] = {"pattern_identical": all(e[0] for e in errs),
                                    "fro": max(e[1] for e in errs), "max": max(e[2] for e in errs),
                                    "per_problem": len(errs) > 1, "bound": 1e-6}
     elif world == 1:
         line["fp64"] = {"skipped": "pass --fp64-steps K to time the all-FP64 path on this workload"}
-    # the same one-sided algorithm (classes, closed forms, fixed-point scatter) in FP64 arithmetic:
-    # the ratio to it is what the precision alone buys
+    # the one-sided pass in FP64 arithmetic by name (every structural slot kept): classes and polygon
+    # structure by the same certified FP32 geometry as the headline, points, moments and sums in FP64
     A1 = None
     if world == 1 and not args.no_fp64 and args.workload in ("c1", "c2", "c3", "c5"):
         problems1, _ = workload(args, "fp64-onesided")
         p1, s1, st1, _, clk1, sess1 = timed_session(problems1, args.fp64_steps, 1, flush, dev)
         A1 = [sess1.download(i) for i in range(len(problems1))]
         sess1.close()
-        a1 = algorithmic_flops(st1, dict(problems1[0][2], precision="mixed"), kernel0) / (st1["ms_quad"] / 1000.0) / 1e12
         line["fp64_same_algorithm"] = {
             "value": p1 / s1, "unit": "pairs/s", "steps": args.fp64_steps, "ms_per_step": 1000.0 * s1 / args.fp64_steps,
             "mixed_over_fp64_same_algorithm": value / (p1 / s1),
             "phase_ms": {"dual+bfs+pairs+color": st1["ms_bfs"], "pattern": st1["ms_pattern"],
                          "quadrature+scatter": st1["ms_quad"], "finish": st1["ms_finish"]},
-            "roofline": {"bound": "fp64", "achieved": a1, "peak": peak64, "unit": "TFLOP/s", "frac": a1 / peak64,
-                         "note": "the mixed path's FLOP model over the FP64 instance's quadrature phase"},
+            "roofline": fp64_roofline(st1, problems1[0][2], kernel0, dim0, peak64),
             "note": "precision \"fp64-onesided\": the headline's one-sided pass, closed forms and fixed-point sums "
                     "in FP64 arithmetic (classes and polygon structure by the certified FP32 geometry), every "
                     "structural slot kept; the FP64 arm beside it takes the same pass where it applies",

@@ -50,3 +50,18 @@ def test_flop_model_counts_items():
     # the general kernels count the inner-point loops
     par = bench.algorithmic_flops(st, _conf("retriangulate"), {"function": "parabola"})
     assert par == 100 * (12 + 7 * 198) + 900 * (11 + 7 * (51 + 7))
+
+
+def test_fp64_pass_flops_and_roofline():
+    st = {"n_pairs": 100, "n_items_in": 500, "n_items_cut": 100, "n_subtri": 900, "slot_map": 1, "ms_quad": 1.0}
+    c = {"function": "constant"}
+    retri = bench.fp64_pass_flops(st, _conf("retriangulate", precision="fp64"), c)
+    assert retri == 100 * 31 + 100 * 189 + 400 * 29
+    assert bench.fp64_pass_flops(st, _conf("retriangulate", nPx=16), c) == retri + 100 * 7
+    assert bench.fp64_pass_flops(st, _conf("baryCenter", nPx=11), {"function": "constant3D"}, 3) == 100 * (2 + 4 + 16 + 12 + 10)
+    assert bench.fp64_pass_flops(st, _conf("retriangulate"), {"function": "parabola"}) is None
+    r = bench.fp64_roofline(st, _conf("retriangulate", precision="fp64"), c, 2, 2.0)
+    assert r["achieved"] == pytest.approx(retri / 1e-3 / 1e12) and r["frac"] == pytest.approx(r["achieved"] / 2.0)
+    assert bench.fp64_roofline(st, _conf("retriangulate"), {"function": "parabola"}, 2, 2.0)["frac"] is None
+    general = bench.fp64_roofline(dict(st, slot_map=0), _conf("retriangulate", precision="fp64"), c, 2, 2.0)
+    assert general["achieved"] == pytest.approx(bench.algorithmic_flops(st, _conf("retriangulate", precision="fp64"), c) / 1e-3 / 1e12)
