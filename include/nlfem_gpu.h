@@ -42,9 +42,11 @@ extern "C" {
 /* arithmetic of the quadrature */
 #define NLFEM_PREC_FP64 0       /* all FP64 */
 #define NLFEM_PREC_MIXED 1      /* FP32 quadrature, FP64 cut geometry and accumulation */
-#define NLFEM_PREC_FP64_ONESIDED 2 /* the one-sided FP64 pass by name (2D retriangulate only), every
-                                      structural slot kept; NLFEM_PREC_FP64 takes the same pass where
-                                      it applies */
+#define NLFEM_PREC_FP64_ONESIDED 2 /* the one-sided FP64 pass by name (2D retriangulate only, elements of at
+                                      most 512 horizons), every structural slot kept; NLFEM_PREC_FP64
+                                      takes the same pass where the certified FP32 geometry decides its
+                                      classes (elements of at most 16 horizons) and the general pass
+                                      elsewhere */
 
 /* One assembly problem. Arrays are borrowed host pointers, row-major. */
 typedef struct nlfem_problem {

@@ -63,7 +63,8 @@ __device__ __forceinline__ float kernel_f32_r2(const ProbParams &P, float r2) {
 // the outer rule at points that differ from lane to lane: from shared memory (the constant cache
 // serves one address at a time). Five blocks
 // per SM at 96 registers: 4 and 6 were 1.1 and 0.4 ms slower at 6 * 32^3 tetrahedra, 1.26e8 pairs, where
-// the pass takes 10.2 ms (15.7 with the constant cache and group sums by shuffles).
+// the pass took 10.2 ms (15.7 with the constant cache and group sums by shuffles; 8.6 now that batches of near
+// pairs find no classes).
 template <int DIM, bool CK>
 __global__ void __launch_bounds__(BARY_THREADS, CK ? 5 : 4) k_pass_bary(MixArgs ma, Rule rule, PassRule pr) {
     constexpr int dV = DIM + 1, NS = dV * (dV + 1) / 2, RN = DIM + 2;

@@ -15,10 +15,11 @@
 //   * Cut items (and, for other kernels, inside items) are listed pair by pair, so a pair's items
 //     are neighbours: full warps integrate the items, then full warps fold them, one (pair, output)
 //     per lane, instead of every lane walking all outer points.
-// Measured (quadrature phase, against the two-sided colored pass that the path used before): constant
-// kernel, 2 * 128^2 triangles, delta = 0.1, 2.56e7 pairs: 21.4 ms against 1725 ms; 2 * 32^2
-// triangles: 0.52 against 66.6 ms; parabola, 2 * 57^2: 5.4 against 257 ms; fractional, 2 * 40^2:
-// 9.6 against about 540 ms. The FP64 pipe is 70 to 89% busy in these.
+// Measured (quadrature phase, against the two-sided colored pass): constant kernel, 2 * 128^2
+// triangles, delta = 0.1, 2.56e7 pairs: 19.3 ms against 1740 ms; 2 * 32^2 triangles: 0.45 against 66.6 ms;
+// parabola, 2 * 57^2, delta = 0.12: 5.2 against 257 ms; fractional, 2 * 40^2: 8.1 and 5.1 for the close
+// pairs against 568 ms. The FP64 pipe is 70 to 90% busy in these. With one integer per slot the first
+// took 18.6 ms: 0.4 ms of the rest are the second integers' sums, 0.3 the moments' origin.
 //
 // Sums. Every contribution is cut into 64-bit integers that are added with integer atomics, so the
 // result does not depend on the order of the warps. The unit of a slot (t, v) of termNonloc
@@ -302,7 +303,8 @@ struct F64Poly {
 // quotient, per cap a reciprocal square root. In reference coordinates vertices are constants and
 // a crossing is its root. Against the exact routine, which takes both roots of all three edges with
 // their divisions for every item, that is about a third of the FP64 instructions: with the closed
-// moments of f64_item 51.5 -> 20.5 ms on 2 * 128^2 triangles (constant kernel). False where a decision
+// moments of f64_item the pass went from 51.5 to 20.5 ms on 2 * 128^2 triangles (constant kernel) when
+// this came. False where a decision
 // is within its margin. LATE takes such an item's polygon from the exact routine instead, and is false
 // where that holds less than 1e-5 of the partner (f64_item_exact then; above, every sum of the item is
 // far above its rounding).

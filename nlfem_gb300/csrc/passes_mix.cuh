@@ -47,7 +47,7 @@ struct MixWarp {
 // joins that writer's entry. Others (two vertices with the same low bits) have an entry of their own: a
 // vertex may have several entries, and the users' integer sums allow that. Against one __match_any_sync
 // per local vertex a vertex has one entry instead of up to three; k_pass_near2d at n = 256, delta = 0.1:
-// 18.8 against 19.7 ms.
+// 18.8 against 19.7 ms (9.8 since the lists came in element order).
 constexpr int GROUP_TAB = 512;
 template <int DV>
 struct VertexGroups {

@@ -819,7 +819,7 @@ static int session_init(Session &S, const nlfem_problem *probs, int n, bool syst
             return fail(NLFEM_ERR_UNSUPPORTED, "precision \"fp64-onesided\" covers the 2D retriangulate rule "
                                                "without domain-decomposition weights");
         // FP64: the one-sided pass where it covers every problem of the call and its rule's tables
-        // fit an SM's shared memory (16 to 41 times the colored passes' speed on 2 * 32^2 to 2 * 128^2
+        // fit an SM's shared memory (65 to 71 times the colored passes' speed on 2 * 32^2 to 2 * 128^2
         // triangles, see passes_f64.cuh), the colored passes for everything else
         bool all_f64 = system && S.prec == PREC_F64 && (all_retri || all_bary);
         S.cert = system;
