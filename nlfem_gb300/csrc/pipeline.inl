@@ -1542,6 +1542,7 @@ static int run_pattern(Session &S) {
     ENS(S.rowptr, sizeof(long long) * (nV + 1));
     CK(cudaMemsetAsync(S.marks.p, 0, sizeof(unsigned) * (size_t)nwarps * S.maxNV, S.st));
     RowArgs a;
+    memset(&a, 0, sizeof(a));
     a.T32 = S.T32.get<int>(); a.labT = S.labT.get<int>(); a.labV = S.labV.get<int>();
     a.vprob = S.vprob.get<int>(); a.vel = S.vel.get<int>(); a.pB = S.pB.get<int>(); a.inA = S.inA.get<int>();
     a.vptr = S.vptr.get<long long>(); a.out_ptr = S.out_ptr.get<long long>();

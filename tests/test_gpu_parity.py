@@ -1606,3 +1606,36 @@ def test_threads_of_different_sizes(nl):
     for t in threads:
         t.join()
     assert not errors, errors[:4]
+
+
+@pytest.mark.parametrize("case", ["fp64", "mixed", "bary_fp64", "bary_mixed", "label_fp64", "dim3_fp64", "dim3_mixed"])
+def test_pattern_of_meshes_too_large_for_bitmaps(nl, orc, case):
+    """From 819,200 vertices on, a problem's vertex bitmap leaves shared memory and the rows are built from marks in
+    global memory. A small mesh numbered behind unused vertices takes that path, in the passes that read pair
+    arrays: its rows are those of the mesh by itself."""
+    from nlfem_gb300 import meshes, _lib
+    prec = case.split("_")[-1]
+    k = {"function": "constant", "horizon": 0.12, "outputdim": 1}
+    if case.startswith("dim3"):
+        m, c, k["function"] = cube_mesh(4, 0.1, jitter=0.15, seed=3), conf3d(prec), "constant3D"
+        k["horizon"] = 0.3
+    else:
+        m = labeled_mesh(12) if case.startswith("label") else square_mesh(13, 0.1, jitter=0.2, seed=3)
+        c = conf2d(method="baryCenter" if case.startswith("bary") else "retriangulate", precision=prec)
+        if case.startswith("label"):
+            k["function"] = "labeled"
+    pad = 820000
+    v = np.vstack([np.zeros((pad, m["vertices"].shape[1])), m["vertices"]])
+    v[:pad] = m["vertices"][0]
+    big = meshes.mesh_dict(v, m["elements"] + pad, m["elementLabels"])
+    A = nl.stiffnessMatrix(big, k, c).tocsr()
+    st = _lib.stats()
+    B = nl.stiffnessMatrix(dict(m), k, c).tocsr()
+    assert A.indptr[pad] == 0 and st["n_pairs"] == _lib.stats()["n_pairs"]
+    C = A[pad:, pad:]
+    assert C.nnz == A.nnz and same_pattern(C, B)
+    if prec == "mixed":
+        assert abs(C - B).max() < 1e-6 * abs(B).max()
+    else:
+        fro, mx = rel_errors(C, orc.assemble(m, k, c)["A"])
+        assert fro < FP64_TOL and mx < FP64_TOL, (fro, mx)
